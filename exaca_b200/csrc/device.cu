@@ -14,10 +14,11 @@
 //          critical lengths), mask updates of its active neighbours, and for those the
 //          solidification re-check.
 // Stretches of cycles run in one persistent cooperative kernel (k_cycles) whose blocks meet at
-// bounded grid-wide barriers between the passes; the last block to reach the end of a cycle
-// starts the next one. In k_cycles each block runs the claim steps of the records it flagged right
-// after its own growth (a shared-memory queue); a grid-wide claim pass runs only in a cycle where
-// some block's queue overflowed. The same passes also run as separate kernels (per-pass timing).
+// bounded grid-wide barriers, two per cycle: after the claims and after the captures. Each block runs
+// the claim steps of the records it flagged right after its own growth (a shared-memory queue; a
+// grid-wide claim pass runs only in a cycle where some block's queue overflowed), and captures the
+// winners among its own claims. The start of the next cycle runs under the capture pass, in a few
+// warps of their own. The same passes also run as separate kernels (per-pass timing).
 // The claim rule reproduces the Kokkos-Serial loop order exactly: serial visits active cells in
 // ascending index and captures flip Liquid to Active in place, so the capturer of a cell is the
 // lowest-index claimant, and an active cell sees a neighbour as liquid iff it was liquid at the
@@ -74,7 +75,18 @@ constexpr unsigned int kMaskKeep = 1u << 29;  // this cycle, a neighbour was cap
 // capture pass's re-check needs no CritTimeStep (a record's eligibility only changes at a layer
 // change, which rebuilds the list)
 constexpr unsigned int kMaskGrown = 1u << 28;
+// a neighbour nucleated at the start of this cycle: the growth pass drops the directions that are no
+// longer liquid from the mask (set only inside the persistent kernel, between two of its cycles)
+constexpr unsigned int kMaskNuc = 1u << 27;
 constexpr unsigned int kDirBits = (1u << 26) - 1;
+// CellType of a liquid cell that nucleates at the start of the next cycle unless it is claimed in
+// this one; two codes, alternating by cycle, so that the captures of a cycle tell the sites that fire
+// after it (no longer liquid for a captured cell's mask) from those marked for the cycle after that
+// (still liquid). Only inside the persistent kernel: no mark is left when it ends.
+constexpr int8_t kMark0 = 8;
+__device__ __forceinline__ int8_t mark_code(int cycle_index) { return (int8_t)(kMark0 + (cycle_index & 1)); }
+// liquid at the start of the current cycle, for a pass in which claims are being made
+__device__ __forceinline__ bool liquid_type(int8_t t) { return t == kLiquid || t == kTemporaryUpdate || t >= kMark0; }
 constexpr int kErrGrowthTable = 1;
 constexpr int kErrListOverflow = 2;
 constexpr int kErrBounds = 4;
@@ -315,34 +327,26 @@ __device__ float capture_cell(const DomainDesc &D, unsigned int c, unsigned int 
     double n0 = __shfl_sync(gmask, nq, 0, kLanes), n1 = __shfl_sync(gmask, nq, 1, kLanes),
            n2 = __shfl_sync(gmask, nq, 2, kLanes);
     double ParaT = (n0 * x0 + n1 * y0 + n2 * z0) / (n0 * Diag1X + n1 * Diag1Y + n2 * Diag1Z);
-    double TX[3], TY[3], TZ[3];
-    TX[0] = cxold + ParaT * Diag1X;
-    TY[0] = cyold + ParaT * Diag1Y;
-    TZ[0] = czold + ParaT * Diag1Z;
-    TX[1] = cxold + ParaT * Diag2X;
-    TY[1] = cyold + ParaT * Diag2Y;
-    TZ[1] = czold + ParaT * Diag2Z;
-    TX[2] = cxold + ParaT * Diag3X;
-    TY[2] = cyold + ParaT * Diag3Y;
-    TZ[2] = czold + ParaT * Diag3Z;
+    const double TX0 = cxold + ParaT * Diag1X, TY0 = cyold + ParaT * Diag1Y, TZ0 = czold + ParaT * Diag1Z;
+    const double TX1 = cxold + ParaT * Diag2X, TY1 = cyold + ParaT * Diag2Y, TZ1 = czold + ParaT * Diag2Z;
+    const double TX2 = cxold + ParaT * Diag3X, TY2 = cyold + ParaT * Diag3Y, TZ2 = czold + ParaT * Diag3Z;
     // Dist[0..2] on lanes 0..2
-    const double tqx = q3 == 0 ? TX[0] : (q3 == 1 ? TX[1] : TX[2]), tqy = q3 == 0 ? TY[0] : (q3 == 1 ? TY[1] : TY[2]),
-                 tqz = q3 == 0 ? TZ[0] : (q3 == 1 ? TZ[1] : TZ[2]);
+    const double tqx = q3 == 0 ? TX0 : (q3 == 1 ? TX1 : TX2), tqy = q3 == 0 ? TY0 : (q3 == 1 ? TY1 : TY2),
+                 tqz = q3 == 0 ? TZ0 : (q3 == 1 ? TZ1 : TZ2);
     const float distq =
         sqrtf((float)(((tqx - xp) * (tqx - xp)) + ((tqy - yp) * (tqy - yp)) + ((tqz - zp) * (tqz - zp))));
-    double Dist[3];
-    Dist[0] = __shfl_sync(gmask, distq, 0, kLanes);
-    Dist[1] = __shfl_sync(gmask, distq, 1, kLanes);
-    Dist[2] = __shfl_sync(gmask, distq, 2, kLanes);
-    int x = (Dist[0] < Dist[1]);
-    int y = (Dist[1] < Dist[2]);
-    int z = (Dist[2] < Dist[0]);
+    const double Dist0 = __shfl_sync(gmask, distq, 0, kLanes), Dist1 = __shfl_sync(gmask, distq, 1, kLanes),
+                 Dist2 = __shfl_sync(gmask, distq, 2, kLanes);
+    int x = (Dist0 < Dist1);
+    int y = (Dist1 < Dist2);
+    int z = (Dist2 < Dist0);
+    // 0, 1 or 2; the points idx, idx + 1 and idx + 2 (mod 3) by selects, without a local array
     int idx = 2 * (z - y) * z + (y - x) * y;
-    double mindist = Dist[idx];
-    double xc = TX[idx], yc = TY[idx], zc = TZ[idx];
-    int i1 = (idx + 1) % 3, i2 = (idx + 2) % 3;
-    double x1 = TX[i1], y1 = TY[i1], z1 = TZ[i1];
-    double x2 = TX[i2], y2 = TY[i2], z2 = TZ[i2];
+    const bool p0 = idx == 0, p1 = idx == 1;
+    double mindist = p0 ? Dist0 : (p1 ? Dist1 : Dist2);
+    double xc = p0 ? TX0 : (p1 ? TX1 : TX2), yc = p0 ? TY0 : (p1 ? TY1 : TY2), zc = p0 ? TZ0 : (p1 ? TZ1 : TZ2);
+    double x1 = p0 ? TX1 : (p1 ? TX2 : TX0), y1 = p0 ? TY1 : (p1 ? TY2 : TY0), z1 = p0 ? TZ1 : (p1 ? TZ2 : TZ0);
+    double x2 = p0 ? TX2 : (p1 ? TX0 : TX1), y2 = p0 ? TY2 : (p1 ? TY0 : TY1), z2 = p0 ? TZ2 : (p1 ? TZ0 : TZ1);
     // D1..D4 on lanes 0..3: D1 = |p - v2|, D2 = |c - v2|, D3 = |p - v1|, D4 = |c - v1|
     const int q4 = sub & 3;
     const double ax = (q4 & 1) ? xc : xp, ay = (q4 & 1) ? yc : yp, az = (q4 & 1) ? zc : zp;
@@ -464,7 +468,6 @@ __device__ __forceinline__ void lists_start(PoolState *P, bool close, int *cur_o
             appended += __shfl_down_sync(0xffffffffu, appended, o);
         }
         if (lane == 0) {
-            P->claim_overflow = 0;
             if (close) {
                 // the capture pass reserved its new records' slots past the count of list `cur`
                 const unsigned long long grown = (cur ? cnt1 : cnt0) + appended;
@@ -533,9 +536,104 @@ __device__ __forceinline__ DomainStart load_start(const DomainDesc &D) {
     return s;
 }
 
-// Cycle start of domain d by one warp (all lanes call with the same arguments).
+// The descriptor fields that a nucleation needs.
+struct NucleationView {
+    int32_t *gid;
+    const int32_t *cts_run;
+    float *dl, *doc, *cdl;
+    const float *cdl_table;
+    unsigned int *pos;
+    int mx, my, z_end, xoff, yoff;
+};
+__device__ __forceinline__ NucleationView nucleation_view(const DomainDesc &D) {
+    return NucleationView{D.gid, D.cts_run, D.dl, D.doc, D.cdl, D.cdl_table, D.pos, D.mx, D.my, D.z_end, D.xoff, D.yoff};
+}
+
+// Nucleation of one site by a warp (src/CAupdate.cpp:100-194), one round of loads: lanes 0-12 copy the
+// fresh octahedron's critical lengths, lane n < 26 reads neighbour n's type and list position; an
+// active neighbour's record goes to on_neighbour(position, direction from the site). The record goes
+// to `slot` (ULLONG_MAX: none) of the list given.
+template <class OnNeighbour>
+__device__ __forceinline__ void nucleate_site(const NucleationView &V, int8_t *ctype, ActiveRec *rec, unsigned int *rdom,
+                                              unsigned int *rstat, unsigned long long *rmin2, unsigned int dom,
+                                              unsigned int site, int site_gid, int cts, unsigned long long slot,
+                                              OnNeighbour &&on_neighbour) {
+    const unsigned int lane = threadIdx.x & 31;
+    const int plane = V.mx * V.my;
+    const unsigned int z = site / (unsigned int)plane;
+    const unsigned int rem = site - z * (unsigned int)plane;
+    const int rx = (int)(rem / (unsigned int)V.my), ry = (int)(rem - (unsigned int)rx * (unsigned int)V.my), rz = (int)z;
+    const unsigned int valid = edge_mask(rx, ry, rz, V.mx, V.my, V.z_end);
+    int ori = (abs(site_gid) - 1) % 10000;
+    if (ori < 0)
+        ori += 10000;
+    float2 row = make_float2(0.0f, 0.0f);
+    if (lane < 13)
+        row = reinterpret_cast<const float2 *>(V.cdl_table + 26 * ori)[lane];
+    const bool nb = lane < 26 && ((valid >> lane) & 1u);
+    int8_t nb_type = kLiquid;
+    unsigned int nb_pos = 0;
+    if (nb) {
+        const long long a = (long long)site + nb_offset((int)lane, plane, V.my);
+        nb_type = __ldcg(ctype + a);
+        nb_pos = __ldcg(V.pos + a);
+    }
+    if (lane < 13)
+        reinterpret_cast<float2 *>(V.cdl + 26ull * site)[lane] = row;
+    if (lane == 0) {
+        V.dl[site] = 0.01f;
+        V.doc[3ull * site + 0] = (float)((double)(rx + V.xoff) + 0.5);
+        V.doc[3ull * site + 1] = (float)((double)(ry + V.yoff) + 0.5);
+        V.doc[3ull * site + 2] = (float)((double)rz + 0.5);
+        if (slot != ULLONG_MAX) {
+            ActiveRec r;
+            r.cell = site;
+            r.dl = 0.01f;
+            r.cdl_min = 0.0f;
+            r.cts = cts;
+            rec[slot] = r;
+            rdom[slot] = dom;
+            rstat[slot] = kMaskFresh;
+            rmin2[slot] = kNoMin2;
+            V.pos[site] = (unsigned int)slot;
+        }
+        ctype[site] = kActive;
+    }
+    if (nb && nb_type == kActive)
+        on_neighbour(nb_pos, (int)lane);
+    __syncwarp();
+}
+
+// Marks the liquid sites from `mark` on that are due by `cycle` (one warp); returns the first site not
+// due. Sites are sorted by time, so the due ones form a prefix.
+__device__ __forceinline__ int mark_sites(DomainDesc &D, const DomainStart &s, int mark, int cycle, int8_t code,
+                                          int layer_no, long long active_size) {
+    const unsigned int lane = threadIdx.x & 31;
+    while (mark < s.n_nuclei) {
+        const int idx = mark + (int)lane;
+        const int t = idx < s.n_nuclei ? __ldg(s.nuc_time + idx) : INT_MAX;
+        const int l = idx < s.n_nuclei ? __ldg(s.nuc_loc + idx) : -1;
+        const bool due = t <= cycle;
+        const int n_due = __popc(__ballot_sync(0xffffffffu, due));
+        if (n_due == 0)
+            break;
+        if (due) {
+            if (l < 0 || l >= active_size)
+                atomicOr(&D.error, kErrBounds);
+            else if (__ldcg(s.ctype + l) == kLiquid && D.layer[l] <= layer_no)
+                s.ctype[l] = code;
+        }
+        mark += n_due;
+        if (n_due < 32)
+            break;
+    }
+    return mark;
+}
+
+// Cycle start of domain d by one warp (all lanes call with the same arguments). With `mark` the sites
+// due at the next cycle's start are marked for start_next.
 __device__ __forceinline__ void start_domain(PoolState *P, DomainDesc &D, const DomainStart &s, unsigned int d,
-                                             int cur, unsigned long long &nucleated) {
+                                             int cur, bool mark, unsigned long long &nucleated) {
     const unsigned int lane = threadIdx.x & 31;
     if (s.ctype == nullptr || s.done)
         return;
@@ -549,12 +647,8 @@ __device__ __forceinline__ void start_domain(PoolState *P, DomainDesc &D, const 
     int cursor = s.cursor0, fired_total = 0;
     // round 2: the rest of the descriptor goes out with the first batch of sites
     const int8_t *const layer = D.layer;
-    int32_t *const gid = D.gid;
-    const int32_t *const cts_run = D.cts_run;
-    float *const dl = D.dl, *const doc = D.doc, *const cdl = D.cdl;
-    const float *const cdl_table = D.cdl_table;
-    unsigned int *const pos = D.pos;
-    const int layer_no = D.layer_no, mx = D.mx, my = D.my, z_end = D.z_end, xoff = D.xoff, yoff = D.yoff;
+    const NucleationView V = nucleation_view(D);
+    const int layer_no = D.layer_no;
     const long long active_size = D.active_size;
     const unsigned int epoch0 = __ldcg(&D.epoch);
     const int nn0 = __ldcg(&D.nn);
@@ -590,67 +684,24 @@ __device__ __forceinline__ void start_domain(PoolState *P, DomainDesc &D, const 
                 loc = (unsigned int)l;
                 const int8_t site_type = __ldcg(s.ctype + loc);
                 const int site_layer = layer[loc];
-                h = __ldcg(gid + loc);
-                cts = cts_run[loc];
+                h = __ldcg(V.gid + loc);
+                cts = V.cts_run[loc];
                 fire = site_type == kLiquid && site_layer <= layer_no;
             }
         }
         // list slots of the firing sites (one atomic; it completes under round 4)
         const unsigned long long my_slot = fire ? warp_reserve(&P->cnt[cur], cap, &P->error) : ULLONG_MAX;
-        // round 4, one firing site at a time with the whole warp: lanes 0-12 copy the fresh
-        // octahedron's critical lengths (src/CAupdate.cpp:100-194), lane n < 26 reads neighbour n's
-        // type and list position (an active neighbour drops the site from its liquid mask)
-        const int plane = mx * my;
+        // round 4, one firing site at a time with the whole warp; an active neighbour drops the site
+        // from its liquid mask
         for (unsigned int todo = __ballot_sync(0xffffffffu, fire); todo; todo &= todo - 1) {
             const int src = __ffs(todo) - 1;
-            const unsigned int site = __shfl_sync(0xffffffffu, loc, src);
-            const int site_gid = __shfl_sync(0xffffffffu, h, src);
-            const unsigned int z = site / (unsigned int)plane;
-            const unsigned int rem = site - z * (unsigned int)plane;
-            const int rx = (int)(rem / (unsigned int)my), ry = (int)(rem - (unsigned int)rx * (unsigned int)my),
-                      rz = (int)z;
-            const unsigned int valid = edge_mask(rx, ry, rz, mx, my, z_end);
-            int ori = (abs(site_gid) - 1) % 10000;
-            if (ori < 0)
-                ori += 10000;
-            float2 row = make_float2(0.0f, 0.0f);
-            if (lane < 13)
-                row = reinterpret_cast<const float2 *>(cdl_table + 26 * ori)[lane];
-            const bool nb = lane < 26 && ((valid >> lane) & 1u);
-            int8_t nb_type = kLiquid;
-            unsigned int nb_pos = 0;
-            if (nb) {
-                const long long a = (long long)site + nb_offset((int)lane, plane, my);
-                nb_type = __ldcg(s.ctype + a);
-                nb_pos = __ldcg(pos + a);
-            }
-            const unsigned long long slot = __shfl_sync(0xffffffffu, my_slot, src);
-            if (lane < 13)
-                reinterpret_cast<float2 *>(cdl + 26ull * site)[lane] = row;
-            if (lane == 0) {
-                dl[site] = 0.01f;
-                doc[3ull * site + 0] = (float)((double)(rx + xoff) + 0.5);
-                doc[3ull * site + 1] = (float)((double)(ry + yoff) + 0.5);
-                doc[3ull * site + 2] = (float)((double)rz + 0.5);
-            }
-            if (lane == (unsigned int)src) {
-                if (slot != ULLONG_MAX) {
-                    ActiveRec r;
-                    r.cell = site;
-                    r.dl = 0.01f;
-                    r.cdl_min = 0.0f;
-                    r.cts = cts;
-                    P->rec[cur][slot] = r;
-                    P->rdom[cur][slot] = d;
-                    rstat[slot] = kMaskFresh;
-                    P->rmin2[cur][slot] = kNoMin2;
-                    pos[site] = (unsigned int)slot;
-                }
-                s.ctype[site] = kActive;
-            }
-            if (nb && nb_type == kActive && nb_pos < cap)
-                atomicAnd(rstat + nb_pos, ~(1u << nb_opp((int)lane)));
-            __syncwarp();
+            nucleate_site(V, s.ctype, P->rec[cur], P->rdom[cur], rstat, P->rmin2[cur], d,
+                          __shfl_sync(0xffffffffu, loc, src), __shfl_sync(0xffffffffu, h, src),
+                          __shfl_sync(0xffffffffu, cts, src), __shfl_sync(0xffffffffu, my_slot, src),
+                          [&](unsigned int nb_pos, int l) {
+                              if (nb_pos < cap)
+                                  atomicAnd(rstat + nb_pos, ~(1u << nb_opp(l)));
+                          });
         }
         fired_total += __popc(__ballot_sync(0xffffffffu, fire));
         cursor += n_due;
@@ -676,6 +727,7 @@ __device__ __forceinline__ void start_domain(PoolState *P, DomainDesc &D, const 
             }
         }
     }
+    const int marked = mark && !ended ? mark_sites(D, s, cursor, cycle + 1, mark_code(1), layer_no, active_size) : cursor;
     if (lane == 0 && ended) {
         D.cycle = (s.cycle0 + 999) / 1000 * 1000;
         D.done = 1;
@@ -684,6 +736,7 @@ __device__ __forceinline__ void start_domain(PoolState *P, DomainDesc &D, const 
         D.cycle = cycle;
         D.epoch = epoch0 + 1;
         D.nuc_cursor = cursor;
+        D.nuc_mark = marked;
         D.nn = nn0 + fired_total;
         D.liquid = liquid0 - fired_total;
         nucleated += fired_total;
@@ -692,13 +745,13 @@ __device__ __forceinline__ void start_domain(PoolState *P, DomainDesc &D, const 
 
 // Cycle start, per-domain part, across the grid: warps first_warp, first_warp + warp_stride, ...
 // take one domain each (the current list was settled by begin_lists before a grid-wide meeting).
-__device__ __noinline__ void begin_domains(PoolState *P, DomainDesc *desc, int n_domains, int first_warp,
-                                           int warp_stride) {
+__device__ __noinline__ void begin_domains(PoolState *P, DomainDesc *desc, int n_domains, int first_warp, int warp_stride,
+                                           bool mark) {
     const int cur = __ldcg(&P->cur);
     unsigned long long nucleated = 0;
     for (int d = first_warp; d < n_domains; d += warp_stride) {
         const DomainStart s = load_start(desc[d]);
-        start_domain(P, desc[d], s, (unsigned int)d, cur, nucleated);
+        start_domain(P, desc[d], s, (unsigned int)d, cur, mark, nucleated);
     }
     if ((threadIdx.x & 31) == 0 && nucleated)
         atomicAdd(&P->stat[0][kStatNucleated], nucleated);
@@ -706,8 +759,9 @@ __device__ __noinline__ void begin_domains(PoolState *P, DomainDesc *desc, int n
 
 // Cycle start by one block: the pool part in warp 0 while every warp loads its first domain's
 // descriptor, then the domains with the block's warps. With `close` it first ends the previous
-// cycle (finish_capture).
-__device__ __noinline__ void begin_cycle(PoolState *P, bool close, DomainDesc *desc, int n_domains, AliveSet alive) {
+// cycle (finish_capture); `mark` as start_domain.
+__device__ __noinline__ void begin_cycle(PoolState *P, bool close, DomainDesc *desc, int n_domains, AliveSet alive,
+                                         bool mark) {
     __shared__ int s_cur;
     const int w = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
     const int n = alive.n < 0 ? n_domains : alive.n;
@@ -722,13 +776,13 @@ __device__ __noinline__ void begin_cycle(PoolState *P, bool close, DomainDesc *d
         const int d = alive.n < 0 ? i : alive.idx[i];
         if (i != w)
             s = load_start(desc[d]);
-        start_domain(P, desc[d], s, (unsigned int)d, cur, nucleated);
+        start_domain(P, desc[d], s, (unsigned int)d, cur, mark, nucleated);
     }
     if ((threadIdx.x & 31) == 0 && nucleated)
         atomicAdd(&P->stat[0][kStatNucleated], nucleated);
 }
 
-__global__ void k_step_begin(PoolState *P) { begin_cycle(P, false, P->desc, P->n_domains, AliveSet{-1, {}}); }
+__global__ void k_step_begin(PoolState *P) { begin_cycle(P, false, P->desc, P->n_domains, AliveSet{-1, {}}, false); }
 
 // ---------------------------------------------------------------------------------------------
 // One CA cycle after its start (begin_cycle) is three passes over the pool:
@@ -753,9 +807,12 @@ constexpr int kBatchChoices[2] = {2, 4};
 constexpr int kLaneChoices[2] = {4, 8};
 constexpr int kErrBarrier = 8;
 
+// Work counts of one thread, added to the pool's at the end of a kernel and, in the persistent one,
+// every kStatCycles cycles (32 bits hold a thread's records of that many cycles).
+constexpr int kStatCycles = 512;
 struct CycleStats {
-    unsigned long long listed = 0, grown = 0, dropped = 0, flagged = 0, claims = 0, rows = 0, fresh = 0,
-                       captured = 0, rechecks = 0;
+    unsigned int listed = 0, grown = 0, dropped = 0, flagged = 0, claims = 0, rows = 0, fresh = 0, captured = 0,
+                 rechecks = 0;
 };
 
 __device__ void flush_stats(PoolState *P, const CycleStats &st) {
@@ -766,52 +823,83 @@ __device__ void flush_stats(PoolState *P, const CycleStats &st) {
     block_stats(P, st.rechecks, 0, kStatRechecks, kStatRechecks);
 }
 
-// Growth step of one record with its liquid mask and growth increment loaded. Returns 0: drop
-// the record, 1: keep it unchanged (not eligible yet), 2: keep the updated record.
-// eff_min: the cached minimum critical length, or the second-smallest one once the minimum's
-// neighbour is no longer liquid (both are lower bounds of the current liquid neighbours' lengths).
-__device__ __forceinline__ int grow_record(DomainDesc &D, ActiveRec &r, unsigned int m, double inc, bool inc_ok,
-                                           float eff_min, CycleStats &st) {
-    const unsigned int c = r.cell;
-    st.listed++;
-    if (D.done || (m & kMaskDead)) {
-        // finished domain, or solidified by last cycle's re-check (a retired domain's records point
-        // at the placeholder descriptor, which has no fields)
-        if (D.dl)
-            D.dl[c] = r.dl;
-        return 0;
+// What a kernel reads again and again, in shared memory: the pool's pointers and the descriptor of
+// one domain (the one with the most cells among few). A grid-wide meeting leaves L1 empty, so a
+// pointer read from global memory costs a round trip to L2 before the load that needs it goes out.
+// The copy's dynamic fields are those of the kernel's start; the persistent kernel refreshes cycle
+// and epoch every cycle.
+struct PassCtx {
+    ActiveRec *rec[2];
+    unsigned int *rdom[2], *rstat[2];
+    unsigned long long *rmin2[2];
+    DomainDesc *desc;
+    unsigned long long *tgt;
+    unsigned long long capacity, segment, shard_cap; // segment: entries of tgt a block may fill
+    long long hot_skipped;                           // cycles the hot domain's jumps skipped
+    int extras;
+    unsigned int hot;
+    DomainDesc hot_desc;
+};
+
+// Fills X (all threads of the block call; a block barrier follows before X is read).
+__device__ __forceinline__ void load_ctx(const PoolState *P, PassCtx &X, unsigned int hot) {
+    static_assert(sizeof(DomainDesc) % 8 == 0, "copied in 8-byte words");
+    const unsigned long long *src = reinterpret_cast<const unsigned long long *>(P->desc + hot);
+    unsigned long long *dst = reinterpret_cast<unsigned long long *>(&X.hot_desc);
+    for (unsigned int w = threadIdx.x; w < sizeof(DomainDesc) / 8; w += blockDim.x)
+        dst[w] = __ldcg(src + w);
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < 2; q++) {
+            X.rec[q] = P->rec[q];
+            X.rdom[q] = P->rdom[q];
+            X.rstat[q] = P->rstat[q];
+            X.rmin2[q] = P->rmin2[q];
+        }
+        X.desc = P->desc;
+        X.tgt = P->tgt;
+        X.capacity = P->capacity;
+        X.segment = P->tgt_len / gridDim.x;
+        X.shard_cap = P->shard_cap;
+        X.extras = P->extras;
+        X.hot = hot;
+        const DomainDesc &D = P->desc[hot];
+        long long skipped = 0;
+        for (int j = 0; j < D.n_jumps; j++)
+            skipped += (long long)D.jump_hi[j] - D.jump_lo[j];
+        X.hot_skipped = skipped;
     }
-    if (!(D.cycle > r.cts))
-        return 1; // cts is INT_MAX outside the window and for LayerID > layer
-    st.grown++;
-    if (!inc_ok)
-        atomicOr(&D.error, kErrGrowthTable);
-    const float dl = (float)((double)r.dl + inc);
-    r.dl = dl;
-    if ((m & kMaskFresh) || dl >= eff_min) {
-        r.cdl_min = __uint_as_float(kNeedsClaim);
-        st.flagged++;
-        return 2;
-    }
-    if ((m & kDirBits) == 0) {
-        // no liquid neighbour: LCount stays 0 (src/CAupdate.cpp:722-725)
-        D.ctype[c] = kSolid;
-        D.dl[c] = dl;
-        return 0;
-    }
-    return 2;
 }
 
-// The descriptor fields a growth step reads for every record, in registers: for the pool's first
-// domain they are loaded once per growth pass, for the others per record.
+// Domain dom's descriptor: the shared copy for the hot domain. Static fields, and cycle / epoch.
+__device__ __forceinline__ const DomainDesc &desc_of(const PassCtx &X, unsigned int dom) {
+    return dom == X.hot ? X.hot_desc : X.desc[dom];
+}
+
+// A domain's dynamic fields in one load, past L1.
+struct DomainDyn {
+    int cycle;
+    unsigned int epoch;
+    int nuc_cursor, done;
+};
+__device__ __forceinline__ DomainDyn load_dyn(const DomainDesc &D) {
+    static_assert(offsetof(DomainDesc, cycle) % 16 == 0 && offsetof(DomainDesc, epoch) == offsetof(DomainDesc, cycle) + 4 &&
+                      offsetof(DomainDesc, nuc_cursor) == offsetof(DomainDesc, cycle) + 8 &&
+                      offsetof(DomainDesc, done) == offsetof(DomainDesc, cycle) + 12,
+                  "cycle, epoch, nuc_cursor and done are one 16-byte vector");
+    const int4 v = __ldcg(reinterpret_cast<const int4 *>(&D.cycle));
+    return DomainDyn{v.x, (unsigned int)v.y, v.z, v.w};
+}
+
+// The descriptor fields a growth step reads for every record, in registers: for the hot domain they
+// are loaded once per growth pass, for the others per record.
 struct GrowView {
-    DomainDesc *D;
+    const DomainDesc *D;
     const double *growth;
     long long e_cycle; // executed cycles up to the current one
     int cycle, growth_len;
     bool done, jumps, zero_du;
 };
-__device__ __forceinline__ GrowView grow_view(DomainDesc &D) {
+__device__ __forceinline__ GrowView grow_view(const DomainDesc &D) {
     GrowView v;
     v.D = &D;
     v.growth = D.growth;
@@ -823,22 +911,39 @@ __device__ __forceinline__ GrowView grow_view(DomainDesc &D) {
     v.zero_du = D.zero_du != 0;
     return v;
 }
+__device__ __forceinline__ GrowView hot_view(const PassCtx &X, const DomainDyn &dyn) {
+    GrowView v;
+    v.D = &X.hot_desc;
+    v.growth = X.hot_desc.growth;
+    v.cycle = dyn.cycle;
+    v.e_cycle = dyn.cycle - X.hot_skipped; // every jump ends below the current cycle
+    v.growth_len = X.hot_desc.growth_len;
+    v.done = dyn.done != 0;
+    v.jumps = X.hot_desc.n_jumps > 0;
+    v.zero_du = X.hot_desc.zero_du != 0;
+    return v;
+}
 
-// grow_record with the per-record descriptor fields from a view
-__device__ __forceinline__ int grow_record(const GrowView &v, ActiveRec &r, unsigned int m, double inc, bool inc_ok,
-                                           float eff_min, CycleStats &st) {
+// Growth step of one record with its liquid mask and growth increment loaded. Returns 0: drop
+// the record, 1: keep it unchanged (not eligible yet), 2: keep the updated record.
+// eff_min: the cached minimum critical length, or the second-smallest one once the minimum's
+// neighbour is no longer liquid (both are lower bounds of the current liquid neighbours' lengths).
+__device__ __forceinline__ int grow_record(const PassCtx &X, const GrowView &v, unsigned int dom, ActiveRec &r,
+                                           unsigned int m, double inc, bool inc_ok, float eff_min, CycleStats &st) {
     const unsigned int c = r.cell;
     st.listed++;
     if (v.done || (m & kMaskDead)) {
+        // finished domain, or solidified by last cycle's re-check (a retired domain's records point
+        // at the placeholder descriptor, which has no fields)
         if (v.D->dl)
             v.D->dl[c] = r.dl;
         return 0;
     }
     if (!(v.cycle > r.cts))
-        return 1;
+        return 1; // cts is INT_MAX outside the window and for LayerID > layer
     st.grown++;
     if (!inc_ok)
-        atomicOr(&v.D->error, kErrGrowthTable);
+        atomicOr(&X.desc[dom].error, kErrGrowthTable);
     const float dl = (float)((double)r.dl + inc);
     r.dl = dl;
     if ((m & kMaskFresh) || dl >= eff_min) {
@@ -847,11 +952,26 @@ __device__ __forceinline__ int grow_record(const GrowView &v, ActiveRec &r, unsi
         return 2;
     }
     if ((m & kDirBits) == 0) {
+        // no liquid neighbour: LCount stays 0 (src/CAupdate.cpp:722-725)
         v.D->ctype[c] = kSolid;
         v.D->dl[c] = dl;
         return 0;
     }
     return 2;
+}
+
+// The mask of a record next to cells that nucleated at the start of this cycle: without the
+// directions that are no longer liquid (the nucleated cells; every other change cleared its bit).
+__device__ __noinline__ unsigned int drop_nucleated(const DomainDesc &D, unsigned int c, unsigned int m) {
+    const int plane = D.mx * D.my, my = D.my;
+    const int8_t *ct = D.ctype + c;
+    unsigned int gone = 0;
+    for (unsigned int bits = m & kDirBits; bits; bits &= bits - 1) {
+        const int l = __ffs(bits) - 1;
+        if (!liquid_type(__ldcg(ct + nb_offset(l, plane, my))))
+            gone |= 1u << l;
+    }
+    return m & ~(gone | kMaskNuc);
 }
 
 __device__ __forceinline__ float effective_min(const ActiveRec &r, unsigned int m, unsigned long long min2) {
@@ -873,24 +993,6 @@ __device__ __forceinline__ void load_growth(const GrowView &v, const ActiveRec &
         nu = 0;
     ok = nu >= 0 && nu < v.growth_len;
     inc = (ok && v.cycle > r.cts) ? __ldg(table + nu) : 0.0;
-}
-
-__device__ __forceinline__ void load_growth(const DomainDesc &D, const ActiveRec &r, double &inc, bool &ok,
-                                            bool extras) {
-    // undercooling after the executed updates since the liquidus (src/CAupdate.cpp:236-237), plus
-    // those of earlier layers; the growth table of the cell's UndercoolingChange value
-    long long nu = executed_upto(D, D.cycle) - executed_upto(D, r.cts);
-    const double *table = D.growth;
-    if (extras) {
-        if (D.nu_base)
-            nu += __ldg(D.nu_base + r.cell);
-        if (D.du_class)
-            table += (size_t)__ldg(D.du_class + r.cell) * (size_t)D.growth_len;
-    }
-    if (D.zero_du && D.du[r.cell] == 0.0f)
-        nu = 0;
-    ok = nu >= 0 && nu < D.growth_len;
-    inc = (ok && D.cycle > r.cts) ? __ldg(table + nu) : 0.0;
 }
 
 // Records the growth pass hands to the claim pass go to a global queue together with the state the
@@ -921,6 +1023,15 @@ __device__ __forceinline__ unsigned long long warp_reserve_n(unsigned long long 
     return base + incl - n;
 }
 
+// A claim of cell c in the current cycle: later epochs and lower cells compare lower.
+__device__ __forceinline__ unsigned long long claim_key(const DomainDesc &D, unsigned int c) {
+    return ((unsigned long long)(0xffffffffu - D.epoch) << 32) | (unsigned long long)c;
+}
+// A listed claim: domain, direction from the claimant and claimed cell.
+__device__ __forceinline__ unsigned long long claim_entry_of(unsigned int dom, int l, unsigned int t) {
+    return ((unsigned long long)dom << 37) | ((unsigned long long)l << 32) | t;
+}
+
 // Claim work of queue entry k. Returns the directions of the cells it claimed. All loads of the entry
 // (critical-length row, neighbour types) go out in one round.
 // A record the growth pass flagged for a claim step: its list position, cell, domain, liquid mask
@@ -930,12 +1041,15 @@ struct ClaimItem {
     float dl;
 };
 
-__device__ __forceinline__ unsigned int claim_record(PoolState *P, ActiveRec *recs, const ClaimItem &it,
-                                                     CycleStats &st, unsigned long long &tombs) {
+// With kIssue the claims go out here; otherwise the caller issues them (block_claims).
+template <bool kIssue>
+__device__ __forceinline__ unsigned int claim_record(const PassCtx &X, int app, const ClaimItem &it, CycleStats &st,
+                                                     unsigned int &tombs) {
     const unsigned int i = it.pos, c = it.cell, dom = it.dom;
     unsigned int m = it.mask;
     const float dl = it.dl;
-    DomainDesc &D = P->desc[dom];
+    const DomainDesc &D = desc_of(X, dom);
+    ActiveRec *recs = X.rec[app];
     const int plane = D.mx * D.my, my = D.my;
     // the 26 critical lengths as 7 aligned 16-byte loads: a row (26 * 4 * c bytes in) starts on a
     // 16-byte boundary for even c and 8 bytes past one for odd c, which read from 8 bytes before it
@@ -970,9 +1084,9 @@ __device__ __forceinline__ unsigned int claim_record(PoolState *P, ActiveRec *re
         for (int l = 0; l < 26; l++) {
             const bool v = (valid >> l) & 1u;
             const int8_t nt = __ldcg(ct + (v ? nb_offset(l, plane, my) : 0));
-            m |= (v && (nt == kLiquid || nt == kTemporaryUpdate)) ? (1u << l) : 0u;
+            m |= (v && liquid_type(nt)) ? (1u << l) : 0u;
         }
-        P->rstat[P->pending][i] = m | kMaskGrown; // a flagged record was grown this cycle
+        X.rstat[app][i] = m | kMaskGrown; // a flagged record was grown this cycle
     }
     if ((m & kDirBits) == 0) {
         // no liquid neighbour: LCount stays 0 (src/CAupdate.cpp:722-725)
@@ -1007,18 +1121,20 @@ __device__ __forceinline__ unsigned int claim_record(PoolState *P, ActiveRec *re
         }
     }
     recs[i].cdl_min = nm;
-    P->rmin2[P->pending][i] = ((unsigned long long)d1 << 32) | __float_as_uint(nm2);
+    X.rmin2[app][i] = ((unsigned long long)d1 << 32) | __float_as_uint(nm2);
     if (reach) {
         // claims (src/CAupdate.cpp:336-352): the lowest index wins. Nothing waits for them: every
         // claimant lists its claim and the capture pass keeps the winner's. A claimed cell reads
         // TemporaryUpdate until its capture makes it active, as in the reference's capture
         // (src/CAupdate.cpp:343-352).
-        const unsigned long long key = ((unsigned long long)(0xffffffffu - D.epoch) << 32) | (unsigned long long)c;
-        unsigned long long *base = D.claim + c;
-        for (unsigned int bits = reach; bits; bits &= bits - 1) {
-            const int nb = nb_offset(__ffs(bits) - 1, plane, my);
-            atomicMin(base + nb, key);
-            D.ctype[c + nb] = kTemporaryUpdate;
+        if (kIssue) {
+            const unsigned long long key = claim_key(D, c);
+            unsigned long long *base = D.claim + c;
+            for (unsigned int bits = reach; bits; bits &= bits - 1) {
+                const int nb = nb_offset(__ffs(bits) - 1, plane, my);
+                atomicMin(base + nb, key);
+                D.ctype[c + nb] = kTemporaryUpdate;
+            }
         }
         st.claims += __popc(reach);
     }
@@ -1026,11 +1142,12 @@ __device__ __forceinline__ unsigned int claim_record(PoolState *P, ActiveRec *re
 }
 
 // The claim step of global claim-queue entry k.
-__device__ __forceinline__ unsigned int claim_entry(PoolState *P, ActiveRec *recs, unsigned long long k,
-                                                    CycleStats &st, unsigned long long &tombs) {
+template <bool kIssue>
+__device__ __forceinline__ unsigned int claim_entry(const PoolState *P, const PassCtx &X, int app, unsigned long long k,
+                                                    CycleStats &st, unsigned int &tombs) {
     const ClaimItem it{__ldcg(P->qpos + k), __ldcg(P->qcell + k), __ldcg(P->qdom + k), __ldcg(P->qmask + k),
                        __ldcg(P->qdl + k)};
-    return claim_record(P, recs, it, st, tombs);
+    return claim_record<kIssue>(X, app, it, st, tombs);
 }
 
 // Lists the claims of one record per lane (all lanes of the warp call; reach 0: none) for the
@@ -1046,20 +1163,41 @@ __device__ __forceinline__ void list_claims(PoolState *P, unsigned int shard, un
         unsigned long long t = pos;
         for (unsigned int bits = reach; bits; bits &= bits - 1) {
             const int l = __ffs(bits) - 1;
-            P->tgt[t++] = ((unsigned long long)dom << 37) | ((unsigned long long)l << 32) |
-                          (unsigned int)((long long)cell + nb_offset(l, plane, my));
+            P->tgt[t++] = claim_entry_of(dom, l, (unsigned int)((long long)cell + nb_offset(l, plane, my)));
         }
     }
 }
 
-// The flagged records of a block wait in shared memory for the block's own claim step, which starts
-// as soon as the block has grown its records (no grid-wide wait between growth and claims). A
-// block that flags more than kBlockQueue records in a cycle sends the rest to the global queue,
-// whose claim pass then runs after a grid-wide barrier (a flag tells every block).
+// The persistent kernel's working set of one block in shared memory. The records a block flags wait
+// in its queue for its own claim step, which starts as soon as the block has grown its records (no
+// grid-wide wait between growth and claims); records beyond kBlockQueue go to the global queue,
+// whose claim pass then runs after a grid-wide barrier (a flag tells every block). The claims a block
+// makes stay in its own list up to the capture pass, where the same block keeps the winners and
+// captures them: nothing about a claim goes through global memory but the claim word itself. Claims
+// beyond kBlockClaims go to the block's segment of PoolState::tgt.
 constexpr int kBlockQueue = 1280;
-struct BlockQueue {
-    ClaimItem *items;    // kBlockQueue entries in shared memory
-    unsigned int *count; // in shared memory; may exceed kBlockQueue (the excess went global)
+constexpr int kBlockClaims = 1024;
+// A winning claim, with the state of its claimant that the capture starts from.
+struct WinItem {
+    unsigned int t, c;    // captured cell, claimant
+    unsigned int dom_dir; // (domain << 5) | direction from the claimant
+    int h, cts;           // claimant's GrainID, CritTimeStep of t
+    float docx, docy, docz;
+};
+struct BlockShared {
+    union {
+        ClaimItem items[kBlockQueue]; // growth and claims
+        WinItem wins[kBlock];         // capture
+    };
+    unsigned long long claims[kBlockClaims];
+    unsigned int n_items;  // may exceed kBlockQueue (the excess went global)
+    unsigned int n_claims; // may exceed kBlockClaims (the excess is in the block's segment)
+    unsigned int n_wins;
+    unsigned int n_first;    // cells of the hot domain this block was the first to claim this cycle
+    unsigned int n_tombs;    // records dropped this cycle
+    unsigned int n_appended; // records appended this cycle (captures and nucleations)
+    unsigned long long slot; // first record slot of the block's captures in this round
+    PassCtx X;
 };
 
 // Puts the flagged records of one growth step into the claim queue (all lanes of the warp call).
@@ -1088,7 +1226,7 @@ __device__ __forceinline__ void queue_flagged(PoolState *P, unsigned int shard, 
 // the global queue (all lanes of the warp call). Every slot below kBlockQueue that a warp reserves
 // is written in the same step, so the block's claim step reads only this cycle's records.
 template <int kBatch>
-__device__ __forceinline__ void block_queue_flagged(PoolState *P, BlockQueue bq, unsigned int shard, unsigned int nf,
+__device__ __forceinline__ void block_queue_flagged(PoolState *P, BlockShared &B, unsigned int shard, unsigned int nf,
                                                     unsigned int flagged, const unsigned long long *idx,
                                                     const ActiveRec *r, const unsigned int *dom, const unsigned int *m) {
     const unsigned int lane = threadIdx.x & 31;
@@ -1102,7 +1240,7 @@ __device__ __forceinline__ void block_queue_flagged(PoolState *P, BlockQueue bq,
     const unsigned int total = __shfl_sync(0xffffffffu, incl, 31);
     unsigned int base = 0;
     if (lane == 31 && total)
-        base = atomicAdd(bq.count, total);
+        base = atomicAdd(&B.n_items, total);
     base = __shfl_sync(0xffffffffu, base, 31);
     const unsigned int first = base + incl - nf; // this lane's first slot
     unsigned int e = first, n_global = 0;
@@ -1110,7 +1248,7 @@ __device__ __forceinline__ void block_queue_flagged(PoolState *P, BlockQueue bq,
     for (int q = 0; q < kBatch; q++)
         if (flagged & (1u << q)) {
             if (e < (unsigned int)kBlockQueue)
-                bq.items[e] = ClaimItem{(unsigned int)idx[q], r[q].cell, dom[q], m[q], r[q].dl};
+                B.items[e] = ClaimItem{(unsigned int)idx[q], r[q].cell, dom[q], m[q], r[q].dl};
             else
                 n_global++;
             e++;
@@ -1137,46 +1275,117 @@ __device__ __forceinline__ void block_queue_flagged(PoolState *P, BlockQueue bq,
     }
 }
 
+// Puts the claims of one record per lane (all lanes of the warp call; reach 0: none) into the block's list.
+__device__ __forceinline__ void push_claims(PoolState *P, BlockShared &B, unsigned int reach, unsigned int dom,
+                                            unsigned int cell) {
+    const unsigned int lane = threadIdx.x & 31, n = __popc(reach);
+    unsigned int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (unsigned)o)
+            incl += v;
+    }
+    unsigned int base = 0;
+    if (lane == 31 && incl)
+        base = atomicAdd(&B.n_claims, incl);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    if (reach) {
+        const DomainDesc &D = desc_of(B.X, dom);
+        const int plane = D.mx * D.my, my = D.my;
+        unsigned int e = base + incl - n;
+        for (unsigned int bits = reach; bits; bits &= bits - 1, e++) {
+            const int l = __ffs(bits) - 1;
+            const unsigned long long v = claim_entry_of(dom, l, (unsigned int)((long long)cell + nb_offset(l, plane, my)));
+            if (e < (unsigned int)kBlockClaims) {
+                B.claims[e] = v;
+            }
+            else {
+                const unsigned long long k = e - kBlockClaims;
+                if (k < B.X.segment)
+                    B.X.tgt[blockIdx.x * B.X.segment + k] = v;
+                else
+                    atomicOr(&P->error, kErrListOverflow);
+            }
+        }
+    }
+}
+
+// Claims of the block's list, and claim i of them (all threads agree after a block barrier).
+__device__ __forceinline__ unsigned int claim_count(const BlockShared &B) {
+    const unsigned long long most = kBlockClaims + B.X.segment;
+    return B.n_claims < most ? B.n_claims : (unsigned int)most;
+}
+__device__ __forceinline__ unsigned long long claim_at(const BlockShared &B, unsigned int i) {
+    return i < (unsigned int)kBlockClaims ? B.claims[i] : __ldcg(B.X.tgt + blockIdx.x * B.X.segment + (i - kBlockClaims));
+}
+
+// Issues the claims [first, claim_count) of the block's list, one per thread (src/CAupdate.cpp:336-352;
+// all threads of the block call, after a block barrier). A claim that finds an older epoch in the
+// claim word is the first on its cell, which is captured in this cycle: one liquid cell less, known
+// before the capture pass. The hot domain's are counted in shared memory.
+__device__ __forceinline__ void issue_claims(BlockShared &B, unsigned int first) {
+    const unsigned int n = claim_count(B);
+    unsigned int firsts = 0;
+    for (unsigned int i = first + threadIdx.x; i < n; i += kBlock) {
+        const unsigned long long e = claim_at(B, i);
+        const unsigned int dom = (unsigned int)(e >> 37), t = (unsigned int)e;
+        const DomainDesc &D = desc_of(B.X, dom);
+        const unsigned int c = (unsigned int)((long long)t - nb_offset((int)((e >> 32) & 31u), D.mx * D.my, D.my));
+        const unsigned long long key = claim_key(D, c);
+        const unsigned long long old = atomicMin(D.claim + t, key);
+        D.ctype[t] = kTemporaryUpdate;
+        if ((old >> 32) != (key >> 32)) {
+            if (dom == B.X.hot)
+                firsts++;
+            else
+                atomicAdd((unsigned long long *)&B.X.desc[dom].liquid_shard[i & (kLiquidShards - 1)],
+                          (unsigned long long)(-1ll));
+        }
+    }
+    firsts = __reduce_add_sync(0xffffffffu, firsts);
+    if ((threadIdx.x & 31) == 0 && firsts)
+        atomicAdd(&B.n_first, firsts);
+}
+
 // The block's claim step over its queue (all threads of the block call, after the block's growth).
-__device__ __forceinline__ void block_claims(PoolState *P, BlockQueue bq, unsigned int shard, CycleStats &st,
-                                             unsigned long long &tombs) {
+__device__ __forceinline__ void block_claims(PoolState *P, BlockShared &B, int app, CycleStats &st,
+                                             unsigned int &tombs) {
     __syncthreads();
-    // one store per block: every warp of the grid storing to this flag once its block's queue was
-    // full serialised on one L2 slice
-    if (threadIdx.x == 0 && *bq.count > (unsigned int)kBlockQueue)
-        P->claim_overflow = 1;
-    const unsigned int n = min(*bq.count, (unsigned int)kBlockQueue);
-    ActiveRec *recs = P->rec[P->pending];
+    const unsigned int n = min(B.n_items, (unsigned int)kBlockQueue);
+    if (n == 0)
+        return;
     const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (unsigned int k0 = warp * 32; k0 < n; k0 += kBlock) {
         const unsigned int k = k0 + lane;
         unsigned int reach = 0, dom = 0, cell = 0;
         if (k < n) {
-            const ClaimItem it = bq.items[k];
-            reach = claim_record(P, recs, it, st, tombs);
+            const ClaimItem it = B.items[k];
+            reach = claim_record<false>(B.X, app, it, st, tombs);
             dom = it.dom;
             cell = it.cell;
         }
-        list_claims(P, shard, reach, dom, cell);
+        push_claims(P, B, reach, dom, cell);
     }
+    __syncthreads();
+    issue_claims(B, 0);
 }
 
 // Growth step of a compaction cycle: the survivors are written to the other list (rare; kept out of
 // line).
-__device__ __noinline__ void compact_pass(PoolState *P, int cur, unsigned long long gw, unsigned long long nw,
-                                         unsigned long long n, CycleStats &st, const BlockQueue *bq) {
+__device__ __noinline__ void compact_pass(PoolState *P, const PassCtx &X, int cur, unsigned long long gw,
+                                         unsigned long long nw, unsigned long long n, const DomainDyn &dyn,
+                                         CycleStats &st, BlockShared *B) {
     const unsigned int lane = threadIdx.x & 31;
-    DomainDesc *desc = P->desc;
-    const bool extras = P->extras;
-    const ActiveRec *in = P->rec[cur];
-    const unsigned int *in_dom = P->rdom[cur];
-    const unsigned int *in_stat = P->rstat[cur];
-    const unsigned long long *in_min2 = P->rmin2[cur];
+    const ActiveRec *in = X.rec[cur];
+    const unsigned int *in_dom = X.rdom[cur];
+    const unsigned int *in_stat = X.rstat[cur];
+    const unsigned long long *in_min2 = X.rmin2[cur];
     const int nxt = cur ^ 1;
-    ActiveRec *out = P->rec[nxt];
-    unsigned int *out_dom = P->rdom[nxt];
-    unsigned int *out_stat = P->rstat[nxt];
-    unsigned long long *out_min2 = P->rmin2[nxt];
+    ActiveRec *out = X.rec[nxt];
+    unsigned int *out_dom = X.rdom[nxt];
+    unsigned int *out_stat = X.rstat[nxt];
+    unsigned long long *out_min2 = X.rmin2[nxt];
     const unsigned long long groups = (n + 31) / 32;
     for (unsigned long long g = gw; g < groups; g += nw) {
         unsigned long long i = g * 32 + lane;
@@ -1192,10 +1401,13 @@ __device__ __noinline__ void compact_pass(PoolState *P, int cur, unsigned long l
             m = __ldcg(in_stat + i) & ~kMaskKeep;
             mn2 = __ldcg(in_min2 + i);
             if (r.cell != kTombstone) {
+                if (m & kMaskNuc)
+                    m = drop_nucleated(desc_of(X, dom), r.cell, m);
+                const GrowView view = dom == X.hot ? hot_view(X, dyn) : grow_view(X.desc[dom]);
                 double inc;
                 bool ok;
-                load_growth(desc[dom], r, inc, ok, extras);
-                const int a = grow_record(desc[dom], r, m, inc, ok, effective_min(r, m, mn2), st);
+                load_growth(view, r, inc, ok, X.extras);
+                const int a = grow_record(X, view, dom, r, m, inc, ok, effective_min(r, m, mn2), st);
                 keep = a != 0;
                 if (a == 2)
                     m |= kMaskGrown;
@@ -1203,19 +1415,19 @@ __device__ __noinline__ void compact_pass(PoolState *P, int cur, unsigned long l
                     st.dropped++;
             }
         }
-        const unsigned long long pos = warp_reserve_n(&P->cnt[nxt], P->capacity, &P->error, keep ? 1u : 0u);
+        const unsigned long long pos = warp_reserve_n(&P->cnt[nxt], X.capacity, &P->error, keep ? 1u : 0u);
         const bool placed = keep && pos != ULLONG_MAX;
         if (placed) {
             out[pos] = r;
             out_dom[pos] = dom;
             out_stat[pos] = m;
             out_min2[pos] = mn2;
-            desc[dom].pos[r.cell] = (unsigned int)pos;
+            desc_of(X, dom).pos[r.cell] = (unsigned int)pos;
         }
         const bool flag = placed && __float_as_uint(r.cdl_min) == kNeedsClaim;
         unsigned long long idx = pos;
-        if (bq)
-            block_queue_flagged<1>(P, *bq, (unsigned int)(gw % kShards), flag ? 1u : 0u, flag ? 1u : 0u, &idx, &r,
+        if (B)
+            block_queue_flagged<1>(P, *B, (unsigned int)(gw % kShards), flag ? 1u : 0u, flag ? 1u : 0u, &idx, &r,
                                    &dom, &m);
         else
             queue_flagged<1>(P, (unsigned int)(gw % kShards), flag ? 1u : 0u, flag ? 1u : 0u, &idx, &r, &dom, &m);
@@ -1226,39 +1438,38 @@ __device__ __noinline__ void compact_pass(PoolState *P, int cur, unsigned long l
 // group g to warp g % (number of warps of the grid), consecutive warps on different blocks: the
 // records appended by the last capture pass, which all need a fresh mask and claims, spread over
 // every SM. No block-wide synchronisation.
-template <int kBatch, bool kBlockClaims> __device__ void grow_pass(PoolState *P, CycleStats &st, unsigned int hot = 0) {
-    const int cur = P->cur;
-    const unsigned long long n = P->cnt[cur];
+// With kOwnClaims (B given) the block's flagged records go to its queue and their claim steps follow
+// here. cur is the list to read, n its length; with `compact` the survivors go to the other list.
+template <int kBatch, bool kOwnClaims>
+__device__ void grow_pass(PoolState *P, PassCtx &X, BlockShared *B, int cur, unsigned long long n, bool compact,
+                          CycleStats &st, unsigned int &tombs) {
     const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned long long nw = (unsigned long long)gridDim.x * (kBlock / 32);
     const unsigned long long gw = (unsigned long long)warp * gridDim.x + blockIdx.x;
     const unsigned int shard = (unsigned int)(gw % kShards);
-    __shared__ ClaimItem s_items[kBlockClaims ? kBlockQueue : 1];
-    __shared__ unsigned int s_count;
-    const BlockQueue bq{s_items, &s_count};
-    if (kBlockClaims) {
-        if (threadIdx.x == 0)
-            s_count = 0;
-        __syncthreads();
+    const unsigned int hot = X.hot;
+    const DomainDyn dyn = load_dyn(X.desc[hot]);
+    if (kOwnClaims && threadIdx.x == 0) {
+        // read by the block's claim step, after its first barrier
+        X.hot_desc.cycle = dyn.cycle;
+        X.hot_desc.epoch = dyn.epoch;
     }
-    if (P->compact) {
-        compact_pass(P, cur, gw, nw, n, st, kBlockClaims ? &bq : nullptr);
-        if (kBlockClaims) {
-            unsigned long long claim_tombs = 0; // a compacted list starts without dropped records
-            block_claims(P, bq, shard, st, claim_tombs);
+    if (compact) {
+        compact_pass(P, X, cur, gw, nw, n, dyn, st, kOwnClaims ? B : nullptr);
+        if (kOwnClaims) {
+            unsigned int claim_tombs = 0; // a compacted list starts without dropped records
+            block_claims(P, *B, cur ^ 1, st, claim_tombs);
         }
         return;
     }
-    ActiveRec *in = P->rec[cur];
-    const unsigned int *in_dom = P->rdom[cur];
-    unsigned int *in_stat = P->rstat[cur];
-    const unsigned long long *in_min2 = P->rmin2[cur];
-    DomainDesc *desc = P->desc;
-    const bool extras = P->extras;
-    unsigned long long tombs = 0;
+    ActiveRec *in = X.rec[cur];
+    const unsigned int *in_dom = X.rdom[cur];
+    unsigned int *in_stat = X.rstat[cur];
+    const unsigned long long *in_min2 = X.rmin2[cur];
+    const bool extras = X.extras;
     const unsigned long long groups = (n + 31) / 32;
-    // the growth fields of one domain (the one with the most cells among few) held in registers
-    const GrowView v0 = grow_view(desc[hot]);
+    // the growth fields of the hot domain held in registers
+    const GrowView v0 = hot_view(X, dyn);
     // records are updated in place; dropped ones become tombstones
     for (unsigned long long g0 = gw; g0 < groups; g0 += kBatch * nw) {
         ActiveRec r[kBatch];
@@ -1287,15 +1498,17 @@ template <int kBatch, bool kBlockClaims> __device__ void grow_pass(PoolState *P,
             inc[q] = 0.0;
             ok[q] = true;
             if (r[q].cell != kTombstone) {
-                if (m[q] & kMaskKeep) {
+                if (m[q] & (kMaskKeep | kMaskNuc)) {
                     // the neighbour verdict of the previous cycle does not carry over
                     m[q] &= ~kMaskKeep;
+                    if (m[q] & kMaskNuc)
+                        m[q] = drop_nucleated(desc_of(X, dom[q]), r[q].cell, m[q]);
                     in_stat[idx[q]] = m[q];
                 }
                 if (dom[q] == hot)
                     load_growth(v0, r[q], inc[q], ok[q], extras);
                 else
-                    load_growth(grow_view(desc[dom[q]]), r[q], inc[q], ok[q], extras);
+                    load_growth(grow_view(X.desc[dom[q]]), r[q], inc[q], ok[q], extras);
             }
         }
         unsigned int flagged = 0;
@@ -1303,9 +1516,10 @@ template <int kBatch, bool kBlockClaims> __device__ void grow_pass(PoolState *P,
         for (int q = 0; q < kBatch; q++) {
             if (r[q].cell == kTombstone)
                 continue;
-            const int a = dom[q] == hot ? grow_record(v0, r[q], m[q], inc[q], ok[q], effective_min(r[q], m[q], mn2[q]), st)
-                                      : grow_record(grow_view(desc[dom[q]]), r[q], m[q], inc[q], ok[q],
-                                                    effective_min(r[q], m[q], mn2[q]), st);
+            const float eff_min = effective_min(r[q], m[q], mn2[q]);
+            const int a = dom[q] == hot
+                              ? grow_record(X, v0, dom[q], r[q], m[q], inc[q], ok[q], eff_min, st)
+                              : grow_record(X, grow_view(X.desc[dom[q]]), dom[q], r[q], m[q], inc[q], ok[q], eff_min, st);
             if (a == 0) {
                 in[idx[q]].cell = kTombstone;
                 in[idx[q]].cdl_min = 0.0f;
@@ -1322,19 +1536,21 @@ template <int kBatch, bool kBlockClaims> __device__ void grow_pass(PoolState *P,
                     flagged |= 1u << q;
             }
         }
-        if (kBlockClaims)
-            block_queue_flagged<kBatch>(P, bq, shard, __popc(flagged), flagged, idx, r, dom, m);
+        if (kOwnClaims)
+            block_queue_flagged<kBatch>(P, *B, shard, __popc(flagged), flagged, idx, r, dom, m);
         else
             queue_flagged<kBatch>(P, shard, __popc(flagged), flagged, idx, r, dom, m);
     }
-    if (kBlockClaims)
-        block_claims(P, bq, shard, st, tombs);
-    // dropped records stay as tombstones of the in-place list until the next compaction
-#pragma unroll
-    for (int o = 16; o; o >>= 1)
-        tombs += __shfl_down_sync(0xffffffffu, tombs, o);
-    if (lane == 0 && tombs)
-        atomicAdd(&P->tomb_s[gw % kShards].v, tombs);
+    if (kOwnClaims)
+        block_claims(P, *B, cur, st, tombs);
+}
+
+// Dropped records stay as tombstones of the in-place list until the next compaction; the separate
+// kernels count them in shards.
+__device__ __forceinline__ void add_tombs(PoolState *P, unsigned int tombs) {
+    tombs = __reduce_add_sync(0xffffffffu, tombs);
+    if ((threadIdx.x & 31) == 0 && tombs)
+        atomicAdd(&P->tomb_s[(blockIdx.x + (threadIdx.x >> 5)) % kShards].v, (unsigned long long)tombs);
 }
 
 // Exclusive prefix of the shard counts in shared memory (all threads of the block call).
@@ -1367,122 +1583,89 @@ __device__ __forceinline__ unsigned long long shard_entry(const unsigned long lo
     return (unsigned long long)lo * cap + (k - pre[lo]);
 }
 
-// One queue entry per thread, consecutive warps on different blocks; every claim is listed.
-__device__ void claim_pass(PoolState *P, CycleStats &st) {
+// One queue entry per thread, consecutive warps on different blocks; every claim is listed, in the
+// block's own list (B, persistent kernel) or the sharded global one.
+template <bool kOwnClaims>
+__device__ void claim_pass(PoolState *P, PassCtx &X, BlockShared *B, int app, CycleStats &st, unsigned int &tombs) {
     __shared__ unsigned long long s_pre[kShards + 1];
     shard_prefix(P->qcnt_s, s_pre);
     const unsigned long long nq = s_pre[kShards];
-    const unsigned long long cap = P->shard_cap;
-    ActiveRec *recs = P->rec[P->pending];
+    const unsigned long long cap = X.shard_cap;
     const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned long long nw = (unsigned long long)gridDim.x * (kBlock / 32);
     const unsigned long long gw = (unsigned long long)warp * gridDim.x + blockIdx.x;
-    unsigned long long tombs = 0;
+    const unsigned int listed = kOwnClaims ? claim_count(*B) : 0u; // claims of the block's own queue
+    if (kOwnClaims)
+        __syncthreads();
     for (unsigned long long k0 = gw * 32; k0 < nq; k0 += nw * 32) {
         const unsigned long long k = k0 + lane;
         unsigned int reach = 0, dom = 0, cell = 0;
         if (k < nq) {
             const unsigned long long e = shard_entry(s_pre, cap, k);
-            reach = claim_entry(P, recs, e, st, tombs);
+            reach = claim_entry<!kOwnClaims>(P, X, app, e, st, tombs);
             dom = __ldcg(P->qdom + e);
             cell = __ldcg(P->qcell + e);
         }
-        list_claims(P, (unsigned int)(gw % kShards), reach, dom, cell);
+        if (kOwnClaims)
+            push_claims(P, *B, reach, dom, cell);
+        else
+            list_claims(P, (unsigned int)(gw % kShards), reach, dom, cell);
     }
-    if (!P->compact) {
-#pragma unroll
-        for (int o = 16; o; o >>= 1)
-            tombs += __shfl_down_sync(0xffffffffu, tombs, o);
-        if (lane == 0 && tombs)
-            atomicAdd(&P->tomb_s[gw % kShards].v, tombs);
+    if (kOwnClaims) {
+        __syncthreads();
+        issue_claims(*B, listed);
     }
 }
 
-template <int kCaptureLanes> __device__ void capture_pass(PoolState *P, CycleStats &st) {
-    __shared__ unsigned long long s_pre[kShards + 1];
-    shard_prefix(P->tcnt_s, s_pre);
-    const int app = P->pending; // list of the next cycle
-    const unsigned long long T = s_pre[kShards];
-    const unsigned long long cap = P->shard_cap;
-    // records of the cells active at the start of the cycle lie below base; claim j of the cycle
-    // gets record slot base + j (a tombstone unless it won), and the count grows by T when the
-    // cycle finishes
-    const unsigned long long base = P->cnt[app];
-    if (base + T > P->capacity) {
-        if (threadIdx.x == 0 && blockIdx.x == 0)
-            atomicOr(&P->error, kErrListOverflow);
-        return;
-    }
-    DomainDesc *desc = P->desc;
-    unsigned long long losers = 0;
-    unsigned int *rs = P->rstat[app];
-    constexpr int kGroups = 32 / kCaptureLanes;
-    constexpr int kPer = (26 + kCaptureLanes - 1) / kCaptureLanes;
-    const int lane = threadIdx.x & 31;
-    const int grp = lane / kCaptureLanes, sub = lane % kCaptureLanes;
-    // consecutive claims on different blocks (spread over all SMs)
-    const unsigned long long ngroups = (unsigned long long)gridDim.x * (kBlock / 32) * kGroups;
-    const unsigned long long g0 = ((unsigned long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * kGroups + grp;
-    for (unsigned long long j = g0; j < T; j += ngroups) {
-        const unsigned long long e = __ldcg(P->tgt + shard_entry(s_pre, cap, j));
-        const unsigned int t = (unsigned int)e;
-        const int l = (int)((e >> 32) & 31u);
-        const unsigned int dom = (unsigned int)(e >> 37);
-        DomainDesc &D = desc[dom];
+// Captures cell w.t by its winning claimant with a group of kLanes lanes (on: the group has a winner;
+// every group of the block calls): the new octahedron, the masks of the captured cell's active
+// neighbours and their solidification re-checks, and the new record in slot slot_of() of list `app`
+// (ULLONG_MAX: none). Records of the cells active at the start of the cycle lie below base. A cell of
+// type also_liquid (a mark of the cycle after next, or kLiquid) is liquid in the next cycle.
+template <int kLanes, class SlotOf>
+__device__ __forceinline__ void capture_group(const PassCtx &X, int app, unsigned long long base, const WinItem &w,
+                                              bool on, int8_t also_liquid, SlotOf &&slot_of, CycleStats &st) {
+    constexpr int kPer = (26 + kLanes - 1) / kLanes;
+    const int lane = threadIdx.x & 31, grp = lane / kLanes, sub = lane % kLanes;
+    const unsigned int group = (kLanes == 32 ? 0xffffffffu : ((1u << kLanes) - 1u)) << (grp * kLanes);
+    const unsigned int t = w.t, c = w.c, dom = w.dom_dir >> 5;
+    const int l = (int)(w.dom_dir & 31u);
+    const DomainDesc &D = desc_of(X, dom);
+    unsigned int *rs = X.rstat[app];
+    unsigned int a[kPer], p[kPer], old[kPer];
+    bool act[kPer];
+    unsigned int liq = 0, d1 = 0xffffffffu;
+    float mn = __int_as_float(0x7f800000), mn2 = mn, new_dl = 0.0f;
+    if (on) {
+        // Lane `sub` takes the neighbour slots sub, sub + kLanes, ... (slot_dir): a load instruction's
+        // lanes read neighbours in few rows of three consecutive cells.
         const int plane = D.mx * D.my, my = D.my;
-        const unsigned int c = (unsigned int)((long long)t - nb_offset(l, plane, my)); // the claimant
-        // Every load of the capture and of the re-checks goes out in one round; only the group of
-        // the winning claim (the lowest claimant index) continues. Lane `sub` takes the neighbour
-        // slots sub, sub + kCaptureLanes, ... (slot_dir): a load instruction's lanes read
-        // neighbours in few rows of three consecutive cells.
-        const unsigned long long key = __ldcg(D.claim + t);
-        const int cts_t = __ldg(D.cts_run + t);
-        const int h = __ldcg(D.gid + c);
-        const float docx = __ldcg(D.doc + 3ull * c + 0), docy = __ldcg(D.doc + 3ull * c + 1),
-                    docz = __ldcg(D.doc + 3ull * c + 2);
         int tx, ty, tz;
         cell_coords(D, t, tx, ty, tz);
         const unsigned int valid = neighbour_mask(D, tx, ty, tz);
-        unsigned int a[kPer], p[kPer], old[kPer];
         int8_t ct[kPer];
-        bool act[kPer];
 #pragma unroll
         for (int k = 0; k < kPer; k++) {
-            const int ln = slot_dir(sub + k * kCaptureLanes);
+            const int ln = slot_dir(sub + k * kLanes);
             act[k] = ln < 26 && (valid & (1u << ln));
             a[k] = (unsigned int)((long long)t + (act[k] ? nb_offset(ln, plane, my) : 0));
             ct[k] = __ldcg(D.ctype + a[k]);
             p[k] = __ldcg(D.pos + a[k]);
         }
-        if ((unsigned int)key != c) {
-            // a lower-index claimant captures t; this claim's slot stays a dropped record
-            if (sub == 0) {
-                P->rec[app][base + j].cell = kTombstone;
-                P->rec[app][base + j].cdl_min = 0.0f;
-                losers++;
-            }
-            continue;
-        }
-        const unsigned int w = c;
         // The captured cell's liquid-neighbour mask, as its first claim step would build it from the
         // neighbour types at the start of a later cycle: the neighbours still liquid (a neighbour
         // claimed in this cycle reads TemporaryUpdate, or active once captured). Later captures and
         // nucleations clear bits of it as of every other record's (it lies below later cycles' base).
-        unsigned int liq = 0;
 #pragma unroll
         for (int k = 0; k < kPer; k++)
-            if (act[k] && ct[k] == kLiquid)
-                liq |= 1u << slot_dir(sub + k * kCaptureLanes);
-        {
-            const unsigned int group = (kCaptureLanes == 32 ? 0xffffffffu : ((1u << kCaptureLanes) - 1u))
-                                       << (grp * kCaptureLanes);
+            if (act[k] && (ct[k] == kLiquid || ct[k] == also_liquid))
+                liq |= 1u << slot_dir(sub + k * kLanes);
 #pragma unroll
-            for (int o = kCaptureLanes / 2; o; o >>= 1)
-                liq |= __shfl_xor_sync(group, liq, o);
-        }
+        for (int o = kLanes / 2; o; o >>= 1)
+            liq |= __shfl_xor_sync(group, liq, o);
         // Serial order (src/CAupdate.cpp:333-334, 722-725): active cell a saw the captured cell t
-        // as liquid iff t's capturer w does not precede a. a keeps a liquid neighbour iff it has an
-        // unclaimed one (a set mask bit that nobody clears) or a claimed one with w >= a. Every
+        // as liquid iff t's capturer c does not precede a. a keeps a liquid neighbour iff it has an
+        // unclaimed one (a set mask bit that nobody clears) or a claimed one with c >= a. Every
         // claimed liquid neighbour clears its own bit exactly once, so the update that clears the
         // last direction bit sees the final verdict: KEEP is always set before the clear of the
         // same update, and an update's two atomics reach the word in program order. Only records of
@@ -1493,70 +1676,199 @@ template <int kCaptureLanes> __device__ void capture_pass(PoolState *P, CycleSta
             act[k] = act[k] && ct[k] == kActive && p[k] < base;
 #pragma unroll
         for (int k = 0; k < kPer; k++)
-            if (act[k] && w >= a[k])
+            if (act[k] && c >= a[k])
                 atomicOr(rs + p[k], kMaskKeep);
 #pragma unroll
         for (int k = 0; k < kPer; k++) {
             old[k] = 0;
             if (act[k])
-                old[k] = atomicAnd(rs + p[k], ~(1u << nb_opp(slot_dir(sub + k * kCaptureLanes))));
+                old[k] = atomicAnd(rs + p[k], ~(1u << nb_opp(slot_dir(sub + k * kLanes))));
         }
         // The new record's cached minimum critical length over its liquid neighbours, with its
         // direction and the second-smallest (the state a claim step leaves), so that its first claim
         // step runs only once its DiagonalLength reaches a liquid neighbour.
-        float mn = __int_as_float(0x7f800000), mn2 = mn;
-        unsigned int d1 = 0xffffffffu;
-        const float new_dl =
-            capture_cell<kCaptureLanes>(D, c, t, l, sub, h, docx, docy, docz, liq, mn, d1, mn2);
-        {
-            const unsigned int group = (kCaptureLanes == 32 ? 0xffffffffu : ((1u << kCaptureLanes) - 1u))
-                                       << (grp * kCaptureLanes);
+        new_dl = capture_cell<kLanes>(D, c, t, l, sub, w.h, w.docx, w.docy, w.docz, liq, mn, d1, mn2);
 #pragma unroll
-            for (int o = kCaptureLanes / 2; o; o >>= 1) {
-                const float omn = __shfl_xor_sync(group, mn, o), omn2 = __shfl_xor_sync(group, mn2, o);
-                const unsigned int od1 = __shfl_xor_sync(group, d1, o);
-                if (omn < mn || (omn == mn && od1 < d1)) {
-                    mn2 = fminf(omn2, mn);
-                    mn = omn;
-                    d1 = od1;
-                }
-                else {
-                    mn2 = fminf(mn2, omn);
-                }
+        for (int o = kLanes / 2; o; o >>= 1) {
+            const float omn = __shfl_xor_sync(group, mn, o), omn2 = __shfl_xor_sync(group, mn2, o);
+            const unsigned int od1 = __shfl_xor_sync(group, d1, o);
+            if (omn < mn || (omn == mn && od1 < d1)) {
+                mn2 = fminf(omn2, mn);
+                mn = omn;
+                d1 = od1;
+            }
+            else {
+                mn2 = fminf(mn2, omn);
             }
         }
-        if (sub == 0) {
+    }
+    const unsigned long long slot = slot_of();
+    if (!on)
+        return;
+    if (sub == 0) {
+        if (slot != ULLONG_MAX) {
             ActiveRec r;
             r.cell = t;
             r.dl = new_dl;
             r.cdl_min = mn;
-            r.cts = cts_t;
-            P->rec[app][base + j] = r;
-            P->rdom[app][base + j] = dom;
-            rs[base + j] = liq;
-            P->rmin2[app][base + j] = ((unsigned long long)d1 << 32) | __float_as_uint(mn2);
-            D.pos[t] = (unsigned int)(base + j);
-            // read as active by the growth pass of the next cycle, after the octahedron is written
-            D.ctype[t] = kActive;
-            atomicAdd((unsigned long long *)&D.liquid_shard[(blockIdx.x + j) & (kLiquidShards - 1)],
-                      (unsigned long long)(-1ll));
-            st.captured++;
+            r.cts = w.cts;
+            X.rec[app][slot] = r;
+            X.rdom[app][slot] = dom;
+            rs[slot] = liq;
+            X.rmin2[app][slot] = ((unsigned long long)d1 << 32) | __float_as_uint(mn2);
+            D.pos[t] = (unsigned int)slot;
         }
+        // read as active by the growth pass of the next cycle, after the octahedron is written
+        D.ctype[t] = kActive;
+        st.captured++;
+    }
 #pragma unroll
-        for (int k = 0; k < kPer; k++) {
-            if (!act[k])
-                continue;
-            const unsigned int bit = 1u << nb_opp(slot_dir(sub + k * kCaptureLanes));
-            if ((old[k] & (kMaskFresh | kMaskDead)) || (old[k] & kDirBits) != bit || (old[k] & kMaskKeep))
-                continue;
-            // a lost its last liquid neighbour; it solidifies if it was grown this cycle (cycle >
-            // its CritTimeStep, src/CAupdate.cpp:257-261)
-            if (old[k] & kMaskGrown) {
-                st.rechecks++;
-                D.ctype[a[k]] = kSolid;
-                atomicOr(rs + p[k], kMaskDead);
-            }
+    for (int k = 0; k < kPer; k++) {
+        if (!act[k])
+            continue;
+        const unsigned int bit = 1u << nb_opp(slot_dir(sub + k * kLanes));
+        if ((old[k] & (kMaskFresh | kMaskDead)) || (old[k] & kDirBits) != bit || (old[k] & kMaskKeep))
+            continue;
+        // a lost its last liquid neighbour; it solidifies if it was grown this cycle (cycle >
+        // its CritTimeStep, src/CAupdate.cpp:257-261)
+        if (old[k] & kMaskGrown) {
+            st.rechecks++;
+            D.ctype[a[k]] = kSolid;
+            atomicOr(rs + p[k], kMaskDead);
         }
+    }
+}
+
+// Listed claim e: whether it won (the lowest claimant index holds the claim word) and its capture's
+// starting state, in one round of loads.
+__device__ __forceinline__ bool load_win(const PassCtx &X, unsigned long long e, WinItem &w) {
+    const unsigned int dom = (unsigned int)(e >> 37);
+    const int l = (int)((e >> 32) & 31u);
+    const DomainDesc &D = desc_of(X, dom);
+    w.t = (unsigned int)e;
+    w.c = (unsigned int)((long long)w.t - nb_offset(l, D.mx * D.my, D.my));
+    w.dom_dir = (dom << 5) | (unsigned int)l;
+    const unsigned long long key = __ldcg(D.claim + w.t);
+    w.cts = __ldg(D.cts_run + w.t);
+    w.h = __ldcg(D.gid + w.c);
+    w.docx = __ldcg(D.doc + 3ull * w.c + 0);
+    w.docy = __ldcg(D.doc + 3ull * w.c + 1);
+    w.docz = __ldcg(D.doc + 3ull * w.c + 2);
+    return (unsigned int)key == w.c;
+}
+
+// A barrier of the block's first `threads` threads (a multiple of 32).
+__device__ __forceinline__ void capture_sync(unsigned int threads) {
+    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+}
+
+// The captures of the block's winners in B.wins by its first `threads` threads, kLanes lanes each.
+template <int kLanes>
+__device__ __forceinline__ void capture_wins(BlockShared &B, unsigned int threads, unsigned int n_wins, int app,
+                                             unsigned long long base, int8_t also_liquid, CycleStats &st) {
+    const unsigned int n_groups = threads / kLanes, grp = threadIdx.x / kLanes;
+    for (unsigned int first = 0; first < n_wins; first += n_groups) {
+        const unsigned int i = first + grp;
+        const bool on = i < n_wins;
+        WinItem w{};
+        if (on)
+            w = B.wins[i];
+        capture_group<kLanes>(
+            B.X, app, base, w, on, also_liquid,
+            [&]() -> unsigned long long {
+                if (first == 0)
+                    capture_sync(threads); // the block's slots are reserved
+                return B.slot == ULLONG_MAX ? ULLONG_MAX : B.slot + i;
+            },
+            st);
+    }
+}
+
+// Capture pass of the persistent kernel, by the first `threads` threads of the block (its other warps
+// start the domains' next cycle). Each block keeps the winners among its own claims (one per
+// thread), reserves their record slots with one atomic (which completes under the captures) and
+// captures them. A block with few winners spends a whole warp on each: its time is then one chain
+// of loads and geometry, and a wider group shortens the chain (one neighbour and one critical
+// length per lane); with many, narrower groups keep the chains of a block in one round.
+template <int kLanes>
+__device__ void capture_block(PoolState *P, BlockShared &B, unsigned int threads, int app, unsigned long long base,
+                              unsigned long long *appended, int8_t also_liquid, CycleStats &st) {
+    const unsigned int n = claim_count(B), lane = threadIdx.x & 31;
+    for (unsigned int r0 = 0; r0 < n; r0 += threads) {
+        const unsigned int i = r0 + threadIdx.x;
+        WinItem w;
+        const bool win = i < n && load_win(B.X, claim_at(B, i), w);
+        const unsigned int winners = __ballot_sync(0xffffffffu, win);
+        unsigned int first = 0;
+        if (lane == 0 && winners)
+            first = atomicAdd(&B.n_wins, __popc(winners));
+        first = __shfl_sync(0xffffffffu, first, 0);
+        if (win)
+            B.wins[first + __popc(winners & ((1u << lane) - 1u))] = w;
+        capture_sync(threads);
+        const unsigned int n_wins = B.n_wins;
+        if (threadIdx.x == threads - 32) {
+            unsigned long long slot = ULLONG_MAX;
+            if (n_wins) {
+                atomicAdd(&B.n_appended, n_wins);
+                slot = base + atomicAdd(appended, (unsigned long long)n_wins);
+                if (slot + n_wins > B.X.capacity) {
+                    atomicOr(&P->error, kErrListOverflow);
+                    slot = ULLONG_MAX;
+                }
+            }
+            B.slot = slot;
+        }
+        if (n_wins * 32 <= threads)
+            capture_wins<32>(B, threads, n_wins, app, base, also_liquid, st);
+        else if (kLanes < 8 && n_wins * 8 <= threads)
+            capture_wins<8>(B, threads, n_wins, app, base, also_liquid, st);
+        else
+            capture_wins<kLanes>(B, threads, n_wins, app, base, also_liquid, st);
+        if (r0 + threads < n) {
+            capture_sync(threads);
+            if (threadIdx.x == 0)
+                B.n_wins = 0;
+            capture_sync(threads);
+        }
+    }
+}
+
+// Capture pass over the sharded claim list (the separate kernels): claim j of the cycle gets record
+// slot base + j (a tombstone unless it won), and the count grows by T when the cycle finishes.
+template <int kCaptureLanes> __device__ void capture_pass(PoolState *P, const PassCtx &X, CycleStats &st) {
+    __shared__ unsigned long long s_pre[kShards + 1];
+    shard_prefix(P->tcnt_s, s_pre);
+    const int app = P->pending; // list of the next cycle
+    const unsigned long long T = s_pre[kShards];
+    const unsigned long long cap = P->shard_cap;
+    const unsigned long long base = P->cnt[app];
+    if (base + T > P->capacity) {
+        if (threadIdx.x == 0 && blockIdx.x == 0)
+            atomicOr(&P->error, kErrListOverflow);
+        return;
+    }
+    unsigned long long losers = 0;
+    constexpr int kGroups = 32 / kCaptureLanes;
+    const int lane = threadIdx.x & 31;
+    const int grp = lane / kCaptureLanes, sub = lane % kCaptureLanes;
+    // consecutive claims on different blocks (spread over all SMs)
+    const unsigned long long ngroups = (unsigned long long)gridDim.x * (kBlock / 32) * kGroups;
+    const unsigned long long g0 = ((unsigned long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * kGroups + grp;
+    for (unsigned long long j = g0; j < T; j += ngroups) {
+        WinItem w;
+        const bool win = load_win(X, __ldcg(P->tgt + shard_entry(s_pre, cap, j)), w);
+        if (!win && sub == 0) {
+            // a lower-index claimant captures t; this claim's slot stays a dropped record
+            P->rec[app][base + j].cell = kTombstone;
+            P->rec[app][base + j].cdl_min = 0.0f;
+            losers++;
+        }
+        capture_group<kCaptureLanes>(
+            X, app, base, w, win, (int8_t)kLiquid, [&]() -> unsigned long long { return base + j; }, st);
+        if (win && sub == 0)
+            atomicAdd((unsigned long long *)&X.desc[w.dom_dir >> 5].liquid_shard[(blockIdx.x + j) & (kLiquidShards - 1)],
+                      (unsigned long long)(-1ll));
     }
     // every lane reaches this point
 #pragma unroll
@@ -1583,22 +1895,37 @@ __device__ void finish_capture(PoolState *P) {
 }
 
 template <int kBatch> __global__ void __launch_bounds__(kBlock) k_grow(PoolState *P) {
+    __shared__ PassCtx X;
+    load_ctx(P, X, 0);
+    __syncthreads();
     CycleStats st;
-    grow_pass<kBatch, false>(P, st);
+    unsigned int tombs = 0;
+    const int cur = P->cur;
+    grow_pass<kBatch, false>(P, X, nullptr, cur, P->cnt[cur], P->compact != 0, st, tombs);
+    add_tombs(P, tombs);
     flush_stats(P, st);
 }
 
 __global__ void __launch_bounds__(kBlock) k_claim(PoolState *P) {
+    __shared__ PassCtx X;
+    load_ctx(P, X, 0);
+    __syncthreads();
     CycleStats st;
-    claim_pass(P, st);
+    unsigned int tombs = 0;
+    claim_pass<false>(P, X, nullptr, P->pending, st, tombs);
+    if (!P->compact) // a compacted list starts without dropped records
+        add_tombs(P, tombs);
     flush_stats(P, st);
 }
 
 // Capture pass as its own kernel; the last block to finish closes the cycle and, with kBegin,
 // starts the next one.
 template <bool kBegin, int kLanes> __global__ void __launch_bounds__(kBlock) k_capture_pass(PoolState *P) {
+    __shared__ PassCtx X;
+    load_ctx(P, X, 0);
+    __syncthreads();
     CycleStats st;
-    capture_pass<kLanes>(P, st);
+    capture_pass<kLanes>(P, X, st);
     flush_stats(P, st);
     __shared__ int s_last;
     __threadfence(); // this block's writes are visible device-wide before it is counted
@@ -1613,7 +1940,7 @@ template <bool kBegin, int kLanes> __global__ void __launch_bounds__(kBlock) k_c
         if (threadIdx.x == 0)
             P->blocks_done = 0;
         if (kBegin)
-            begin_cycle(P, true, P->desc, P->n_domains, AliveSet{-1, {}});
+            begin_cycle(P, true, P->desc, P->n_domains, AliveSet{-1, {}}, false);
         else
             finish_capture(P);
     }
@@ -1621,25 +1948,28 @@ template <bool kBegin, int kLanes> __global__ void __launch_bounds__(kBlock) k_c
 
 // ---------------------------------------------------------------------------------------------
 // Grid-wide meeting point of the persistent kernel (all blocks co-resident: cooperative launch).
-// Arrival is an acq_rel atomic on a counter, release an st.release of the next generation; the
-// last block to arrive runs `serial` with the whole block before it releases the others. Every
-// wait is bounded: after kMeetTimeoutNs (or kMeetSpinCap polls) the block sets kErrBarrier and
+// Meeting k uses word k % 3: every block adds 2^56 (one arrival) and its share of what the grid
+// needs to know (release), and polls the word (acquire) until every block has arrived; the low 56
+// bits are then the sums over the grid, so the counts travel with the arrivals and no block works
+// alone while the others wait. With the last block running the cycle's start before it released the
+// others through a second word, an idle cycle took 9.7 us on 148 blocks. The word of meeting k + 2
+// was last polled for meeting k - 1, which every block has passed once meeting k is complete: block
+// 0 clears it then, before its own next arrival.
+// Every wait is bounded: after kMeetTimeoutNs (or kMeetSpinCap polls) the block sets kErrBarrier and
 // the kernel ends.
 constexpr unsigned long long kMeetTimeoutNs = 1000000000ull;
 constexpr unsigned int kMeetSpinCap = 1u << 26;
+constexpr int kMeetShift = 56;
+constexpr int kMeetMaxGrid = 255; // arrivals in the top byte
+constexpr unsigned long long kMeetSums = (1ull << kMeetShift) - 1;
 
-__device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int *p) {
-    unsigned int v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ unsigned int atom_add_acq_rel_u32(unsigned int *p, unsigned int v) {
-    unsigned int old;
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-    return old;
-}
-__device__ __forceinline__ void st_release_u32(unsigned int *p, unsigned int v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void red_release_u64(unsigned long long *p, unsigned long long v) {
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
@@ -1647,103 +1977,289 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-// With P->timeline set, meeting point `tag` records its first arrival, last arrival and release.
-template <class F> __device__ bool grid_meet(PoolState *P, int tag, F &&serial) {
-    __shared__ unsigned int s_gen;
-    __shared__ int s_state; // 0: released, 1: last to arrive, 2: gave up waiting
+// Meeting number k (counted by the caller). share() gives this block's sums, in thread 0 after the
+// block's other threads have arrived. total: the grid's sums. With tl set, meeting point `tag`
+// records its first and last arrival and when block 0 left it. False: gave up waiting.
+template <class Share>
+__device__ bool grid_meet(PoolState *P, unsigned int &k, unsigned long long *tl, int tag, Share &&share,
+                          unsigned long long &total) {
+    __shared__ unsigned long long s_word;
     __syncthreads();
     if (threadIdx.x == 0) {
-        const unsigned int gen = ld_acquire_u32(&P->bar_gen);
-        const unsigned int prev = atom_add_acq_rel_u32(&P->bar_count, 1u);
-        unsigned long long *tl = tag >= 0 ? P->timeline : nullptr;
-        if (tl && prev == 0)
-            tl[3 * tag + 0] = global_ns();
-        int state = 0;
-        if (prev == gridDim.x - 1) {
-            state = 1;
-            if (tl)
-                tl[3 * tag + 1] = global_ns();
+        unsigned long long *word = &P->meet.word[k % 3].v;
+        const unsigned long long add = (1ull << kMeetShift) + share();
+        if (tl) {
+            const unsigned long long now = global_ns();
+            atomicMin(tl + 3 * tag + 0, now);
+            atomicMax(tl + 3 * tag + 1, now);
         }
-        else {
+        red_release_u64(word, add);
+        unsigned long long v = ld_acquire_u64(word);
+        if ((v >> kMeetShift) != gridDim.x) {
             const unsigned long long t0 = global_ns();
             unsigned int it = 0;
-            while (ld_acquire_u32(&P->bar_gen) == gen) {
+            while (((v = ld_acquire_u64(word)) >> kMeetShift) != gridDim.x) {
                 ++it;
                 if (it >= kMeetSpinCap || ((it & 255u) == 0 && global_ns() - t0 > kMeetTimeoutNs)) {
                     atomicOr(&P->error, kErrBarrier);
-                    state = 2;
+                    v = 0;
                     break;
                 }
-                __nanosleep(32);
             }
         }
-        s_gen = gen;
-        s_state = state;
+        if (blockIdx.x == 0 && v) {
+            P->meet.word[(k + 2) % 3].v = 0;
+            if (tl)
+                tl[3 * tag + 2] = global_ns();
+        }
+        s_word = v;
     }
     __syncthreads();
-    const int state = s_state;
-    if (state == 1) {
-        serial();
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            if (P->timeline && tag >= 0)
-                P->timeline[3 * tag + 2] = global_ns();
-            P->bar_count = 0;
-            st_release_u32(&P->bar_gen, s_gen + 1u);
-        }
+    k++;
+    total = s_word & kMeetSums;
+    return s_word != 0;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Start of domain d's cycle c + 1 (launch-local index) by one warp, while the rest of the grid runs
+// the capture pass of cycle c: the device-side termination check, the cycle advance and the
+// nucleation of the sites whose time has come, as start_domain does at the start of a launch. What
+// makes that possible:
+//   - the liquid count after cycle c is known before the captures (issue_claims counts the cells
+//     claimed; `claimed` are the hot domain's);
+//   - a site that fires was marked (mark_code) during the capture pass before this one, when its
+//     type was liquid. A claim made since has overwritten the mark, so the site fires iff the mark
+//     is still there, and the captures, which see the mark or the site already active, leave it out
+//     of a captured cell's liquid mask either way;
+//   - a firing site flags its active neighbours' records (kMaskNuc) instead of clearing their mask
+//     bits, which still count in cycle c; the growth pass of cycle c + 1 clears them.
+// Sites due in cycle c + 2 are marked at the end.
+__device__ __noinline__ void start_next(PoolState *P, BlockShared &B, unsigned int d, unsigned long long claimed, int app,
+                                        unsigned long long base, unsigned long long *appended, int c, int n_cycles) {
+    DomainDesc &D = B.X.desc[d];
+    const unsigned int lane = threadIdx.x & 31;
+    const DomainStart s = load_start(D);
+    if (s.ctype == nullptr || s.done)
+        return;
+    const long long liquid0 = __ldcg(&D.liquid) - (long long)claimed;
+    if (c + 1 >= n_cycles) {
+        if (lane == 0)
+            D.liquid = liquid0;
+        return;
     }
-    return state != 2;
+    // rest of the descriptor
+    const NucleationView V = nucleation_view(D);
+    const int mark0 = __ldcg(&D.nuc_mark), nn0 = __ldcg(&D.nn), layer_no = D.layer_no;
+    const long long active_size = D.active_size;
+    const unsigned int epoch0 = __ldcg(&D.epoch);
+    const bool check = s.check_mode && s.cycle0 > 0 && s.cycle0 % 1000 == 0;
+    const bool probe = s.check_mode && (s.cycle0 & 63) == 0;
+    const int dry_since = probe ? __ldcg(&D.dry_since) : 0;
+    const int cts_max = probe ? D.cts_max : INT_MAX;
+    long long liquid = 1;
+    if (check || probe) {
+        liquid = lane < kLiquidShards ? __ldcg(&D.liquid_shard[lane]) : 0;
+#pragma unroll
+        for (int o = 16; o; o >>= 1)
+            liquid += __shfl_xor_sync(0xffffffffu, liquid, o);
+        liquid += liquid0;
+    }
+    if (check && liquid == 0) {
+        // src/CAupdate.cpp:782-783: no superheated or undercooled liquid left
+        if (lane == 0) {
+            D.liquid = liquid0;
+            D.done = 1;
+        }
+        return;
+    }
+    const int cycle = s.cycle0 + 1;
+    int fired_total = 0;
+    for (int q = s.cursor0; q < mark0; q += 32) {
+        const int idx = q + (int)lane;
+        const int l = idx < mark0 ? __ldg(s.nuc_loc + idx) : -1;
+        bool fire = false;
+        int h = 0, cts = 0;
+        if (l >= 0 && l < active_size) {
+            fire = __ldcg(s.ctype + l) == mark_code(c + 1);
+            h = __ldcg(V.gid + l);
+            cts = V.cts_run[l];
+        }
+        const unsigned int firing = __ballot_sync(0xffffffffu, fire);
+        if (!firing)
+            continue;
+        const unsigned int n_fire = __popc(firing);
+        unsigned long long slot0 = 0;
+        if (lane == 0) {
+            slot0 = base + atomicAdd(appended, (unsigned long long)n_fire);
+            atomicAdd(&B.n_appended, n_fire);
+            if (slot0 + n_fire > B.X.capacity) {
+                atomicOr(&P->error, kErrListOverflow);
+                slot0 = ULLONG_MAX;
+            }
+        }
+        slot0 = __shfl_sync(0xffffffffu, slot0, 0);
+        for (unsigned int todo = firing; todo; todo &= todo - 1) {
+            const int src = __ffs(todo) - 1;
+            const unsigned int rank = __popc(firing & ((1u << src) - 1u));
+            nucleate_site(V, s.ctype, B.X.rec[app], B.X.rdom[app], B.X.rstat[app], B.X.rmin2[app], d,
+                          (unsigned int)__shfl_sync(0xffffffffu, l, src), __shfl_sync(0xffffffffu, h, src),
+                          __shfl_sync(0xffffffffu, cts, src), slot0 == ULLONG_MAX ? ULLONG_MAX : slot0 + rank,
+                          [&](unsigned int nb_pos, int) {
+                              if (nb_pos < base)
+                                  atomicOr(B.X.rstat[app] + nb_pos, kMaskNuc);
+                          });
+        }
+        fired_total += (int)n_fire;
+    }
+    bool ended = false;
+    if (probe && s.cycle0 - 2 >= cts_max && liquid == 0 && fired_total == 0) {
+        // see start_domain
+        if (dry_since != 0)
+            ended = true;
+        else if (lane == 0)
+            D.dry_since = s.cycle0;
+    }
+    const int mark = (c + 2 < n_cycles && !ended) ? mark_sites(D, s, mark0, cycle + 1, mark_code(c + 2), layer_no, active_size)
+                                                   : mark0;
+    if (lane != 0)
+        return;
+    D.liquid = liquid0 - fired_total;
+    if (ended) {
+        D.cycle = (s.cycle0 + 999) / 1000 * 1000;
+        D.done = 1;
+        return;
+    }
+    D.cycle = cycle;
+    D.epoch = epoch0 + 1;
+    D.nuc_cursor = mark0;
+    D.nuc_mark = mark;
+    D.nn = nn0 + fired_total;
+    if (fired_total)
+        atomicAdd(&P->stat[blockIdx.x & (kStatShards - 1)][kStatNucleated], (unsigned long long)fired_total);
 }
 
 // n_cycles complete CA cycles (start, grow/claim, capture) in one cooperative launch.
 template <int kLanes, int kBatch>
 __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles, AliveSet alive) {
+    __shared__ BlockShared B;
     CycleStats st;
-    // with many running domains, their per-cycle start (termination, nucleation) runs across the
-    // grid (the descriptors and their number change only between launches); with a few, one block
-    // starts them, and the first one's growth fields stay in registers
+    // the start of the launch's first cycle: one block for a few domains, a warp per domain across
+    // the grid for many; later cycles are started under the capture pass (start_next)
     DomainDesc *const desc = P->desc;
     const int n_domains = P->n_domains;
-    const bool spread = alive.n < 0 && n_domains > kSerialDomains;
-    const unsigned int hot = alive.n > 0 ? (unsigned int)alive.idx[0] : 0u;
-    const int gwarp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarp = gridDim.x * (kBlock / 32);
-    bool ok = grid_meet(P, 0, [&] {
+    const bool spread = alive.n < 0;
+    const int n_start = spread ? n_domains : alive.n;
+    unsigned long long *const tl = P->timeline;
+    unsigned int meet = 0;
+    unsigned long long total = 0;
+    const auto no_share = [] { return 0ull; };
+    if (threadIdx.x == 0)
+        B.n_items = B.n_claims = B.n_wins = B.n_first = B.n_tombs = B.n_appended = 0;
+    if (blockIdx.x == 0) {
         if (spread)
             begin_lists(P, false);
         else
-            begin_cycle(P, false, desc, n_domains, alive);
-    });
-    if (ok && spread) {
-        begin_domains(P, desc, n_domains, gwarp, nwarp);
-        ok = grid_meet(P, -1, [] {});
+            begin_cycle(P, false, desc, n_domains, alive, n_cycles > 1);
     }
+    bool ok = grid_meet(P, meet, tl, 0, no_share, total);
+    if (ok && spread) {
+        begin_domains(P, desc, n_domains, (threadIdx.x >> 5) * gridDim.x + blockIdx.x, gridDim.x * (kBlock / 32),
+                      n_cycles > 1);
+        ok = grid_meet(P, meet, nullptr, 0, no_share, total);
+    }
+    load_ctx(P, B.X, alive.n > 0 ? (unsigned int)alive.idx[0] : 0u);
+    // the list's state, the same in every block
+    int cur = __ldcg(&P->cur);
+    unsigned long long n = __ldcg(&P->cnt[cur]), tombs = __ldcg(&P->tombs);
+    // the warps that start domains: the last of the blocks 0 .. n_start - 1
+    const int start_warps = min(8, (n_start + (int)gridDim.x - 1) / (int)gridDim.x);
+    const unsigned int threads = (int)blockIdx.x < n_start ? (unsigned int)(kBlock - 32 * start_warps) : (unsigned int)kBlock;
+    __syncthreads();
     for (int c = 0; ok && c < n_cycles; c++) {
+        if (c % kStatCycles == kStatCycles - 1) {
+            flush_stats(P, st);
+            st = CycleStats();
+        }
+        // compact when dropped records exceed a quarter of the list, as lists_start
+        const bool compact = tombs * 4 > n;
+        const int app = compact ? cur ^ 1 : cur; // list of the next cycle
         // growth with each block's claims right after its own growth; the global claim pass only
         // when some block's queue overflowed this cycle (the same answer for every block)
-        grow_pass<kBatch, true>(P, st, hot);
-        ok = grid_meet(P, 3 * c + 1, [] {});
+        unsigned int dropped = 0;
+        grow_pass<kBatch, true>(P, B.X, &B, cur, n, compact, st, dropped);
+        dropped = __reduce_add_sync(0xffffffffu, dropped);
+        if ((threadIdx.x & 31) == 0 && dropped)
+            atomicAdd(&B.n_tombs, dropped);
+        constexpr int kOverflowShift = 40; // sums: first claims of the hot domain, blocks that overflowed
+        const auto claim_share = [&] {
+            const unsigned long long v = B.n_first;
+            B.n_first = 0;
+            return v;
+        };
+        ok = grid_meet(
+            P, meet, tl, 3 * c + 1,
+            [&] { return claim_share() + (B.n_items > (unsigned int)kBlockQueue ? 1ull << kOverflowShift : 0ull); }, total);
         if (!ok)
             break;
-        if (__ldcg(&P->claim_overflow)) {
-            claim_pass(P, st);
-            ok = grid_meet(P, 3 * c + 2, [] {});
+        unsigned long long claimed = total & ((1ull << kOverflowShift) - 1);
+        const bool overflow = (total >> kOverflowShift) != 0;
+        if (overflow) {
+            dropped = 0;
+            claim_pass<true>(P, B.X, &B, app, st, dropped);
+            dropped = __reduce_add_sync(0xffffffffu, dropped);
+            if ((threadIdx.x & 31) == 0 && dropped)
+                atomicAdd(&B.n_tombs, dropped);
+            ok = grid_meet(P, meet, tl, 3 * c + 2, claim_share, total);
             if (!ok)
                 break;
+            claimed += total;
         }
-        capture_pass<kLanes>(P, st);
-        const bool more = c + 1 < n_cycles;
-        ok = grid_meet(P, 3 * c + 3, [&] {
-            if (!more)
-                finish_capture(P);
-            else if (spread)
-                begin_lists(P, true);
-            else
-                begin_cycle(P, true, desc, n_domains, alive);
-        });
-        if (ok && more && spread) {
-            begin_domains(P, desc, n_domains, gwarp, nwarp);
-            ok = grid_meet(P, -1, [] {});
+        const unsigned long long base = compact ? __ldcg(&P->cnt[app]) : n;
+        if (blockIdx.x == 0 && threadIdx.x < 32) {
+            // counters that the grid has done with, or needs from the next meeting on
+            if (threadIdx.x == 0) {
+                P->meet.appended[(c + 1) % 3].v = 0;
+                if (compact)
+                    P->cnt[cur] = 0;
+            }
+            if (overflow)
+                P->qcnt_s[threadIdx.x].v = 0;
         }
+        unsigned long long *const appended = &P->meet.appended[c % 3].v;
+        if (threadIdx.x >= threads) {
+            const unsigned int w = (threadIdx.x - threads) / 32;
+            for (int i = (int)(w * gridDim.x + blockIdx.x); i < n_start; i += start_warps * (int)gridDim.x) {
+                const unsigned int d = spread ? (unsigned int)i : (unsigned int)alive.idx[i];
+                start_next(P, B, d, d == B.X.hot ? claimed : 0ull, app, base, appended, c, n_cycles);
+            }
+        }
+        else {
+            capture_block<kLanes>(P, B, threads, app, base, appended, mark_code(c + 2), st);
+        }
+        // sums: records appended (36 bits: list positions have 32), records dropped (20 bits; only
+        // the compaction's timing depends on them, so a block adds at most its share of the field)
+        constexpr int kTombShift = 36;
+        ok = grid_meet(
+            P, meet, tl, 3 * c + 3,
+            [&] {
+                const unsigned int most = ((1u << (kMeetShift - kTombShift)) - 1u) / gridDim.x;
+                const unsigned long long v = B.n_appended + ((unsigned long long)min(B.n_tombs, most) << kTombShift);
+                B.n_items = B.n_claims = B.n_wins = B.n_tombs = B.n_appended = 0;
+                return v;
+            },
+            total);
+        n = base + (total & ((1ull << kTombShift) - 1));
+        if (n > B.X.capacity)
+            n = B.X.capacity; // overflowed: flagged
+        tombs = (compact ? 0 : tombs) + (total >> kTombShift);
+        cur = app;
+    }
+    if (ok && blockIdx.x == 0 && threadIdx.x == 0) {
+        P->cur = P->pending = cur;
+        P->cnt[cur] = n;
+        P->cnt[cur ^ 1] = 0;
+        P->tombs = tombs;
+        P->compact = 0;
     }
     flush_stats(P, st);
 }
@@ -1754,7 +2270,9 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
 __global__ void __launch_bounds__(kBlock) k_meet_probe(PoolState *P) {
     if (blockIdx.x == 0)
         return;
-    grid_meet(P, -1, [] {});
+    unsigned int k = 0;
+    unsigned long long total;
+    grid_meet(P, k, nullptr, 0, [] { return 0ull; }, total);
 }
 
 // Compiled launch shapes: {capture lanes, growth batch} for kLaneChoices x kBatchChoices.
@@ -2275,7 +2793,9 @@ Pool::Pool(int device, size_t budget_bytes, unsigned long long list_capacity)
     // a shard takes the entries of 1/kShards of the warps: room for its share of the list plus slack
     ps.shard_cap = capacity_ / kShards + 8192;
     const size_t qn = (size_t)kShards * ps.shard_cap;
-    CUDA_OK(cudaMalloc(&ps.tgt, qn * sizeof(unsigned long long)));
+    // the persistent kernel splits the claim list into one segment per block of its grid
+    ps.tgt_len = qn + 4096ull * (unsigned long long)num_sms_;
+    CUDA_OK(cudaMalloc(&ps.tgt, ps.tgt_len * sizeof(unsigned long long)));
     CUDA_OK(cudaMalloc(&ps.qpos, qn * sizeof(unsigned int)));
     CUDA_OK(cudaMalloc(&ps.qcell, qn * sizeof(unsigned int)));
     CUDA_OK(cudaMalloc(&ps.qdom, qn * sizeof(unsigned int)));
@@ -2643,7 +3163,7 @@ void Pool::retire(int slot) {
 void Pool::launch_persistent(int n) {
     cudaStream_t st = S(stream_);
     // the meeting point starts at zero arrivals (a launch that gave up waiting may have left some)
-    CUDA_OK(cudaMemsetAsync((char *)dstate_ + offsetof(PoolState, bar_count), 0, 2 * sizeof(unsigned int), st));
+    CUDA_OK(cudaMemsetAsync((char *)dstate_ + offsetof(PoolState, meet), 0, sizeof(PoolState::meet), st));
     PoolState *ps = dstate_;
     // the domains still running at the last state read, when few (the one with most cells first);
     // one that ends during the launch is still started and returns at once, as in the spread start
@@ -2674,7 +3194,7 @@ void Pool::launch_persistent(int n) {
         grid_div_ = (last_records_ > 0 && last_records_ < kHalfGridRecords) ? 2 : 1;
     else if (!grid_tuned_)
         grid_div_ = (last_records_ > 0 && last_records_ < kSmallGridRecords) ? 16 : 1;
-    const int grid = std::max(1, grid_cycles_[variant_] / grid_div_);
+    const int grid = std::max(1, std::min(kMeetMaxGrid, grid_cycles_[variant_]) / grid_div_);
     CUDA_OK(cudaLaunchCooperativeKernel(kStepKernel[variant_].cycles, dim3(grid), dim3(kBlock), args, 0, st));
     launches_ += 1;
 }
@@ -2764,7 +3284,7 @@ void Pool::sync_state() {
 int Pool::check_bounded_wait() {
     CUDA_OK(cudaSetDevice(device_));
     cudaStream_t st = S(stream_);
-    CUDA_OK(cudaMemsetAsync((char *)dstate_ + offsetof(PoolState, bar_count), 0, 2 * sizeof(unsigned int), st));
+    CUDA_OK(cudaMemsetAsync((char *)dstate_ + offsetof(PoolState, meet), 0, sizeof(PoolState::meet), st));
     PoolState *ps = dstate_;
     void *args[] = {&ps};
     CUDA_OK(cudaLaunchCooperativeKernel((const void *)k_meet_probe, dim3(2), dim3(kBlock), args, 0, st));
@@ -2774,7 +3294,7 @@ int Pool::check_bounded_wait() {
     const int zero = 0;
     CUDA_OK(cudaMemcpyAsync((char *)dstate_ + offsetof(PoolState, error), &zero, sizeof(int), cudaMemcpyHostToDevice,
                             st));
-    CUDA_OK(cudaMemsetAsync((char *)dstate_ + offsetof(PoolState, bar_count), 0, 2 * sizeof(unsigned int), st));
+    CUDA_OK(cudaMemsetAsync((char *)dstate_ + offsetof(PoolState, meet), 0, sizeof(PoolState::meet), st));
     CUDA_OK(cudaStreamSynchronize(st));
     return flags;
 }
@@ -2872,14 +3392,17 @@ void Pool::profile_persistent(int n, double us[7]) {
     const size_t words = 3 * (3 * (size_t)n + 1);
     unsigned long long *dtl = nullptr;
     CUDA_OK(cudaMalloc(&dtl, words * sizeof(unsigned long long)));
-    CUDA_OK(cudaMemsetAsync(dtl, 0, words * sizeof(unsigned long long), st));
+    // first arrivals take the minimum, last arrivals the maximum, departures are stored
+    std::vector<unsigned long long> tl(words, 0);
+    for (size_t m = 0; m < words; m += 3)
+        tl[m] = ULLONG_MAX;
+    CUDA_OK(cudaMemcpyAsync(dtl, tl.data(), words * sizeof(unsigned long long), cudaMemcpyHostToDevice, st));
     CUDA_OK(cudaMemcpyAsync((char *)dstate_ + offsetof(PoolState, timeline), &dtl, sizeof(dtl),
                             cudaMemcpyHostToDevice, st));
     step(n);
     unsigned long long *none = nullptr;
     CUDA_OK(cudaMemcpyAsync((char *)dstate_ + offsetof(PoolState, timeline), &none, sizeof(none),
                             cudaMemcpyHostToDevice, st));
-    std::vector<unsigned long long> tl(words);
     CUDA_OK(cudaMemcpyAsync(tl.data(), dtl, words * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
     CUDA_OK(cudaStreamSynchronize(st));
     CUDA_OK(cudaFree(dtl));

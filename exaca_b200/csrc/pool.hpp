@@ -85,14 +85,15 @@ struct DomainDesc {
     float du_value;
     int zero_du; // 1 if a cell that can become active has UndercoolingChange 0 (U stays 0 there)
     int cts_max; // check_mode domains: the largest CritTimeStep of any cell
-    // dynamic state
-    int cycle;
+    // dynamic state; the growth pass reads the first four as one 16-byte vector
+    alignas(16) int cycle;
     unsigned int epoch;
     int nuc_cursor;
     int done;
     int nn;
     int error;
     int n_jumps;
+    int nuc_mark; // persistent kernel: sites [nuc_cursor, nuc_mark) are marked to nucleate at the next cycle's start
     int dry_since; // check_mode domains past cts_max: the first cycle start that found no liquid (0: none)
     long long liquid; // liquid cells of layer 0, less the nucleations (captures are in liquid_shard)
     long long liquid_shard[kLiquidShards]; // minus the captures, spread over shards to avoid contention
@@ -125,9 +126,11 @@ struct PoolState {
     // shard s holds entries [s * shard_cap, s * shard_cap + qcnt_s[s])
     unsigned int *qpos, *qcell, *qdom, *qmask;
     float *qdl;
-    // claims this cycle, (domain << 37) | (direction << 32) | claimed cell; shard s holds entries
-    // [s * shard_cap, s * shard_cap + tcnt_s[s])
+    // claims this cycle, (domain << 37) | (direction << 32) | claimed cell. Separate kernels: shard s
+    // holds entries [s * shard_cap, s * shard_cap + tcnt_s[s]). Persistent kernel: block b of a grid
+    // of g keeps the claims that its shared-memory list does not hold from entry b * (tgt_len / g).
     unsigned long long *tgt;
+    unsigned long long tgt_len;
     unsigned long long shard_cap;
     ShardCounter qcnt_s[kShards];
     ShardCounter tcnt_s[kShards];
@@ -141,13 +144,13 @@ struct PoolState {
     int error;
     int n_domains;
     int extras; // 1 once a domain with per-cell growth extras (several layers or undercooling values) was admitted
-    int claim_overflow; // 1: a block's claim queue overflowed this cycle, so the global claim pass runs
-    int pad;
     DomainDesc *desc;
     unsigned long long stat[kStatShards][kNumStats];
     unsigned int blocks_done;      // last-block detection of the separate capture kernel
-    unsigned int bar_count;        // grid-wide meeting point of the persistent kernel: arrivals
-    unsigned int bar_gen;          // and generation
+    struct {
+        ShardCounter word[3];     // grid-wide meeting points of the persistent kernel, in turn
+        ShardCounter appended[3]; // records appended by a cycle's captures and nucleations, in turn
+    } meet;
     unsigned long long *timeline;  // optional: per meeting point {first arrival, last arrival, release} (ns)
     unsigned long long work[2];    // spare counters
 };

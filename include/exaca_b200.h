@@ -152,9 +152,9 @@ int exaca_pool_autotune(exaca_pool *pool, int trial_cycles, int *config, double 
 int exaca_pool_timed_step(exaca_pool *pool, int n_cycles, double *ms);
 /* exaca_pool_step with the persistent kernel's device timeline on (globaltimer at every grid-wide
  * meeting point); waits and returns per-cycle averages in microseconds: us[7] = {growth pass done in
- * the first block, in the last block; claim pass first, last; capture pass first, last; end of the
- * cycle and start of the next (run by the last block alone)}. Pass times count from the release of
- * the previous meeting point. */
+ * the first block, in the last block; claim pass first, last; capture pass (with the start of the
+ * next cycle) first, last; last arrival at the end of the cycle to the first block's departure}. Pass
+ * times count from the departure from the previous meeting point. */
 int exaca_pool_profile_persistent(exaca_pool *pool, int n_cycles, double *us);
 /* Device error flags, as exaca_domain_status.error reports them. */
 #define EXACA_FLAG_GROWTH_TABLE 1  /* undercooling count beyond the growth table */
