@@ -88,8 +88,9 @@ struct DomainDesc {
     // dynamic state; the growth pass reads the first four as one 16-byte vector
     alignas(16) int cycle;
     unsigned int epoch;
-    int nuc_cursor;
+    int next_start; // persistent kernel: the first cycle whose start has to be run (no claims before it)
     int done;
+    int nuc_cursor;
     int nn;
     int error;
     int n_jumps;
@@ -150,6 +151,7 @@ struct PoolState {
     struct {
         ShardCounter word[3];     // grid-wide meeting points of the persistent kernel, in turn
         ShardCounter appended[3]; // records appended by a cycle's captures and nucleations, in turn
+        ShardCounter min_cts[3];  // smallest CritTimeStep (an int) of the records of a cycle's idle blocks, in turn
     } meet;
     unsigned long long *timeline;  // optional: per meeting point {first arrival, last arrival, release} (ns)
     unsigned long long work[2];    // spare counters

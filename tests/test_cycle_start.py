@@ -91,3 +91,22 @@ def test_queue_and_claim_list_overflow(lib, config):
         res.append(pool.copy_out(slot) + (st.nn, st.liquid))
         pool.close()
     assert all(np.array_equal(a, b) for a, b in zip(*res))
+
+
+@pytest.mark.parametrize("dtn", [3.0, 60.0])
+def test_cycles_that_do_nothing(lib, tmp_path, dtn):
+    # one seed in a corner of a wide, late front: stretches of cycles without an eligible record,
+    # without claims, and (dtn 60) ended by a nucleation; stepped across them in every way
+    inp = directional(tmp_path, nx=9, ny=8, nz=30, G=5e6, R=2e5, density=3e3, dtn=dtn, N=25, frac=0.03)
+    p = ex.Problem.from_file(inp)
+    o = Oracle(inp)
+    o.step(2000)
+    for chunks in ((2000,), (1, 2, 997, 1000), tuple([37] * 54 + [2])):
+        assert sum(chunks) == 2000
+        pool = ex.Pool(0, list_capacity=p.geometry.active_size)
+        slot = pool.admit(p, device_check=False)
+        for n in chunks:
+            pool.step(n)
+        assert pool.status(slot).cycle == 2000
+        equal(pool, slot, o, f"chunks {chunks[:4]}")
+        pool.close()
