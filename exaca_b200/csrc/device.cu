@@ -818,6 +818,11 @@ constexpr unsigned int kNeedsClaim = 0xffffffffu; // NaN pattern in ActiveRec::c
 // capture pass.
 constexpr int kBatchChoices[2] = {2, 4};
 constexpr int kLaneChoices[2] = {4, 8};
+// The persistent kernels of the wider capture groups also hold the code for blocks with few records,
+// claims or captures (a warp for each, one group of records per warp): short lists are a chain of
+// dependent instructions, and the 8-lane shapes are the faster ones there anyway. The 4-lane shapes,
+// faster on long lists, go without it: with both, spills cost 512^3 3 % (41.3 vs 40.0 us per cycle).
+constexpr int kFewLanes = 8;
 constexpr int kErrBarrier = 8;
 
 // Work counts of one thread, added to the pool's at the end of a kernel and, in the persistent one,
@@ -1040,10 +1045,13 @@ __device__ __forceinline__ unsigned long long warp_reserve_n(unsigned long long 
 __device__ __forceinline__ unsigned long long claim_key(const DomainDesc &D, unsigned int c) {
     return ((unsigned long long)(0xffffffffu - D.epoch) << 32) | (unsigned long long)c;
 }
-// A listed claim: domain, direction from the claimant and claimed cell.
+// A listed claim: domain (13 bits), direction from the claimant and claimed cell; in a block's own
+// list also 1 + the entry of BlockShared::claimants that holds the claimant's state (0: none).
+constexpr int kClaimantShift = 50;
 __device__ __forceinline__ unsigned long long claim_entry_of(unsigned int dom, int l, unsigned int t) {
     return ((unsigned long long)dom << 37) | ((unsigned long long)l << 32) | t;
 }
+__device__ __forceinline__ unsigned int claim_domain(unsigned long long e) { return (unsigned int)(e >> 37) & 0x1fffu; }
 
 // Claim work of queue entry k. Returns the directions of the cells it claimed. All loads of the entry
 // (critical-length row, neighbour types) go out in one round.
@@ -1203,6 +1211,10 @@ struct BlockShared {
         WinItem wins[kBlock];         // capture
     };
     unsigned long long claims[kBlockClaims];
+    struct {
+        int h;        // GrainID
+        float doc[3]; // DOCenter
+    } claimants[kBlock / 32];
     unsigned int n_items;  // may exceed kBlockQueue (the excess went global)
     unsigned int n_claims; // may exceed kBlockClaims (the excess is in the block's segment)
     unsigned int n_wins;
@@ -1344,7 +1356,7 @@ __device__ __forceinline__ void issue_claims(BlockShared &B, unsigned int first)
     unsigned int firsts = 0;
     for (unsigned int i = first + threadIdx.x; i < n; i += kBlock) {
         const unsigned long long e = claim_at(B, i);
-        const unsigned int dom = (unsigned int)(e >> 37), t = (unsigned int)e;
+        const unsigned int dom = claim_domain(e), t = (unsigned int)e;
         const DomainDesc &D = desc_of(B.X, dom);
         const unsigned int c = (unsigned int)((long long)t - nb_offset((int)((e >> 32) & 31u), D.mx * D.my, D.my));
         const unsigned long long key = claim_key(D, c);
@@ -1363,7 +1375,97 @@ __device__ __forceinline__ void issue_claims(BlockShared &B, unsigned int first)
         atomicAdd(&B.n_first, firsts);
 }
 
+// The claim step of the block's item `i` by a whole warp: claim_record, push_claims and issue_claims with
+// one direction per lane, and the claimant's state loaded for the capture. A block with a few flagged
+// records has one chain of dependent instructions to wait for, most of them issued for one lane each in
+// the record-per-lane form (26 lengths compared in turn, the list positions, two block barriers).
+__device__ __forceinline__ void claim_warp(BlockShared &B, int app, unsigned int i, CycleStats &st, unsigned int &tombs) {
+    const unsigned int lane = threadIdx.x & 31;
+    const ClaimItem it = B.items[i];
+    const unsigned int c = it.cell, dom = it.dom;
+    unsigned int m = it.mask;
+    const DomainDesc &D = desc_of(B.X, dom);
+    const int plane = D.mx * D.my, my = D.my;
+    constexpr unsigned int kInf = 0x7f800000u;
+    // lanes 0-25: the critical lengths; 26: GrainID; 27-29: DOCenter
+    unsigned int v = kInf;
+    if (lane < 26)
+        v = __float_as_uint(__ldcg(D.cdl + 26ull * c + lane));
+    else if (lane == 26)
+        v = (unsigned int)__ldcg(D.gid + c);
+    else if (lane < 30)
+        v = __float_as_uint(__ldcg(D.doc + 3ull * c + (lane - 27)));
+    if (m & kMaskFresh) {
+        // as claim_record
+        int rx, ry, rz;
+        cell_coords(D, c, rx, ry, rz);
+        const bool nb = (neighbour_mask(D, rx, ry, rz) >> lane) & 1u;
+        m = __ballot_sync(0xffffffffu, nb && liquid_type(__ldcg(D.ctype + c + (nb ? nb_offset((int)lane, plane, my) : 0))));
+        if (lane == 0) {
+            st.fresh++;
+            B.X.rstat[app][it.pos] = m | kMaskGrown;
+        }
+    }
+    ActiveRec *rec = B.X.rec[app] + it.pos;
+    if ((m & kDirBits) == 0) {
+        // no liquid neighbour: LCount stays 0 (src/CAupdate.cpp:722-725)
+        if (lane == 0) {
+            D.ctype[c] = kSolid;
+            D.dl[c] = it.dl;
+            rec->cell = kTombstone;
+            rec->cdl_min = 0.0f;
+            st.dropped++;
+            tombs++;
+        }
+        return;
+    }
+    const bool liquid = lane < 26 && ((m >> lane) & 1u), reached = liquid && it.dl >= __uint_as_float(v);
+    const unsigned int reach = __ballot_sync(0xffffffffu, reached);
+    if (reach) {
+        unsigned int e = 0;
+        if (lane == 0)
+            e = atomicAdd(&B.n_claims, __popc(reach)); // at most 26 per warp: within kBlockClaims
+        e = __shfl_sync(0xffffffffu, e, 0) + __popc(reach & ((1u << lane) - 1u));
+        bool first = false;
+        if (reached) {
+            const unsigned int t = (unsigned int)((long long)c + nb_offset((int)lane, plane, my));
+            const unsigned long long key = claim_key(D, c);
+            const unsigned long long old = atomicMin(D.claim + t, key);
+            D.ctype[t] = kTemporaryUpdate;
+            B.claims[e] = claim_entry_of(dom, (int)lane, t) | ((unsigned long long)(i + 1) << kClaimantShift);
+            first = (old >> 32) != (key >> 32);
+            if (first && dom != B.X.hot)
+                atomicAdd((unsigned long long *)&B.X.desc[dom].liquid_shard[lane & (kLiquidShards - 1)],
+                          (unsigned long long)(-1ll));
+        }
+        if (lane == 26)
+            B.claimants[i].h = (int)v;
+        else if (lane > 26 && lane < 30)
+            B.claimants[i].doc[lane - 27] = __uint_as_float(v);
+        const unsigned int firsts = __popc(__ballot_sync(0xffffffffu, first && dom == B.X.hot));
+        if (lane == 0) {
+            st.claims += __popc(reach);
+            if (firsts)
+                atomicAdd(&B.n_first, firsts);
+        }
+    }
+    // the cached minimum over the liquid neighbours not reached, its lowest direction and the
+    // second-smallest: lengths are not negative, so their bits order as the values do (a NaN counts
+    // as +inf, which the comparisons of claim_record skip as well)
+    const unsigned int b = liquid && !reached ? min(v, kInf) : kInf;
+    const unsigned int nm = __reduce_min_sync(0xffffffffu, b);
+    const unsigned int d1 = nm == kInf ? 0xffffffffu : (unsigned int)__ffs(__ballot_sync(0xffffffffu, b == nm)) - 1u;
+    const unsigned int nm2 = __reduce_min_sync(0xffffffffu, lane == d1 ? kInf : b);
+    if (lane == 0) {
+        st.rows++;
+        rec->cdl_min = __uint_as_float(nm);
+        B.X.rmin2[app][it.pos] = ((unsigned long long)d1 << 32) | nm2;
+    }
+}
+
 // The block's claim step over its queue (all threads of the block call, after the block's growth).
+// kFew: with a warp per record when there are few (short chains; see claim_warp).
+template <bool kFew>
 __device__ __forceinline__ void block_claims(PoolState *P, BlockShared &B, int app, CycleStats &st,
                                              unsigned int &tombs) {
     __syncthreads();
@@ -1371,6 +1473,11 @@ __device__ __forceinline__ void block_claims(PoolState *P, BlockShared &B, int a
     if (n == 0)
         return;
     const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (kFew && n <= (unsigned int)(kBlock / 32)) {
+        if (warp < n)
+            claim_warp(B, app, warp, st, tombs);
+        return;
+    }
     for (unsigned int k0 = warp * 32; k0 < n; k0 += kBlock) {
         const unsigned int k = k0 + lane;
         unsigned int reach = 0, dom = 0, cell = 0;
@@ -1453,33 +1560,12 @@ __device__ __noinline__ void compact_pass(PoolState *P, const PassCtx &X, int cu
 // group g to warp g % (number of warps of the grid), consecutive warps on different blocks: the
 // records appended by the last capture pass, which all need a fresh mask and claims, spread over
 // every SM. No block-wide synchronisation.
-// With kOwnClaims (B given) the block's flagged records go to its queue and their claim steps follow
-// here. cur is the list to read, n its length; with `compact` the survivors go to the other list.
+// Growth of the list's groups of 32 records, kBatch groups per warp in flight (see grow_pass).
 template <int kBatch, bool kOwnClaims>
-__device__ void grow_pass(PoolState *P, PassCtx &X, BlockShared *B, const DomainDyn &dyn, int cur, unsigned long long n,
-                          bool compact, CycleStats &st, unsigned int &tombs) {
-    const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned long long nw = (unsigned long long)gridDim.x * (kBlock / 32);
-    const unsigned long long gw = (unsigned long long)warp * gridDim.x + blockIdx.x;
-    const unsigned int shard = (unsigned int)(gw % kShards);
-    const unsigned int hot = X.hot;
-    if (kOwnClaims && threadIdx.x == 0) {
-        // read by the block's claim step, after its first barrier
-        X.hot_desc.cycle = dyn.cycle;
-        X.hot_desc.epoch = dyn.epoch;
-    }
-    if (compact) {
-        compact_pass(P, X, cur, gw, nw, n, dyn, st, kOwnClaims ? B : nullptr);
-        if (kOwnClaims) {
-            B->busy = 1;
-            unsigned int claim_tombs = 0; // a compacted list starts without dropped records
-            block_claims(P, *B, cur ^ 1, st, claim_tombs);
-        }
-        return;
-    }
-    // whether a record was grown or dropped, and the smallest CritTimeStep of the others
-    bool busy = false;
-    int min_cts = INT_MAX;
+__device__ __forceinline__ void grow_groups(PoolState *P, const PassCtx &X, BlockShared *B, const DomainDyn &dyn, int cur,
+                                            unsigned long long n, unsigned long long gw, unsigned long long nw,
+                                            CycleStats &st, unsigned int &tombs, bool &busy, int &min_cts) {
+    const unsigned int lane = threadIdx.x & 31, shard = (unsigned int)(gw % kShards), hot = X.hot;
     ActiveRec *in = X.rec[cur];
     const unsigned int *in_dom = X.rdom[cur];
     unsigned int *in_stat = X.rstat[cur];
@@ -1563,6 +1649,38 @@ __device__ void grow_pass(PoolState *P, PassCtx &X, BlockShared *B, const Domain
         else
             queue_flagged<kBatch>(P, shard, __popc(flagged), flagged, idx, r, dom, m);
     }
+}
+
+// With kOwnClaims (B given) the block's flagged records go to its queue and their claim steps follow
+// here. cur is the list to read, n its length; with `compact` the survivors go to the other list.
+template <int kBatch, bool kOwnClaims, bool kFew>
+__device__ void grow_pass(PoolState *P, PassCtx &X, BlockShared *B, const DomainDyn &dyn, int cur, unsigned long long n,
+                          bool compact, CycleStats &st, unsigned int &tombs) {
+    const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned long long nw = (unsigned long long)gridDim.x * (kBlock / 32);
+    const unsigned long long gw = (unsigned long long)warp * gridDim.x + blockIdx.x;
+    if (kOwnClaims && threadIdx.x == 0) {
+        // read by the block's claim step, after its first barrier
+        X.hot_desc.cycle = dyn.cycle;
+        X.hot_desc.epoch = dyn.epoch;
+    }
+    if (compact) {
+        compact_pass(P, X, cur, gw, nw, n, dyn, st, kOwnClaims ? B : nullptr);
+        if (kOwnClaims) {
+            B->busy = 1;
+            unsigned int claim_tombs = 0; // a compacted list starts without dropped records
+            block_claims<kFew>(P, *B, cur ^ 1, st, claim_tombs);
+        }
+        return;
+    }
+    // whether a record was grown or dropped, and the smallest CritTimeStep of the others
+    bool busy = false;
+    int min_cts = INT_MAX;
+    // one group per warp at most: the shorter code for one group is the shorter chain
+    if (kFew && (n + 31) / 32 <= nw)
+        grow_groups<1, kOwnClaims>(P, X, B, dyn, cur, n, gw, nw, st, tombs, busy, min_cts);
+    else
+        grow_groups<kBatch, kOwnClaims>(P, X, B, dyn, cur, n, gw, nw, st, tombs, busy, min_cts);
     if (kOwnClaims) {
         busy = __any_sync(0xffffffffu, busy);
         min_cts = __reduce_min_sync(0xffffffffu, min_cts);
@@ -1572,7 +1690,7 @@ __device__ void grow_pass(PoolState *P, PassCtx &X, BlockShared *B, const Domain
             else if (min_cts != INT_MAX)
                 atomicMin(&B->min_cts, min_cts);
         }
-        block_claims(P, *B, cur, st, tombs);
+        block_claims<kFew>(P, *B, cur, st, tombs);
     }
 }
 
@@ -1653,9 +1771,10 @@ __device__ void claim_pass(PoolState *P, PassCtx &X, BlockShared *B, int app, Cy
 // neighbours and their solidification re-checks, and the new record in slot slot_of() of list `app`
 // (ULLONG_MAX: none). Records of the cells active at the start of the cycle lie below base. A cell of
 // type also_liquid (a mark of the cycle after next, or kLiquid) is liquid in the next cycle.
-template <int kLanes, class SlotOf>
+// won() says whether the claim has won, after the neighbours' loads have gone out.
+template <int kLanes, class Won, class SlotOf>
 __device__ __forceinline__ void capture_group(const PassCtx &X, int app, unsigned long long base, const WinItem &w,
-                                              bool on, int8_t also_liquid, SlotOf &&slot_of, CycleStats &st) {
+                                              bool on, int8_t also_liquid, Won &&won, SlotOf &&slot_of, CycleStats &st) {
     constexpr int kPer = (26 + kLanes - 1) / kLanes;
     const int lane = threadIdx.x & 31, grp = lane / kLanes, sub = lane % kLanes;
     const unsigned int group = (kLanes == 32 ? 0xffffffffu : ((1u << kLanes) - 1u)) << (grp * kLanes);
@@ -1664,6 +1783,7 @@ __device__ __forceinline__ void capture_group(const PassCtx &X, int app, unsigne
     const DomainDesc &D = desc_of(X, dom);
     unsigned int *rs = X.rstat[app];
     unsigned int a[kPer], p[kPer], old[kPer];
+    int8_t ct[kPer];
     bool act[kPer];
     unsigned int liq = 0, d1 = 0xffffffffu;
     float mn = __int_as_float(0x7f800000), mn2 = mn, new_dl = 0.0f;
@@ -1674,7 +1794,6 @@ __device__ __forceinline__ void capture_group(const PassCtx &X, int app, unsigne
         int tx, ty, tz;
         cell_coords(D, t, tx, ty, tz);
         const unsigned int valid = neighbour_mask(D, tx, ty, tz);
-        int8_t ct[kPer];
 #pragma unroll
         for (int k = 0; k < kPer; k++) {
             const int ln = slot_dir(sub + k * kLanes);
@@ -1683,6 +1802,9 @@ __device__ __forceinline__ void capture_group(const PassCtx &X, int app, unsigne
             ct[k] = __ldcg(D.ctype + a[k]);
             p[k] = __ldcg(D.pos + a[k]);
         }
+        on = won();
+    }
+    if (on) {
         // The captured cell's liquid-neighbour mask, as its first claim step would build it from the
         // neighbour types at the start of a later cycle: the neighbours still liquid (a neighbour
         // claimed in this cycle reads TemporaryUpdate, or active once captured). Later captures and
@@ -1691,9 +1813,14 @@ __device__ __forceinline__ void capture_group(const PassCtx &X, int app, unsigne
         for (int k = 0; k < kPer; k++)
             if (act[k] && (ct[k] == kLiquid || ct[k] == also_liquid))
                 liq |= 1u << slot_dir(sub + k * kLanes);
+        if (kLanes == 32) {
+            liq = __reduce_or_sync(0xffffffffu, liq);
+        }
+        else {
 #pragma unroll
-        for (int o = kLanes / 2; o; o >>= 1)
-            liq |= __shfl_xor_sync(group, liq, o);
+            for (int o = kLanes / 2; o; o >>= 1)
+                liq |= __shfl_xor_sync(group, liq, o);
+        }
         // Serial order (src/CAupdate.cpp:333-334, 722-725): active cell a saw the captured cell t
         // as liquid iff t's capturer c does not precede a. a keeps a liquid neighbour iff it has an
         // unclaimed one (a set mask bit that nobody clears) or a claimed one with c >= a. Every
@@ -1719,17 +1846,28 @@ __device__ __forceinline__ void capture_group(const PassCtx &X, int app, unsigne
         // direction and the second-smallest (the state a claim step leaves), so that its first claim
         // step runs only once its DiagonalLength reaches a liquid neighbour.
         new_dl = capture_cell<kLanes>(D, c, t, l, sub, w.h, w.docx, w.docy, w.docz, liq, mn, d1, mn2);
+        if (kLanes == 32) {
+            // one direction per lane (lane = direction), lengths not negative: by their bits
+            const unsigned int b = __float_as_uint(mn);
+            const unsigned int nm = __reduce_min_sync(0xffffffffu, b);
+            const unsigned int holds = __ballot_sync(0xffffffffu, b == nm);
+            d1 = nm == 0x7f800000u ? 0xffffffffu : (unsigned int)__ffs(holds) - 1u;
+            mn = __uint_as_float(nm);
+            mn2 = __uint_as_float(__reduce_min_sync(0xffffffffu, (unsigned int)lane == d1 ? 0x7f800000u : b));
+        }
+        else {
 #pragma unroll
-        for (int o = kLanes / 2; o; o >>= 1) {
-            const float omn = __shfl_xor_sync(group, mn, o), omn2 = __shfl_xor_sync(group, mn2, o);
-            const unsigned int od1 = __shfl_xor_sync(group, d1, o);
-            if (omn < mn || (omn == mn && od1 < d1)) {
-                mn2 = fminf(omn2, mn);
-                mn = omn;
-                d1 = od1;
-            }
-            else {
-                mn2 = fminf(mn2, omn);
+            for (int o = kLanes / 2; o; o >>= 1) {
+                const float omn = __shfl_xor_sync(group, mn, o), omn2 = __shfl_xor_sync(group, mn2, o);
+                const unsigned int od1 = __shfl_xor_sync(group, d1, o);
+                if (omn < mn || (omn == mn && od1 < d1)) {
+                    mn2 = fminf(omn2, mn);
+                    mn = omn;
+                    d1 = od1;
+                }
+                else {
+                    mn2 = fminf(mn2, omn);
+                }
             }
         }
     }
@@ -1773,7 +1911,7 @@ __device__ __forceinline__ void capture_group(const PassCtx &X, int app, unsigne
 // Listed claim e: whether it won (the lowest claimant index holds the claim word) and its capture's
 // starting state, in one round of loads.
 __device__ __forceinline__ bool load_win(const PassCtx &X, unsigned long long e, WinItem &w) {
-    const unsigned int dom = (unsigned int)(e >> 37);
+    const unsigned int dom = claim_domain(e);
     const int l = (int)((e >> 32) & 31u);
     const DomainDesc &D = desc_of(X, dom);
     w.t = (unsigned int)e;
@@ -1805,7 +1943,7 @@ __device__ __forceinline__ void capture_wins(BlockShared &B, unsigned int thread
         if (on)
             w = B.wins[i];
         capture_group<kLanes>(
-            B.X, app, base, w, on, also_liquid,
+            B.X, app, base, w, on, also_liquid, [] { return true; },
             [&]() -> unsigned long long {
                 if (first == 0)
                     capture_sync(threads); // the block's slots are reserved
@@ -1821,10 +1959,68 @@ __device__ __forceinline__ void capture_wins(BlockShared &B, unsigned int thread
 // captures them. A block with few winners spends a whole warp on each: its time is then one chain
 // of loads and geometry, and a wider group shortens the chain (one neighbour and one critical
 // length per lane); with many, narrower groups keep the chains of a block in one round.
+//
+// A block with no more claims than warps gives each claim a warp at once: the winner test and every
+// load of the capture go out in one round, without a block barrier (the losers' loads are wasted).
+
+// Claim i of the block's list by one warp.
+__device__ __forceinline__ void capture_claim(PoolState *P, BlockShared &B, unsigned int i, int app, unsigned long long base,
+                                              unsigned long long *appended, int8_t also_liquid, CycleStats &st) {
+    const unsigned long long e = claim_at(B, i);
+    const unsigned int dom = claim_domain(e), held = (unsigned int)(e >> kClaimantShift);
+    const int l = (int)((e >> 32) & 31u);
+    const DomainDesc &D = desc_of(B.X, dom);
+    WinItem w;
+    w.t = (unsigned int)e;
+    w.c = (unsigned int)((long long)w.t - nb_offset(l, D.mx * D.my, D.my));
+    w.dom_dir = (dom << 5) | (unsigned int)l;
+    const unsigned long long key = __ldcg(D.claim + w.t);
+    w.cts = __ldg(D.cts_run + w.t);
+    if (held) {
+        w.h = B.claimants[held - 1].h;
+        w.docx = B.claimants[held - 1].doc[0];
+        w.docy = B.claimants[held - 1].doc[1];
+        w.docz = B.claimants[held - 1].doc[2];
+    }
+    else {
+        w.h = __ldcg(D.gid + w.c);
+        w.docx = __ldcg(D.doc + 3ull * w.c + 0);
+        w.docy = __ldcg(D.doc + 3ull * w.c + 1);
+        w.docz = __ldcg(D.doc + 3ull * w.c + 2);
+    }
+    const bool leader = (threadIdx.x & 31) == 0;
+    unsigned long long slot = 0;
+    capture_group<32>(
+        B.X, app, base, w, true, also_liquid,
+        [&] {
+            const bool win = (unsigned int)key == w.c;
+            if (win && leader) {
+                // completes under the capture
+                slot = base + atomicAdd(appended, 1ull);
+                atomicAdd(&B.n_appended, 1u);
+            }
+            return win;
+        },
+        [&]() -> unsigned long long {
+            if (leader && slot >= B.X.capacity) {
+                atomicOr(&P->error, kErrListOverflow);
+                return ULLONG_MAX;
+            }
+            return slot;
+        },
+        st);
+}
+
 template <int kLanes>
 __device__ void capture_block(PoolState *P, BlockShared &B, unsigned int threads, int app, unsigned long long base,
                               unsigned long long *appended, int8_t also_liquid, CycleStats &st) {
     const unsigned int n = claim_count(B), lane = threadIdx.x & 31;
+    constexpr bool kFew = kLanes >= kFewLanes;
+    if (kFew && n * 32 <= threads) {
+        if (threadIdx.x / 32 < n)
+            capture_claim(P, B, threadIdx.x / 32, app, base, appended, also_liquid, st);
+        return;
+    }
     for (unsigned int r0 = 0; r0 < n; r0 += threads) {
         const unsigned int i = r0 + threadIdx.x;
         WinItem w;
@@ -1850,7 +2046,7 @@ __device__ void capture_block(PoolState *P, BlockShared &B, unsigned int threads
             }
             B.slot = slot;
         }
-        if (n_wins * 32 <= threads)
+        if (kFew && n_wins * 32 <= threads)
             capture_wins<32>(B, threads, n_wins, app, base, also_liquid, st);
         else if (kLanes < 8 && n_wins * 8 <= threads)
             capture_wins<8>(B, threads, n_wins, app, base, also_liquid, st);
@@ -1896,7 +2092,8 @@ template <int kCaptureLanes> __device__ void capture_pass(PoolState *P, const Pa
             losers++;
         }
         capture_group<kCaptureLanes>(
-            X, app, base, w, win, (int8_t)kLiquid, [&]() -> unsigned long long { return base + j; }, st);
+            X, app, base, w, win, (int8_t)kLiquid, [] { return true; },
+            [&]() -> unsigned long long { return base + j; }, st);
         if (win && sub == 0)
             atomicAdd((unsigned long long *)&X.desc[w.dom_dir >> 5].liquid_shard[(blockIdx.x + j) & (kLiquidShards - 1)],
                       (unsigned long long)(-1ll));
@@ -1932,7 +2129,7 @@ template <int kBatch> __global__ void __launch_bounds__(kBlock) k_grow(PoolState
     CycleStats st;
     unsigned int tombs = 0;
     const int cur = P->cur;
-    grow_pass<kBatch, false>(P, X, nullptr, load_dyn(X.desc[0]), cur, P->cnt[cur], P->compact != 0, st, tombs);
+    grow_pass<kBatch, false, false>(P, X, nullptr, load_dyn(X.desc[0]), cur, P->cnt[cur], P->compact != 0, st, tombs);
     add_tombs(P, tombs);
     flush_stats(P, st);
 }
@@ -2242,7 +2439,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
         // growth with each block's claims right after its own growth; the global claim pass only
         // when some block's queue overflowed this cycle (the same answer for every block)
         unsigned int dropped = 0;
-        grow_pass<kBatch, true>(P, B.X, &B, dyn, cur, n, compact, st, dropped);
+        grow_pass<kBatch, true, (kLanes >= kFewLanes)>(P, B.X, &B, dyn, cur, n, compact, st, dropped);
         dropped = __reduce_add_sync(0xffffffffu, dropped);
         if ((threadIdx.x & 31) == 0 && dropped)
             atomicAdd(&B.n_tombs, dropped);

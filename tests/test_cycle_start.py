@@ -110,3 +110,22 @@ def test_cycles_that_do_nothing(lib, tmp_path, dtn):
         assert pool.status(slot).cycle == 2000
         equal(pool, slot, o, f"chunks {chunks[:4]}")
         pool.close()
+
+
+@pytest.mark.parametrize("config", [0, 2, 3])
+@pytest.mark.parametrize("n,frac,divisor", [(12, 0.02, 0), (20, 0.15, 32), (26, 0.3, 32), (26, 0.3, 16)])
+def test_few_and_many_per_block(lib, tmp_path, config, n, frac, divisor):
+    # from no record of a block to more than its warps (16), its threads and beyond: on 4 or 9 blocks
+    # the flagged records and claims per block run over every such edge as the front grows
+    inp = directional(tmp_path, nx=n, ny=n - 1, nz=n, density=800, sigma=0.4, N=14, frac=frac)
+    p = ex.Problem.from_file(inp)
+    o = Oracle(inp)
+    pool = ex.Pool(0, list_capacity=p.geometry.active_size)
+    pool.set_config(config)
+    pool.set_grid(divisor)
+    slot = pool.admit(p, device_check=False)
+    for k in (30, 90, 200):
+        pool.step(k)
+        o.step(k)
+        equal(pool, slot, o, f"{k} cycles on")
+    pool.close()
