@@ -78,6 +78,7 @@ constexpr unsigned int kMaskGrown = 1u << 28;
 // a neighbour nucleated at the start of this cycle: the growth pass drops the directions that are no
 // longer liquid from the mask (set only inside the persistent kernel, between two of its cycles)
 constexpr unsigned int kMaskNuc = 1u << 27;
+constexpr unsigned int kMaskTomb = 1u << 26; // a dropped record (the whole status word)
 constexpr unsigned int kDirBits = (1u << 26) - 1;
 // CellType of a liquid cell that nucleates at the start of the next cycle unless it is claimed in
 // this one; two codes, alternating by cycle, so that the captures of a cycle tell the sites that fire
@@ -94,8 +95,17 @@ constexpr int kErrBounds = 4;
 // the blocks of two 256-thread ones, so half the arrivals at every grid-wide meeting, and a claim
 // step of up to 512 flagged records per block in one round.
 constexpr int kBlock = 512;
-// rmin2 of a record whose minimum direction is not known: the cached minimum alone applies
-constexpr unsigned long long kNoMin2 = 0xffffffffull << 32;
+// A record's domain word: its domain, and in the upper half the direction of the cached minimum critical
+// length (kNoDir: not known, or there is none; the cached minimum alone applies).
+constexpr unsigned int kNoDir = 31u;
+__device__ __forceinline__ unsigned int dom_word(unsigned int dom, unsigned int dir) { return dom | (min(dir, kNoDir) << 16); }
+__device__ __forceinline__ unsigned int word_dom(unsigned int w) { return w & 0xffffu; }
+// The cached minimum, or the second-smallest length once the minimum's neighbour is no longer liquid (both
+// are lower bounds of the current liquid neighbours' lengths).
+__device__ __forceinline__ float effective_min(float cdl_min, float min2, unsigned int m, unsigned int w) {
+    const unsigned int d1 = w >> 16;
+    return d1 < 26u && !((m >> d1) & 1u) ? min2 : cdl_min;
+}
 
 __device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b : a; } // std::min
 __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; } // std::max
@@ -269,164 +279,19 @@ __device__ __forceinline__ long long domain_liquid(const DomainDesc &D) {
     return v;
 }
 
-// ---------------------------------------------------------------------------------------------
-// Capture of liquid cell t by active cell c through neighbour direction l
-// (src/CAupdate.cpp:353-563, 713-717).
-// Cooperative over kLanes lanes: the group's lanes share the geometry, each independent division
-// and square root of a set (the three angles, normal components, distances and direction
-// components, the four side lengths, the two projections) evaluated once, on its own lane, with the
-// reference's expression, and passed to the others by shuffles; lane `sub` computes critical
-// lengths sub, sub + kLanes, ...; lane 0 of the group writes the scalar state. Returns the new
-// DiagonalLength. Over the directions in `liq` among the lane's own,
-// (mn, d1, mn2) receive the smallest critical length, its lowest direction and the second-smallest
-// (+inf and 0xffffffff where there is none), as a claim step's scan would find them.
-template <int kLanes>
-__device__ float capture_cell(const DomainDesc &D, unsigned int c, unsigned int t, int l, int sub, int h, float docx,
-                              float docy, float docz, unsigned int liq, float &mn, unsigned int &d1, float &mn2) {
-    int rx, ry, rz;
-    cell_coords(D, c, rx, ry, rz);
-    const int GlobalX = rx + D.xoff, GlobalY = ry + D.yoff, GlobalZ = rz;
-    int ori = (abs(h) - 1) % 10000;
-    if (ori < 0)
-        ori += 10000;
-    const float *g = D.guv + 9 * ori;
-    const float g0 = g[0], g1 = g[1], g2 = g[2], g3 = g[3], g4 = g[4], g5 = g[5], g6 = g[6], g7 = g[7], g8 = g[8];
-    const double cxold = docx;
-    const double cyold = docy;
-    const double czold = docz;
-    double xp = GlobalX + nb_dx(l) + 0.5;
-    double yp = GlobalY + nb_dy(l) + 0.5;
-    double zp = GlobalZ + nb_dz(l) + 0.5;
-    double x0 = xp - cxold;
-    double y0 = yp - cyold;
-    double z0 = zp - czold;
-    static_assert(kLanes >= 4 && kLanes <= 32, "the geometry spreads over at least four lanes");
-    const unsigned int gmask = (kLanes == 32 ? 0xffffffffu : ((1u << kLanes) - 1u))
-                               << ((int)(threadIdx.x & 31) / kLanes * kLanes);
-    double mag0 = sqrtf((float)(x0 * x0 + y0 * y0 + z0 * z0));
-    // Angle1..3 on lanes 0..2 (src/CAupdate.cpp:382-393), their signs by ballot
-    const int q3 = sub < 3 ? sub : 0;
-    const float ga = q3 == 0 ? g0 : (q3 == 1 ? g3 : g6), gb = q3 == 0 ? g1 : (q3 == 1 ? g4 : g7),
-                gc = q3 == 0 ? g2 : (q3 == 1 ? g5 : g8);
-    double Angle = (ga * x0 + gb * y0 + gc * z0) / mag0;
-    const unsigned int neg = __ballot_sync(gmask, Angle < 0) >> ((int)(threadIdx.x & 31) / kLanes * kLanes);
-    float s1 = (float)(2 * (int)(neg & 1u) - 1);
-    float s2 = (float)(2 * (int)((neg >> 1) & 1u) - 1);
-    float s3 = (float)(2 * (int)((neg >> 2) & 1u) - 1);
-    double Diag1X = g0 * s1, Diag1Y = g1 * s1, Diag1Z = g2 * s1;
-    double Diag2X = g3 * s2, Diag2Y = g4 * s2, Diag2Z = g5 * s2;
-    double Diag3X = g6 * s3, Diag3Y = g7 * s3, Diag3Z = g8 * s3;
-    double U1x = Diag2X - Diag1X, U1y = Diag2Y - Diag1Y, U1z = Diag2Z - Diag1Z;
-    double U2x = Diag3X - Diag1X, U2y = Diag3Y - Diag1Y, U2z = Diag3Z - Diag1Z;
-    double UUx = U1y * U2z - U1z * U2y;
-    double UUy = U1z * U2x - U1x * U2z;
-    double UUz = U1x * U2y - U1y * U2x;
-    double NDem = sqrtf((float)(UUx * UUx + UUy * UUy + UUz * UUz));
-    // n0..n2 on lanes 0..2
-    const double nq = (q3 == 0 ? UUx : (q3 == 1 ? UUy : UUz)) / NDem;
-    double n0 = __shfl_sync(gmask, nq, 0, kLanes), n1 = __shfl_sync(gmask, nq, 1, kLanes),
-           n2 = __shfl_sync(gmask, nq, 2, kLanes);
-    double ParaT = (n0 * x0 + n1 * y0 + n2 * z0) / (n0 * Diag1X + n1 * Diag1Y + n2 * Diag1Z);
-    const double TX0 = cxold + ParaT * Diag1X, TY0 = cyold + ParaT * Diag1Y, TZ0 = czold + ParaT * Diag1Z;
-    const double TX1 = cxold + ParaT * Diag2X, TY1 = cyold + ParaT * Diag2Y, TZ1 = czold + ParaT * Diag2Z;
-    const double TX2 = cxold + ParaT * Diag3X, TY2 = cyold + ParaT * Diag3Y, TZ2 = czold + ParaT * Diag3Z;
-    // Dist[0..2] on lanes 0..2
-    const double tqx = q3 == 0 ? TX0 : (q3 == 1 ? TX1 : TX2), tqy = q3 == 0 ? TY0 : (q3 == 1 ? TY1 : TY2),
-                 tqz = q3 == 0 ? TZ0 : (q3 == 1 ? TZ1 : TZ2);
-    const float distq =
-        sqrtf((float)(((tqx - xp) * (tqx - xp)) + ((tqy - yp) * (tqy - yp)) + ((tqz - zp) * (tqz - zp))));
-    const double Dist0 = __shfl_sync(gmask, distq, 0, kLanes), Dist1 = __shfl_sync(gmask, distq, 1, kLanes),
-                 Dist2 = __shfl_sync(gmask, distq, 2, kLanes);
-    int x = (Dist0 < Dist1);
-    int y = (Dist1 < Dist2);
-    int z = (Dist2 < Dist0);
-    // 0, 1 or 2; the points idx, idx + 1 and idx + 2 (mod 3) by selects, without a local array
-    int idx = 2 * (z - y) * z + (y - x) * y;
-    const bool p0 = idx == 0, p1 = idx == 1;
-    double mindist = p0 ? Dist0 : (p1 ? Dist1 : Dist2);
-    double xc = p0 ? TX0 : (p1 ? TX1 : TX2), yc = p0 ? TY0 : (p1 ? TY1 : TY2), zc = p0 ? TZ0 : (p1 ? TZ1 : TZ2);
-    double x1 = p0 ? TX1 : (p1 ? TX2 : TX0), y1 = p0 ? TY1 : (p1 ? TY2 : TY0), z1 = p0 ? TZ1 : (p1 ? TZ2 : TZ0);
-    double x2 = p0 ? TX2 : (p1 ? TX0 : TX1), y2 = p0 ? TY2 : (p1 ? TY0 : TY1), z2 = p0 ? TZ2 : (p1 ? TZ0 : TZ1);
-    // D1..D4 on lanes 0..3: D1 = |p - v2|, D2 = |c - v2|, D3 = |p - v1|, D4 = |c - v1|
-    const int q4 = sub & 3;
-    const double ax = (q4 & 1) ? xc : xp, ay = (q4 & 1) ? yc : yp, az = (q4 & 1) ? zc : zp;
-    const double bx = (q4 & 2) ? x1 : x2, by = (q4 & 2) ? y1 : y2, bz = (q4 & 2) ? z1 : z2;
-    const float dq = sqrtf((float)(((ax - bx) * (ax - bx)) + ((ay - by) * (ay - by)) + ((az - bz) * (az - bz))));
-    double D1 = __shfl_sync(gmask, dq, 0, kLanes);
-    double D2 = __shfl_sync(gmask, dq, 1, kLanes);
-    double D3 = __shfl_sync(gmask, dq, 2, kLanes);
-    double D4 = __shfl_sync(gmask, dq, 3, kLanes);
-    double I1 = 0, I2 = D2, J1 = 0, J2 = D4;
-    if (mindist != 0) {
-        // I1 on lane 0, J1 on lane 1
-        const bool j = sub & 1;
-        const double ex = j ? x1 : x2, ey = j ? y1 : y2, ez = j ? z1 : z2;
-        const double Da = j ? D3 : D1, Db = j ? D4 : D2;
-        const double ij = Da * ((xp - ex) * (xc - ex) + (yp - ey) * (yc - ey) + (zp - ez) * (zc - ez)) / (Da * Db);
-        I1 = __shfl_sync(gmask, ij, 0, kLanes);
-        I2 = D2 - I1;
-        J1 = __shfl_sync(gmask, ij, 1, kLanes);
-        J2 = D4 - J1;
-    }
-    const double sqrt3 = sqrt(3.0);
-    double L12 = 0.5 * (dmin(I1, sqrt3) + dmin(I2, sqrt3));
-    double L13 = 0.5 * (dmin(J1, sqrt3) + dmin(J2, sqrt3));
-    double NewODiagL = sqrt(2.0) * dmax(L12, L13);
-    double cd0 = xc - cxold, cd1 = yc - cyold, cd2 = zc - czold;
-    double nd = sqrt(cd0 * cd0 + cd1 * cd1 + cd2 * cd2);
-    // uv0..uv2 on lanes 0..2
-    const double uvq = (q3 == 0 ? cd0 : (q3 == 1 ? cd1 : cd2)) / nd;
-    double uv0 = __shfl_sync(gmask, uvq, 0, kLanes), uv1 = __shfl_sync(gmask, uvq, 1, kLanes),
-           uv2 = __shfl_sync(gmask, uvq, 2, kLanes);
-    double cx = xc - NewODiagL * uv0;
-    double cy = yc - NewODiagL * uv1;
-    double cz = zc - NewODiagL * uv2;
-    if (sub == 0) {
-        D.gid[t] = h;
-        D.dl[t] = (float)NewODiagL;
-        D.doc[3ull * t + 0] = (float)cx;
-        D.doc[3ull * t + 1] = (float)cy;
-        D.doc[3ull * t + 2] = (float)cz;
-    }
-    // face normals: float sums of the unit-vector components (src/CAupdate.cpp:526-551)
-    double Fx[4], Fy[4], Fz[4];
-    Fx[0] = g0 + g3 + g6;
-    Fx[1] = g0 - g3 + g6;
-    Fx[2] = g0 + g3 - g6;
-    Fx[3] = g0 - g3 - g6;
-    Fy[0] = g1 + g4 + g7;
-    Fy[1] = g1 - g4 + g7;
-    Fy[2] = g1 + g4 - g7;
-    Fy[3] = g1 - g4 - g7;
-    Fz[0] = g2 + g5 + g8;
-    Fz[1] = g2 - g5 + g8;
-    Fz[2] = g2 + g5 - g8;
-    Fz[3] = g2 - g5 - g8;
-#pragma unroll 1
-    for (int n = sub; n < 26; n += kLanes) {
-        double a0 = xp + nb_dx(n) - cx;
-        double b0 = yp + nb_dy(n) - cy;
-        double d0 = zp + nb_dz(n) - cz;
-        double q0 = a0 * Fx[0] + b0 * Fy[0] + d0 * Fz[0];
-        double q1 = a0 * Fx[1] + b0 * Fy[1] + d0 * Fz[1];
-        double q2 = a0 * Fx[2] + b0 * Fy[2] + d0 * Fz[2];
-        double q3 = a0 * Fx[3] + b0 * Fy[3] + d0 * Fz[3];
-        double m = dmax(dmax(fabs(q0), fabs(q1)), dmax(fabs(q2), fabs(q3)));
-        const float v = (float)m;
-        D.cdl[26ull * t + n] = v;
-        if ((liq >> n) & 1u) {
-            if (v < mn) {
-                mn2 = mn;
-                mn = v;
-                d1 = (unsigned int)n;
-            }
-            else if (v < mn2) {
-                mn2 = v;
-            }
-        }
-    }
-    return (float)NewODiagL;
+// One list of active-cell records (PoolState).
+struct RecordList {
+    ActiveRec *rec;
+    unsigned int *cell, *dom;
+    float *min2;
+    RecordBody *body;
+    unsigned int body_cap; // records below it have a body
+};
+__device__ __forceinline__ RecordList list_of(const PoolState *P, int q) {
+    return RecordList{P->rec[q], P->rcell[q], P->rdom[q], P->rmin2[q], P->body[q], P->body_cap};
 }
+// GrainID (bits) and DOCenter of a body as one vector
+__device__ __forceinline__ float4 &body_head(RecordBody &b) { return *reinterpret_cast<float4 *>(&b); }
 
 // ---------------------------------------------------------------------------------------------
 // Start of a CA cycle (src/runCA.cpp:290-298, src/CAupdate.cpp:67-200): list swap, device-side
@@ -552,10 +417,9 @@ __device__ __forceinline__ NucleationView nucleation_view(const DomainDesc &D) {
 // Nucleation of one site by a warp (src/CAupdate.cpp:100-194), one round of loads: lanes 0-12 copy the
 // fresh octahedron's critical lengths, lane n < 26 reads neighbour n's type and list position; an
 // active neighbour's record goes to on_neighbour(position, direction from the site). The record goes
-// to `slot` (ULLONG_MAX: none) of the list given.
+// to `slot` (ULLONG_MAX: none) of list L.
 template <class OnNeighbour>
-__device__ __forceinline__ void nucleate_site(const NucleationView &V, int8_t *ctype, ActiveRec *rec, unsigned int *rdom,
-                                              unsigned int *rstat, unsigned long long *rmin2, unsigned int dom,
+__device__ __forceinline__ void nucleate_site(const NucleationView &V, int8_t *ctype, const RecordList &L, unsigned int dom,
                                               unsigned int site, int site_gid, int cts, unsigned long long slot,
                                               OnNeighbour &&on_neighbour) {
     const unsigned int lane = threadIdx.x & 31;
@@ -578,25 +442,28 @@ __device__ __forceinline__ void nucleate_site(const NucleationView &V, int8_t *c
         nb_type = __ldcg(ctype + a);
         nb_pos = __ldcg(V.pos + a);
     }
-    if (lane < 13)
+    const bool has_body = slot < L.body_cap;
+    if (lane < 13) {
         reinterpret_cast<float2 *>(V.cdl + 26ull * site)[lane] = row;
+        if (has_body)
+            reinterpret_cast<float2 *>(L.body[slot].cdl)[lane] = row;
+    }
     if (lane == 0) {
+        const float cx = (float)((double)(rx + V.xoff) + 0.5), cy = (float)((double)(ry + V.yoff) + 0.5),
+                    cz = (float)((double)rz + 0.5);
         V.dl[site] = 0.01f;
-        V.doc[3ull * site + 0] = (float)((double)(rx + V.xoff) + 0.5);
-        V.doc[3ull * site + 1] = (float)((double)(ry + V.yoff) + 0.5);
-        V.doc[3ull * site + 2] = (float)((double)rz + 0.5);
+        V.doc[3ull * site + 0] = cx;
+        V.doc[3ull * site + 1] = cy;
+        V.doc[3ull * site + 2] = cz;
         if (slot != ULLONG_MAX) {
-            ActiveRec r;
-            r.cell = site;
-            r.dl = 0.01f;
-            r.cdl_min = 0.0f;
-            r.cts = cts;
-            rec[slot] = r;
-            rdom[slot] = dom;
-            rstat[slot] = kMaskFresh;
-            rmin2[slot] = kNoMin2;
+            L.rec[slot] = ActiveRec{0.01f, 0.0f, cts, kMaskFresh};
+            L.cell[slot] = site;
+            L.dom[slot] = dom_word(dom, kNoDir);
+            L.min2[slot] = 0.0f;
             V.pos[site] = (unsigned int)slot;
         }
+        if (has_body)
+            body_head(L.body[slot]) = make_float4(__int_as_float(site_gid), cx, cy, cz);
         ctype[site] = kActive;
     }
     if (nb && nb_type == kActive)
@@ -673,7 +540,7 @@ __device__ __forceinline__ void start_domain(PoolState *P, DomainDesc &D, const 
     const int cts_max = probe ? D.cts_max : INT_MAX;
     long long dry = probe && lane < kLiquidShards ? __ldcg(&D.liquid_shard[lane]) : 0;
     const unsigned long long cap = P->capacity;
-    unsigned int *const rstat = P->rstat[cur];
+    const RecordList L = list_of(P, cur);
     // src/CAupdate.cpp:76-198: sites with cycle >= NucleationTimes that are still liquid
     while (cursor < s.n_nuclei) {
         const int idx = cursor + (int)lane;
@@ -707,12 +574,12 @@ __device__ __forceinline__ void start_domain(PoolState *P, DomainDesc &D, const 
         // from its liquid mask
         for (unsigned int todo = __ballot_sync(0xffffffffu, fire); todo; todo &= todo - 1) {
             const int src = __ffs(todo) - 1;
-            nucleate_site(V, s.ctype, P->rec[cur], P->rdom[cur], rstat, P->rmin2[cur], d,
+            nucleate_site(V, s.ctype, L, d,
                           __shfl_sync(0xffffffffu, loc, src), __shfl_sync(0xffffffffu, h, src),
                           __shfl_sync(0xffffffffu, cts, src), __shfl_sync(0xffffffffu, my_slot, src),
                           [&](unsigned int nb_pos, int l) {
                               if (nb_pos < cap)
-                                  atomicAnd(rstat + nb_pos, ~(1u << nb_opp(l)));
+                                  atomicAnd(&L.rec[nb_pos].stat, ~(1u << nb_opp(l)));
                           });
         }
         fired_total += __popc(__ballot_sync(0xffffffffu, fire));
@@ -812,17 +679,17 @@ __global__ void k_step_begin(PoolState *P) { begin_cycle(P, false, P->desc, P->n
 //               critical length, and re-checks the captured cell's active neighbours.
 // They run as three kernels per cycle (k_grow, k_claim, k_capture_pass) or, for stretches of
 // cycles, inside the persistent cooperative kernel k_cycles with grid-wide barriers between them.
-constexpr unsigned int kNeedsClaim = 0xffffffffu; // NaN pattern in ActiveRec::cdl_min
-// Launch-shape parameters (template arguments of the passes; the pool's tuner picks among the
-// compiled combinations): records per lane in flight in the growth pass, lanes per claim in the
-// capture pass.
+// Records per lane in flight in the growth pass (template argument).
 constexpr int kBatchChoices[2] = {2, 4};
-constexpr int kLaneChoices[2] = {4, 8};
-// The persistent kernels of the wider capture groups also hold the code for blocks with few records,
-// claims or captures (a warp for each, one group of records per warp): short lists are a chain of
-// dependent instructions, and the 8-lane shapes are the faster ones there anyway. The 4-lane shapes,
-// faster on long lists, go without it: with both, spills cost 512^3 3 % (41.3 vs 40.0 us per cycle).
-constexpr int kFewLanes = 8;
+// The persistent kernel has a family of code for each range of list lengths (a kernel that held it all
+// would be short of registers and of instruction cache: each pass runs once per cycle, and what a warp
+// waits for is mostly the next instruction, not memory):
+//   kLongList   hundreds of flagged records and captures per block and cycle: a lane per flagged record,
+//               six captures' neighbours in flight per warp, two or four records per lane in the growth.
+//   kMidList    tens of them: eight lanes per flagged record.
+//   kShortList  as kMidList, and for blocks with no more claims than warps a warp per claim.
+// Pool::shape_for chooses by the list's length.
+enum { kLongList, kMidList, kShortList };
 constexpr int kErrBarrier = 8;
 
 // Work counts of one thread, added to the pool's at the end of a kernel and, in the persistent one,
@@ -847,9 +714,7 @@ __device__ void flush_stats(PoolState *P, const CycleStats &st) {
 // The copy's dynamic fields are those of the kernel's start; the persistent kernel refreshes cycle
 // and epoch every cycle.
 struct PassCtx {
-    ActiveRec *rec[2];
-    unsigned int *rdom[2], *rstat[2];
-    unsigned long long *rmin2[2];
+    RecordList list[2];
     DomainDesc *desc;
     unsigned long long *tgt;
     unsigned long long capacity, segment, shard_cap; // segment: entries of tgt a block may fill
@@ -867,12 +732,8 @@ __device__ __forceinline__ void load_ctx(const PoolState *P, PassCtx &X, unsigne
     for (unsigned int w = threadIdx.x; w < sizeof(DomainDesc) / 8; w += blockDim.x)
         dst[w] = __ldcg(src + w);
     if (threadIdx.x == 0) {
-        for (int q = 0; q < 2; q++) {
-            X.rec[q] = P->rec[q];
-            X.rdom[q] = P->rdom[q];
-            X.rstat[q] = P->rstat[q];
-            X.rmin2[q] = P->rmin2[q];
-        }
+        for (int q = 0; q < 2; q++)
+            X.list[q] = list_of(P, q);
         X.desc = P->desc;
         X.tgt = P->tgt;
         X.capacity = P->capacity;
@@ -893,6 +754,13 @@ __device__ __forceinline__ const DomainDesc &desc_of(const PassCtx &X, unsigned 
     return dom == X.hot ? X.hot_desc : X.desc[dom];
 }
 
+// The 26 critical lengths of record `pos` (cell `cell` of domain D): of its body, else the cell's own.
+// Both hold the same values; the bodies of a long front lie in a few dozen MB, the rows of its cells
+// all over an array of 104 bytes per cell.
+__device__ __forceinline__ const float *row_of(const RecordList &L, const DomainDesc &D, unsigned int pos, unsigned int cell) {
+    return pos < L.body_cap ? L.body[pos].cdl : D.cdl + 26ull * cell;
+}
+
 // A domain's dynamic fields in one load, past L1.
 struct DomainDyn {
     int cycle;
@@ -908,74 +776,103 @@ __device__ __forceinline__ DomainDyn load_dyn(const DomainDesc &D) {
     return DomainDyn{v.x, (unsigned int)v.y, v.z, v.w};
 }
 
-// The descriptor fields a growth step reads for every record, in registers: for the hot domain they
-// are loaded once per growth pass, for the others per record.
+// What the growth of a domain's records needs of its descriptor: for the hot domain loaded once per
+// growth pass, for the others per record (two 16-byte vectors of one 32-byte sector).
 struct GrowView {
-    const DomainDesc *D;
     const double *growth;
-    long long e_cycle; // executed cycles up to the current one
-    int cycle, growth_len;
-    bool done, jumps, zero_du;
+    int e_cycle; // executed cycles up to the current one
+    int cycle;   // kDoneCycle: the domain has ended
+    int growth_len;
+    bool zero_du, jumps;
 };
+constexpr int kDoneCycle = INT_MIN;
 __device__ __forceinline__ GrowView grow_view(const DomainDesc &D) {
-    GrowView v;
-    v.D = &D;
-    v.growth = D.growth;
-    v.cycle = D.cycle;
-    v.e_cycle = executed_upto(D, v.cycle);
-    v.growth_len = D.growth_len;
-    v.done = D.done != 0;
-    v.jumps = D.n_jumps > 0;
-    v.zero_du = D.zero_du != 0;
-    return v;
+    static_assert(offsetof(DomainDesc, growth) % 32 == 0 && offsetof(DomainDesc, growth_len) == offsetof(DomainDesc, growth) + 8 &&
+                      offsetof(DomainDesc, zero_du) == offsetof(DomainDesc, growth) + 12 &&
+                      offsetof(DomainDesc, n_jumps) == offsetof(DomainDesc, growth) + 14 &&
+                      offsetof(DomainDesc, cycle) == offsetof(DomainDesc, growth) + 16,
+                  "growth, growth_len, zero_du, n_jumps and the dynamic fields are one 32-byte sector");
+    const int4 v = __ldcg(reinterpret_cast<const int4 *>(&D.growth));
+    const DomainDyn dyn = load_dyn(D);
+    GrowView g;
+    g.growth = reinterpret_cast<const double *>((unsigned long long)(unsigned int)v.x | ((unsigned long long)(unsigned int)v.y << 32));
+    g.growth_len = v.z;
+    g.zero_du = (v.w & 0xffff) != 0;
+    g.jumps = ((unsigned int)v.w >> 16) != 0;
+    g.cycle = dyn.done ? kDoneCycle : dyn.cycle;
+    g.e_cycle = g.jumps ? (int)executed_upto(D, dyn.cycle) : dyn.cycle;
+    return g;
 }
 __device__ __forceinline__ GrowView hot_view(const PassCtx &X, const DomainDyn &dyn) {
-    GrowView v;
-    v.D = &X.hot_desc;
-    v.growth = X.hot_desc.growth;
-    v.cycle = dyn.cycle;
-    v.e_cycle = dyn.cycle - X.hot_skipped; // every jump ends below the current cycle
-    v.growth_len = X.hot_desc.growth_len;
-    v.done = dyn.done != 0;
-    v.jumps = X.hot_desc.n_jumps > 0;
-    v.zero_du = X.hot_desc.zero_du != 0;
-    return v;
+    GrowView g;
+    g.growth = X.hot_desc.growth;
+    g.growth_len = X.hot_desc.growth_len;
+    g.zero_du = X.hot_desc.zero_du != 0;
+    g.jumps = X.hot_desc.n_jumps != 0;
+    g.cycle = dyn.done ? kDoneCycle : dyn.cycle;
+    g.e_cycle = dyn.cycle - (int)X.hot_skipped; // every jump ends below the current cycle
+    return g;
 }
 
-// Growth step of one record with its liquid mask and growth increment loaded. Returns 0: drop
-// the record, 1: keep it unchanged (not eligible yet), 2: keep the updated record.
-// eff_min: the cached minimum critical length, or the second-smallest one once the minimum's
-// neighbour is no longer liquid (both are lower bounds of the current liquid neighbours' lengths).
-__device__ __forceinline__ int grow_record(const PassCtx &X, const GrowView &v, unsigned int dom, ActiveRec &r,
-                                           unsigned int m, double inc, bool inc_ok, float eff_min, CycleStats &st) {
-    const unsigned int c = r.cell;
-    st.listed++;
-    if (v.done || (m & kMaskDead)) {
-        // finished domain, or solidified by last cycle's re-check (a retired domain's records point
-        // at the placeholder descriptor, which has no fields)
-        if (v.D->dl)
-            v.D->dl[c] = r.dl;
-        return 0;
+// The diagonal's growth this cycle of a record of domain D: the table entry of the undercooling after
+// the executed updates since the liquidus (src/CAupdate.cpp:236-237), plus those of earlier layers;
+// the table of the cell's UndercoolingChange value. kNoGrowth beyond the table; 0 if not eligible.
+constexpr double kNoGrowth = -1.0;
+__device__ __forceinline__ double load_growth(const GrowView &g, const DomainDesc &D, unsigned int cell, int cts,
+                                              bool extras) {
+    if (!(g.cycle > cts))
+        return 0.0;
+    int nu = g.e_cycle - (g.jumps ? (int)executed_upto(D, cts) : max(cts, 0));
+    const double *table = g.growth;
+    if (extras) {
+        if (D.nu_base)
+            nu += __ldg(D.nu_base + cell);
+        if (D.du_class)
+            table += (size_t)__ldg(D.du_class + cell) * (size_t)g.growth_len;
     }
-    if (!(v.cycle > r.cts))
-        return 1; // cts is INT_MAX outside the window and for LayerID > layer
+    if (g.zero_du && D.du[cell] == 0.0f)
+        nu = 0;
+    return (unsigned int)nu < (unsigned int)g.growth_len ? __ldg(table + nu) : kNoGrowth;
+}
+
+// Growth step of one record (status m, growth increment inc, its domain's cycle).
+enum GrowAction {
+    kDrop,  // dropped: finished domain, solidified by last cycle's re-check, or no liquid neighbour
+    kWait,  // not eligible yet: unchanged
+    kGrown, // r.dl grown
+    kFlag   // grown, and its claim step is due: the mask must be built or the diagonal reached the
+            // applicable lower bound of the liquid neighbours' critical lengths
+};
+__device__ __forceinline__ GrowAction grow_record(const PassCtx &X, int cycle, unsigned int cell, unsigned int dom, ActiveRec &r,
+                                                  unsigned int m, double inc, float bound, CycleStats &st) {
+    st.listed++;
+    if (cycle == kDoneCycle || (m & kMaskDead)) {
+        // a retired domain's records point at the placeholder descriptor, which has no fields
+        float *dl = desc_of(X, dom).dl;
+        if (dl)
+            dl[cell] = r.dl;
+        return kDrop;
+    }
+    if (!(cycle > r.cts))
+        return kWait; // cts is INT_MAX outside the window and for LayerID > layer
     st.grown++;
-    if (!inc_ok)
+    if (inc < 0.0) {
         atomicOr(&X.desc[dom].error, kErrGrowthTable);
-    const float dl = (float)((double)r.dl + inc);
-    r.dl = dl;
-    if ((m & kMaskFresh) || dl >= eff_min) {
-        r.cdl_min = __uint_as_float(kNeedsClaim);
+        inc = 0.0;
+    }
+    r.dl = (float)((double)r.dl + inc);
+    if ((m & kMaskFresh) || r.dl >= bound) {
         st.flagged++;
-        return 2;
+        return kFlag;
     }
     if ((m & kDirBits) == 0) {
         // no liquid neighbour: LCount stays 0 (src/CAupdate.cpp:722-725)
-        v.D->ctype[c] = kSolid;
-        v.D->dl[c] = dl;
-        return 0;
+        const DomainDesc &D = desc_of(X, dom);
+        D.ctype[cell] = kSolid;
+        D.dl[cell] = r.dl;
+        return kDrop;
     }
-    return 2;
+    return kGrown;
 }
 
 // The mask of a record next to cells that nucleated at the start of this cycle: without the
@@ -990,27 +887,6 @@ __device__ __noinline__ unsigned int drop_nucleated(const DomainDesc &D, unsigne
             gone |= 1u << l;
     }
     return m & ~(gone | kMaskNuc);
-}
-
-__device__ __forceinline__ float effective_min(const ActiveRec &r, unsigned int m, unsigned long long min2) {
-    const unsigned int d1 = (unsigned int)(min2 >> 32);
-    return (d1 >= 26u || ((m >> d1) & 1u)) ? r.cdl_min : __uint_as_float((unsigned int)min2);
-}
-
-// load_growth with the per-record descriptor fields from a view
-__device__ __forceinline__ void load_growth(const GrowView &v, const ActiveRec &r, double &inc, bool &ok, bool extras) {
-    long long nu = v.e_cycle - (v.jumps ? executed_upto(*v.D, r.cts) : (r.cts <= 0 ? 0ll : (long long)r.cts));
-    const double *table = v.growth;
-    if (extras) {
-        if (v.D->nu_base)
-            nu += __ldg(v.D->nu_base + r.cell);
-        if (v.D->du_class)
-            table += (size_t)__ldg(v.D->du_class + r.cell) * (size_t)v.growth_len;
-    }
-    if (v.zero_du && v.D->du[r.cell] == 0.0f)
-        nu = 0;
-    ok = nu >= 0 && nu < v.growth_len;
-    inc = (ok && v.cycle > r.cts) ? __ldg(table + nu) : 0.0;
 }
 
 // Records the growth pass hands to the claim pass go to a global queue together with the state the
@@ -1045,39 +921,159 @@ __device__ __forceinline__ unsigned long long warp_reserve_n(unsigned long long 
 __device__ __forceinline__ unsigned long long claim_key(const DomainDesc &D, unsigned int c) {
     return ((unsigned long long)(0xffffffffu - D.epoch) << 32) | (unsigned long long)c;
 }
-// A listed claim: domain (13 bits), direction from the claimant and claimed cell; in a block's own
-// list also 1 + the entry of BlockShared::claimants that holds the claimant's state (0: none).
+// A listed claim: domain (13 bits), direction from the claimant and claimed cell; in a block's own list
+// also 1 + the entry of BlockShared::claimants that holds the claimant's state (0: none).
 constexpr int kClaimantShift = 50;
 __device__ __forceinline__ unsigned long long claim_entry_of(unsigned int dom, int l, unsigned int t) {
     return ((unsigned long long)dom << 37) | ((unsigned long long)l << 32) | t;
 }
 __device__ __forceinline__ unsigned int claim_domain(unsigned long long e) { return (unsigned int)(e >> 37) & 0x1fffu; }
 
-// Claim work of queue entry k. Returns the directions of the cells it claimed. All loads of the entry
-// (critical-length row, neighbour types) go out in one round.
-// A record the growth pass flagged for a claim step: its list position, cell, domain, liquid mask
-// and grown DiagonalLength.
+// A record the growth pass flagged for a claim step: its list position, domain, liquid mask and grown
+// DiagonalLength.
 struct ClaimItem {
-    unsigned int pos, cell, dom, mask;
+    unsigned int pos, dom, mask;
     float dl;
 };
 
-// With kIssue the claims go out here; otherwise the caller issues them (block_claims).
-template <bool kIssue>
-__device__ __forceinline__ unsigned int claim_record(const PassCtx &X, int app, const ClaimItem &it, CycleStats &st,
-                                                     unsigned int &tombs) {
-    const unsigned int i = it.pos, c = it.cell, dom = it.dom;
+// What a claim step leaves in one lane: the directions of its four that the record reaches, the claimant.
+struct ClaimLane {
+    unsigned int reach;       // bit j: direction dir0 + j
+    int dir0;
+    unsigned int cell, dom;
+};
+
+// The claim step of one flagged record by eight lanes (on: the group has one; every lane of the warp calls,
+// src/CAupdate.cpp:320-352): lanes 1-7 read four critical lengths each (lane 0 the rest
+// of the body), so a record is one 128-byte line in one load instruction of its group, and each lane compares four
+// lengths. (A record per lane, 26 lengths compared in turn from seven uncoalesced 16-byte loads, took
+// 3.7 us of a 256^3 cycle, its code 3000 instructions.)
+__device__ __forceinline__ ClaimLane claim_group(const PassCtx &X, int app, const ClaimItem &it, bool on, CycleStats &st,
+                                                 unsigned int &tombs) {
+    const unsigned int lane = threadIdx.x & 31, sub = lane & 7u, group = 0xffu << (lane & 24u);
+    const RecordList &L = X.list[app];
+    ClaimLane out{0u, 4 * (int)sub - 4, 0u, it.dom};
+    if (!on)
+        return out;
+    const DomainDesc &D = desc_of(X, it.dom);
+    ActiveRec *const rec = L.rec + it.pos;
+    const unsigned int c = __ldcg(L.cell + it.pos); // a body does not wait for it
+    out.cell = c;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (it.pos < L.body_cap) {
+        static_assert(offsetof(RecordBody, cdl) == 16, "GrainID and DOCenter, then the lengths");
+        v = __ldcg(reinterpret_cast<const float4 *>(L.body + it.pos) + sub);
+    }
+    else if (sub) {
+        const float *row = D.cdl + 26ull * c + out.dir0;
+        v.x = __ldcg(row);
+        v.y = __ldcg(row + 1);
+        if (sub < 7) {
+            v.z = __ldcg(row + 2);
+            v.w = __ldcg(row + 3);
+        }
+    }
+    unsigned int m = it.mask;
+    if (m & kMaskFresh) {
+        // liquid neighbours from the 26 neighbour types (src/CAupdate.cpp:320-334); no other thread
+        // writes this cell's mask now, captures and nucleations clear bits later. A cell claimed in
+        // this same step (TemporaryUpdate) is still liquid.
+        int rx, ry, rz;
+        cell_coords(D, c, rx, ry, rz);
+        const unsigned int valid = neighbour_mask(D, rx, ry, rz);
+        const int plane = D.mx * D.my;
+        m = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int l = out.dir0 + j;
+            if (l >= 0 && l < 26 && ((valid >> l) & 1u) && liquid_type(__ldcg(D.ctype + c + nb_offset(l, plane, D.my))))
+                m |= 1u << l;
+        }
+#pragma unroll
+        for (int o = 4; o; o >>= 1)
+            m |= __shfl_xor_sync(group, m, o);
+        if (sub == 0) {
+            st.fresh++;
+            rec->stat = m | kMaskGrown; // a flagged record was grown this cycle
+        }
+    }
+    m &= kDirBits;
+    if (m == 0) {
+        // no liquid neighbour: LCount stays 0 (src/CAupdate.cpp:722-725)
+        if (sub == 0) {
+            D.ctype[c] = kSolid;
+            D.dl[c] = it.dl;
+            rec->stat = kMaskTomb;
+            st.dropped++;
+            tombs++;
+        }
+        return out;
+    }
+    // Every reached cell is claimed and captured within this cycle, so the cached minimum only
+    // covers the liquid neighbours not reached (+inf when none is left).
+    const unsigned int mine = sub ? m >> out.dir0 : 0u;
+    const float f[4] = {v.x, v.y, v.z, v.w};
+    float mn = __int_as_float(0x7f800000), mn2 = mn;
+    unsigned int d1 = 0xffffffffu;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        if ((mine >> j) & 1u) {
+            if (it.dl >= f[j]) {
+                out.reach |= 1u << j;
+            }
+            else if (f[j] < mn) {
+                mn2 = mn;
+                mn = f[j];
+                d1 = (unsigned int)(out.dir0 + j);
+            }
+            else if (f[j] < mn2) {
+                mn2 = f[j];
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 4; o; o >>= 1) {
+        const float omn = __shfl_xor_sync(group, mn, o), omn2 = __shfl_xor_sync(group, mn2, o);
+        const unsigned int od1 = __shfl_xor_sync(group, d1, o);
+        if (omn < mn || (omn == mn && od1 < d1)) {
+            mn2 = fminf(omn2, mn);
+            mn = omn;
+            d1 = od1;
+        }
+        else {
+            mn2 = fminf(mn2, omn);
+        }
+    }
+    if (sub == 0) {
+        st.rows++;
+        rec->cdl_min = mn;
+        L.min2[it.pos] = mn2;
+        L.dom[it.pos] = dom_word(it.dom, d1);
+    }
+    return out;
+}
+
+// The claim step of one flagged record by one lane: the form for blocks with hundreds of flagged
+// records, whose loads are all in flight in one round. Returns the directions of the cells it reaches,
+// which the caller claims (push_claims, issue_claims).
+__device__ __forceinline__ unsigned int claim_record(const PassCtx &X, int app, const ClaimItem &it, unsigned int &c,
+                                                     CycleStats &st, unsigned int &tombs) {
+    const unsigned int i = it.pos, dom = it.dom;
     unsigned int m = it.mask;
     const float dl = it.dl;
     const DomainDesc &D = desc_of(X, dom);
-    ActiveRec *recs = X.rec[app];
+    const RecordList &L = X.list[app];
+    c = __ldcg(L.cell + i); // a body's row does not wait for it
+    ActiveRec *recs = L.rec;
     const int plane = D.mx * D.my, my = D.my;
-    // the 26 critical lengths as 7 aligned 16-byte loads: a row (26 * 4 * c bytes in) starts on a
-    // 16-byte boundary for even c and 8 bytes past one for odd c, which read from 8 bytes before it
+    // the 26 critical lengths as 7 aligned 16-byte loads: a cell's own row (26 * 4 * c bytes in) starts
+    // on a 16-byte boundary for even c and 8 bytes past one for odd c, which read from 8 bytes before it
     // (the previous row's end). The 8 bytes read past an even row lie in the array, or for the last
-    // row in the slot's next field array (sub-arrays start on 256-byte boundaries).
-    const bool odd = c & 1u;
-    const float4 *row = reinterpret_cast<const float4 *>(D.cdl + 26ull * c - (odd ? 2 : 0));
+    // row in the slot's next field array (sub-arrays start on 256-byte boundaries). A body's row is
+    // even, with 8 bytes of its own after it.
+    const float *const lengths = row_of(L, D, i, c);
+    const bool odd = (reinterpret_cast<unsigned long long>(lengths) & 8u) != 0;
+    const float4 *row = reinterpret_cast<const float4 *>(lengths - (odd ? 2 : 0));
     float f[28];
 #pragma unroll
     for (int q = 0; q < 7; q++) {
@@ -1107,14 +1103,13 @@ __device__ __forceinline__ unsigned int claim_record(const PassCtx &X, int app, 
             const int8_t nt = __ldcg(ct + (v ? nb_offset(l, plane, my) : 0));
             m |= (v && liquid_type(nt)) ? (1u << l) : 0u;
         }
-        X.rstat[app][i] = m | kMaskGrown; // a flagged record was grown this cycle
+        recs[i].stat = m | kMaskGrown; // a flagged record was grown this cycle
     }
     if ((m & kDirBits) == 0) {
         // no liquid neighbour: LCount stays 0 (src/CAupdate.cpp:722-725)
         D.ctype[c] = kSolid;
         D.dl[c] = dl;
-        recs[i].cell = kTombstone;
-        recs[i].cdl_min = 0.0f;
+        recs[i].stat = kMaskTomb;
         st.dropped++;
         tombs++;
         return 0;
@@ -1142,51 +1137,12 @@ __device__ __forceinline__ unsigned int claim_record(const PassCtx &X, int app, 
         }
     }
     recs[i].cdl_min = nm;
-    X.rmin2[app][i] = ((unsigned long long)d1 << 32) | __float_as_uint(nm2);
+    L.min2[i] = nm2;
+    L.dom[i] = dom_word(dom, d1);
     if (reach) {
-        // claims (src/CAupdate.cpp:336-352): the lowest index wins. Nothing waits for them: every
-        // claimant lists its claim and the capture pass keeps the winner's. A claimed cell reads
-        // TemporaryUpdate until its capture makes it active, as in the reference's capture
-        // (src/CAupdate.cpp:343-352).
-        if (kIssue) {
-            const unsigned long long key = claim_key(D, c);
-            unsigned long long *base = D.claim + c;
-            for (unsigned int bits = reach; bits; bits &= bits - 1) {
-                const int nb = nb_offset(__ffs(bits) - 1, plane, my);
-                atomicMin(base + nb, key);
-                D.ctype[c + nb] = kTemporaryUpdate;
-            }
-        }
         st.claims += __popc(reach);
     }
     return reach;
-}
-
-// The claim step of global claim-queue entry k.
-template <bool kIssue>
-__device__ __forceinline__ unsigned int claim_entry(const PoolState *P, const PassCtx &X, int app, unsigned long long k,
-                                                    CycleStats &st, unsigned int &tombs) {
-    const ClaimItem it{__ldcg(P->qpos + k), __ldcg(P->qcell + k), __ldcg(P->qdom + k), __ldcg(P->qmask + k),
-                       __ldcg(P->qdl + k)};
-    return claim_record<kIssue>(X, app, it, st, tombs);
-}
-
-// Lists the claims of one record per lane (all lanes of the warp call; reach 0: none) for the
-// capture pass, as (domain << 37) | (direction << 32) | claimed cell, in shard `shard`.
-__device__ __forceinline__ void list_claims(PoolState *P, unsigned int shard, unsigned int reach, unsigned int dom,
-                                            unsigned int cell) {
-    const unsigned long long cap = P->shard_cap;
-    unsigned long long pos = warp_reserve_n(&P->tcnt_s[shard].v, cap, &P->error, __popc(reach));
-    if (reach && pos != ULLONG_MAX) {
-        pos += (unsigned long long)shard * cap;
-        const DomainDesc &D = P->desc[dom];
-        const int plane = D.mx * D.my, my = D.my;
-        unsigned long long t = pos;
-        for (unsigned int bits = reach; bits; bits &= bits - 1) {
-            const int l = __ffs(bits) - 1;
-            P->tgt[t++] = claim_entry_of(dom, l, (unsigned int)((long long)cell + nb_offset(l, plane, my)));
-        }
-    }
 }
 
 // The persistent kernel's working set of one block in shared memory. The records a block flags wait
@@ -1198,50 +1154,62 @@ __device__ __forceinline__ void list_claims(PoolState *P, unsigned int shard, un
 // beyond kBlockClaims go to the block's segment of PoolState::tgt.
 constexpr int kBlockQueue = 1280;
 constexpr int kBlockClaims = 1024;
+constexpr int kFreeSlots = 1024;
 // A winning claim, with the state of its claimant that the capture starts from.
 struct WinItem {
     unsigned int t, c;    // captured cell, claimant
     unsigned int dom_dir; // (domain << 5) | direction from the claimant
     int h, cts;           // claimant's GrainID, CritTimeStep of t
     float docx, docy, docz;
+    unsigned int slot; // of the new record (kNoRecord: none)
 };
+// What the geometry and the neighbours of a capture leave for its last stage.
+struct CaptureItem {
+    double cx, cy, cz; // centre of the new octahedron
+    float dl;          // and its DiagonalLength
+    unsigned int liq;  // the captured cell's liquid neighbours
+};
+constexpr int kCaptureItems = 128; // captures a block has in hand at a time
+
 struct BlockShared {
     union {
         ClaimItem items[kBlockQueue]; // growth and claims
         WinItem wins[kBlock];         // capture
     };
     unsigned long long claims[kBlockClaims];
-    struct {
-        int h;        // GrainID
-        float doc[3]; // DOCenter
-    } claimants[kBlock / 32];
+    unsigned int claim_pos[kBlockClaims]; // the claimant's record
+    CaptureItem captures[kCaptureItems];
+    float4 claimants[kBlock / 32]; // GrainID (bits) and DOCenter, kept by claim_warp for capture_claim
     unsigned int n_items;  // may exceed kBlockQueue (the excess went global)
     unsigned int n_claims; // may exceed kBlockClaims (the excess is in the block's segment)
     unsigned int n_wins;
     unsigned int n_first;    // cells of the hot domain this block was the first to claim this cycle
-    unsigned int n_tombs;    // records dropped this cycle
     unsigned int n_appended; // records appended this cycle (captures and nucleations)
+    // Positions of dropped records that this block's captures may use again: those that it dropped
+    // itself in this launch, and those that its growth met on the launch's first pass. n_free may
+    // exceed kFreeSlots (the excess waits for a compaction); the captures of a cycle take the last
+    // n_taken of them.
+    unsigned int n_free, n_taken;
+    int tombs; // change of the list's number of dropped records, not yet told to the grid
+    unsigned int free_slots[kFreeSlots];
     unsigned int busy;       // a record of the block was grown or dropped this cycle
     int min_cts;             // smallest CritTimeStep of the block's other records, while it is not busy
-    unsigned long long slot; // first record slot of the block's captures in this round
     PassCtx X;
 };
 
 // Puts the flagged records of one growth step into the claim queue (all lanes of the warp call).
 template <int kBatch>
 __device__ __forceinline__ void queue_flagged(PoolState *P, unsigned int shard, unsigned int nf, unsigned int flagged,
-                                              const unsigned long long *idx, const ActiveRec *r,
-                                              const unsigned int *dom, const unsigned int *m) {
+                                              const unsigned int *idx, const ActiveRec *r, const unsigned int *dom) {
     unsigned long long k = warp_reserve_n(&P->qcnt_s[shard].v, P->shard_cap, &P->error, nf);
     if (nf && k != ULLONG_MAX) {
         k += (unsigned long long)shard * P->shard_cap;
 #pragma unroll
         for (int q = 0; q < kBatch; q++) {
             if (flagged & (1u << q)) {
-                P->qpos[k] = (unsigned int)idx[q];
-                P->qcell[k] = r[q].cell;
-                P->qdom[k] = dom[q];
-                P->qmask[k] = m[q];
+                P->qpos[k] = idx[q];
+                P->qdom[k] = word_dom(dom[q]);
+                P->qmask[k] = r[q].stat;
                 P->qdl[k] = r[q].dl;
                 k++;
             }
@@ -1253,58 +1221,54 @@ __device__ __forceinline__ void queue_flagged(PoolState *P, unsigned int shard, 
 // the global queue (all lanes of the warp call). Every slot below kBlockQueue that a warp reserves
 // is written in the same step, so the block's claim step reads only this cycle's records.
 template <int kBatch>
-__device__ __forceinline__ void block_queue_flagged(PoolState *P, BlockShared &B, unsigned int shard, unsigned int nf,
-                                                    unsigned int flagged, const unsigned long long *idx,
-                                                    const ActiveRec *r, const unsigned int *dom, const unsigned int *m) {
-    const unsigned int lane = threadIdx.x & 31;
-    unsigned int incl = nf;
+__device__ __forceinline__ void block_queue_flagged(PoolState *P, BlockShared &B, unsigned int shard, unsigned int flagged,
+                                                    const unsigned int *idx, const ActiveRec *r, const unsigned int *dom) {
+    const unsigned int lane = threadIdx.x & 31, below = (1u << lane) - 1u;
+    unsigned int who[kBatch], total = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= (unsigned)o)
-            incl += v;
+    for (int q = 0; q < kBatch; q++) {
+        who[q] = __ballot_sync(0xffffffffu, (flagged >> q) & 1u);
+        total += __popc(who[q]);
     }
-    const unsigned int total = __shfl_sync(0xffffffffu, incl, 31);
+    if (total == 0)
+        return;
     unsigned int base = 0;
-    if (lane == 31 && total)
+    if (lane == 0)
         base = atomicAdd(&B.n_items, total);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    const unsigned int first = base + incl - nf; // this lane's first slot
-    unsigned int e = first, n_global = 0;
+    base = __shfl_sync(0xffffffffu, base, 0);
+    unsigned int first = base;
 #pragma unroll
-    for (int q = 0; q < kBatch; q++)
-        if (flagged & (1u << q)) {
-            if (e < (unsigned int)kBlockQueue)
-                B.items[e] = ClaimItem{(unsigned int)idx[q], r[q].cell, dom[q], m[q], r[q].dl};
-            else
-                n_global++;
-            e++;
-        }
-    if (__any_sync(0xffffffffu, n_global != 0)) {
-        unsigned long long k = warp_reserve_n(&P->qcnt_s[shard].v, P->shard_cap, &P->error, n_global);
-        if (n_global && k != ULLONG_MAX) {
-            k += (unsigned long long)shard * P->shard_cap;
-            e = first;
-#pragma unroll
-            for (int q = 0; q < kBatch; q++)
-                if (flagged & (1u << q)) {
-                    if (e >= (unsigned int)kBlockQueue) {
-                        P->qpos[k] = (unsigned int)idx[q];
-                        P->qcell[k] = r[q].cell;
-                        P->qdom[k] = dom[q];
-                        P->qmask[k] = m[q];
-                        P->qdl[k] = r[q].dl;
-                        k++;
-                    }
-                    e++;
-                }
-        }
+    for (int q = 0; q < kBatch; q++) {
+        const unsigned int e = first + __popc(who[q] & below);
+        if (((flagged >> q) & 1u) && e < (unsigned int)kBlockQueue)
+            B.items[e] = ClaimItem{idx[q], word_dom(dom[q]), r[q].stat, r[q].dl};
+        first += __popc(who[q]);
     }
+    if (base + total > (unsigned int)kBlockQueue) {
+        unsigned int beyond = 0;
+        first = base;
+#pragma unroll
+        for (int q = 0; q < kBatch; q++) {
+            if (((flagged >> q) & 1u) && first + __popc(who[q] & below) >= (unsigned int)kBlockQueue)
+                beyond |= 1u << q;
+            first += __popc(who[q]);
+        }
+        queue_flagged<kBatch>(P, shard, __popc(beyond), beyond, idx, r, dom);
+    }
+}
+
+// Claims of the block's list, and claim i of them (all threads agree after a block barrier).
+__device__ __forceinline__ unsigned int claim_count(const BlockShared &B) {
+    const unsigned long long most = kBlockClaims + B.X.segment;
+    return B.n_claims < most ? B.n_claims : (unsigned int)most;
+}
+__device__ __forceinline__ unsigned long long claim_at(const BlockShared &B, unsigned int i) {
+    return i < (unsigned int)kBlockClaims ? B.claims[i] : __ldcg(B.X.tgt + blockIdx.x * B.X.segment + (i - kBlockClaims));
 }
 
 // Puts the claims of one record per lane (all lanes of the warp call; reach 0: none) into the block's list.
 __device__ __forceinline__ void push_claims(PoolState *P, BlockShared &B, unsigned int reach, unsigned int dom,
-                                            unsigned int cell) {
+                                            unsigned int cell, unsigned int pos) {
     const unsigned int lane = threadIdx.x & 31, n = __popc(reach);
     unsigned int incl = n;
 #pragma unroll
@@ -1326,6 +1290,7 @@ __device__ __forceinline__ void push_claims(PoolState *P, BlockShared &B, unsign
             const unsigned long long v = claim_entry_of(dom, l, (unsigned int)((long long)cell + nb_offset(l, plane, my)));
             if (e < (unsigned int)kBlockClaims) {
                 B.claims[e] = v;
+                B.claim_pos[e] = pos;
             }
             else {
                 const unsigned long long k = e - kBlockClaims;
@@ -1336,15 +1301,6 @@ __device__ __forceinline__ void push_claims(PoolState *P, BlockShared &B, unsign
             }
         }
     }
-}
-
-// Claims of the block's list, and claim i of them (all threads agree after a block barrier).
-__device__ __forceinline__ unsigned int claim_count(const BlockShared &B) {
-    const unsigned long long most = kBlockClaims + B.X.segment;
-    return B.n_claims < most ? B.n_claims : (unsigned int)most;
-}
-__device__ __forceinline__ unsigned long long claim_at(const BlockShared &B, unsigned int i) {
-    return i < (unsigned int)kBlockClaims ? B.claims[i] : __ldcg(B.X.tgt + blockIdx.x * B.X.segment + (i - kBlockClaims));
 }
 
 // Issues the claims [first, claim_count) of the block's list, one per thread (src/CAupdate.cpp:336-352;
@@ -1375,21 +1331,25 @@ __device__ __forceinline__ void issue_claims(BlockShared &B, unsigned int first)
         atomicAdd(&B.n_first, firsts);
 }
 
-// The claim step of the block's item `i` by a whole warp: claim_record, push_claims and issue_claims with
-// one direction per lane, and the claimant's state loaded for the capture. A block with a few flagged
-// records has one chain of dependent instructions to wait for, most of them issued for one lane each in
-// the record-per-lane form (26 lengths compared in turn, the list positions, two block barriers).
+// The claim step of the block's item `i` by a whole warp: one direction per lane (claim_group and make_claims
+// in one), the shortest chain for a block with no more flagged records than warps.
 __device__ __forceinline__ void claim_warp(BlockShared &B, int app, unsigned int i, CycleStats &st, unsigned int &tombs) {
     const unsigned int lane = threadIdx.x & 31;
     const ClaimItem it = B.items[i];
-    const unsigned int c = it.cell, dom = it.dom;
+    const unsigned int dom = it.dom;
     unsigned int m = it.mask;
     const DomainDesc &D = desc_of(B.X, dom);
     const int plane = D.mx * D.my, my = D.my;
     constexpr unsigned int kInf = 0x7f800000u;
+    const RecordList &L = B.X.list[app];
+    const unsigned int c = __ldcg(L.cell + it.pos); // a body does not wait for it
     // lanes 0-25: the critical lengths; 26: GrainID; 27-29: DOCenter
     unsigned int v = kInf;
-    if (lane < 26)
+    if (it.pos < L.body_cap) {
+        if (lane < 30)
+            v = __float_as_uint(__ldcg(reinterpret_cast<const float *>(L.body + it.pos) + (lane < 26 ? 4 + lane : lane - 26)));
+    }
+    else if (lane < 26)
         v = __float_as_uint(__ldcg(D.cdl + 26ull * c + lane));
     else if (lane == 26)
         v = (unsigned int)__ldcg(D.gid + c);
@@ -1403,17 +1363,16 @@ __device__ __forceinline__ void claim_warp(BlockShared &B, int app, unsigned int
         m = __ballot_sync(0xffffffffu, nb && liquid_type(__ldcg(D.ctype + c + (nb ? nb_offset((int)lane, plane, my) : 0))));
         if (lane == 0) {
             st.fresh++;
-            B.X.rstat[app][it.pos] = m | kMaskGrown;
+            L.rec[it.pos].stat = m | kMaskGrown;
         }
     }
-    ActiveRec *rec = B.X.rec[app] + it.pos;
+    ActiveRec *rec = L.rec + it.pos;
     if ((m & kDirBits) == 0) {
         // no liquid neighbour: LCount stays 0 (src/CAupdate.cpp:722-725)
         if (lane == 0) {
             D.ctype[c] = kSolid;
             D.dl[c] = it.dl;
-            rec->cell = kTombstone;
-            rec->cdl_min = 0.0f;
+            rec->stat = kMaskTomb;
             st.dropped++;
             tombs++;
         }
@@ -1433,15 +1392,14 @@ __device__ __forceinline__ void claim_warp(BlockShared &B, int app, unsigned int
             const unsigned long long old = atomicMin(D.claim + t, key);
             D.ctype[t] = kTemporaryUpdate;
             B.claims[e] = claim_entry_of(dom, (int)lane, t) | ((unsigned long long)(i + 1) << kClaimantShift);
+            B.claim_pos[e] = it.pos;
             first = (old >> 32) != (key >> 32);
             if (first && dom != B.X.hot)
                 atomicAdd((unsigned long long *)&B.X.desc[dom].liquid_shard[lane & (kLiquidShards - 1)],
                           (unsigned long long)(-1ll));
         }
-        if (lane == 26)
-            B.claimants[i].h = (int)v;
-        else if (lane > 26 && lane < 30)
-            B.claimants[i].doc[lane - 27] = __uint_as_float(v);
+        if (lane >= 26 && lane < 30)
+            reinterpret_cast<unsigned int *>(&B.claimants[i])[lane - 26] = v;
         const unsigned int firsts = __popc(__ballot_sync(0xffffffffu, first && dom == B.X.hot));
         if (lane == 0) {
             st.claims += __popc(reach);
@@ -1459,38 +1417,146 @@ __device__ __forceinline__ void claim_warp(BlockShared &B, int app, unsigned int
     if (lane == 0) {
         st.rows++;
         rec->cdl_min = __uint_as_float(nm);
-        B.X.rmin2[app][it.pos] = ((unsigned long long)d1 << 32) | nm2;
+        L.min2[it.pos] = __uint_as_float(nm2);
+        L.dom[it.pos] = dom_word(dom, d1);
     }
 }
 
-// The block's claim step over its queue (all threads of the block call, after the block's growth).
-// kFew: with a warp per record when there are few (short chains; see claim_warp).
-template <bool kFew>
-__device__ __forceinline__ void block_claims(PoolState *P, BlockShared &B, int app, CycleStats &st,
-                                             unsigned int &tombs) {
+// Makes a warp's claims (src/CAupdate.cpp:336-352): the lowest index wins. Nothing waits for the outcome:
+// every claim is listed, in the block's own list, and the capture pass keeps the winner's. A claimed cell
+// reads TemporaryUpdate until its capture makes it active, as in the reference's capture
+// (src/CAupdate.cpp:343-352). A claim that finds an older epoch in the claim word is the first on its
+// cell, which is captured in this cycle: one liquid cell less, known before the capture pass. The hot
+// domain's are counted in shared memory.
+__device__ __forceinline__ void make_claims(PoolState *P, BlockShared &B, const ClaimLane &cl, unsigned int pos,
+                                            CycleStats &st) {
+    const unsigned int lane = threadIdx.x & 31, below = (1u << lane) - 1u;
+    unsigned int who[4], total = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        who[j] = __ballot_sync(0xffffffffu, (cl.reach >> j) & 1u);
+        total += __popc(who[j]);
+    }
+    if (total == 0)
+        return;
+    unsigned int base = 0;
+    if (lane == 0)
+        base = atomicAdd(&B.n_claims, total);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    unsigned int firsts = 0;
+    if (cl.reach) {
+        const DomainDesc &D = desc_of(B.X, cl.dom);
+        const int plane = D.mx * D.my, my = D.my;
+        const unsigned long long key = claim_key(D, cl.cell);
+        unsigned long long old[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            old[j] = key;
+            if ((cl.reach >> j) & 1u) {
+                const unsigned int t = (unsigned int)((long long)cl.cell + nb_offset(cl.dir0 + j, plane, my));
+                old[j] = atomicMin(D.claim + t, key);
+                D.ctype[t] = kTemporaryUpdate;
+                const unsigned int e = base + __popc(who[j] & below);
+                const unsigned long long v = claim_entry_of(cl.dom, cl.dir0 + j, t);
+                if (e < (unsigned int)kBlockClaims) {
+                    B.claims[e] = v;
+                    B.claim_pos[e] = pos;
+                }
+                else if (e - kBlockClaims < B.X.segment) {
+                    B.X.tgt[blockIdx.x * B.X.segment + (e - kBlockClaims)] = v;
+                }
+                else {
+                    atomicOr(&P->error, kErrListOverflow);
+                }
+            }
+            base += __popc(who[j]);
+        }
+        st.claims += __popc(cl.reach);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            firsts += (old[j] >> 32) != (key >> 32) ? 1u : 0u;
+        if (firsts && cl.dom != B.X.hot) {
+            atomicAdd((unsigned long long *)&B.X.desc[cl.dom].liquid_shard[lane & (kLiquidShards - 1)],
+                      (unsigned long long)(-(long long)firsts));
+            firsts = 0;
+        }
+    }
+    firsts = __reduce_add_sync(0xffffffffu, firsts);
+    if (lane == 0 && firsts)
+        atomicAdd(&B.n_first, firsts);
+}
+
+// The block's claim step over its queue (all threads of the block call, after the block's growth). In the
+// families for shorter lists a warp per record where there are no more of them than warps, else eight lanes per
+// record, consecutive records on different warps. Without it a record per lane: at 512^3 (270 flagged
+// records per block and cycle) 39.0 us per cycle against 45.2 with eight lanes, whose four rounds wait for
+// memory in turn; at 256^3 (67) eight lanes take 18.95 against 20.0.
+template <int kFamily>
+__device__ __forceinline__ void block_claims(PoolState *P, BlockShared &B, int app, CycleStats &st, unsigned int &tombs) {
     __syncthreads();
     const unsigned int n = min(B.n_items, (unsigned int)kBlockQueue);
     if (n == 0)
         return;
-    const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (kFew && n <= (unsigned int)(kBlock / 32)) {
+    constexpr unsigned int kWarps = kBlock / 32;
+    const unsigned int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+    if (kFamily != kLongList && n <= kWarps) {
         if (warp < n)
             claim_warp(B, app, warp, st, tombs);
-        return;
     }
-    for (unsigned int k0 = warp * 32; k0 < n; k0 += kBlock) {
-        const unsigned int k = k0 + lane;
-        unsigned int reach = 0, dom = 0, cell = 0;
-        if (k < n) {
-            const ClaimItem it = B.items[k];
-            reach = claim_record<false>(B.X, app, it, st, tombs);
-            dom = it.dom;
-            cell = it.cell;
+    else if (kFamily != kLongList) {
+        for (unsigned int k0 = warp; k0 < n; k0 += 4 * kWarps) {
+            const unsigned int k = k0 + lane / 8 * kWarps;
+            const bool on = k < n;
+            ClaimItem it{};
+            if (on)
+                it = B.items[k];
+            const ClaimLane cl = claim_group(B.X, app, it, on, st, tombs);
+            make_claims(P, B, cl, it.pos, st);
         }
-        push_claims(P, B, reach, dom, cell);
     }
-    __syncthreads();
-    issue_claims(B, 0);
+    else {
+        for (unsigned int k0 = warp * 32; k0 < n; k0 += kBlock) {
+            const unsigned int k = k0 + lane;
+            unsigned int reach = 0, cell = 0;
+            ClaimItem it{};
+            if (k < n) {
+                it = B.items[k];
+                reach = claim_record(B.X, app, it, cell, st, tombs);
+            }
+            push_claims(P, B, reach, it.dom, cell, it.pos);
+        }
+        __syncthreads();
+        issue_claims(B, 0);
+    }
+}
+
+// The bodies of a warp's surviving records (one per lane, `moves`) to their new positions: a body at a
+// time by eight lanes, four in flight; from the cell's own fields where the record had none.
+__device__ __forceinline__ void move_bodies(const RecordList &from, const RecordList &to, const PassCtx &X, bool moves,
+                                            unsigned int i, unsigned int pos, unsigned int cell, unsigned int dom) {
+    const unsigned int lane = threadIdx.x & 31;
+    unsigned int todo = __ballot_sync(0xffffffffu, moves && i < from.body_cap);
+    const unsigned int gather = __ballot_sync(0xffffffffu, moves && i >= from.body_cap);
+    while (todo) {
+        // the lane's own body: the (lane / 8)-th of the next four
+        unsigned int pick = todo;
+        for (unsigned int k = 0; k < lane / 8 && pick; k++)
+            pick &= pick - 1;
+        const int src = pick ? __ffs(pick) - 1 : 0;
+        const unsigned int si = __shfl_sync(0xffffffffu, i, src), sp = __shfl_sync(0xffffffffu, pos, src);
+        if (pick)
+            reinterpret_cast<float4 *>(to.body + sp)[lane & 7] = __ldcg(reinterpret_cast<const float4 *>(from.body + si) + (lane & 7));
+        for (int k = 0; k < 4 && todo; k++)
+            todo &= todo - 1;
+    }
+    if (gather && moves && i >= from.body_cap) {
+        const DomainDesc &D = desc_of(X, dom);
+        RecordBody &b = to.body[pos];
+        body_head(b) = make_float4(__int_as_float(__ldcg(D.gid + cell)), __ldcg(D.doc + 3ull * cell), __ldcg(D.doc + 3ull * cell + 1),
+                             __ldcg(D.doc + 3ull * cell + 2));
+        for (int l = 0; l < 26; l++)
+            b.cdl[l] = __ldcg(D.cdl + 26ull * cell + l);
+    }
 }
 
 // Growth step of a compaction cycle: the survivors are written to the other list (rare; kept out of
@@ -1499,60 +1565,54 @@ __device__ __noinline__ void compact_pass(PoolState *P, const PassCtx &X, int cu
                                          unsigned long long nw, unsigned long long n, const DomainDyn &dyn,
                                          CycleStats &st, BlockShared *B) {
     const unsigned int lane = threadIdx.x & 31;
-    const ActiveRec *in = X.rec[cur];
-    const unsigned int *in_dom = X.rdom[cur];
-    const unsigned int *in_stat = X.rstat[cur];
-    const unsigned long long *in_min2 = X.rmin2[cur];
     const int nxt = cur ^ 1;
-    ActiveRec *out = X.rec[nxt];
-    unsigned int *out_dom = X.rdom[nxt];
-    unsigned int *out_stat = X.rstat[nxt];
-    unsigned long long *out_min2 = X.rmin2[nxt];
+    const RecordList &from = X.list[cur], &to = X.list[nxt];
     const unsigned long long groups = (n + 31) / 32;
     for (unsigned long long g = gw; g < groups; g += nw) {
-        unsigned long long i = g * 32 + lane;
-        bool keep = false;
-        ActiveRec r;
-        r.cell = kTombstone;
-        unsigned int dom = 0, m = 0;
-        unsigned long long mn2 = kNoMin2;
+        const unsigned long long i = g * 32 + lane;
+        bool keep = false, flag = false;
+        ActiveRec r{};
+        unsigned int cell = 0, word = 0, dom = 0;
+        float mn2 = 0.0f;
         if (i < n) {
-            const int4 v = __ldcg(reinterpret_cast<const int4 *>(in + i));
+            const int4 v = __ldcg(reinterpret_cast<const int4 *>(from.rec + i));
             r = *reinterpret_cast<const ActiveRec *>(&v);
-            dom = __ldcg(in_dom + i);
-            m = __ldcg(in_stat + i) & ~kMaskKeep;
-            mn2 = __ldcg(in_min2 + i);
-            if (r.cell != kTombstone) {
-                if (m & kMaskNuc)
-                    m = drop_nucleated(desc_of(X, dom), r.cell, m);
+            cell = __ldcg(from.cell + i);
+            word = __ldcg(from.dom + i);
+            dom = word_dom(word);
+            mn2 = __ldcg(from.min2 + i);
+            if (!(r.stat & kMaskTomb)) {
+                r.stat &= ~kMaskKeep;
+                if (r.stat & kMaskNuc)
+                    r.stat = drop_nucleated(desc_of(X, dom), cell, r.stat);
                 const GrowView view = dom == X.hot ? hot_view(X, dyn) : grow_view(X.desc[dom]);
-                double inc;
-                bool ok;
-                load_growth(view, r, inc, ok, X.extras);
-                const int a = grow_record(X, view, dom, r, m, inc, ok, effective_min(r, m, mn2), st);
-                keep = a != 0;
-                if (a == 2)
-                    m |= kMaskGrown;
+                const double inc = load_growth(view, desc_of(X, dom), cell, r.cts, X.extras);
+                const GrowAction a = grow_record(X, view.cycle, cell, dom, r, r.stat, inc,
+                                                 effective_min(r.cdl_min, mn2, r.stat, word), st);
+                keep = a != kDrop;
+                flag = a == kFlag;
+                if (a >= kGrown)
+                    r.stat |= kMaskGrown;
                 if (!keep)
                     st.dropped++;
             }
         }
         const unsigned long long pos = warp_reserve_n(&P->cnt[nxt], X.capacity, &P->error, keep ? 1u : 0u);
-        const bool placed = keep && pos != ULLONG_MAX;
-        if (placed) {
-            out[pos] = r;
-            out_dom[pos] = dom;
-            out_stat[pos] = m;
-            out_min2[pos] = mn2;
-            desc_of(X, dom).pos[r.cell] = (unsigned int)pos;
+        if (!(keep && pos != ULLONG_MAX))
+            flag = false;
+        else {
+            to.rec[pos] = r;
+            to.cell[pos] = cell;
+            to.dom[pos] = word;
+            to.min2[pos] = mn2;
+            desc_of(X, dom).pos[cell] = (unsigned int)pos;
         }
-        const bool flag = placed && __float_as_uint(r.cdl_min) == kNeedsClaim;
-        unsigned long long idx = pos;
+        move_bodies(from, to, X, keep && pos < to.body_cap, (unsigned int)i, (unsigned int)pos, cell, dom);
+        const unsigned int idx = (unsigned int)pos;
         if (B)
-            block_queue_flagged<1>(P, *B, (unsigned int)(gw % kShards), flag ? 1u : 0u, flag ? 1u : 0u, &idx, &r,
-                                   &dom, &m);
+            block_queue_flagged<1>(P, *B, (unsigned int)(gw % kShards), flag ? 1u : 0u, &idx, &r, &word);
         else
-            queue_flagged<1>(P, (unsigned int)(gw % kShards), flag ? 1u : 0u, flag ? 1u : 0u, &idx, &r, &dom, &m);
+            queue_flagged<1>(P, (unsigned int)(gw % kShards), flag ? 1u : 0u, flag ? 1u : 0u, &idx, &r, &word);
     }
 }
 
@@ -1560,102 +1620,183 @@ __device__ __noinline__ void compact_pass(PoolState *P, const PassCtx &X, int cu
 // group g to warp g % (number of warps of the grid), consecutive warps on different blocks: the
 // records appended by the last capture pass, which all need a fresh mask and claims, spread over
 // every SM. No block-wide synchronisation.
-// Growth of the list's groups of 32 records, kBatch groups per warp in flight (see grow_pass).
-template <int kBatch, bool kOwnClaims>
+// The position of a dropped record, for one of the block's later captures.
+__device__ __forceinline__ void push_free(BlockShared &B, unsigned int pos) {
+    const unsigned int e = atomicAdd(&B.n_free, 1u);
+    if (e < (unsigned int)kFreeSlots)
+        B.free_slots[e] = pos;
+}
+
+// Growth step of one record by one lane, every case of it: other domains, per-cell growth extras, cycle
+// jumps, records that leave the list, masks to clear. Returns what became of it, its list entry updated.
+struct GrowResult {
+    GrowAction action;
+    unsigned int stat;
+    float dl;
+};
+template <bool kOwnClaims>
+__device__ __forceinline__ GrowResult grow_any(const PassCtx &X, BlockShared *B, const DomainDyn &dyn, int cur, unsigned int idx,
+                                             ActiveRec r, unsigned int cell, unsigned int word, float min2, CycleStats &st) {
+    const RecordList &L = X.list[cur];
+    const unsigned int dom = word_dom(word), before = r.stat;
+    // the neighbour verdict of the previous cycle does not carry over
+    r.stat &= ~kMaskKeep;
+    if (r.stat & kMaskNuc)
+        r.stat = drop_nucleated(desc_of(X, dom), cell, r.stat);
+    const GrowView v = dom == X.hot ? hot_view(X, dyn) : grow_view(X.desc[dom]);
+    const double inc = load_growth(v, desc_of(X, dom), cell, r.cts, X.extras);
+    const GrowAction a =
+        grow_record(X, v.cycle, cell, dom, r, r.stat, inc, effective_min(r.cdl_min, min2, r.stat, word), st);
+    if (a == kDrop) {
+        L.rec[idx].stat = kMaskTomb;
+        if (kOwnClaims)
+            push_free(*B, idx);
+        st.dropped++;
+        return GrowResult{a, kMaskTomb, r.dl};
+    }
+    if (a >= kGrown) {
+        r.stat |= kMaskGrown;
+        L.rec[idx].dl = r.dl;
+    }
+    if (r.stat != before)
+        L.rec[idx].stat = r.stat;
+    return GrowResult{a, r.stat, r.dl};
+}
+// The same out of line: one copy for the groups of a batch, which reach it rarely.
+template <bool kOwnClaims>
+__device__ __noinline__ GrowResult grow_slow(const PassCtx &X, BlockShared *B, DomainDyn dyn, int cur, unsigned int idx,
+                                             ActiveRec r, unsigned int cell, unsigned int word, float min2, CycleStats &st) {
+    return grow_any<kOwnClaims>(X, B, dyn, cur, idx, r, cell, word, min2, st);
+}
+
+// Growth of the list's groups of 32 records, kBatch groups per warp in flight (see grow_pass). A record
+// costs 24 bytes read (its 16-byte vector with the status word, its domain word and the second bound)
+// and 4 written. Nearly every record of the hot domain takes the short path below (about 70 instead of
+// 250 instructions per group of 32): eligible or waiting, with liquid neighbours. The others go through
+// grow_slow, lane by lane. kCells (the shapes for short lists, where a round of loads more shows): the
+// cell comes with the record, for 4 bytes more, so that the slow path does not wait for it and the short
+// one takes domains with per-cell growth extras, jumps and zero UndercoolingChange too; without it the
+// increment of a short-path record is one entry of the domain's table.
+template <int kBatch, bool kOwnClaims, bool kCells>
 __device__ __forceinline__ void grow_groups(PoolState *P, const PassCtx &X, BlockShared *B, const DomainDyn &dyn, int cur,
-                                            unsigned long long n, unsigned long long gw, unsigned long long nw,
+                                            unsigned int n, unsigned int gw, unsigned int nw, bool first_pass,
                                             CycleStats &st, unsigned int &tombs, bool &busy, int &min_cts) {
-    const unsigned int lane = threadIdx.x & 31, shard = (unsigned int)(gw % kShards), hot = X.hot;
-    ActiveRec *in = X.rec[cur];
-    const unsigned int *in_dom = X.rdom[cur];
-    unsigned int *in_stat = X.rstat[cur];
-    const unsigned long long *in_min2 = X.rmin2[cur];
-    const bool extras = X.extras;
-    const unsigned long long groups = (n + 31) / 32;
-    // the growth fields of the hot domain held in registers
+    const unsigned int lane = threadIdx.x & 31, shard = gw % kShards;
+    const RecordList &L = X.list[cur];
+    ActiveRec *const in = L.rec;
+    const unsigned int *const in_dom = L.dom, *const in_cell = L.cell;
+    const float *const in_min2 = L.min2;
+    const unsigned int groups = (n + 31) / 32;
+    // the growth fields of the hot domain in registers; without the short path no record matches `hot`
     const GrowView v0 = hot_view(X, dyn);
+    const bool extras = X.extras, plain = !extras && !v0.jumps && !v0.zero_du;
+    const unsigned int hot = v0.cycle != kDoneCycle && (kCells || plain) ? X.hot : 0xffffffffu;
+    const int cycle = v0.cycle;
+    const double *const table = v0.growth + v0.e_cycle;
     // records are updated in place; dropped ones become tombstones
-    for (unsigned long long g0 = gw; g0 < groups; g0 += kBatch * nw) {
+    for (unsigned int g0 = gw; g0 < groups; g0 += kBatch * nw) {
         ActiveRec r[kBatch];
-        unsigned int dom[kBatch], m[kBatch];
-        unsigned long long idx[kBatch], mn2[kBatch];
+        unsigned int word[kBatch], cell[kBatch], idx[kBatch];
+        float min2[kBatch];
         double inc[kBatch];
-        bool ok[kBatch];
 #pragma unroll
         for (int q = 0; q < kBatch; q++) {
-            idx[q] = (g0 + (unsigned long long)q * nw) * 32 + lane;
-            r[q].cell = kTombstone;
-            dom[q] = 0;
-            m[q] = 0;
-            mn2[q] = kNoMin2;
-            if (idx[q] < n) {
+            idx[q] = (g0 + q * nw) * 32 + lane;
+            r[q].stat = kMaskTomb;
+            if (g0 + q * nw < groups && idx[q] < n) {
                 // streamed once per cycle: through L2 only
                 const int4 v = __ldcg(reinterpret_cast<const int4 *>(in + idx[q]));
                 r[q] = *reinterpret_cast<const ActiveRec *>(&v);
-                dom[q] = __ldcg(in_dom + idx[q]);
-                m[q] = __ldcg(in_stat + idx[q]);
-                mn2[q] = __ldcg(in_min2 + idx[q]);
+                word[q] = __ldcg(in_dom + idx[q]);
+                min2[q] = __ldcg(in_min2 + idx[q]);
+                if (kCells)
+                    cell[q] = __ldcg(in_cell + idx[q]);
             }
         }
+        // the short path: grows, or waits for its CritTimeStep
+        unsigned int grows = 0, waits = 0;
 #pragma unroll
         for (int q = 0; q < kBatch; q++) {
+            const unsigned int m = r[q].stat;
             inc[q] = 0.0;
-            ok[q] = true;
-            if (r[q].cell != kTombstone) {
-                if (m[q] & (kMaskKeep | kMaskNuc)) {
-                    // the neighbour verdict of the previous cycle does not carry over
-                    m[q] &= ~kMaskKeep;
-                    if (m[q] & kMaskNuc)
-                        m[q] = drop_nucleated(desc_of(X, dom[q]), r[q].cell, m[q]);
-                    in_stat[idx[q]] = m[q];
+            if (!(m & (kMaskTomb | kMaskDead | kMaskNuc | kMaskFresh)) && (m & kDirBits) && word_dom(word[q]) == hot) {
+                if (cycle > r[q].cts) {
+                    if (kCells && !plain) {
+                        inc[q] = load_growth(v0, X.hot_desc, cell[q], r[q].cts, extras);
+                        if (inc[q] >= 0.0)
+                            grows |= 1u << q;
+                    }
+                    else {
+                        const int from = max(r[q].cts, 0);
+                        if ((unsigned int)(v0.e_cycle - from) < (unsigned int)v0.growth_len) {
+                            grows |= 1u << q;
+                            inc[q] = __ldg(table - from);
+                        }
+                    }
                 }
-                if (dom[q] == hot)
-                    load_growth(v0, r[q], inc[q], ok[q], extras);
-                else
-                    load_growth(grow_view(X.desc[dom[q]]), r[q], inc[q], ok[q], extras);
+                else if (!(m & kMaskKeep)) {
+                    waits |= 1u << q;
+                    min_cts = min(min_cts, r[q].cts);
+                }
             }
         }
         unsigned int flagged = 0;
 #pragma unroll
         for (int q = 0; q < kBatch; q++) {
-            if (r[q].cell == kTombstone)
-                continue;
-            const float eff_min = effective_min(r[q], m[q], mn2[q]);
-            const int a = dom[q] == hot
-                              ? grow_record(X, v0, dom[q], r[q], m[q], inc[q], ok[q], eff_min, st)
-                              : grow_record(X, grow_view(X.desc[dom[q]]), dom[q], r[q], m[q], inc[q], ok[q], eff_min, st);
-            if (a == 1)
-                min_cts = min(min_cts, r[q].cts);
-            else
-                busy = true;
-            if (a == 0) {
-                in[idx[q]].cell = kTombstone;
-                in[idx[q]].cdl_min = 0.0f;
-                st.dropped++;
-                tombs++;
-            }
-            else if (a == 2) {
-                *reinterpret_cast<float2 *>(&in[idx[q]].dl) = make_float2(r[q].dl, r[q].cdl_min);
-                if (!(m[q] & kMaskGrown)) {
-                    m[q] |= kMaskGrown;
-                    in_stat[idx[q]] = m[q];
-                }
-                if (__float_as_uint(r[q].cdl_min) == kNeedsClaim)
+            if ((grows >> q) & 1u) {
+                const unsigned int m = (r[q].stat & ~kMaskKeep) | kMaskGrown;
+                r[q].dl = (float)((double)r[q].dl + inc[q]);
+                in[idx[q]].dl = r[q].dl;
+                if (m != r[q].stat)
+                    in[idx[q]].stat = m;
+                r[q].stat = m;
+                if (r[q].dl >= effective_min(r[q].cdl_min, min2[q], m, word[q])) {
                     flagged |= 1u << q;
+                    if (!kCells && idx[q] < L.body_cap) // the claim step's line, on its way to L2 meanwhile
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(L.body + idx[q]));
+                }
             }
         }
+        st.listed += __popc(grows | waits);
+        st.grown += __popc(grows);
+        st.flagged += __popc(flagged);
+        busy = busy || grows != 0;
+#pragma unroll
+        for (int q = 0; q < kBatch; q++) {
+            if (((grows | waits) >> q) & 1u)
+                continue;
+            if (r[q].stat & kMaskTomb) {
+                if (kOwnClaims && first_pass && g0 + q * nw < groups && idx[q] < n)
+                    push_free(*B, idx[q]);
+                continue;
+            }
+            const unsigned int c = kCells ? cell[q] : __ldcg(in_cell + idx[q]);
+            const GrowResult a = kBatch == 1 ? grow_any<kOwnClaims>(X, B, dyn, cur, idx[q], r[q], c, word[q], min2[q], st)
+                                             : grow_slow<kOwnClaims>(X, B, dyn, cur, idx[q], r[q], c, word[q], min2[q], st);
+            r[q].stat = a.stat;
+            r[q].dl = a.dl;
+            if (a.action == kWait) {
+                min_cts = min(min_cts, r[q].cts);
+                continue;
+            }
+            busy = true;
+            if (a.action == kDrop)
+                tombs++;
+            else if (a.action == kFlag)
+                flagged |= 1u << q;
+        }
         if (kOwnClaims)
-            block_queue_flagged<kBatch>(P, *B, shard, __popc(flagged), flagged, idx, r, dom, m);
+            block_queue_flagged<kBatch>(P, *B, shard, flagged, idx, r, word);
         else
-            queue_flagged<kBatch>(P, shard, __popc(flagged), flagged, idx, r, dom, m);
+            queue_flagged<kBatch>(P, shard, __popc(flagged), flagged, idx, r, word);
     }
 }
 
 // With kOwnClaims (B given) the block's flagged records go to its queue and their claim steps follow
 // here. cur is the list to read, n its length; with `compact` the survivors go to the other list.
-template <int kBatch, bool kOwnClaims, bool kFew>
+template <int kBatch, bool kOwnClaims, int kFamily>
 __device__ void grow_pass(PoolState *P, PassCtx &X, BlockShared *B, const DomainDyn &dyn, int cur, unsigned long long n,
-                          bool compact, CycleStats &st, unsigned int &tombs) {
+                          bool compact, bool first_pass, CycleStats &st, unsigned int &tombs) {
     const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned long long nw = (unsigned long long)gridDim.x * (kBlock / 32);
     const unsigned long long gw = (unsigned long long)warp * gridDim.x + blockIdx.x;
@@ -1669,7 +1810,7 @@ __device__ void grow_pass(PoolState *P, PassCtx &X, BlockShared *B, const Domain
         if (kOwnClaims) {
             B->busy = 1;
             unsigned int claim_tombs = 0; // a compacted list starts without dropped records
-            block_claims<kFew>(P, *B, cur ^ 1, st, claim_tombs);
+            block_claims<kFamily>(P, *B, cur ^ 1, st, claim_tombs);
         }
         return;
     }
@@ -1677,10 +1818,12 @@ __device__ void grow_pass(PoolState *P, PassCtx &X, BlockShared *B, const Domain
     bool busy = false;
     int min_cts = INT_MAX;
     // one group per warp at most: the shorter code for one group is the shorter chain
-    if (kFew && (n + 31) / 32 <= nw)
-        grow_groups<1, kOwnClaims>(P, X, B, dyn, cur, n, gw, nw, st, tombs, busy, min_cts);
+    if (kFamily != kLongList && (n + 31) / 32 <= nw)
+        grow_groups<1, kOwnClaims, true>(P, X, B, dyn, cur, (unsigned int)n, (unsigned int)gw, (unsigned int)nw, first_pass, st,
+                                   tombs, busy, min_cts);
     else
-        grow_groups<kBatch, kOwnClaims>(P, X, B, dyn, cur, n, gw, nw, st, tombs, busy, min_cts);
+        grow_groups<kBatch, kOwnClaims, kFamily != kLongList>(P, X, B, dyn, cur, (unsigned int)n, (unsigned int)gw, (unsigned int)nw, first_pass,
+                                        st, tombs, busy, min_cts);
     if (kOwnClaims) {
         busy = __any_sync(0xffffffffu, busy);
         min_cts = __reduce_min_sync(0xffffffffu, min_cts);
@@ -1690,7 +1833,7 @@ __device__ void grow_pass(PoolState *P, PassCtx &X, BlockShared *B, const Domain
             else if (min_cts != INT_MAX)
                 atomicMin(&B->min_cts, min_cts);
         }
-        block_claims<kFew>(P, *B, cur, st, tombs);
+        block_claims<kFamily>(P, *B, cur, st, tombs);
     }
 }
 
@@ -1732,8 +1875,9 @@ __device__ __forceinline__ unsigned long long shard_entry(const unsigned long lo
     return (unsigned long long)lo * cap + (k - pre[lo]);
 }
 
-// One queue entry per thread, consecutive warps on different blocks; every claim is listed, in the
-// block's own list (B, persistent kernel) or the sharded global one.
+// The claim steps of the global queue, eight lanes per entry, consecutive warps on different blocks;
+// every claim is listed, in the block's own list (B, persistent kernel) or, as (domain << 37) |
+// (direction << 32) | claimed cell, in the sharded global one.
 template <bool kOwnClaims>
 __device__ void claim_pass(PoolState *P, PassCtx &X, BlockShared *B, int app, CycleStats &st, unsigned int &tombs) {
     __shared__ unsigned long long s_pre[kShards + 1];
@@ -1743,186 +1887,318 @@ __device__ void claim_pass(PoolState *P, PassCtx &X, BlockShared *B, int app, Cy
     const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned long long nw = (unsigned long long)gridDim.x * (kBlock / 32);
     const unsigned long long gw = (unsigned long long)warp * gridDim.x + blockIdx.x;
-    const unsigned int listed = kOwnClaims ? claim_count(*B) : 0u; // claims of the block's own queue
-    if (kOwnClaims)
-        __syncthreads();
-    for (unsigned long long k0 = gw * 32; k0 < nq; k0 += nw * 32) {
-        const unsigned long long k = k0 + lane;
-        unsigned int reach = 0, dom = 0, cell = 0;
-        if (k < nq) {
+    for (unsigned long long k0 = gw * 4; k0 < nq; k0 += nw * 4) {
+        const unsigned long long k = k0 + lane / 8;
+        const bool on = k < nq;
+        ClaimItem it{};
+        if (on) {
             const unsigned long long e = shard_entry(s_pre, cap, k);
-            reach = claim_entry<!kOwnClaims>(P, X, app, e, st, tombs);
-            dom = __ldcg(P->qdom + e);
-            cell = __ldcg(P->qcell + e);
+            it = ClaimItem{__ldcg(P->qpos + e), __ldcg(P->qdom + e), __ldcg(P->qmask + e), __ldcg(P->qdl + e)};
         }
-        if (kOwnClaims)
-            push_claims(P, *B, reach, dom, cell);
-        else
-            list_claims(P, (unsigned int)(gw % kShards), reach, dom, cell);
-    }
-    if (kOwnClaims) {
-        __syncthreads();
-        issue_claims(*B, listed);
-    }
-}
-
-// Captures cell w.t by its winning claimant with a group of kLanes lanes (on: the group has a winner;
-// every group of the block calls): the new octahedron, the masks of the captured cell's active
-// neighbours and their solidification re-checks, and the new record in slot slot_of() of list `app`
-// (ULLONG_MAX: none). Records of the cells active at the start of the cycle lie below base. A cell of
-// type also_liquid (a mark of the cycle after next, or kLiquid) is liquid in the next cycle.
-// won() says whether the claim has won, after the neighbours' loads have gone out.
-template <int kLanes, class Won, class SlotOf>
-__device__ __forceinline__ void capture_group(const PassCtx &X, int app, unsigned long long base, const WinItem &w,
-                                              bool on, int8_t also_liquid, Won &&won, SlotOf &&slot_of, CycleStats &st) {
-    constexpr int kPer = (26 + kLanes - 1) / kLanes;
-    const int lane = threadIdx.x & 31, grp = lane / kLanes, sub = lane % kLanes;
-    const unsigned int group = (kLanes == 32 ? 0xffffffffu : ((1u << kLanes) - 1u)) << (grp * kLanes);
-    const unsigned int t = w.t, c = w.c, dom = w.dom_dir >> 5;
-    const int l = (int)(w.dom_dir & 31u);
-    const DomainDesc &D = desc_of(X, dom);
-    unsigned int *rs = X.rstat[app];
-    unsigned int a[kPer], p[kPer], old[kPer];
-    int8_t ct[kPer];
-    bool act[kPer];
-    unsigned int liq = 0, d1 = 0xffffffffu;
-    float mn = __int_as_float(0x7f800000), mn2 = mn, new_dl = 0.0f;
-    if (on) {
-        // Lane `sub` takes the neighbour slots sub, sub + kLanes, ... (slot_dir): a load instruction's
-        // lanes read neighbours in few rows of three consecutive cells.
-        const int plane = D.mx * D.my, my = D.my;
-        int tx, ty, tz;
-        cell_coords(D, t, tx, ty, tz);
-        const unsigned int valid = neighbour_mask(D, tx, ty, tz);
-#pragma unroll
-        for (int k = 0; k < kPer; k++) {
-            const int ln = slot_dir(sub + k * kLanes);
-            act[k] = ln < 26 && (valid & (1u << ln));
-            a[k] = (unsigned int)((long long)t + (act[k] ? nb_offset(ln, plane, my) : 0));
-            ct[k] = __ldcg(D.ctype + a[k]);
-            p[k] = __ldcg(D.pos + a[k]);
-        }
-        on = won();
-    }
-    if (on) {
-        // The captured cell's liquid-neighbour mask, as its first claim step would build it from the
-        // neighbour types at the start of a later cycle: the neighbours still liquid (a neighbour
-        // claimed in this cycle reads TemporaryUpdate, or active once captured). Later captures and
-        // nucleations clear bits of it as of every other record's (it lies below later cycles' base).
-#pragma unroll
-        for (int k = 0; k < kPer; k++)
-            if (act[k] && (ct[k] == kLiquid || ct[k] == also_liquid))
-                liq |= 1u << slot_dir(sub + k * kLanes);
-        if (kLanes == 32) {
-            liq = __reduce_or_sync(0xffffffffu, liq);
+        const ClaimLane cl = claim_group(X, app, it, on, st, tombs);
+        if (kOwnClaims) {
+            make_claims(P, *B, cl, it.pos, st);
         }
         else {
-#pragma unroll
-            for (int o = kLanes / 2; o; o >>= 1)
-                liq |= __shfl_xor_sync(group, liq, o);
-        }
-        // Serial order (src/CAupdate.cpp:333-334, 722-725): active cell a saw the captured cell t
-        // as liquid iff t's capturer c does not precede a. a keeps a liquid neighbour iff it has an
-        // unclaimed one (a set mask bit that nobody clears) or a claimed one with c >= a. Every
-        // claimed liquid neighbour clears its own bit exactly once, so the update that clears the
-        // last direction bit sees the final verdict: KEEP is always set before the clear of the
-        // same update, and an update's two atomics reach the word in program order. Only records of
-        // cells active at the start of the cycle (positions below base) take part: a neighbour
-        // captured in this same cycle reads as liquid, or has no record below base.
-#pragma unroll
-        for (int k = 0; k < kPer; k++)
-            act[k] = act[k] && ct[k] == kActive && p[k] < base;
-#pragma unroll
-        for (int k = 0; k < kPer; k++)
-            if (act[k] && c >= a[k])
-                atomicOr(rs + p[k], kMaskKeep);
-#pragma unroll
-        for (int k = 0; k < kPer; k++) {
-            old[k] = 0;
-            if (act[k])
-                old[k] = atomicAnd(rs + p[k], ~(1u << nb_opp(slot_dir(sub + k * kLanes))));
-        }
-        // The new record's cached minimum critical length over its liquid neighbours, with its
-        // direction and the second-smallest (the state a claim step leaves), so that its first claim
-        // step runs only once its DiagonalLength reaches a liquid neighbour.
-        new_dl = capture_cell<kLanes>(D, c, t, l, sub, w.h, w.docx, w.docy, w.docz, liq, mn, d1, mn2);
-        if (kLanes == 32) {
-            // one direction per lane (lane = direction), lengths not negative: by their bits
-            const unsigned int b = __float_as_uint(mn);
-            const unsigned int nm = __reduce_min_sync(0xffffffffu, b);
-            const unsigned int holds = __ballot_sync(0xffffffffu, b == nm);
-            d1 = nm == 0x7f800000u ? 0xffffffffu : (unsigned int)__ffs(holds) - 1u;
-            mn = __uint_as_float(nm);
-            mn2 = __uint_as_float(__reduce_min_sync(0xffffffffu, (unsigned int)lane == d1 ? 0x7f800000u : b));
-        }
-        else {
-#pragma unroll
-            for (int o = kLanes / 2; o; o >>= 1) {
-                const float omn = __shfl_xor_sync(group, mn, o), omn2 = __shfl_xor_sync(group, mn2, o);
-                const unsigned int od1 = __shfl_xor_sync(group, d1, o);
-                if (omn < mn || (omn == mn && od1 < d1)) {
-                    mn2 = fminf(omn2, mn);
-                    mn = omn;
-                    d1 = od1;
+            const unsigned int shard = (unsigned int)(gw % kShards);
+            unsigned long long pos = warp_reserve_n(&P->tcnt_s[shard].v, cap, &P->error, __popc(cl.reach));
+            if (cl.reach) {
+                const DomainDesc &D = desc_of(X, cl.dom);
+                const unsigned long long key = claim_key(D, cl.cell);
+                for (unsigned int bits = cl.reach; bits; bits &= bits - 1) {
+                    const int l = cl.dir0 + __ffs(bits) - 1;
+                    const unsigned int t = (unsigned int)((long long)cl.cell + nb_offset(l, D.mx * D.my, D.my));
+                    atomicMin(D.claim + t, key);
+                    D.ctype[t] = kTemporaryUpdate;
+                    if (pos != ULLONG_MAX)
+                        P->tgt[shard * cap + pos++] = claim_entry_of(cl.dom, l, t);
                 }
-                else {
-                    mn2 = fminf(mn2, omn);
-                }
+                st.claims += __popc(cl.reach);
             }
         }
     }
-    const unsigned long long slot = slot_of();
-    if (!on)
-        return;
-    if (sub == 0) {
-        if (slot != ULLONG_MAX) {
-            ActiveRec r;
-            r.cell = t;
-            r.dl = new_dl;
-            r.cdl_min = mn;
-            r.cts = w.cts;
-            X.rec[app][slot] = r;
-            X.rdom[app][slot] = dom;
-            rs[slot] = liq;
-            X.rmin2[app][slot] = ((unsigned long long)d1 << 32) | __float_as_uint(mn2);
-            D.pos[t] = (unsigned int)slot;
-        }
-        // read as active by the growth pass of the next cycle, after the octahedron is written
-        D.ctype[t] = kActive;
-        st.captured++;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Capture of liquid cell t by active cell c (src/CAupdate.cpp:353-563, 713-717), in three parts: the
+// geometry (one thread per capture), the neighbours of the captured cell, and the critical lengths.
+
+// The new octahedron, from the claimant's GrainID and centre, with the reference's expressions.
+__device__ __forceinline__ void capture_geometry(const DomainDesc &D, unsigned int t, int h, float docx, float docy,
+                                                 float docz, CaptureItem &out) {
+    int rx, ry, rz;
+    cell_coords(D, t, rx, ry, rz);
+    int ori = (abs(h) - 1) % 10000;
+    if (ori < 0)
+        ori += 10000;
+    const float *g = D.guv + 9 * ori;
+    const float g0 = g[0], g1 = g[1], g2 = g[2], g3 = g[3], g4 = g[4], g5 = g[5], g6 = g[6], g7 = g[7], g8 = g[8];
+    const double cxold = docx, cyold = docy, czold = docz;
+    const double xp = (rx + D.xoff) + 0.5, yp = (ry + D.yoff) + 0.5, zp = rz + 0.5;
+    const double x0 = xp - cxold, y0 = yp - cyold, z0 = zp - czold;
+    const double mag0 = sqrtf((float)(x0 * x0 + y0 * y0 + z0 * z0));
+    // Angle1..3 (src/CAupdate.cpp:382-393) matter by their signs alone: that of the dot product, without
+    // the division by the distance, unless the quotient could vanish
+    const auto negative = [&](float a, float b, float c) {
+        const double dot = a * x0 + b * y0 + c * z0;
+        return (dot < -1e-200 && mag0 < 1e30) || dot / mag0 < 0;
+    };
+    const float s1 = negative(g0, g1, g2) ? 1.0f : -1.0f, s2 = negative(g3, g4, g5) ? 1.0f : -1.0f,
+                s3 = negative(g6, g7, g8) ? 1.0f : -1.0f;
+    double Diag1X = g0 * s1, Diag1Y = g1 * s1, Diag1Z = g2 * s1;
+    double Diag2X = g3 * s2, Diag2Y = g4 * s2, Diag2Z = g5 * s2;
+    double Diag3X = g6 * s3, Diag3Y = g7 * s3, Diag3Z = g8 * s3;
+    double U1x = Diag2X - Diag1X, U1y = Diag2Y - Diag1Y, U1z = Diag2Z - Diag1Z;
+    double U2x = Diag3X - Diag1X, U2y = Diag3Y - Diag1Y, U2z = Diag3Z - Diag1Z;
+    double UUx = U1y * U2z - U1z * U2y;
+    double UUy = U1z * U2x - U1x * U2z;
+    double UUz = U1x * U2y - U1y * U2x;
+    double NDem = sqrtf((float)(UUx * UUx + UUy * UUy + UUz * UUz));
+    double n0 = UUx / NDem, n1 = UUy / NDem, n2 = UUz / NDem;
+    double ParaT = (n0 * x0 + n1 * y0 + n2 * z0) / (n0 * Diag1X + n1 * Diag1Y + n2 * Diag1Z);
+    const double TX0 = cxold + ParaT * Diag1X, TY0 = cyold + ParaT * Diag1Y, TZ0 = czold + ParaT * Diag1Z;
+    const double TX1 = cxold + ParaT * Diag2X, TY1 = cyold + ParaT * Diag2Y, TZ1 = czold + ParaT * Diag2Z;
+    const double TX2 = cxold + ParaT * Diag3X, TY2 = cyold + ParaT * Diag3Y, TZ2 = czold + ParaT * Diag3Z;
+    const auto distance = [](double ax, double ay, double az, double bx, double by, double bz) -> double {
+        return sqrtf((float)(((ax - bx) * (ax - bx)) + ((ay - by) * (ay - by)) + ((az - bz) * (az - bz))));
+    };
+    const double Dist0 = distance(TX0, TY0, TZ0, xp, yp, zp), Dist1 = distance(TX1, TY1, TZ1, xp, yp, zp),
+                 Dist2 = distance(TX2, TY2, TZ2, xp, yp, zp);
+    int x = (Dist0 < Dist1);
+    int y = (Dist1 < Dist2);
+    int z = (Dist2 < Dist0);
+    // 0, 1 or 2; the points idx, idx + 1 and idx + 2 (mod 3) by selects, without a local array
+    int idx = 2 * (z - y) * z + (y - x) * y;
+    const bool p0 = idx == 0, p1 = idx == 1;
+    double mindist = p0 ? Dist0 : (p1 ? Dist1 : Dist2);
+    double xc = p0 ? TX0 : (p1 ? TX1 : TX2), yc = p0 ? TY0 : (p1 ? TY1 : TY2), zc = p0 ? TZ0 : (p1 ? TZ1 : TZ2);
+    double x1 = p0 ? TX1 : (p1 ? TX2 : TX0), y1 = p0 ? TY1 : (p1 ? TY2 : TY0), z1 = p0 ? TZ1 : (p1 ? TZ2 : TZ0);
+    double x2 = p0 ? TX2 : (p1 ? TX0 : TX1), y2 = p0 ? TY2 : (p1 ? TY0 : TY1), z2 = p0 ? TZ2 : (p1 ? TZ0 : TZ1);
+    double D1 = distance(xp, yp, zp, x2, y2, z2), D2 = distance(xc, yc, zc, x2, y2, z2);
+    double D3 = distance(xp, yp, zp, x1, y1, z1), D4 = distance(xc, yc, zc, x1, y1, z1);
+    double I1 = 0, I2 = D2, J1 = 0, J2 = D4;
+    if (mindist != 0) {
+        I1 = D1 * ((xp - x2) * (xc - x2) + (yp - y2) * (yc - y2) + (zp - z2) * (zc - z2)) / (D1 * D2);
+        I2 = D2 - I1;
+        J1 = D3 * ((xp - x1) * (xc - x1) + (yp - y1) * (yc - y1) + (zp - z1) * (zc - z1)) / (D3 * D4);
+        J2 = D4 - J1;
     }
+    const double sqrt3 = sqrt(3.0);
+    double L12 = 0.5 * (dmin(I1, sqrt3) + dmin(I2, sqrt3));
+    double L13 = 0.5 * (dmin(J1, sqrt3) + dmin(J2, sqrt3));
+    double NewODiagL = sqrt(2.0) * dmax(L12, L13);
+    double cd0 = xc - cxold, cd1 = yc - cyold, cd2 = zc - czold;
+    double nd = sqrt(cd0 * cd0 + cd1 * cd1 + cd2 * cd2);
+    double uv0 = cd0 / nd, uv1 = cd1 / nd, uv2 = cd2 / nd;
+    out.cx = xc - NewODiagL * uv0;
+    out.cy = yc - NewODiagL * uv1;
+    out.cz = zc - NewODiagL * uv2;
+    out.dl = (float)NewODiagL;
+}
+
+// The critical lengths of capture w by a group of `per` lanes (a power of two; group: their mask), and with
+// them the new record, in slot w.slot of list L.
+__device__ __forceinline__ void capture_lengths(const DomainDesc &D, const RecordList &L, const WinItem &w,
+                                                const CaptureItem &o, int per, int sub, unsigned int group,
+                                                CycleStats &st) {
+    const unsigned int t = w.t, dom = w.dom_dir >> 5;
+    int rx, ry, rz;
+    cell_coords(D, t, rx, ry, rz);
+    const double xp = (rx + D.xoff) + 0.5, yp = (ry + D.yoff) + 0.5, zp = rz + 0.5;
+    int ori = (abs(w.h) - 1) % 10000;
+    if (ori < 0)
+        ori += 10000;
+    const float *g = D.guv + 9 * ori;
+    const float g0 = g[0], g1 = g[1], g2 = g[2], g3 = g[3], g4 = g[4], g5 = g[5], g6 = g[6], g7 = g[7], g8 = g[8];
+    const double cx = o.cx, cy = o.cy, cz = o.cz;
+    const bool has_body = w.slot < L.body_cap;
+    float *const row = D.cdl + 26ull * t, *const body_row = L.body[has_body ? w.slot : 0].cdl;
+    // face normals: float sums of the unit-vector components (src/CAupdate.cpp:526-551)
+    double Fx[4], Fy[4], Fz[4];
+    Fx[0] = g0 + g3 + g6;
+    Fx[1] = g0 - g3 + g6;
+    Fx[2] = g0 + g3 - g6;
+    Fx[3] = g0 - g3 - g6;
+    Fy[0] = g1 + g4 + g7;
+    Fy[1] = g1 - g4 + g7;
+    Fy[2] = g1 + g4 - g7;
+    Fy[3] = g1 - g4 - g7;
+    Fz[0] = g2 + g5 + g8;
+    Fz[1] = g2 - g5 + g8;
+    Fz[2] = g2 + g5 - g8;
+    Fz[3] = g2 - g5 - g8;
+    // the new record's cached minimum over its liquid neighbours, with its direction and the
+    // second-smallest (the state a claim step leaves), so that its first claim step runs only once
+    // its DiagonalLength reaches a liquid neighbour
+    float mn = __int_as_float(0x7f800000), mn2 = mn;
+    unsigned int d1 = 0xffffffffu;
+#pragma unroll 1
+    for (int n = sub; n < 26; n += per) {
+        double a0 = xp + nb_dx(n) - cx;
+        double b0 = yp + nb_dy(n) - cy;
+        double d0 = zp + nb_dz(n) - cz;
+        double q0 = a0 * Fx[0] + b0 * Fy[0] + d0 * Fz[0];
+        double q1 = a0 * Fx[1] + b0 * Fy[1] + d0 * Fz[1];
+        double q2 = a0 * Fx[2] + b0 * Fy[2] + d0 * Fz[2];
+        double q3 = a0 * Fx[3] + b0 * Fy[3] + d0 * Fz[3];
+        double m = dmax(dmax(fabs(q0), fabs(q1)), dmax(fabs(q2), fabs(q3)));
+        const float v = (float)m;
+        row[n] = v;
+        if (has_body)
+            body_row[n] = v;
+        if ((o.liq >> n) & 1u) {
+            if (v < mn) {
+                mn2 = mn;
+                mn = v;
+                d1 = (unsigned int)n;
+            }
+            else if (v < mn2) {
+                mn2 = v;
+            }
+        }
+    }
+#pragma unroll 1
+    for (int k = per / 2; k; k >>= 1) {
+        const float omn = __shfl_xor_sync(group, mn, k), omn2 = __shfl_xor_sync(group, mn2, k);
+        const unsigned int od1 = __shfl_xor_sync(group, d1, k);
+        if (omn < mn || (omn == mn && od1 < d1)) {
+            mn2 = fminf(omn2, mn);
+            mn = omn;
+            d1 = od1;
+        }
+        else {
+            mn2 = fminf(mn2, omn);
+        }
+    }
+    if (sub != 0)
+        return;
+    D.gid[t] = w.h;
+    D.dl[t] = o.dl;
+    D.doc[3ull * t + 0] = (float)cx;
+    D.doc[3ull * t + 1] = (float)cy;
+    D.doc[3ull * t + 2] = (float)cz;
+    if (has_body)
+        body_head(L.body[w.slot]) = make_float4(__int_as_float(w.h), (float)cx, (float)cy, (float)cz);
+    if (w.slot != kNoRecord) {
+        L.rec[w.slot] = ActiveRec{o.dl, mn, w.cts, o.liq};
+        L.cell[w.slot] = t;
+        L.dom[w.slot] = dom_word(dom, d1);
+        L.min2[w.slot] = mn2;
+        D.pos[t] = w.slot;
+    }
+    // read as active by the growth pass of the next cycle, after the octahedron is written
+    D.ctype[t] = kActive;
+    st.captured++;
+}
+
+// The neighbours of captured cell w.t by a warp, lane s < 26 the neighbour of slot s (slot_dir: a load
+// instruction's lanes read neighbours in few rows of three consecutive cells): the cell's liquid mask,
+// and the masks and solidification re-checks of its active neighbours. kN captures at a time, their
+// loads in flight together. Records of the cells active at the start of the cycle lie below base; a cell
+// of type also_liquid (a mark of the cycle after next, or kLiquid) is liquid in the next cycle.
+template <int kN>
+__device__ __forceinline__ void capture_neighbours(const PassCtx &X, int app, unsigned long long base, const WinItem *wins,
+                                                   CaptureItem *items, unsigned int first, unsigned int stride,
+                                                   unsigned int n, int8_t also_liquid, CycleStats &st) {
+    const unsigned int lane = threadIdx.x & 31;
+    const int dir = slot_dir((int)lane);
+    const bool has = dir < 26;
+    const int dx = has ? nb_dx(dir) : 0, dy = has ? nb_dy(dir) : 0, dz = has ? nb_dz(dir) : 0;
+    const unsigned int dir_bit = has ? 1u << dir : 0u, opp_bit = has ? 1u << nb_opp(dir) : 0u;
+    ActiveRec *const rec = X.list[app].rec;
+    for (unsigned int i0 = first; i0 < n; i0 += kN * stride) {
+        int8_t ct[kN];
+        unsigned int p[kN], a[kN], c[kN], old[kN];
+        bool in[kN];
 #pragma unroll
-    for (int k = 0; k < kPer; k++) {
-        if (!act[k])
-            continue;
-        const unsigned int bit = 1u << nb_opp(slot_dir(sub + k * kLanes));
-        if ((old[k] & (kMaskFresh | kMaskDead)) || (old[k] & kDirBits) != bit || (old[k] & kMaskKeep))
-            continue;
-        // a lost its last liquid neighbour; it solidifies if it was grown this cycle (cycle >
-        // its CritTimeStep, src/CAupdate.cpp:257-261)
-        if (old[k] & kMaskGrown) {
+        for (int k = 0; k < kN; k++) {
+            const unsigned int i = i0 + k * stride;
+            in[k] = false;
+            ct[k] = kWall;
+            p[k] = kNoRecord;
+            a[k] = c[k] = 0;
+            if (i < n) {
+                const DomainDesc &D = desc_of(X, wins[i].dom_dir >> 5);
+                const unsigned int t = wins[i].t;
+                c[k] = wins[i].c;
+                int tx, ty, tz;
+                cell_coords(D, t, tx, ty, tz);
+                in[k] = (neighbour_mask(D, tx, ty, tz) & dir_bit) != 0;
+                a[k] = (unsigned int)((long long)t + (in[k] ? (dz * D.mx + dx) * D.my + dy : 0));
+                if (in[k]) {
+                    ct[k] = __ldcg(D.ctype + a[k]);
+                    p[k] = __ldcg(D.pos + a[k]);
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kN; k++) {
+            const unsigned int i = i0 + k * stride;
+            if (i >= n) // the whole warp agrees
+                break;
+            // The captured cell's liquid-neighbour mask, as its first claim step would build it from the
+            // neighbour types at the start of a later cycle: the neighbours still liquid (a neighbour
+            // claimed in this cycle reads TemporaryUpdate, or active once captured). Later captures and
+            // nucleations clear bits of it as of every other record's.
+            const unsigned int liq =
+                __reduce_or_sync(0xffffffffu, in[k] && (ct[k] == kLiquid || ct[k] == also_liquid) ? dir_bit : 0u);
+            if (lane == 0)
+                items[i].liq = liq;
+            // Serial order (src/CAupdate.cpp:333-334, 722-725): active cell a saw the captured cell t
+            // as liquid iff t's capturer c does not precede a. a keeps a liquid neighbour iff it has an
+            // unclaimed one (a set mask bit that nobody clears) or a claimed one with c >= a. Every
+            // claimed liquid neighbour clears its own bit exactly once, so the update that clears the
+            // last direction bit sees the final verdict: KEEP is always set before the clear of the
+            // same update, and an update's two atomics reach the word in program order. Only records of
+            // cells active at the start of the cycle (positions below base) need to take part. A neighbour
+            // captured in this same cycle may show up too, as active with a position used again: its mask
+            // has no bit for t (claimed when it was built), so the clear finds none and no re-check
+            // follows, and a KEEP set after its record was written goes with the next growth step.
+            in[k] = in[k] && ct[k] == kActive && p[k] < base;
+            if (in[k] && c[k] >= a[k])
+                atomicOr(&rec[p[k]].stat, kMaskKeep);
+            old[k] = in[k] ? atomicAnd(&rec[p[k]].stat, ~opp_bit) : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < kN; k++) {
+            if (!in[k] || (old[k] & (kMaskFresh | kMaskDead | kMaskKeep)) || (old[k] & kDirBits) != opp_bit ||
+                !(old[k] & kMaskGrown))
+                continue;
+            // a lost its last liquid neighbour; it solidifies if it was grown this cycle (cycle >
+            // its CritTimeStep, src/CAupdate.cpp:257-261)
             st.rechecks++;
-            D.ctype[a[k]] = kSolid;
-            atomicOr(rs + p[k], kMaskDead);
+            desc_of(X, wins[i0 + k * stride].dom_dir >> 5).ctype[a[k]] = kSolid;
+            atomicOr(&rec[p[k]].stat, kMaskDead);
         }
     }
 }
 
 // Listed claim e: whether it won (the lowest claimant index holds the claim word) and its capture's
-// starting state, in one round of loads.
-__device__ __forceinline__ bool load_win(const PassCtx &X, unsigned long long e, WinItem &w) {
+// starting state, in one round of loads. pos: the claimant's record in list L (kNoRecord: not known).
+__device__ __forceinline__ bool load_win(const PassCtx &X, const RecordList &L, unsigned long long e, unsigned int pos,
+                                         WinItem &w) {
     const unsigned int dom = claim_domain(e);
     const int l = (int)((e >> 32) & 31u);
     const DomainDesc &D = desc_of(X, dom);
     w.t = (unsigned int)e;
     w.c = (unsigned int)((long long)w.t - nb_offset(l, D.mx * D.my, D.my));
     w.dom_dir = (dom << 5) | (unsigned int)l;
+    w.slot = kNoRecord;
     const unsigned long long key = __ldcg(D.claim + w.t);
     w.cts = __ldg(D.cts_run + w.t);
-    w.h = __ldcg(D.gid + w.c);
-    w.docx = __ldcg(D.doc + 3ull * w.c + 0);
-    w.docy = __ldcg(D.doc + 3ull * w.c + 1);
-    w.docz = __ldcg(D.doc + 3ull * w.c + 2);
+    if (pos < L.body_cap) {
+        const float4 head = __ldcg(&body_head(L.body[pos]));
+        w.h = __float_as_int(head.x);
+        w.docx = head.y;
+        w.docy = head.z;
+        w.docz = head.w;
+    }
+    else {
+        w.h = __ldcg(D.gid + w.c);
+        w.docx = __ldcg(D.doc + 3ull * w.c + 0);
+        w.docy = __ldcg(D.doc + 3ull * w.c + 1);
+        w.docz = __ldcg(D.doc + 3ull * w.c + 2);
+    }
     return (unsigned int)key == w.c;
 }
 
@@ -1931,92 +2207,239 @@ __device__ __forceinline__ void capture_sync(unsigned int threads) {
     asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
 }
 
-// The captures of the block's winners in B.wins by its first `threads` threads, kLanes lanes each.
-template <int kLanes>
-__device__ __forceinline__ void capture_wins(BlockShared &B, unsigned int threads, unsigned int n_wins, int app,
-                                             unsigned long long base, int8_t also_liquid, CycleStats &st) {
-    const unsigned int n_groups = threads / kLanes, grp = threadIdx.x / kLanes;
-    for (unsigned int first = 0; first < n_wins; first += n_groups) {
-        const unsigned int i = first + grp;
-        const bool on = i < n_wins;
-        WinItem w{};
-        if (on)
-            w = B.wins[i];
-        capture_group<kLanes>(
-            B.X, app, base, w, on, also_liquid, [] { return true; },
-            [&]() -> unsigned long long {
-                if (first == 0)
-                    capture_sync(threads); // the block's slots are reserved
-                return B.slot == ULLONG_MAX ? ULLONG_MAX : B.slot + i;
-            },
-            st);
+// The critical lengths of captures 0 .. n - 1 by the block's first `threads` threads.
+__device__ __forceinline__ void capture_lengths_of(const PassCtx &X, const WinItem *w, const CaptureItem *items, unsigned int n,
+                                                   unsigned int threads, int app, CycleStats &st) {
+    unsigned int per = 32;
+    while (per > 4 && n * per > threads)
+        per >>= 1;
+    const unsigned int lane = threadIdx.x & 31, in_group = lane & (per - 1u);
+    const unsigned int group = (per == 32 ? 0xffffffffu : ((1u << per) - 1u)) << (lane - in_group);
+    for (unsigned int i = threadIdx.x / per; i < n; i += threads / per)
+        capture_lengths(desc_of(X, w[i].dom_dir >> 5), X.list[app], w[i], items[i], (int)per, (int)in_group, group, st);
+}
+
+// Captures of n winners by the block's first `threads` threads (at least 256), at most kCaptureItems at a
+// time, in two stages with a barrier between them. First the geometry, one thread per capture in the
+// first warps, while the other warps do the neighbours, a warp per capture: neither needs the other, and
+// the geometry of a whole block is one chain (its nine divisions and nine roots of a capture overlap)
+// instead of one per group of lanes. Then the critical lengths, as many lanes per capture (4-32) as the
+// block has threads. alloc(wins, m), called by one warp in the first stage, sets the slots of m winners.
+// kN: captures whose neighbours a warp has in flight.
+template <int kN, class Alloc>
+__device__ __forceinline__ void capture_winners(const PassCtx &X, WinItem *wins, CaptureItem *items, unsigned int threads,
+                                                unsigned int n, int app, unsigned long long base, int8_t also_liquid,
+                                                Alloc &&alloc, CycleStats &st) {
+    const unsigned int warp = threadIdx.x / 32, n_warps = threads / 32;
+    for (unsigned int first = 0; first < n; first += kCaptureItems) {
+        const unsigned int m = min(n - first, (unsigned int)kCaptureItems), geometry_warps = (m + 31) / 32;
+        WinItem *const w = wins + first;
+        if (warp < geometry_warps) {
+            if (threadIdx.x < m) {
+                const WinItem &q = w[threadIdx.x];
+                capture_geometry(desc_of(X, q.dom_dir >> 5), q.t, q.h, q.docx, q.docy, q.docz, items[threadIdx.x]);
+            }
+        }
+        else {
+            if (warp == n_warps - 1)
+                alloc(w, m);
+            capture_neighbours<kN>(X, app, base, w, items, warp - geometry_warps, n_warps - geometry_warps, m, also_liquid,
+                                   st);
+        }
+        capture_sync(threads);
+        capture_lengths_of(X, w, items, m, threads, app, st);
+        if (first + kCaptureItems < n)
+            capture_sync(threads);
+    }
+}
+
+// Record slots for m captures of the block (one warp calls): the block's free slots first, the others
+// appended to the list (one atomic on the grid's counter, which completes under the captures' first stage).
+__device__ __forceinline__ void take_slots(PoolState *P, BlockShared &B, WinItem *w, unsigned int m, unsigned long long base,
+                                           unsigned long long *appended) {
+    const unsigned int lane = threadIdx.x & 31;
+    const unsigned int free = min(B.n_free, (unsigned int)kFreeSlots), taken = min(B.n_taken, free);
+    const unsigned int reused = min(m, free - taken);
+    __syncwarp();
+    unsigned long long s0 = 0;
+    if (lane == 0) {
+        B.n_taken += m;
+        if (reused < m) {
+            s0 = base + atomicAdd(appended, (unsigned long long)(m - reused));
+            atomicAdd(&B.n_appended, m - reused);
+        }
+    }
+    s0 = __shfl_sync(0xffffffffu, s0, 0);
+    for (unsigned int k = lane; k < m; k += 32) {
+        unsigned int slot = kNoRecord;
+        if (k < reused)
+            slot = B.free_slots[free - taken - 1u - k];
+        else if (s0 + (k - reused) < B.X.capacity)
+            slot = (unsigned int)(s0 + (k - reused));
+        else
+            atomicOr(&P->error, kErrListOverflow);
+        w[k].slot = slot;
+    }
+}
+
+// Claim i of the block's list by a whole warp, lane n < 26 direction n: the shortest chain for a block that
+// has no more claims than warps. The winner test and every load go out in one round (held: the claimant's
+// state was kept by its claim step, so the orientation does not wait for it either), the independent
+// divisions and roots of the geometry run on lanes of their own, with capture_geometry's expressions on
+// the same operands.
+__device__ __forceinline__ void capture_claim(PoolState *P, BlockShared &B, unsigned int i, int app, unsigned long long base,
+                                              unsigned long long *appended, int8_t also_liquid, CycleStats &st) {
+    constexpr unsigned int kAll = 0xffffffffu;
+    const unsigned int lane = threadIdx.x & 31;
+    const unsigned long long e = claim_at(B, i);
+    const unsigned int dom = claim_domain(e), held = (unsigned int)(e >> kClaimantShift), t = (unsigned int)e;
+    const DomainDesc &D = desc_of(B.X, dom);
+    const RecordList &L = B.X.list[app];
+    const int plane = D.mx * D.my, my = D.my;
+    const unsigned int c = (unsigned int)((long long)t - nb_offset((int)((e >> 32) & 31u), plane, my));
+    const unsigned long long key = __ldcg(D.claim + t);
+    const int cts = __ldg(D.cts_run + t);
+    float4 head;
+    if (held) {
+        head = B.claimants[held - 1];
+    }
+    else {
+        const unsigned int pos = B.claim_pos[i];
+        const bool body = pos < L.body_cap;
+        const float *doc = body ? L.body[pos].doc : D.doc + 3ull * c;
+        head = make_float4(__int_as_float(__ldcg(body ? &L.body[pos].h : D.gid + c)), __ldcg(doc), __ldcg(doc + 1),
+                           __ldcg(doc + 2));
+    }
+    const int h = __float_as_int(head.x);
+    int rx, ry, rz;
+    cell_coords(D, t, rx, ry, rz);
+    const bool nb = (neighbour_mask(D, rx, ry, rz) >> lane) & 1u;
+    const unsigned int a = (unsigned int)((long long)t + (nb ? nb_offset((int)lane, plane, my) : 0));
+    const int8_t ct = __ldcg(D.ctype + a);
+    const unsigned int p = __ldcg(D.pos + a);
+    int ori = (abs(h) - 1) % 10000;
+    if (ori < 0)
+        ori += 10000;
+    const float *g = D.guv + 9 * ori;
+    const float g0 = g[0], g1 = g[1], g2 = g[2], g3 = g[3], g4 = g[4], g5 = g[5], g6 = g[6], g7 = g[7], g8 = g[8];
+    if ((unsigned int)key != c)
+        return; // a lower-index claimant captures t
+    // the record's slot; the atomic completes under the capture
+    unsigned int taken = 0, n_free = 0;
+    unsigned long long appended_at = 0;
+    if (lane == 0) {
+        n_free = min(B.n_free, (unsigned int)kFreeSlots);
+        taken = atomicAdd(&B.n_taken, 1u);
+        if (taken >= n_free) {
+            appended_at = base + atomicAdd(appended, 1ull);
+            atomicAdd(&B.n_appended, 1u);
+        }
+    }
+    // liquid mask, the neighbours' masks (see capture_neighbours)
+    const unsigned int liq = __reduce_or_sync(kAll, nb && (ct == kLiquid || ct == also_liquid) ? 1u << lane : 0u);
+    const bool act = nb && ct == kActive && p < base;
+    const unsigned int opp = act ? 1u << nb_opp((int)lane) : 0u;
+    if (act && c >= a)
+        atomicOr(&L.rec[p].stat, kMaskKeep);
+    const unsigned int old = act ? atomicAnd(&L.rec[p].stat, ~opp) : 0u;
+    // geometry (capture_geometry)
+    const int q3 = lane < 3 ? (int)lane : 0;
+    const double cxold = head.y, cyold = head.z, czold = head.w;
+    const double xp = (rx + D.xoff) + 0.5, yp = (ry + D.yoff) + 0.5, zp = rz + 0.5;
+    const double x0 = xp - cxold, y0 = yp - cyold, z0 = zp - czold;
+    const double mag0 = sqrtf((float)(x0 * x0 + y0 * y0 + z0 * z0));
+    const float ga = q3 == 0 ? g0 : (q3 == 1 ? g3 : g6), gb = q3 == 0 ? g1 : (q3 == 1 ? g4 : g7),
+                gc = q3 == 0 ? g2 : (q3 == 1 ? g5 : g8);
+    const double dot = ga * x0 + gb * y0 + gc * z0;
+    const unsigned int neg = __ballot_sync(kAll, (dot < -1e-200 && mag0 < 1e30) || dot / mag0 < 0);
+    const float s1 = (neg & 1u) ? 1.0f : -1.0f, s2 = (neg & 2u) ? 1.0f : -1.0f, s3 = (neg & 4u) ? 1.0f : -1.0f;
+    double Diag1X = g0 * s1, Diag1Y = g1 * s1, Diag1Z = g2 * s1;
+    double Diag2X = g3 * s2, Diag2Y = g4 * s2, Diag2Z = g5 * s2;
+    double Diag3X = g6 * s3, Diag3Y = g7 * s3, Diag3Z = g8 * s3;
+    double U1x = Diag2X - Diag1X, U1y = Diag2Y - Diag1Y, U1z = Diag2Z - Diag1Z;
+    double U2x = Diag3X - Diag1X, U2y = Diag3Y - Diag1Y, U2z = Diag3Z - Diag1Z;
+    double UUx = U1y * U2z - U1z * U2y;
+    double UUy = U1z * U2x - U1x * U2z;
+    double UUz = U1x * U2y - U1y * U2x;
+    double NDem = sqrtf((float)(UUx * UUx + UUy * UUy + UUz * UUz));
+    const double nq = (q3 == 0 ? UUx : (q3 == 1 ? UUy : UUz)) / NDem;
+    double n0 = __shfl_sync(kAll, nq, 0), n1 = __shfl_sync(kAll, nq, 1), n2 = __shfl_sync(kAll, nq, 2);
+    double ParaT = (n0 * x0 + n1 * y0 + n2 * z0) / (n0 * Diag1X + n1 * Diag1Y + n2 * Diag1Z);
+    const double TX0 = cxold + ParaT * Diag1X, TY0 = cyold + ParaT * Diag1Y, TZ0 = czold + ParaT * Diag1Z;
+    const double TX1 = cxold + ParaT * Diag2X, TY1 = cyold + ParaT * Diag2Y, TZ1 = czold + ParaT * Diag2Z;
+    const double TX2 = cxold + ParaT * Diag3X, TY2 = cyold + ParaT * Diag3Y, TZ2 = czold + ParaT * Diag3Z;
+    const double tqx = q3 == 0 ? TX0 : (q3 == 1 ? TX1 : TX2), tqy = q3 == 0 ? TY0 : (q3 == 1 ? TY1 : TY2),
+                 tqz = q3 == 0 ? TZ0 : (q3 == 1 ? TZ1 : TZ2);
+    const float distq =
+        sqrtf((float)(((tqx - xp) * (tqx - xp)) + ((tqy - yp) * (tqy - yp)) + ((tqz - zp) * (tqz - zp))));
+    const double Dist0 = __shfl_sync(kAll, distq, 0), Dist1 = __shfl_sync(kAll, distq, 1), Dist2 = __shfl_sync(kAll, distq, 2);
+    int x = (Dist0 < Dist1);
+    int y = (Dist1 < Dist2);
+    int z = (Dist2 < Dist0);
+    int idx = 2 * (z - y) * z + (y - x) * y;
+    const bool p0 = idx == 0, p1 = idx == 1;
+    double mindist = p0 ? Dist0 : (p1 ? Dist1 : Dist2);
+    double xc = p0 ? TX0 : (p1 ? TX1 : TX2), yc = p0 ? TY0 : (p1 ? TY1 : TY2), zc = p0 ? TZ0 : (p1 ? TZ1 : TZ2);
+    double x1 = p0 ? TX1 : (p1 ? TX2 : TX0), y1 = p0 ? TY1 : (p1 ? TY2 : TY0), z1 = p0 ? TZ1 : (p1 ? TZ2 : TZ0);
+    double x2 = p0 ? TX2 : (p1 ? TX0 : TX1), y2 = p0 ? TY2 : (p1 ? TY0 : TY1), z2 = p0 ? TZ2 : (p1 ? TZ0 : TZ1);
+    // D1..D4 on lanes 0..3: D1 = |p - v2|, D2 = |c - v2|, D3 = |p - v1|, D4 = |c - v1|
+    const double ax = (lane & 1) ? xc : xp, ay = (lane & 1) ? yc : yp, az = (lane & 1) ? zc : zp;
+    const double bx = (lane & 2) ? x1 : x2, by = (lane & 2) ? y1 : y2, bz = (lane & 2) ? z1 : z2;
+    const float dq = sqrtf((float)(((ax - bx) * (ax - bx)) + ((ay - by) * (ay - by)) + ((az - bz) * (az - bz))));
+    double D1 = __shfl_sync(kAll, dq, 0), D2 = __shfl_sync(kAll, dq, 1), D3 = __shfl_sync(kAll, dq, 2),
+           D4 = __shfl_sync(kAll, dq, 3);
+    double I1 = 0, I2 = D2, J1 = 0, J2 = D4;
+    if (mindist != 0) {
+        // I1 on lane 0, J1 on lane 1
+        const bool j = lane & 1;
+        const double ex = j ? x1 : x2, ey = j ? y1 : y2, ez = j ? z1 : z2;
+        const double Da = j ? D3 : D1, Db = j ? D4 : D2;
+        const double ij = Da * ((xp - ex) * (xc - ex) + (yp - ey) * (yc - ey) + (zp - ez) * (zc - ez)) / (Da * Db);
+        I1 = __shfl_sync(kAll, ij, 0);
+        I2 = D2 - I1;
+        J1 = __shfl_sync(kAll, ij, 1);
+        J2 = D4 - J1;
+    }
+    const double sqrt3 = sqrt(3.0);
+    double L12 = 0.5 * (dmin(I1, sqrt3) + dmin(I2, sqrt3));
+    double L13 = 0.5 * (dmin(J1, sqrt3) + dmin(J2, sqrt3));
+    double NewODiagL = sqrt(2.0) * dmax(L12, L13);
+    double cd0 = xc - cxold, cd1 = yc - cyold, cd2 = zc - czold;
+    double nd = sqrt(cd0 * cd0 + cd1 * cd1 + cd2 * cd2);
+    const double uvq = (q3 == 0 ? cd0 : (q3 == 1 ? cd1 : cd2)) / nd;
+    CaptureItem o;
+    o.cx = xc - NewODiagL * __shfl_sync(kAll, uvq, 0);
+    o.cy = yc - NewODiagL * __shfl_sync(kAll, uvq, 1);
+    o.cz = zc - NewODiagL * __shfl_sync(kAll, uvq, 2);
+    o.dl = (float)NewODiagL;
+    o.liq = liq;
+    taken = __shfl_sync(kAll, taken, 0);
+    n_free = __shfl_sync(kAll, n_free, 0);
+    appended_at = __shfl_sync(kAll, appended_at, 0);
+    unsigned int slot = kNoRecord;
+    if (taken < n_free)
+        slot = B.free_slots[n_free - 1u - taken];
+    else if (appended_at < B.X.capacity)
+        slot = (unsigned int)appended_at;
+    else
+        atomicOr(&P->error, kErrListOverflow);
+    capture_lengths(D, L, WinItem{t, c, dom << 5, h, cts, head.y, head.z, head.w, slot}, o, 32, (int)lane, kAll, st);
+    if (act && !(old & (kMaskFresh | kMaskDead | kMaskKeep)) && (old & kDirBits) == opp && (old & kMaskGrown)) {
+        st.rechecks++;
+        D.ctype[a] = kSolid;
+        atomicOr(&L.rec[p].stat, kMaskDead);
     }
 }
 
 // Capture pass of the persistent kernel, by the first `threads` threads of the block (its other warps
 // start the domains' next cycle). Each block keeps the winners among its own claims (one per
-// thread), reserves their record slots with one atomic (which completes under the captures) and
-// captures them. A block with few winners spends a whole warp on each: its time is then one chain
-// of loads and geometry, and a wider group shortens the chain (one neighbour and one critical
-// length per lane); with many, narrower groups keep the chains of a block in one round.
-//
-// A block with no more claims than warps gives each claim a warp at once: the winner test and every
-// load of the capture go out in one round, without a block barrier (the losers' loads are wasted).
-
-// Claim i of the block's list by one warp.
-__device__ __forceinline__ void capture_claim(PoolState *P, BlockShared &B, unsigned int i, int app, unsigned long long base,
-                                              unsigned long long *appended, int8_t also_liquid, CycleStats &st) {
-    const unsigned long long e = claim_at(B, i);
-    const unsigned int dom = claim_domain(e), held = (unsigned int)(e >> kClaimantShift);
-    const int l = (int)((e >> 32) & 31u);
-    const DomainDesc &D = desc_of(B.X, dom);
-    WinItem w;
-    w.t = (unsigned int)e;
-    w.c = (unsigned int)((long long)w.t - nb_offset(l, D.mx * D.my, D.my));
-    w.dom_dir = (dom << 5) | (unsigned int)l;
-    const unsigned long long key = __ldcg(D.claim + w.t);
-    w.cts = __ldg(D.cts_run + w.t);
-    if (held) {
-        w.h = B.claimants[held - 1].h;
-        w.docx = B.claimants[held - 1].doc[0];
-        w.docy = B.claimants[held - 1].doc[1];
-        w.docz = B.claimants[held - 1].doc[2];
-    }
-    else {
-        w.h = __ldcg(D.gid + w.c);
-        w.docx = __ldcg(D.doc + 3ull * w.c + 0);
-        w.docy = __ldcg(D.doc + 3ull * w.c + 1);
-        w.docz = __ldcg(D.doc + 3ull * w.c + 2);
-    }
-    const bool leader = (threadIdx.x & 31) == 0;
-    unsigned long long slot = 0;
-    capture_group<32>(
-        B.X, app, base, w, true, also_liquid,
-        [&] {
-            const bool win = (unsigned int)key == w.c;
-            if (win && leader) {
-                // completes under the capture
-                slot = base + atomicAdd(appended, 1ull);
-                atomicAdd(&B.n_appended, 1u);
-            }
-            return win;
-        },
-        [&]() -> unsigned long long {
-            if (leader && slot >= B.X.capacity) {
-                atomicOr(&P->error, kErrListOverflow);
-                return ULLONG_MAX;
-            }
-            return slot;
-        },
-        st);
-}
-
-template <int kLanes>
-__device__ void capture_block(PoolState *P, BlockShared &B, unsigned int threads, int app, unsigned long long base,
-                              unsigned long long *appended, int8_t also_liquid, CycleStats &st) {
+// thread) and captures them.
+template <int kFamily>
+__device__ __forceinline__ void capture_block(PoolState *P, BlockShared &B, unsigned int threads, int app,
+                                              unsigned long long base, unsigned long long *appended, int8_t also_liquid,
+                                              CycleStats &st) {
     const unsigned int n = claim_count(B), lane = threadIdx.x & 31;
-    constexpr bool kFew = kLanes >= kFewLanes;
-    if (kFew && n * 32 <= threads) {
+    if (kFamily == kShortList && n * 32 <= threads) {
         if (threadIdx.x / 32 < n)
             capture_claim(P, B, threadIdx.x / 32, app, base, appended, also_liquid, st);
         return;
@@ -2024,7 +2447,8 @@ __device__ void capture_block(PoolState *P, BlockShared &B, unsigned int threads
     for (unsigned int r0 = 0; r0 < n; r0 += threads) {
         const unsigned int i = r0 + threadIdx.x;
         WinItem w;
-        const bool win = i < n && load_win(B.X, claim_at(B, i), w);
+        const bool win = i < n && load_win(B.X, B.X.list[app], claim_at(B, i),
+                                           i < (unsigned int)kBlockClaims ? B.claim_pos[i] : kNoRecord, w);
         const unsigned int winners = __ballot_sync(0xffffffffu, win);
         unsigned int first = 0;
         if (lane == 0 && winners)
@@ -2033,25 +2457,9 @@ __device__ void capture_block(PoolState *P, BlockShared &B, unsigned int threads
         if (win)
             B.wins[first + __popc(winners & ((1u << lane) - 1u))] = w;
         capture_sync(threads);
-        const unsigned int n_wins = B.n_wins;
-        if (threadIdx.x == threads - 32) {
-            unsigned long long slot = ULLONG_MAX;
-            if (n_wins) {
-                atomicAdd(&B.n_appended, n_wins);
-                slot = base + atomicAdd(appended, (unsigned long long)n_wins);
-                if (slot + n_wins > B.X.capacity) {
-                    atomicOr(&P->error, kErrListOverflow);
-                    slot = ULLONG_MAX;
-                }
-            }
-            B.slot = slot;
-        }
-        if (kFew && n_wins * 32 <= threads)
-            capture_wins<32>(B, threads, n_wins, app, base, also_liquid, st);
-        else if (kLanes < 8 && n_wins * 8 <= threads)
-            capture_wins<8>(B, threads, n_wins, app, base, also_liquid, st);
-        else
-            capture_wins<kLanes>(B, threads, n_wins, app, base, also_liquid, st);
+        capture_winners<kFamily == kLongList ? 6 : 2>(
+            B.X, B.wins, B.captures, threads, B.n_wins, app, base, also_liquid,
+            [&](WinItem *q, unsigned int m) { take_slots(P, B, q, m, base, appended); }, st);
         if (r0 + threads < n) {
             capture_sync(threads);
             if (threadIdx.x == 0)
@@ -2061,9 +2469,14 @@ __device__ void capture_block(PoolState *P, BlockShared &B, unsigned int threads
     }
 }
 
-// Capture pass over the sharded claim list (the separate kernels): claim j of the cycle gets record
-// slot base + j (a tombstone unless it won), and the count grows by T when the cycle finishes.
-template <int kCaptureLanes> __device__ void capture_pass(PoolState *P, const PassCtx &X, CycleStats &st) {
+// Capture pass over the sharded claim list (the separate kernels): claim j of the cycle gets record slot
+// base + j (a tombstone unless it won), and the count grows by T when the cycle finishes.
+struct CaptureShared {
+    WinItem wins[kBlock];
+    CaptureItem captures[kCaptureItems];
+    unsigned int n_wins;
+};
+__device__ void capture_pass(PoolState *P, const PassCtx &X, CaptureShared &C, CycleStats &st) {
     __shared__ unsigned long long s_pre[kShards + 1];
     shard_prefix(P->tcnt_s, s_pre);
     const int app = P->pending; // list of the next cycle
@@ -2075,35 +2488,40 @@ template <int kCaptureLanes> __device__ void capture_pass(PoolState *P, const Pa
             atomicOr(&P->error, kErrListOverflow);
         return;
     }
-    unsigned long long losers = 0;
-    constexpr int kGroups = 32 / kCaptureLanes;
-    const int lane = threadIdx.x & 31;
-    const int grp = lane / kCaptureLanes, sub = lane % kCaptureLanes;
+    unsigned int losers = 0;
+    const unsigned int lane = threadIdx.x & 31;
     // consecutive claims on different blocks (spread over all SMs)
-    const unsigned long long ngroups = (unsigned long long)gridDim.x * (kBlock / 32) * kGroups;
-    const unsigned long long g0 = ((unsigned long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * kGroups + grp;
-    for (unsigned long long j = g0; j < T; j += ngroups) {
+    for (unsigned long long j0 = 0; j0 < T; j0 += (unsigned long long)gridDim.x * kBlock) {
+        const unsigned long long j = j0 + (unsigned long long)threadIdx.x * gridDim.x + blockIdx.x;
+        if (threadIdx.x == 0)
+            C.n_wins = 0;
+        __syncthreads();
         WinItem w;
-        const bool win = load_win(X, __ldcg(P->tgt + shard_entry(s_pre, cap, j)), w);
-        if (!win && sub == 0) {
-            // a lower-index claimant captures t; this claim's slot stays a dropped record
-            P->rec[app][base + j].cell = kTombstone;
-            P->rec[app][base + j].cdl_min = 0.0f;
-            losers++;
+        bool win = false;
+        if (j < T) {
+            win = load_win(X, X.list[app], __ldcg(P->tgt + shard_entry(s_pre, cap, j)), kNoRecord, w);
+            w.slot = (unsigned int)(base + j);
+            if (!win) {
+                // a lower-index claimant captures t; this claim's slot stays a dropped record
+                X.list[app].rec[base + j].stat = kMaskTomb;
+                losers++;
+            }
         }
-        capture_group<kCaptureLanes>(
-            X, app, base, w, win, (int8_t)kLiquid, [] { return true; },
-            [&]() -> unsigned long long { return base + j; }, st);
-        if (win && sub == 0)
+        const unsigned int winners = __ballot_sync(0xffffffffu, win);
+        unsigned int first = 0;
+        if (lane == 0 && winners)
+            first = atomicAdd(&C.n_wins, __popc(winners));
+        first = __shfl_sync(0xffffffffu, first, 0);
+        if (win) {
+            C.wins[first + __popc(winners & ((1u << lane) - 1u))] = w;
             atomicAdd((unsigned long long *)&X.desc[w.dom_dir >> 5].liquid_shard[(blockIdx.x + j) & (kLiquidShards - 1)],
                       (unsigned long long)(-1ll));
+        }
+        __syncthreads();
+        capture_winners<2>(X, C.wins, C.captures, kBlock, C.n_wins, app, base, (int8_t)kLiquid, [](WinItem *, unsigned int) {}, st);
+        __syncthreads();
     }
-    // every lane reaches this point
-#pragma unroll
-    for (int o = 16; o; o >>= 1)
-        losers += __shfl_down_sync(0xffffffffu, losers, o);
-    if (lane == 0 && losers)
-        atomicAdd(&P->tomb_s[(blockIdx.x + threadIdx.x) % kShards].v, losers);
+    add_tombs(P, losers);
 }
 
 // End of a cycle: the record slots of this cycle's claims join the list.
@@ -2129,7 +2547,7 @@ template <int kBatch> __global__ void __launch_bounds__(kBlock) k_grow(PoolState
     CycleStats st;
     unsigned int tombs = 0;
     const int cur = P->cur;
-    grow_pass<kBatch, false, false>(P, X, nullptr, load_dyn(X.desc[0]), cur, P->cnt[cur], P->compact != 0, st, tombs);
+    grow_pass<kBatch, false, kLongList>(P, X, nullptr, load_dyn(X.desc[0]), cur, P->cnt[cur], P->compact != 0, false, st, tombs);
     add_tombs(P, tombs);
     flush_stats(P, st);
 }
@@ -2148,12 +2566,13 @@ __global__ void __launch_bounds__(kBlock) k_claim(PoolState *P) {
 
 // Capture pass as its own kernel; the last block to finish closes the cycle and, with kBegin,
 // starts the next one.
-template <bool kBegin, int kLanes> __global__ void __launch_bounds__(kBlock) k_capture_pass(PoolState *P) {
+template <bool kBegin> __global__ void __launch_bounds__(kBlock) k_capture_pass(PoolState *P) {
     __shared__ PassCtx X;
     load_ctx(P, X, 0);
     __syncthreads();
+    __shared__ CaptureShared C;
     CycleStats st;
-    capture_pass<kLanes>(P, X, st);
+    capture_pass(P, X, C, st);
     flush_stats(P, st);
     __shared__ int s_last;
     __threadfence(); // this block's writes are visible device-wide before it is counted
@@ -2253,7 +2672,7 @@ __device__ bool grid_meet(PoolState *P, unsigned int &k, unsigned long long *tl,
 // the capture pass of cycle c: the device-side termination check, the cycle advance and the
 // nucleation of the sites whose time has come, as start_domain does at the start of a launch. What
 // makes that possible:
-//   - the liquid count after cycle c is known before the captures (issue_claims counts the cells
+//   - the liquid count after cycle c is known before the captures (make_claims counts the cells
 //     claimed; `claimed` are the hot domain's);
 //   - a site that fires was marked (mark_code) during the capture pass before this one, when its
 //     type was liquid. A claim made since has overwritten the mark, so the site fires iff the mark
@@ -2305,6 +2724,7 @@ __device__ __noinline__ void start_next(PoolState *P, BlockShared &B, unsigned i
         return;
     }
     const int cycle = s.cycle0 + 1;
+    const RecordList &L = B.X.list[app];
     int fired_total = 0;
     for (int q = s.cursor0; q < mark0; q += 32) {
         const int idx = q + (int)lane;
@@ -2333,12 +2753,12 @@ __device__ __noinline__ void start_next(PoolState *P, BlockShared &B, unsigned i
         for (unsigned int todo = firing; todo; todo &= todo - 1) {
             const int src = __ffs(todo) - 1;
             const unsigned int rank = __popc(firing & ((1u << src) - 1u));
-            nucleate_site(V, s.ctype, B.X.rec[app], B.X.rdom[app], B.X.rstat[app], B.X.rmin2[app], d,
+            nucleate_site(V, s.ctype, L, d,
                           (unsigned int)__shfl_sync(0xffffffffu, l, src), __shfl_sync(0xffffffffu, h, src),
                           __shfl_sync(0xffffffffu, cts, src), slot0 == ULLONG_MAX ? ULLONG_MAX : slot0 + rank,
                           [&](unsigned int nb_pos, int) {
                               if (nb_pos < base)
-                                  atomicOr(B.X.rstat[app] + nb_pos, kMaskNuc);
+                                  atomicOr(&L.rec[nb_pos].stat, kMaskNuc);
                           });
         }
         fired_total += (int)n_fire;
@@ -2379,7 +2799,7 @@ __device__ __noinline__ void start_next(PoolState *P, BlockShared &B, unsigned i
 // is past some record's CritTimeStep or needs its start: they only advance the cycle number. Of the
 // cycles of a 64^3 solve 32 % make no claim (19 % grow nothing), of 3 x 3 spot melts 57 % (57 %), of
 // small three-layer ones 86 % (74 %); an idle cycle took 4.8 us, one with growth and no claim about 7.
-template <int kLanes, int kBatch>
+template <int kFamily, int kBatch>
 __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles, AliveSet alive) {
     __shared__ BlockShared B;
     CycleStats st;
@@ -2395,7 +2815,8 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
     const auto no_share = [] { return 0ull; };
     if (threadIdx.x == 0)
     {
-        B.n_items = B.n_claims = B.n_wins = B.n_first = B.n_tombs = B.n_appended = B.busy = 0;
+        B.n_items = B.n_claims = B.n_wins = B.n_first = B.n_appended = B.n_free = B.n_taken = B.busy = 0;
+        B.tombs = 0;
         B.min_cts = INT_MAX;
     }
     if (blockIdx.x == 0) {
@@ -2439,10 +2860,10 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
         // growth with each block's claims right after its own growth; the global claim pass only
         // when some block's queue overflowed this cycle (the same answer for every block)
         unsigned int dropped = 0;
-        grow_pass<kBatch, true, (kLanes >= kFewLanes)>(P, B.X, &B, dyn, cur, n, compact, st, dropped);
+        grow_pass<kBatch, true, kFamily>(P, B.X, &B, dyn, cur, n, compact, passes == 0, st, dropped);
         dropped = __reduce_add_sync(0xffffffffu, dropped);
         if ((threadIdx.x & 31) == 0 && dropped)
-            atomicAdd(&B.n_tombs, dropped);
+            atomicAdd(&B.tombs, (int)dropped);
         // sums: first claims of the hot domain, blocks whose queue overflowed, blocks that are busy
         constexpr int kOverflowShift = 40, kBusyShift = 48;
         int *const grid_min = reinterpret_cast<int *>(&P->meet.min_cts[passes % 3].v);
@@ -2460,6 +2881,11 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
                     atomicMin(grid_min, B.min_cts);
                 B.n_items = B.busy = 0;
                 B.min_cts = INT_MAX;
+                if (compact) {
+                    // positions in the old list
+                    B.n_free = 0;
+                    B.tombs = 0;
+                }
                 return v;
             },
             total);
@@ -2474,7 +2900,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
             claim_pass<true>(P, B.X, &B, app, st, dropped);
             dropped = __reduce_add_sync(0xffffffffu, dropped);
             if ((threadIdx.x & 31) == 0 && dropped)
-                atomicAdd(&B.n_tombs, dropped);
+                atomicAdd(&B.tombs, (int)dropped);
             ok = grid_meet(P, meet, tl, 3 * c + 2, claim_share, total);
             if (!ok)
                 break;
@@ -2519,24 +2945,29 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
             }
         }
         else {
-            capture_block<kLanes>(P, B, threads, app, base, appended, mark_code(c + 2), st);
+            capture_block<kFamily>(P, B, threads, app, base, appended, mark_code(c + 2), st);
         }
-        // sums: records appended (36 bits: list positions have 32), records dropped (20 bits; only
-        // the compaction's timing depends on them, so a block adds at most its share of the field)
-        constexpr int kTombShift = 36;
+        // sums: records appended (32 bits, as list positions), change of the number of dropped records
+        // (24 bits: 2^15 more from each block, which keeps what exceeds its share for the next time)
+        constexpr int kTombShift = 32, kTombBias = 1 << 15;
         ok = grid_meet(
             P, meet, tl, 3 * c + 3,
             [&] {
-                const unsigned int most = ((1u << (kMeetShift - kTombShift)) - 1u) / gridDim.x;
-                const unsigned long long v = B.n_appended + ((unsigned long long)min(B.n_tombs, most) << kTombShift);
-                B.n_claims = B.n_wins = B.n_tombs = B.n_appended = 0;
+                const unsigned int free = min(B.n_free, (unsigned int)kFreeSlots), reused = min(B.n_taken, free);
+                B.n_free = free - reused;
+                B.tombs -= (int)reused;
+                const int delta = min(max(B.tombs, 1 - kTombBias), kTombBias - 1);
+                const unsigned long long v = B.n_appended + ((unsigned long long)(delta + kTombBias) << kTombShift);
+                B.tombs -= delta;
+                B.n_claims = B.n_wins = B.n_taken = B.n_appended = 0;
                 return v;
             },
             total);
-        n = base + (total & ((1ull << kTombShift) - 1));
+        n = base + (total & 0xffffffffull);
         if (n > B.X.capacity)
             n = B.X.capacity; // overflowed: flagged
-        tombs = (compact ? 0 : tombs) + (total >> kTombShift);
+        const long long change = (long long)(total >> kTombShift) - (long long)gridDim.x * kTombBias;
+        tombs = (unsigned long long)max((long long)(compact ? 0 : tombs) + change, 0ll);
         cur = app;
     }
     if (ok && blockIdx.x == 0 && threadIdx.x == 0) {
@@ -2562,20 +2993,20 @@ __global__ void __launch_bounds__(kBlock) k_meet_probe(PoolState *P) {
     grid_meet(P, k, nullptr, 0, [] { return 0ull; }, total);
 }
 
-// Compiled launch shapes: {capture lanes, growth batch} for kLaneChoices x kBatchChoices.
+// Compiled launch shapes.
 struct StepKernels {
     const void *cycles;
     void (*grow)(PoolState *);
     void (*capture_begin)(PoolState *);
     void (*capture_end)(PoolState *);
 };
-template <int kL, int kB> StepKernels step_kernels() {
-    return {(const void *)k_cycles<kL, kB>, k_grow<kB>, k_capture_pass<true, kL>, k_capture_pass<false, kL>};
+template <int kF, int kB> StepKernels step_kernels() {
+    return {(const void *)k_cycles<kF, kB>, k_grow<kB>, k_capture_pass<true>, k_capture_pass<false>};
 }
-static_assert(kStepVariants == 4, "two lane widths x two batch depths");
+static_assert(kStepVariants == 4, "the shapes below");
 const StepKernels kStepKernel[kStepVariants] = {
-    step_kernels<kLaneChoices[0], kBatchChoices[0]>(), step_kernels<kLaneChoices[0], kBatchChoices[1]>(),
-    step_kernels<kLaneChoices[1], kBatchChoices[0]>(), step_kernels<kLaneChoices[1], kBatchChoices[1]>()};
+    step_kernels<kLongList, kBatchChoices[0]>(), step_kernels<kLongList, kBatchChoices[1]>(),
+    step_kernels<kMidList, kBatchChoices[0]>(), step_kernels<kShortList, kBatchChoices[1]>()};
 
 // ---------------------------------------------------------------------------------------------
 // Census of src/CAupdate.cpp:738-808 for one domain and its current layer; the smallest
@@ -2720,16 +3151,18 @@ __global__ void k_init_active(PoolState *P, int dom, int list_slot) {
         bool listed = act;
         unsigned long long pos = block_reserve(P, list_slot, listed ? 1u : 0u);
         if (listed && pos != ULLONG_MAX) {
-            ActiveRec r;
-            r.cell = (unsigned int)c;
-            r.dl = 0.01f;
-            r.cdl_min = 0.0f;
-            r.cts = D.cts_run[c];
-            P->rec[list_slot][pos] = r;
-            P->rdom[list_slot][pos] = (unsigned int)dom;
-            P->rstat[list_slot][pos] = kMaskFresh;
-            P->rmin2[list_slot][pos] = kNoMin2;
+            const RecordList L = list_of(P, list_slot);
+            L.rec[pos] = ActiveRec{0.01f, 0.0f, D.cts_run[c], kMaskFresh};
+            L.cell[pos] = (unsigned int)c;
+            L.dom[pos] = dom_word((unsigned int)dom, kNoDir);
+            L.min2[pos] = 0.0f;
             D.pos[c] = (unsigned int)pos;
+            if (pos < L.body_cap) {
+                RecordBody &b = L.body[pos];
+                body_head(b) = make_float4(__int_as_float(D.gid[c]), D.doc[3ull * c], D.doc[3ull * c + 1], D.doc[3ull * c + 2]);
+                for (int l = 0; l < 26; l++)
+                    b.cdl[l] = D.cdl[26ull * c + l];
+            }
         }
     }
 }
@@ -2742,8 +3175,8 @@ __global__ void k_drop_domain(PoolState *P, unsigned int dom, unsigned int place
     unsigned int *d = P->rdom[nxt];
     for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (unsigned long long)gridDim.x * blockDim.x)
-        if (d[i] == dom)
-            d[i] = placeholder;
+        if (word_dom(d[i]) == dom)
+            d[i] = dom_word(placeholder, kNoDir);
 }
 
 // Diagonal lengths held in the pending records back to the per-cell arrays.
@@ -2753,11 +3186,11 @@ __global__ void k_flush_records(PoolState *P) {
     for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (unsigned long long)gridDim.x * blockDim.x) {
         const ActiveRec r = P->rec[nxt][i];
-        if (r.cell == kTombstone)
+        if (r.stat & kMaskTomb)
             continue; // a dropped record's other fields are not kept up to date
-        const DomainDesc &D = P->desc[P->rdom[nxt][i]];
+        const DomainDesc &D = P->desc[word_dom(P->rdom[nxt][i])];
         if (D.dl)
-            D.dl[r.cell] = r.dl;
+            D.dl[P->rcell[nxt][i]] = r.dl;
     }
 }
 
@@ -3074,9 +3507,11 @@ Pool::Pool(int device, size_t budget_bytes, unsigned long long list_capacity)
     for (int q = 0; q < 2; q++) {
         CUDA_OK(cudaMalloc(&ps.rec[q], capacity_ * sizeof(ActiveRec)));
         CUDA_OK(cudaMalloc(&ps.rdom[q], capacity_ * sizeof(unsigned int)));
-        CUDA_OK(cudaMalloc(&ps.rstat[q], capacity_ * sizeof(unsigned int)));
-        CUDA_OK(cudaMalloc(&ps.rmin2[q], capacity_ * sizeof(unsigned long long)));
+        CUDA_OK(cudaMalloc(&ps.rcell[q], capacity_ * sizeof(unsigned int)));
+        CUDA_OK(cudaMalloc(&ps.rmin2[q], capacity_ * sizeof(float)));
+        CUDA_OK(cudaMalloc(&ps.body[q], std::min(capacity_, kBodyRecords) * sizeof(RecordBody)));
     }
+    ps.body_cap = (unsigned int)std::min(capacity_, kBodyRecords);
     // a shard takes the entries of 1/kShards of the warps: room for its share of the list plus slack
     ps.shard_cap = capacity_ / kShards + 8192;
     const size_t qn = (size_t)kShards * ps.shard_cap;
@@ -3084,7 +3519,6 @@ Pool::Pool(int device, size_t budget_bytes, unsigned long long list_capacity)
     ps.tgt_len = qn + 4096ull * (unsigned long long)num_sms_;
     CUDA_OK(cudaMalloc(&ps.tgt, ps.tgt_len * sizeof(unsigned long long)));
     CUDA_OK(cudaMalloc(&ps.qpos, qn * sizeof(unsigned int)));
-    CUDA_OK(cudaMalloc(&ps.qcell, qn * sizeof(unsigned int)));
     CUDA_OK(cudaMalloc(&ps.qdom, qn * sizeof(unsigned int)));
     CUDA_OK(cudaMalloc(&ps.qmask, qn * sizeof(unsigned int)));
     CUDA_OK(cudaMalloc(&ps.qdl, qn * sizeof(float)));
@@ -3118,12 +3552,12 @@ Pool::~Pool() {
             for (int q = 0; q < 2; q++) {
                 cudaFree(ps.rec[q]);
                 cudaFree(ps.rdom[q]);
-                cudaFree(ps.rstat[q]);
+                cudaFree(ps.rcell[q]);
                 cudaFree(ps.rmin2[q]);
+                cudaFree(ps.body[q]);
             }
             cudaFree(ps.tgt);
             cudaFree(ps.qpos);
-            cudaFree(ps.qcell);
             cudaFree(ps.qdom);
             cudaFree(ps.qmask);
             cudaFree(ps.qdl);
@@ -3414,7 +3848,8 @@ int Pool::admit(std::shared_ptr<const Problem> pp, int check_mode) {
     k_init_active<<<num_sms_ * 4, 256, 0, st>>>(dstate_, slot, -1);
     CUDA_OK(cudaGetLastError());
     bytes_in_use_ += s.bytes;
-    last_records_ = 0; // the list length is unknown until the next state read
+    // the list's length until the next state read: as then, with the new domain's first active cells
+    last_records_ += p.dir.used ? p.dir.active.size() : 0;
     return slot;
 }
 
@@ -3446,6 +3881,18 @@ void Pool::retire(int slot) {
     s = SlotHost();
 }
 
+// The persistent shape for a list of n records (0: not known). us per cycle of directional solves, long
+// list with two / four records per lane, middle, short: 2.9e4 records 14.9 / 15.8 / 11.9 / 11.7, 5.9e4 15.5
+// / 16.7 / 13.0 / 15.0, 1.7e5 19.7 / 19.9 / 17.5 / 18.8, 3.6e5 24.1 / 25.0 / 24.4 / 26.6, 5e5 27.7 / 28.2
+// / 29.2 / 31.2; whole solves: 64^3 (7e3) 9.9 / 10.2 / 7.9 / 7.6, 512^3 (1e6) 38.4 / 36.8 / 40.5 / 42.1.
+// All co-resident blocks are as fast as fewer, or faster, from 5e3 records on (half of them: 5.4 -> 6.3
+// on 3x3 spot melts), and within 2 % below.
+int Pool::shape_for(unsigned long long n) {
+    if (n == 0)
+        return 2;
+    return n < (1ull << 15) ? 3 : (n < 350000 ? 2 : (n < 700000 ? 0 : 1));
+}
+
 // One cooperative launch of k_cycles over n cycles (the grid is exactly the co-resident blocks).
 void Pool::launch_persistent(int n) {
     cudaStream_t st = S(stream_);
@@ -3468,21 +3915,11 @@ void Pool::launch_persistent(int n) {
         if (host_desc_[alive.idx[i]].active_size > host_desc_[alive.idx[0]].active_size)
             std::swap(alive.idx[0], alive.idx[i]);
     void *args[] = {&ps, &n, &alive};
-    // a sixteenth of the co-resident blocks for a list too short to fill them (fewer arrivals at
-    // every grid-wide meeting; on a many-domain map measured faster below ~8e3 records, slower from
-    // ~1.7e4, and the half grid slower than the full one from ~3e4 up)
-    constexpr unsigned long long kSmallGridRecords = 1ull << 13;
-    // run_plain before its trials: half of them below 2^17 records (its first launch, while the
-    // list grows from the initial front)
-    constexpr unsigned long long kHalfGridRecords = 1ull << 17;
-    if (grid_fixed_)
-        grid_div_ = grid_fixed_;
-    else if (!grid_tuned_ && plain_run_)
-        grid_div_ = (last_records_ > 0 && last_records_ < kHalfGridRecords) ? 2 : 1;
-    else if (!grid_tuned_)
-        grid_div_ = (last_records_ > 0 && last_records_ < kSmallGridRecords) ? 16 : 1;
-    const int grid = std::max(1, std::min(kMeetMaxGrid, grid_cycles_[variant_]) / grid_div_);
-    CUDA_OK(cudaLaunchCooperativeKernel(kStepKernel[variant_].cycles, dim3(grid), dim3(kBlock), args, 0, st));
+    const int v = config_fixed_ && !(tuned_records_ && last_records_ && last_records_ * 4 < tuned_records_)
+                      ? variant_
+                      : shape_for(last_records_);
+    const int grid = std::max(1, std::min(kMeetMaxGrid, grid_cycles_[v]) / std::max(1, grid_fixed_));
+    CUDA_OK(cudaLaunchCooperativeKernel(kStepKernel[v].cycles, dim3(grid), dim3(kBlock), args, 0, st));
     launches_ += 1;
 }
 
@@ -3722,36 +4159,13 @@ void Pool::profile_persistent(int n, double us[7]) {
 void Pool::set_config(int config) {
     apply_config(config);
     config_fixed_ = true;
+    tuned_records_ = 0;
 }
 
 void Pool::set_grid(int divisor) {
     if (divisor < 0 || divisor > 32)
         throw std::invalid_argument("grid divisor must be 0 (automatic) or 1-32");
     grid_fixed_ = divisor;
-}
-
-int Pool::plain_tune(int n) {
-    int best = variant_, best_div = 1;
-    double best_ms = 1e300;
-    grid_tuned_ = true;
-    // the half grid only for lists that are not clearly long (it measured 25 % slower at ~1e6
-    // records, where its trials would cost more than they can find)
-    const int min_div = grid_fixed_ ? grid_fixed_ : 1;
-    const int max_div = grid_fixed_ ? grid_fixed_ : (last_records_ < (1ull << 19) ? 2 : 1);
-    for (int div = min_div; div <= max_div; div++)
-        for (int v = 0; v < kStepVariants; v++) {
-            apply_config(v);
-            grid_div_ = div;
-            const double ms = timed_step(n);
-            if (ms < best_ms) {
-                best_ms = ms;
-                best = v;
-                best_div = div;
-            }
-        }
-    apply_config(best);
-    grid_div_ = best_div;
-    return (max_div - min_div + 1) * kStepVariants * n;
 }
 
 void Pool::apply_config(int config) {
@@ -3783,6 +4197,8 @@ int Pool::autotune(int trial_cycles, double *ms_per_cycle) {
         }
     }
     set_config(best);
+    sync_state();
+    tuned_records_ = last_records_;
     return best;
 }
 
@@ -4013,14 +4429,6 @@ void Pool::copy_out_concurrent(int slot, int32_t *grain_id, int32_t *cell_type) 
 
 int Pool::run_plain(int slot, std::string &log, double *nucl_s, double *capture_s) {
     TraceRange trace("exaca run_plain");
-    // its own grid rule until its trials choose, and the grid they choose holds for this run only
-    // (the short-list rule of chunked stepping would hold a small domain's first 1000 cycles, while
-    // its list grows from the initial front, on a sixteenth of the blocks)
-    struct GridReset {
-        bool &tuned, &plain;
-        ~GridReset() { tuned = plain = false; }
-    } grid_reset{grid_tuned_, plain_run_};
-    plain_run_ = true;
     // src/runCA.cpp:282-411: the layer loop, each layer's cycles until no liquid of the layer is left
     const Problem &p = *slots_.at(slot).problem;
     const bool type_r = p.cfg.simulation_type == "R";
@@ -4033,14 +4441,15 @@ int Pool::run_plain(int slot, std::string &log, double *nucl_s, double *capture_
     CUDA_OK(cudaEventRecord(ev0, S(stream_)));
     sync_state();
     int cycle = host_desc_[slot].cycle;
-    constexpr int kTuneCycles = 50;
     while (true) {
         int n = 1000 - (cycle % 1000);
-        if (!config_fixed_ && cycle % 4000 == 1000 && n == 1000) {
-            // the persistent configuration's speed depends on the domain's active front: time each
-            // launch shape with the full and the half grid for kTuneCycles real cycles at cycle 1000
-            // and every 4000 cycles after; the results do not depend on it
-            n -= plain_tune(kTuneCycles);
+        if (!config_fixed_ && cycle == 0) {
+            // a layer's list grows from its initial front: its length is read, and with it the launch
+            // shape chosen, every 250 cycles of the first 1000
+            for (; n > 250; n -= 250) {
+                step(250);
+                sync_state();
+            }
         }
         step(n);
         sync_state();

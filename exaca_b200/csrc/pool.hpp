@@ -19,7 +19,6 @@ namespace exaca {
 
 constexpr int kMaxJumps = 32;
 constexpr int kStepVariants = 4; // compiled launch shapes of the step passes
-constexpr unsigned int kTombstone = 0xffffffffu;
 constexpr unsigned int kNoRecord = 0xffffffffu;
 constexpr int kLiquidShards = 16;
 // Per-cycle counters that every warp reserves from are split into kShards counters (warp w uses
@@ -49,13 +48,25 @@ enum {
 // One active cell in the compacted list: the state the per-cycle growth pass needs, so that pass
 // streams 16-byte records instead of gathering per-cell arrays.
 struct alignas(16) ActiveRec {
-    float dl;          // DiagonalLength (dl and cdl_min form one aligned 8-byte pair)
+    float dl;          // DiagonalLength
     float cdl_min;     // lower bound of the critical lengths of the cell's liquid neighbours
-    unsigned int cell; // index in the domain; kTombstone for a dropped record
     int cts;           // CritTimeStep
+    unsigned int stat; // liquid-neighbour directions and flags (kMask*), updated atomically by captures
 };
 static_assert(sizeof(ActiveRec) == 16, "ActiveRec is one 16-byte vector");
-static_assert(offsetof(ActiveRec, dl) % 8 == 0, "dl/cdl_min are stored as one float2");
+
+// What a record's claim step and its captures read of its cell, one 128-byte line per record beside the
+// list (the cell's own copies in the domain's arrays are for the caller: copy_octahedra). A 512^3 front's
+// 8e5 records take 100 MB here, within L2 and some 50 pages; their cells' rows lie scattered over
+// 0.7 GB. The first kBodyRecords positions of a list have one; the others read the cell's copies.
+struct alignas(128) RecordBody {
+    int h;         // GrainID
+    float doc[3];  // DOCenter
+    float cdl[26]; // CritDiagonalLength
+    float pad[2];
+};
+static_assert(sizeof(RecordBody) == 128, "RecordBody is one line");
+constexpr unsigned long long kBodyRecords = 1ull << 21;
 
 // Device-resident descriptor of one domain. Static fields are written at admission; dynamic
 // fields are advanced by the step kernels and read back by the host.
@@ -72,28 +83,30 @@ struct DomainDesc {
     unsigned long long *claim; // per active-window cell: (~epoch << 32) | capturer index
     unsigned int *pos;        // per active-window cell: position of its record in the list the next
                               // cycle reads (kNoRecord for cells that never had one)
-    const double *growth;     // growth increment by number of undercooling updates
     const float *guv;         // 9 per orientation
     const float *cdl_table;   // 26 per orientation
     const int32_t *nuc_loc;   // nuclei sorted by nucleation time
     const int32_t *nuc_time;
-    int growth_len;
     int n_nuclei;
     int mx, my, nz, nz_active, xoff, yoff, zbound_high;
     int check_mode; // 1: the device ends the domain at cycle % 1000 == 0 once no liquid is left
     long long domain_size, active_size;
     float du_value;
-    int zero_du; // 1 if a cell that can become active has UndercoolingChange 0 (U stays 0 there)
     int cts_max; // check_mode domains: the largest CritTimeStep of any cell
-    // dynamic state; the growth pass reads the first four as one 16-byte vector
-    alignas(16) int cycle;
+    // what the growth of a record needs, one 32-byte sector: the table, and the first four fields of
+    // the dynamic state
+    alignas(32) const double *growth; // growth increment by number of undercooling updates
+    int growth_len;
+    int16_t zero_du; // 1 if a cell that can become active has UndercoolingChange 0 (U stays 0 there)
+    int16_t n_jumps; // cycle jumps so far (jump_lo, jump_hi)
+    // dynamic state
+    int cycle;
     unsigned int epoch;
     int next_start; // persistent kernel: the first cycle whose start has to be run (no claims before it)
     int done;
     int nuc_cursor;
     int nn;
     int error;
-    int n_jumps;
     int nuc_mark; // persistent kernel: sites [nuc_cursor, nuc_mark) are marked to nucleate at the next cycle's start
     int dry_since; // check_mode domains past cts_max: the first cycle start that found no liquid (0: none)
     long long liquid; // liquid cells of layer 0, less the nucleations (captures are in liquid_shard)
@@ -118,14 +131,15 @@ struct DomainDesc {
 // Pool-level device state.
 struct PoolState {
     ActiveRec *rec[2];           // active-cell records of the current / next cycle
-    unsigned int *rdom[2];       // domain of each record
-    unsigned int *rstat[2];      // per record: liquid-neighbour directions and flags (kMaskFresh: not built)
-    // per record: (direction of the cached minimum critical length << 32) | second-smallest critical
-    // length (float bits), both over the liquid neighbours not reached at the last claim step
-    unsigned long long *rmin2[2];
+    unsigned int *rdom[2];       // domain of each record, and the direction of its cached minimum (dom_word)
+    unsigned int *rcell[2];      // cell of each record (index in the domain)
+    RecordBody *body[2];         // of the first body_cap records
+    unsigned int body_cap;
+    float *rmin2[2];             // second-smallest critical length over the liquid neighbours not reached at
+                                 // the last claim step
     // claim queue: records the growth pass hands to the claim pass, with the state the claim needs;
     // shard s holds entries [s * shard_cap, s * shard_cap + qcnt_s[s])
-    unsigned int *qpos, *qcell, *qdom, *qmask;
+    unsigned int *qpos, *qdom, *qmask;
     float *qdl;
     // claims this cycle, (domain << 37) | (direction << 32) | claimed cell. Separate kernels: shard s
     // holds entries [s * shard_cap, s * shard_cap + tcnt_s[s]). Persistent kernel: block b of a grid
@@ -263,12 +277,10 @@ class Pool {
     // Step configurations: config = mode * kStepVariants + variant. set_config switches; autotune
     // runs trial_cycles real cycles with every configuration (the pool's domains advance), keeps
     // the fastest and returns it; ms_per_cycle (kStepConfigs entries, may be null) gets the trials.
-    // Either fixes the configuration for run_plain, which otherwise picks the fastest persistent
-    // one itself (plain_tune).
+    // Without either, every persistent launch takes the shape for the list's length (shape_for).
     static constexpr int kStepConfigs = 2 * kStepVariants;
     void set_config(int config);
-    // Persistent grid: 0 chooses itself (run_plain's trials, else the list length), 1 all co-resident
-    // blocks, 2 half of them.
+    // Persistent grid: divisor d runs 1/d of the co-resident blocks; 0, all of them.
     void set_grid(int divisor);
     int config() const { return step_mode_ * kStepVariants + variant_; }
     int autotune(int trial_cycles, double *ms_per_cycle);
@@ -323,18 +335,11 @@ class Pool {
     int step_mode_ = 0;
     int variant_ = kStepVariants - 1;
     bool config_fixed_ = false; // set_config or autotune chose the configuration
-    // Persistent grid: all co-resident blocks (grid_div_ 1) or half of them (2), which cuts the
-    // grid-wide meetings' cost when the list is short. run_plain's trials choose it; otherwise it
-    // follows the list length read at the last sync_state.
-    int grid_div_ = 1;
-    bool grid_tuned_ = false;
-    bool plain_run_ = false; // inside run_plain
-    int grid_fixed_ = 0; // set_grid's divisor, 0 when the grid chooses itself
-    unsigned long long last_records_ = 0;
+    int grid_fixed_ = 0; // set_grid's divisor, 0 for every co-resident block
+    unsigned long long last_records_ = 0;  // length of the active list at the last state read
+    unsigned long long tuned_records_ = 0; // and at autotune's; its choice holds down to a quarter of it
+    static int shape_for(unsigned long long records);
     void apply_config(int config);
-    // run_plain's choice: n real cycles with each persistent configuration (and grid), the fastest
-    // kept; returns the cycles run
-    int plain_tune(int n);
     int grid_cycles_[kStepVariants] = {}; // co-resident blocks of each persistent kernel
     int grid_grow_[kStepVariants] = {};
     int grid_capture_[kStepVariants] = {};

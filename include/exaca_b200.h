@@ -134,16 +134,16 @@ int exaca_pool_step(exaca_pool *pool, int n_cycles);
  * result does not depend on the other domains in the pool. */
 int exaca_pool_run_all(exaca_pool *pool, int chunk_cycles, int64_t max_cycles, int64_t *cycles_stepped);
 /* Step configurations (no counterpart in the reference): config = mode * 4 + shape, mode 0 the
- * persistent kernel and 1 a CUDA graph of the per-pass kernels, shape one of the compiled
- * {capture lanes 4|8} x {growth records per lane 2|4}. Results do not depend on the configuration.
- * A configuration set here or chosen by exaca_pool_autotune stays; without either,
- * exaca_pool_run_plain picks the fastest persistent one itself. */
+ * persistent kernel and 1 a CUDA graph of the per-pass kernels; shapes of the persistent kernel: for
+ * long active lists with two (0) and four (1) records per lane in the growth pass, for middle (2) and
+ * for short lists (3); of the pass kernels: two (0, 2) and four (1, 3) records per lane. Results do not
+ * depend on the configuration. A configuration set here stays, one chosen by exaca_pool_autotune until
+ * the list has shrunk to a quarter; without either, each persistent launch takes the shape for the
+ * list's length at the last status read. */
 #define EXACA_STEP_CONFIGS 8
 int exaca_pool_set_config(exaca_pool *pool, int config);
 /* Grid of the persistent kernel (no counterpart in the reference): divisor d in 1-32 runs 1/d of
- * the co-resident blocks (cheaper grid-wide meetings for short active lists), 0 (the default) lets
- * the pool choose (exaca_pool_run_plain's trials, else the active list's length at the last status
- * read). Results do not depend on it. */
+ * the co-resident blocks, 0 (the default) all of them. Results do not depend on it. */
 int exaca_pool_set_grid(exaca_pool *pool, int divisor);
 /* Autotuner: runs trial_cycles real cycles of the pool's domains in every configuration, keeps the
  * fastest; ms_per_cycle (EXACA_STEP_CONFIGS entries, may be NULL) receives the trial times. */
@@ -176,11 +176,8 @@ int exaca_pool_stats(exaca_pool *pool, exaca_pool_stats_t *st);
 int exaca_pool_census(exaca_pool *pool, int slot, exaca_census *c);
 /* Runs one slot to completion exactly as the reference's layer loop (src/runCA.cpp:290-342):
  * 1000-cycle census, termination, type-S cycle jump; progress lines are appended to stdout when
- * verbose is 1. Unless a step configuration was set, it times the four persistent ones (with all
- * and with half of the co-resident blocks, for active lists below 2^19 records) for 50 real cycles
- * each at cycle 1000 of a layer and every 4000 cycles after, and keeps the fastest; before the first
- * trials it runs all co-resident blocks. (exaca_pool_step and exaca_pool_run_all run a sixteenth of
- * them while the active list read at the last status holds fewer than 2^13 records.) */
+ * verbose is 1. Unless a step configuration was set, the launch shape follows the active list's
+ * length, read every 250 cycles of the first 1000 of a layer and every 1000 after. */
 int exaca_pool_run_plain(exaca_pool *pool, int slot, int verbose, int *final_cycle);
 /* Ends the current layer of a multilayer slot and sets up the next: DomainShiftAndResize (the new
  * window from one plane below the lowest active cell to the highest cell of the next layer) and
