@@ -665,20 +665,22 @@ __device__ __noinline__ void begin_cycle(PoolState *P, bool close, DomainDesc *d
 __global__ void k_step_begin(PoolState *P) { begin_cycle(P, false, P->desc, P->n_domains, AliveSet{-1, {}}, false); }
 
 // ---------------------------------------------------------------------------------------------
-// One CA cycle after its start (begin_cycle) is three passes over the pool:
+// One CA cycle after its start is three passes over the pool:
 //   grow        every record of the current list (kBatch per lane, loads issued first): eligibility
 //               and diagonal growth (src/CAupdate.cpp:257-261), drop of finished or
 //               re-check-solidified cells, solidification of cells whose liquid mask is empty. A
 //               record whose mask must still be built, or whose diagonal reached the cached minimum
-//               critical length, goes to the claim queue.
-//   claim       one queue entry per thread: the liquid mask from the 26 neighbour types when it is
-//               not built yet (nucleated and new-layer cells), the critical-length row (7 aligned
-//               16-byte loads) and the claims (src/CAupdate.cpp:320-352); every claim is listed.
-//   capture     kCaptureLanes lanes per listed claim: the winner's group captures the cell
-//               (src/CAupdate.cpp:353-563), builds the new record's liquid mask and cached minimum
-//               critical length, and re-checks the captured cell's active neighbours.
-// They run as three kernels per cycle (k_grow, k_claim, k_capture_pass) or, for stretches of
-// cycles, inside the persistent cooperative kernel k_cycles with grid-wide barriers between them.
+//               critical length, is flagged for the claim pass.
+//   claim       per flagged record: the liquid mask from the 26 neighbour types when it is not built
+//               yet (nucleated and new-layer cells), the critical-length row (from the record's body)
+//               and the claims (src/CAupdate.cpp:320-352); every claim is listed.
+//   capture     per listed claim: the winner captures the cell (src/CAupdate.cpp:353-563), builds the
+//               new record's liquid mask and cached minimum critical length, and re-checks the
+//               captured cell's active neighbours.
+// They run as three kernels per cycle (k_grow, k_claim, k_capture_pass) or, for stretches of cycles,
+// inside the persistent cooperative kernel k_cycles: there a block claims for the records that it
+// flagged and captures for the claims that it listed, the grid meets after the claims and after the
+// captures, and the next cycle's start is spread over warps that have no capture left.
 // Records per lane in flight in the growth pass (template argument).
 constexpr int kBatchChoices[2] = {2, 4};
 // The persistent kernel has a family of code for each range of list lengths (a kernel that held it all
@@ -3544,6 +3546,7 @@ Pool::~Pool() {
     }
     for (auto &kv : tables_) {
         cudaFree(kv.second.guv);
+        cudaFree(kv.second.mis);
         cudaFree(kv.second.cdl_table);
     }
     if (dstate_) {
@@ -4519,53 +4522,78 @@ struct GrainAcc {
     unsigned long long melted, nucleated, top_melted;
     double mis, mis_top;
     unsigned long long hist[kMisorientationBins];
+    unsigned long long grains;
     int gmin, gmax;
 };
 
 struct Region {
-    int x0, x1, y0, y1, z0, z1, mx, my;
-    __device__ __forceinline__ long long count() const {
-        return (long long)(x1 - x0 + 1) * (y1 - y0 + 1) * (z1 - z0 + 1);
-    }
-    // q-th region cell: (k, i, j) of the .vtk grid -> rank-local index (ghost ring offset 1)
-    __device__ __forceinline__ long long cell(long long q, int &k) const {
-        const long long ny_r = y1 - y0 + 1, nx_r = x1 - x0 + 1;
-        const long long j = q % ny_r, t = q / ny_r;
-        const long long i = t % nx_r;
-        k = (int)(t / nx_r) + z0;
-        return (long long)k * mx * my + (i + x0 + 1) * my + (j + y0 + 1);
-    }
+    int x0, x1, y0, y1, z0, z1, mx, my, nz;
 };
 
-__global__ void __launch_bounds__(kBlock) k_grain_region(const int32_t *gid, const int8_t *melted, const float *mis,
-                                                         Region R, GrainAcc *acc) {
-    __shared__ unsigned long long s_hist[kMisorientationBins];
+// A row of the region (fixed z and x) per warp at a time, consecutive lanes on consecutive cells: one
+// division per row instead of four 64-bit ones per cell. Neighbouring cells mostly belong to one grain, so
+// their lanes share a histogram bin and a bitmap bit: the bin is counted once per set of lanes (with an
+// atomic per cell the lanes of a warp queued on one word), the bit set by lanes whose left neighbour has
+// another grain, where it is not set already. melted null: a type-C problem, where every cell off the
+// bottom and top planes and the ghost ring (outside any region) is melted. bits null: gmin / gmax only
+// (the bitmap's range is not known yet), as codes of which gmin holds the complement (both start at zero).
+// 192 x 160 x 128: the call takes 0.12 ms (a launch, a memset and two copies are most of it) instead of 4.5
+// with four divisions and an atomic per cell, a table of arc cosines made per call and the melted flags uploaded.
+__device__ __forceinline__ unsigned int grain_code(int g) { return (unsigned int)g ^ 0x80000000u; } // ordered as g
+
+__global__ void __launch_bounds__(256) k_grain_region(const int32_t *gid, const int8_t *melted, const float *mis, Region R,
+                                                      GrainAcc *acc, unsigned long long *bits, int bits_min,
+                                                      long long n_bits) {
+    __shared__ unsigned int s_hist[kMisorientationBins];
     for (int b = threadIdx.x; b < kMisorientationBins; b += blockDim.x)
         s_hist[b] = 0;
     __syncthreads();
+    const unsigned int lane = threadIdx.x & 31, below = (1u << lane) - 1u;
     unsigned long long m = 0, nuc = 0, top = 0;
     double ms = 0, mt = 0;
-    int gmin = INT_MAX, gmax = INT_MIN;
-    const long long n = R.count();
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        int k;
-        const long long c = R.cell(q, k);
-        const int g = gid[c];
-        gmin = min(gmin, g);
-        gmax = max(gmax, g);
-        if (g < 0)
-            nuc++;
-        if (melted[c] == 1) {
-            int ori = (abs(g) - 1) % 10000;
-            if (ori < 0)
-                ori += 10000;
-            const float a = mis[ori];
-            m++;
-            ms += a;
-            atomicAdd(&s_hist[min((int)a, kMisorientationBins - 1)], 1ull);
-            if (k == R.z1) {
-                top++;
-                mt += a;
+    unsigned int cmin = 0xffffffffu, cmax = 0;
+    const unsigned int nxr = (unsigned int)(R.x1 - R.x0 + 1), rows = nxr * (unsigned int)(R.z1 - R.z0 + 1);
+    const int nyr = R.y1 - R.y0 + 1;
+    for (unsigned int row = blockIdx.x * 8u + threadIdx.x / 32; row < rows; row += gridDim.x * 8u) {
+        const unsigned int kz = row / nxr;
+        const int k = (int)kz + R.z0, i = (int)(row - kz * nxr) + R.x0;
+        const long long c0 = ((long long)k * R.mx + (i + 1)) * R.my + (R.y0 + 1);
+        const bool plane_melted = k != 0 && k != R.nz - 1;
+        for (int j0 = 0; j0 < nyr; j0 += 32) {
+            const bool in = j0 + (int)lane < nyr;
+            const int g = in ? __ldcs(gid + c0 + j0 + lane) : 0;
+            const bool melt = in && (melted ? __ldcs(melted + c0 + j0 + lane) == 1 : plane_melted);
+            if (in) {
+                const unsigned int code = grain_code(g);
+                cmin = min(cmin, code);
+                cmax = max(cmax, code);
+                nuc += g < 0;
+            }
+            int bin = -1;
+            if (melt) {
+                int ori = (abs(g) - 1) % 10000;
+                if (ori < 0)
+                    ori += 10000;
+                const float a = __ldg(mis + ori);
+                m++;
+                ms += a;
+                bin = min((int)a, kMisorientationBins - 1);
+                if (k == R.z1) {
+                    top++;
+                    mt += a;
+                }
+            }
+            const unsigned int same = __match_any_sync(0xffffffffu, bin);
+            if (bin >= 0 && (same & below) == 0)
+                atomicAdd(&s_hist[bin], (unsigned int)__popc(same));
+            if (bits) {
+                const int left = __shfl_up_sync(0xffffffffu, g, 1);
+                const long long off = (long long)g - bits_min;
+                if (in && (lane == 0 || left != g) && off >= 0 && off < n_bits) {
+                    const unsigned long long bit = 1ull << (off & 63);
+                    if (!(bits[off >> 6] & bit))
+                        atomicOr(bits + (off >> 6), bit);
+                }
             }
         }
     }
@@ -4575,10 +4603,10 @@ __global__ void __launch_bounds__(kBlock) k_grain_region(const int32_t *gid, con
         top += __shfl_down_sync(0xffffffffu, top, o);
         ms += __shfl_down_sync(0xffffffffu, ms, o);
         mt += __shfl_down_sync(0xffffffffu, mt, o);
-        gmin = min(gmin, __shfl_down_sync(0xffffffffu, gmin, o));
-        gmax = max(gmax, __shfl_down_sync(0xffffffffu, gmax, o));
     }
-    if ((threadIdx.x & 31) == 0) {
+    cmin = __reduce_min_sync(0xffffffffu, cmin);
+    cmax = __reduce_max_sync(0xffffffffu, cmax);
+    if (lane == 0) {
         if (m)
             atomicAdd(&acc->melted, m);
         if (nuc)
@@ -4589,21 +4617,33 @@ __global__ void __launch_bounds__(kBlock) k_grain_region(const int32_t *gid, con
             atomicAdd(&acc->mis, ms);
         if (mt != 0)
             atomicAdd(&acc->mis_top, mt);
-        atomicMin(&acc->gmin, gmin);
-        atomicMax(&acc->gmax, gmax);
+        if (cmin <= cmax) {
+            // both start at zero: the minimum as the maximum of its complement
+            atomicMax((unsigned int *)&acc->gmin, ~cmin);
+            atomicMax((unsigned int *)&acc->gmax, cmax);
+        }
     }
     __syncthreads();
     for (int b = threadIdx.x; b < kMisorientationBins; b += blockDim.x)
         if (s_hist[b])
-            atomicAdd(&acc->hist[b], s_hist[b]);
+            atomicAdd(&acc->hist[b], (unsigned long long)s_hist[b]);
 }
 
 __global__ void k_grain_bits(const int32_t *gid, Region R, int gmin, unsigned long long *bits) {
-    const long long n = R.count();
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        int k;
-        const long long off = (long long)gid[R.cell(q, k)] - gmin;
-        atomicOr(bits + (off >> 6), 1ull << (off & 63));
+    const unsigned int lane = threadIdx.x & 31;
+    const unsigned int nxr = (unsigned int)(R.x1 - R.x0 + 1), rows = nxr * (unsigned int)(R.z1 - R.z0 + 1);
+    const int nyr = R.y1 - R.y0 + 1;
+    for (unsigned int row = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; row < rows;
+         row += gridDim.x * (blockDim.x / 32)) {
+        const unsigned int kz = row / nxr;
+        const long long c0 =
+            ((long long)((int)kz + R.z0) * R.mx + ((int)(row - kz * nxr) + R.x0 + 1)) * R.my + (R.y0 + 1);
+        for (int j = (int)lane; j < nyr; j += 32) {
+            const long long off = (long long)gid[c0 + j] - gmin;
+            const unsigned long long bit = 1ull << (off & 63);
+            if (!(bits[off >> 6] & bit))
+                atomicOr(bits + (off >> 6), bit);
+        }
     }
 }
 
@@ -4622,7 +4662,6 @@ GrainStats Pool::grain_stats(int slot, const int *region) {
     if (!slot_used(slot))
         throw std::invalid_argument("bad slot");
     const Problem &p = *slots_[slot].problem;
-    materialize_fields(p);
     const Geometry &g = p.g;
     Region R;
     if (region) {
@@ -4636,77 +4675,92 @@ GrainStats Pool::grain_stats(int slot, const int *region) {
         throw std::invalid_argument("region outside the domain");
     R.mx = g.mx;
     R.my = g.my;
-    // per-orientation misorientation to +Z with the reference's expression (GAprint.cpp:38-46)
-    std::vector<float> mis(kNumOrientations);
-    for (int n = 0; n < kNumOrientations; n++) {
-        double amin = 62.7;
-        for (int ll = 0; ll < 3; ll++) {
-            // double acos of the float component, as the reference's unqualified call on a float
-            double a = std::abs((180 / M_PI) * std::acos((double)p.guv[9 * n + 3 * ll + 2]));
-            if (a < amin)
-                amin = a;
+    R.nz = g.nz;
+    tables_for(p);
+    DeviceTables &tb = tables_.at(p.cfg.orientation_file);
+    if (!tb.mis) {
+        // per-orientation misorientation to +Z with the reference's expression (GAprint.cpp:38-46)
+        std::vector<float> mis(kNumOrientations);
+        for (int n = 0; n < kNumOrientations; n++) {
+            double amin = 62.7;
+            for (int ll = 0; ll < 3; ll++) {
+                // double acos of the float component, as the reference's unqualified call on a float
+                double a = std::abs((180 / M_PI) * std::acos((double)p.guv[9 * n + 3 * ll + 2]));
+                if (a < amin)
+                    amin = a;
+            }
+            mis[n] = (float)amin;
         }
-        mis[n] = (float)amin;
+        float *d = nullptr;
+        CUDA_OK(cudaMalloc(&d, mis.size() * sizeof(float)));
+        tb.mis = d;
+        CUDA_OK(cudaMemcpy(d, mis.data(), mis.size() * sizeof(float), cudaMemcpyHostToDevice));
     }
     cudaStream_t st = S(stream_);
     const size_t N = g.domain_size;
-    int8_t *dmel = nullptr;
-    float *dmis = nullptr;
-    GrainAcc *dacc = nullptr;
-    unsigned long long *bits = nullptr, *dcount = nullptr;
+    // a type-C domain's grains are its seeds and nuclei (and 0), its melted cells those off the walls: one
+    // pass; otherwise the melted flags are uploaded and a second pass marks the grains between the first's
+    // smallest and largest
+    const bool known = p.dir.used;
+    long long gmin = -(long long)p.nuclei_loc.size(), gmax = known ? (long long)p.dir.active.size() : 0;
     GrainStats out;
+    GrainAcc acc;
+    char *work = nullptr; // freed in stream order
     try {
-        CUDA_OK(cudaMalloc(&dmel, N));
-        CUDA_OK(cudaMalloc(&dmis, mis.size() * sizeof(float)));
-        CUDA_OK(cudaMalloc(&dacc, sizeof(GrainAcc)));
-        CUDA_OK(cudaMalloc(&dcount, sizeof(unsigned long long)));
-        GrainAcc init;
-        std::memset(&init, 0, sizeof(init));
-        init.gmin = INT_MAX;
-        init.gmax = INT_MIN;
-        CUDA_OK(cudaMemcpyAsync(dmel, p.melted.data(), N, cudaMemcpyHostToDevice, st));
-        CUDA_OK(cudaMemcpyAsync(dmis, mis.data(), mis.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-        CUDA_OK(cudaMemcpyAsync(dacc, &init, sizeof(init), cudaMemcpyHostToDevice, st));
-        CUDA_OK(cudaMemsetAsync(dcount, 0, sizeof(unsigned long long), st));
-        k_grain_region<<<num_sms_ * 4, kBlock, 0, st>>>(host_desc_[slot].gid, dmel, dmis, R, dacc);
+        const int32_t *gid = host_desc_[slot].gid;
+        const auto words = [](long long lo, long long hi) { return (size_t)((hi - lo + 64) / 64); };
+        const size_t nwords = known ? words(gmin, gmax) : 0, flags = known ? 0 : (N + 15) / 16 * 16;
+        constexpr size_t kAccBytes = (sizeof(GrainAcc) + 255) / 256 * 256;
+        CUDA_OK(cudaMallocAsync((void **)&work, kAccBytes + nwords * 8 + flags, st));
+        GrainAcc *dacc = (GrainAcc *)work;
+        unsigned long long *bits = (unsigned long long *)(work + kAccBytes);
+        int8_t *dmel = (int8_t *)(work + kAccBytes + nwords * 8);
+        CUDA_OK(cudaMemsetAsync(work, 0, kAccBytes + nwords * 8, st));
+        if (!known)
+            CUDA_OK(cudaMemcpyAsync(dmel, p.melted.data(), N, cudaMemcpyHostToDevice, st));
+        k_grain_region<<<num_sms_ * 8, 256, 0, st>>>(gid, known ? nullptr : dmel, tb.mis, R, dacc, known ? bits : nullptr,
+                                                     (int)gmin, (long long)nwords * 64);
         CUDA_OK(cudaGetLastError());
-        GrainAcc acc;
+        if (known)
+            k_popcount<<<32, 256, 0, st>>>(bits, (long long)nwords, &dacc->grains);
+        CUDA_OK(cudaGetLastError());
         CUDA_OK(cudaMemcpyAsync(&acc, dacc, sizeof(acc), cudaMemcpyDeviceToHost, st));
         CUDA_OK(cudaStreamSynchronize(st));
-        const long long range = (long long)acc.gmax - acc.gmin + 1;
-        const long long nwords = (range + 63) / 64;
-        CUDA_OK(cudaMalloc(&bits, nwords * 8));
-        CUDA_OK(cudaMemsetAsync(bits, 0, nwords * 8, st));
-        k_grain_bits<<<num_sms_ * 4, kBlock, 0, st>>>(host_desc_[slot].gid, R, acc.gmin, bits);
-        k_popcount<<<num_sms_ * 2, kBlock, 0, st>>>(bits, nwords, dcount);
-        CUDA_OK(cudaGetLastError());
-        unsigned long long count = 0;
-        CUDA_OK(cudaMemcpyAsync(&count, dcount, sizeof(count), cudaMemcpyDeviceToHost, st));
-        CUDA_OK(cudaStreamSynchronize(st));
-        out.region_cells = (long long)(R.x1 - R.x0 + 1) * (R.y1 - R.y0 + 1) * (R.z1 - R.z0 + 1);
-        out.melted_cells = (long long)acc.melted;
-        out.nucleated_cells = (long long)acc.nucleated;
-        out.top_melted = (long long)acc.top_melted;
-        out.n_grains = (long long)count;
-        out.misorientation_sum = acc.mis;
-        out.misorientation_top_sum = acc.mis_top;
-        out.deltax = p.cfg.deltax;
-        for (int b = 0; b < kMisorientationBins; b++)
-            out.hist[b] = acc.hist[b];
+        const long long seen_min = (long long)(int)(~(unsigned int)acc.gmin ^ 0x80000000u),
+                        seen_max = (long long)(int)((unsigned int)acc.gmax ^ 0x80000000u);
+        if (!known || seen_min < gmin || seen_max > gmax) {
+            gmin = seen_min;
+            gmax = seen_max;
+            CUDA_OK(cudaMemsetAsync(&dacc->grains, 0, sizeof(dacc->grains), st));
+            const size_t nw = words(gmin, gmax);
+            unsigned long long *more = nullptr;
+            CUDA_OK(cudaMallocAsync((void **)&more, nw * 8, st));
+            cudaMemsetAsync(more, 0, nw * 8, st);
+            k_grain_bits<<<num_sms_ * 8, 256, 0, st>>>(gid, R, (int)gmin, more);
+            k_popcount<<<32, 256, 0, st>>>(more, (long long)nw, &dacc->grains);
+            const cudaError_t launched = cudaGetLastError();
+            CUDA_OK(cudaFreeAsync(more, st));
+            CUDA_OK(launched);
+            CUDA_OK(cudaMemcpyAsync(&acc.grains, &dacc->grains, sizeof(acc.grains), cudaMemcpyDeviceToHost, st));
+            CUDA_OK(cudaStreamSynchronize(st));
+        }
     }
     catch (...) {
-        cudaFree(dmel);
-        cudaFree(dmis);
-        cudaFree(dacc);
-        cudaFree(bits);
-        cudaFree(dcount);
+        if (work)
+            cudaFreeAsync(work, st);
         throw;
     }
-    cudaFree(dmel);
-    cudaFree(dmis);
-    cudaFree(dacc);
-    cudaFree(bits);
-    cudaFree(dcount);
+    CUDA_OK(cudaFreeAsync(work, st));
+    out.region_cells = (long long)(R.x1 - R.x0 + 1) * (R.y1 - R.y0 + 1) * (R.z1 - R.z0 + 1);
+    out.melted_cells = (long long)acc.melted;
+    out.nucleated_cells = (long long)acc.nucleated;
+    out.top_melted = (long long)acc.top_melted;
+    out.n_grains = (long long)acc.grains;
+    out.misorientation_sum = acc.mis;
+    out.misorientation_top_sum = acc.mis_top;
+    out.deltax = p.cfg.deltax;
+    for (int b = 0; b < kMisorientationBins; b++)
+        out.hist[b] = (long long)acc.hist[b];
     return out;
 }
 

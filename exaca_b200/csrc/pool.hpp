@@ -201,6 +201,7 @@ struct GrainStats {
 
 struct DeviceTables {
     float *guv = nullptr;
+    float *mis = nullptr; // per orientation, its smallest angle to +Z in degrees (first grain_stats)
     float *cdl_table = nullptr;
 };
 
