@@ -253,8 +253,8 @@ class Pool {
     };
     // Issues the transfers on stream (a cudaStream_t) after the work already queued there and
     // returns when every pageable destination holds its data; page-locked destinations take one
-    // DMA each, still in flight at return. Pageable ones go through two 32 MB pinned staging
-    // pieces, the DMA of one overlapping the multi-threaded move out of the other: the driver's
+    // DMA each, still in flight at return. Pageable ones go through two pinned staging
+    // pieces of at most 32 MB, the DMA of one overlapping the multi-threaded move out of the other: the driver's
     // own pageable path moves about 2 GB/s.
     void to_host(const std::vector<HostCopy> &copies, void *stream);
     // writes the diagonal lengths held in the active records back to the per-cell array
@@ -320,6 +320,7 @@ class Pool {
     void *stream_ = nullptr;      // cudaStream_t
     void *copy_stream_ = nullptr; // cudaStream_t of copy_out_concurrent (created on first use)
     void *stage_[2] = {nullptr, nullptr};    // to_host's pinned staging pieces (first use)
+    size_t stage_bytes_ = 0;                 // of each
     void *stage_ev_[2] = {nullptr, nullptr}; // cudaEvent_t marking each piece's DMA
     PoolState *dstate_ = nullptr;
     DomainDesc *ddesc_ = nullptr;
