@@ -48,11 +48,16 @@ static __device__ __align__(256) unsigned char g_census_scratch[kScratchBytes];
 // the current layer are classified (src/CAupdate.cpp:741-752), liquid cells of any other layer are
 // remaining (:754-757); the minimum is taken over the window only (:792-805).
 //
-// 6 bytes are read per cell: sixteen cells per thread and step in 16-byte loads where the three arrays
-// are 16-byte aligned, cell by cell otherwise and at the end. A block sums its counts in shared memory
-// before its six atomics (with six per warp, 24 domains of 1.8e5 cells queued 1200 on each counter): a call
-// on those 24 takes 87 us instead of 97, of which the copies, launches and the caller are most.
-__host__ __device__ inline bool wide_reads(const exaca_cell_fields &d) {
+// 6 bytes are read per cell. kWide, for domains in which every thread has sixteen cells or more: sixteen
+// cells per thread and step in 16-byte loads where the three arrays are 16-byte aligned (cell by cell
+// otherwise and at the end). On smaller domains sixteen cells one after the other are the longer chain
+// (38.9 us per call instead of 32.0 on a few small ones), and a thread takes one at a time.
+// A block sums its counts in shared memory before its six atomics, except on grids of few blocks, whose
+// warps do not queue on a counter: 4 domains of 34^2 x 32 cells (144 blocks each) 42.0 -> 31.9 us per call,
+// 24 of 58^2 x 56 90 -> 73, 2 of 202^2 x 200 113 -> 65, but one of 22^2 x 20 27.2 -> 27.8 with the
+// sums and 27.1 -> 27.1 without.
+constexpr long long kFewBlocks = 64;
+__device__ __forceinline__ bool wide_reads(const exaca_cell_fields &d) {
     return ((reinterpret_cast<unsigned long long>(d.cell_type) | reinterpret_cast<unsigned long long>(d.layer_id) |
              reinterpret_cast<unsigned long long>(d.crit_time_step)) &
             15u) == 0;
@@ -80,6 +85,7 @@ struct CellCount {
     }
 };
 
+template <bool kWide, bool kSums>
 __global__ void __launch_bounds__(kThreads) k_census_cells(const exaca_cell_fields *cells, unsigned long long *acc) {
     const exaca_cell_fields d = cells[blockIdx.y];
     unsigned long long *out = acc + kAccWords * blockIdx.y;
@@ -87,7 +93,7 @@ __global__ void __launch_bounds__(kThreads) k_census_cells(const exaca_cell_fiel
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     CellCount k;
     long long n16 = 0;
-    if (wide_reads(d)) {
+    if (kWide && wide_reads(d)) {
         n16 = d.domain_size / 16;
         for (long long q = tid; q < n16; q += stride) {
             const int4 t16 = __ldcs(reinterpret_cast<const int4 *>(d.cell_type) + q);
@@ -108,17 +114,21 @@ __global__ void __launch_bounds__(kThreads) k_census_cells(const exaca_cell_fiel
     }
     for (long long c = 16 * n16 + tid; c < d.domain_size; c += stride)
         k.cell(d, c, d.cell_type[c], d.layer_id[c], d.crit_time_step[c]);
-    __shared__ unsigned long long s_sum[6];
-    if (threadIdx.x < 6)
-        s_sum[threadIdx.x] = 0;
-    __syncthreads();
+    __shared__ unsigned long long s_sum[kSums ? 6 : 1];
+    if (kSums) {
+        if (threadIdx.x < 6)
+            s_sum[threadIdx.x] = 0;
+        __syncthreads();
+    }
+    unsigned long long *const to = kSums ? s_sum : out;
 #pragma unroll
     for (int q = 0; q < 5; q++) {
-        // a thread counts fewer than 2^32 cells, its warp fewer than 2^37: two halves
-        const unsigned int lo = __reduce_add_sync(0xffffffffu, k.n[q] & 0xffffu),
-                           hi = __reduce_add_sync(0xffffffffu, k.n[q] >> 16);
+        // a thread of the wide kernel counts fewer than 2^32 cells, its warp fewer than 2^37: two halves;
+        // one of the other kernels at most sixteen
+        const unsigned int lo = __reduce_add_sync(0xffffffffu, kWide ? k.n[q] & 0xffffu : k.n[q]),
+                           hi = kWide ? __reduce_add_sync(0xffffffffu, k.n[q] >> 16) : 0u;
         if ((threadIdx.x & 31) == 0 && (lo | hi))
-            atomicAdd(&s_sum[q], ((unsigned long long)hi << 16) + lo);
+            atomicAdd(to + q, ((unsigned long long)hi << 16) + lo);
     }
     unsigned long long neg_mn = k.neg_mn;
     for (int o = 16; o; o >>= 1) {
@@ -126,7 +136,9 @@ __global__ void __launch_bounds__(kThreads) k_census_cells(const exaca_cell_fiel
         neg_mn = v > neg_mn ? v : neg_mn;
     }
     if ((threadIdx.x & 31) == 0 && neg_mn)
-        atomicMax(&s_sum[5], neg_mn);
+        atomicMax(to + 5, neg_mn);
+    if (!kSums)
+        return;
     __syncthreads();
     if (threadIdx.x < 6 && s_sum[threadIdx.x]) {
         if (threadIdx.x < 5)
@@ -162,7 +174,9 @@ void setup(DeviceScratch &s, int device) {
     int sms = 0;
     check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
     cudaFuncAttributes fa;
-    check(cudaFuncGetAttributes(&fa, k_census_cells), "cudaFuncGetAttributes(k_census_cells)");
+    check(cudaFuncGetAttributes(&fa, k_census_cells<true, true>), "cudaFuncGetAttributes(k_census_cells)");
+    check(cudaFuncGetAttributes(&fa, k_census_cells<false, true>), "cudaFuncGetAttributes(k_census_cells)");
+    check(cudaFuncGetAttributes(&fa, k_census_cells<false, false>), "cudaFuncGetAttributes(k_census_cells)");
     s.ptr = static_cast<unsigned char *>(p);
     s.num_sms = sms;
     s.ready = true;
@@ -187,22 +201,21 @@ void census_cells(int device, void *stream, const exaca_cell_fields *domains, in
     setup(s, device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     long long largest = 1;
-    bool wide = true;
-    for (int i = 0; i < n_domains; i++) {
+    for (int i = 0; i < n_domains; i++)
         largest = domains[i].domain_size > largest ? domains[i].domain_size : largest;
-        wide &= wide_reads(domains[i]);
-    }
     unsigned char *desc = s.ptr;
     unsigned long long *acc = reinterpret_cast<unsigned long long *>(s.ptr + kAccOffset);
     try {
         check(cudaMemcpyAsync(desc, domains, n_domains * kDescBytes, cudaMemcpyHostToDevice, st), "descriptor copy");
         check(cudaMemsetAsync(acc, 0, n_domains * kAccWords * sizeof(unsigned long long), st), "accumulator clear");
         long long bx = (4ll * s.num_sms + n_domains - 1) / n_domains;
-        // sixteen cells per thread and step where all can be read so
-        const long long need = (largest / (wide ? 16 : 1) + kThreads - 1) / kThreads;
+        const long long need = (largest + kThreads - 1) / kThreads;
         bx = bx < need ? bx : need;
         bx = bx < 1 ? 1 : bx;
-        k_census_cells<<<dim3((unsigned)bx, (unsigned)n_domains), kThreads, 0, st>>>(
+        const auto kernel = largest >= 16 * bx * kThreads ? k_census_cells<true, true>
+                            : bx >= kFewBlocks            ? k_census_cells<false, true>
+                                                          : k_census_cells<false, false>;
+        kernel<<<dim3((unsigned)bx, (unsigned)n_domains), kThreads, 0, st>>>(
             reinterpret_cast<const exaca_cell_fields *>(desc), acc);
         check(cudaGetLastError(), "k_census_cells launch");
         check(cudaMemcpyAsync(out, acc, n_domains * sizeof(exaca_census), cudaMemcpyDeviceToHost, st), "census copy");
