@@ -805,6 +805,24 @@ __device__ __forceinline__ GrowView grow_view(const DomainDesc &D) {
     g.e_cycle = g.jumps ? (int)executed_upto(D, dyn.cycle) : dyn.cycle;
     return g;
 }
+// What the short growth path needs of a domain without jumps, zero UndercoolingChange or growth extras;
+// cycle kDoneCycle: its records take the general path. A block of the many-domain kernels holds those of
+// the first kViews domains in shared memory, filled at each growth pass (one round of loads). Freed list
+// positions are taken by whichever domain captures next in the block, so the records of a group of 32 come
+// from many domains, and reading their descriptors' sectors per record put every warp's loads on the few
+// L2 sectors that hold them. 256 domains: growth was 76 us per cycle at 2.2e6 records, three times a lone
+// domain's per record; whole maps 1422 -> 1056 ms (96 domains 549 -> 516, 24 domains 418 -> 397). The
+// short path with the fields still read from L2 gained nothing (574 against 547 ms at 96 domains).
+struct alignas(16) ShortView {
+    const double *table; // the growth table from the current cycle's entry, indexed by -CritTimeStep
+    int cycle, len;
+};
+constexpr unsigned int kViews = 320; // what is left of 48 KB
+__device__ __forceinline__ ShortView short_view(const DomainDesc &D, bool extras) {
+    const GrowView g = grow_view(D);
+    const bool plain = !extras && !g.jumps && !g.zero_du && g.cycle != kDoneCycle;
+    return ShortView{g.growth + (plain ? g.cycle : 0), plain ? g.cycle : kDoneCycle, g.growth_len};
+}
 __device__ __forceinline__ GrowView hot_view(const PassCtx &X, const DomainDyn &dyn) {
     GrowView g;
     g.growth = X.hot_desc.growth;
@@ -1679,10 +1697,13 @@ __device__ __noinline__ GrowResult grow_slow(const PassCtx &X, BlockShared *B, D
 // cell comes with the record, for 4 bytes more, so that the slow path does not wait for it and the short
 // one takes domains with per-cell growth extras, jumps and zero UndercoolingChange too; without it the
 // increment of a short-path record is one entry of the domain's table.
-template <int kBatch, bool kOwnClaims, bool kCells>
+// kMany (pools of many domains): every domain's records take the short path, if it has no growth extras,
+// jumps or zero UndercoolingChange; its growth fields come from the block's table of views.
+template <int kBatch, bool kOwnClaims, bool kCells, bool kMany>
 __device__ __forceinline__ void grow_groups(PoolState *P, const PassCtx &X, BlockShared *B, const DomainDyn &dyn, int cur,
                                             unsigned int n, unsigned int gw, unsigned int nw, bool first_pass,
-                                            CycleStats &st, unsigned int &tombs, bool &busy, int &min_cts) {
+                                            CycleStats &st, unsigned int &tombs, bool &busy, int &min_cts,
+                                            const ShortView *views) {
     const unsigned int lane = threadIdx.x & 31, shard = gw % kShards;
     const RecordList &L = X.list[cur];
     ActiveRec *const in = L.rec;
@@ -1721,9 +1742,20 @@ __device__ __forceinline__ void grow_groups(PoolState *P, const PassCtx &X, Bloc
         for (int q = 0; q < kBatch; q++) {
             const unsigned int m = r[q].stat;
             inc[q] = 0.0;
-            if (!(m & (kMaskTomb | kMaskDead | kMaskNuc | kMaskFresh)) && (m & kDirBits) && word_dom(word[q]) == hot) {
-                if (cycle > r[q].cts) {
-                    if (kCells && !plain) {
+            ShortView view{nullptr, kDoneCycle, 0};
+            if (kMany && !(m & kMaskTomb) && word_dom(word[q]) < kViews)
+                view = views[word_dom(word[q])];
+            if (!(m & (kMaskTomb | kMaskDead | kMaskNuc | kMaskFresh)) && (m & kDirBits) &&
+                (kMany ? view.cycle != kDoneCycle : word_dom(word[q]) == hot)) {
+                if ((kMany ? view.cycle : cycle) > r[q].cts) {
+                    if (kMany) {
+                        const int from = max(r[q].cts, 0);
+                        if ((unsigned int)(view.cycle - from) < (unsigned int)view.len) {
+                            grows |= 1u << q;
+                            inc[q] = __ldg(view.table - from);
+                        }
+                    }
+                    else if (kCells && !plain) {
                         inc[q] = load_growth(v0, X.hot_desc, cell[q], r[q].cts, extras);
                         if (inc[q] >= 0.0)
                             grows |= 1u << q;
@@ -1796,9 +1828,10 @@ __device__ __forceinline__ void grow_groups(PoolState *P, const PassCtx &X, Bloc
 
 // With kOwnClaims (B given) the block's flagged records go to its queue and their claim steps follow
 // here. cur is the list to read, n its length; with `compact` the survivors go to the other list.
-template <int kBatch, bool kOwnClaims, int kFamily>
+template <int kBatch, bool kOwnClaims, int kFamily, bool kMany>
 __device__ void grow_pass(PoolState *P, PassCtx &X, BlockShared *B, const DomainDyn &dyn, int cur, unsigned long long n,
-                          bool compact, bool first_pass, CycleStats &st, unsigned int &tombs) {
+                          bool compact, bool first_pass, CycleStats &st, unsigned int &tombs,
+                          const ShortView *views = nullptr) {
     const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned long long nw = (unsigned long long)gridDim.x * (kBlock / 32);
     const unsigned long long gw = (unsigned long long)warp * gridDim.x + blockIdx.x;
@@ -1821,11 +1854,11 @@ __device__ void grow_pass(PoolState *P, PassCtx &X, BlockShared *B, const Domain
     int min_cts = INT_MAX;
     // one group per warp at most: the shorter code for one group is the shorter chain
     if (kFamily != kLongList && (n + 31) / 32 <= nw)
-        grow_groups<1, kOwnClaims, true>(P, X, B, dyn, cur, (unsigned int)n, (unsigned int)gw, (unsigned int)nw, first_pass, st,
-                                   tombs, busy, min_cts);
+        grow_groups<1, kOwnClaims, true, kMany>(P, X, B, dyn, cur, (unsigned int)n, (unsigned int)gw, (unsigned int)nw, first_pass, st,
+                                   tombs, busy, min_cts, views);
     else
-        grow_groups<kBatch, kOwnClaims, kFamily != kLongList>(P, X, B, dyn, cur, (unsigned int)n, (unsigned int)gw, (unsigned int)nw, first_pass,
-                                        st, tombs, busy, min_cts);
+        grow_groups<kBatch, kOwnClaims, kFamily != kLongList, kMany>(P, X, B, dyn, cur, (unsigned int)n, (unsigned int)gw, (unsigned int)nw, first_pass,
+                                        st, tombs, busy, min_cts, views);
     if (kOwnClaims) {
         busy = __any_sync(0xffffffffu, busy);
         min_cts = __reduce_min_sync(0xffffffffu, min_cts);
@@ -2549,7 +2582,7 @@ template <int kBatch> __global__ void __launch_bounds__(kBlock) k_grow(PoolState
     CycleStats st;
     unsigned int tombs = 0;
     const int cur = P->cur;
-    grow_pass<kBatch, false, kLongList>(P, X, nullptr, load_dyn(X.desc[0]), cur, P->cnt[cur], P->compact != 0, false, st, tombs);
+    grow_pass<kBatch, false, kLongList, false>(P, X, nullptr, load_dyn(X.desc[0]), cur, P->cnt[cur], P->compact != 0, false, st, tombs);
     add_tombs(P, tombs);
     flush_stats(P, st);
 }
@@ -2801,15 +2834,16 @@ __device__ __noinline__ void start_next(PoolState *P, BlockShared &B, unsigned i
 // is past some record's CritTimeStep or needs its start: they only advance the cycle number. Of the
 // cycles of a 64^3 solve 32 % make no claim (19 % grow nothing), of 3 x 3 spot melts 57 % (57 %), of
 // small three-layer ones 86 % (74 %); an idle cycle took 4.8 us, one with growth and no claim about 7.
-template <int kFamily, int kBatch>
+template <int kFamily, int kBatch, bool kMany>
 __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles, AliveSet alive) {
     __shared__ BlockShared B;
+    __shared__ ShortView views[kMany ? kViews : 1];
     CycleStats st;
     // the start of the launch's first cycle: one block for a few domains, a warp per domain across
     // the grid for many; later cycles are started under the capture pass (start_next)
     DomainDesc *const desc = P->desc;
     const int n_domains = P->n_domains;
-    const bool spread = alive.n < 0;
+    const bool spread = kMany || alive.n < 0;
     const int n_start = spread ? n_domains : alive.n;
     unsigned long long *const tl = P->timeline;
     unsigned int meet = 0;
@@ -2862,7 +2896,12 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
         // growth with each block's claims right after its own growth; the global claim pass only
         // when some block's queue overflowed this cycle (the same answer for every block)
         unsigned int dropped = 0;
-        grow_pass<kBatch, true, kFamily>(P, B.X, &B, dyn, cur, n, compact, passes == 0, st, dropped);
+        if (kMany) {
+            for (unsigned int d = threadIdx.x; d < min((unsigned int)n_domains, kViews); d += kBlock)
+                views[d] = short_view(B.X.desc[d], B.X.extras);
+            __syncthreads();
+        }
+        grow_pass<kBatch, true, kFamily, kMany>(P, B.X, &B, dyn, cur, n, compact, passes == 0, st, dropped, views);
         dropped = __reduce_add_sync(0xffffffffu, dropped);
         if ((threadIdx.x & 31) == 0 && dropped)
             atomicAdd(&B.tombs, (int)dropped);
@@ -2997,13 +3036,14 @@ __global__ void __launch_bounds__(kBlock) k_meet_probe(PoolState *P) {
 
 // Compiled launch shapes.
 struct StepKernels {
-    const void *cycles;
+    const void *cycles, *cycles_many; // up to kSerialDomains running, more
     void (*grow)(PoolState *);
     void (*capture_begin)(PoolState *);
     void (*capture_end)(PoolState *);
 };
 template <int kF, int kB> StepKernels step_kernels() {
-    return {(const void *)k_cycles<kF, kB>, k_grow<kB>, k_capture_pass<true>, k_capture_pass<false>};
+    return {(const void *)k_cycles<kF, kB, false>, (const void *)k_cycles<kF, kB, true>, k_grow<kB>,
+            k_capture_pass<true>, k_capture_pass<false>};
 }
 static_assert(kStepVariants == 4, "the shapes below");
 const StepKernels kStepKernel[kStepVariants] = {
@@ -3369,12 +3409,15 @@ void Pool::to_host(const std::vector<HostCopy> &copies, void *stream) {
     }
     if (pieces.empty())
         return;
-    // The pieces are as large as the copies need, up to kStageBytes: page-locking 64 MB takes some 20 ms,
-    // half of a 64^3 solve, when a new pool's first results are a megabyte (a new pool's first solve 71 -> 38 ms). They double when larger results come.
-    // No piece is in flight here.
+    // The pieces are as large as this copy or the largest domain's GrainID needs, up to kStageBytes:
+    // page-locking 64 MB takes some 30 ms (a new pool's first 64^3 solve 71 -> 38 ms), but each growth also
+    // waits for what runs on the device. No piece is in flight here.
     size_t need = 0;
     for (const Piece &q : pieces)
         need = std::max(need, q.len);
+    for (const auto &q : slots_)
+        if (q.used)
+            need = std::max(need, (size_t)q.problem->g.domain_size * 4);
     if (need > stage_bytes_) {
         need = std::min(kStageBytes, std::max(2 * stage_bytes_, (need + (size_t(1) << 20) - 1) >> 20 << 20));
         stage_bytes_ = 0;
@@ -3488,6 +3531,9 @@ Pool::Pool(int device, size_t budget_bytes, unsigned long long list_capacity)
     int b = 0;
     for (int v = 0; v < kStepVariants; v++) {
         CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kStepKernel[v].cycles, kBlock, 0));
+        int many = 0;
+        CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&many, kStepKernel[v].cycles_many, kBlock, 0));
+        b = std::min(b, many);
         if (b < 1)
             throw DeviceError("persistent kernel does not fit on an SM");
         grid_cycles_[v] = num_sms_ * b;
@@ -3938,7 +3984,10 @@ void Pool::launch_persistent(int n) {
                       ? variant_
                       : shape_for(last_records_);
     const int grid = std::max(1, std::min(kMeetMaxGrid, grid_cycles_[v]) / std::max(1, grid_fixed_));
-    CUDA_OK(cudaLaunchCooperativeKernel(kStepKernel[v].cycles, dim3(grid), dim3(kBlock), args, 0, st));
+    // many domains: a round of loads more per cycle for the views, which up to kSerialDomains do not repay
+    // (a map of 96: 14.5 -> 15.5 us per cycle with seven running)
+    const void *const kernel = alive.n < 0 ? kStepKernel[v].cycles_many : kStepKernel[v].cycles;
+    CUDA_OK(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kBlock), args, 0, st));
     launches_ += 1;
 }
 

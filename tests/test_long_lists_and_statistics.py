@@ -12,6 +12,7 @@ import pytest
 from helpers import input_path, load_golden
 
 import exaca_b200 as ex
+from exaca_b200 import batch
 
 sys.path.insert(0, os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "oracle"))
 import grain_stats as gs  # noqa: E402
@@ -56,6 +57,38 @@ def test_records_past_the_bodies(lib, large_domains, config):
             g, c = pool.copy_out(s)
             assert np.array_equal(g, gid) and np.array_equal(c, ct), f"domain {k}"
     finally:
+        pool.close()
+
+
+def test_more_domains_than_growth_views(lib):
+    """The last domains lie past the block's table of growth fields and take the general path."""
+    params = batch.process_map(332, seed=12, side=(5, 9), G=(1e6, 4e6), R=(5e5, 1e6), density=(1e15, 1e16))
+    probs = batch.build_problems(params)
+    plain = batch.solve_plain(probs)
+    res = batch.solve_batch(probs, chunk_cycles=250)
+    for i in range(len(probs)):
+        assert res["cycle"][i] == plain["cycle"][i], f"domain {i}"
+        assert np.array_equal(res["grain_id"][i], plain["grain_id"][i]), f"domain {i}"
+        assert np.array_equal(res["cell_type"][i], plain["cell_type"][i]), f"domain {i}"
+
+
+def test_spot_melts_among_many_domains(lib):
+    """A multilayer type-S domain (growth extras: no short path for any domain) among ten type-C ones."""
+    probs = batch.build_problems(batch.process_map(10, seed=13, side=(8, 14), G=(1e6, 4e6), R=(5e5, 1e6)))
+    for case in ("SmallSpotMelt", "SpotMelt3Layers"):
+        spot = ex.Problem.from_file(input_path(case))
+        alone = ex.Pool(0, list_capacity=spot.geometry.active_size)
+        a = alone.admit(spot, device_check=False)
+        pool = ex.Pool(0, list_capacity=1 << 20)
+        s = pool.admit(spot, device_check=False)
+        for p in probs:
+            pool.admit(p, device_check=True)
+        for n in (150, 400):
+            alone.step(n)
+            pool.step(n)
+            for u, v in zip(alone.copy_out(a) + alone.copy_octahedra(a)[:1], pool.copy_out(s) + pool.copy_octahedra(s)[:1]):
+                assert np.array_equal(u, v), (case, n)
+        alone.close()
         pool.close()
 
 
