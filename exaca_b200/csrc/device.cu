@@ -3418,6 +3418,7 @@ void Pool::to_host(const std::vector<HostCopy> &copies, void *stream) {
     for (const auto &q : slots_)
         if (q.used)
             need = std::max(need, (size_t)q.problem->g.domain_size * 4);
+    need = std::min(kStageBytes, need);
     if (need > stage_bytes_) {
         need = std::min(kStageBytes, std::max(2 * stage_bytes_, (need + (size_t(1) << 20) - 1) >> 20 << 20));
         stage_bytes_ = 0;
