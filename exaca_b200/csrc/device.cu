@@ -124,14 +124,24 @@ __device__ __forceinline__ long long executed_upto(const DomainDesc &D, long lon
     return e;
 }
 
-// Block-aggregated reservation of `n` slots per thread on `counter`: one atomicAdd per block. Must
-// be called by every thread of the block. Returns this thread's first slot, or ULLONG_MAX on
-// overflow (the pool error flag is set).
+// What a reservation of [first, first + total) takes past `cap` is given back and flagged. A counter that
+// has reached its limit never falls below it, so every slot below `cap` belongs to one reservation, whose
+// owner writes it, and no counter stays past the array that it counts.
+__device__ __forceinline__ void reserved_past(unsigned long long *counter, unsigned long long cap, int *error,
+                                              unsigned long long first, unsigned long long total) {
+    if (first + total <= cap)
+        return;
+    atomicOr(error, kErrListOverflow);
+    atomicAdd(counter, (first > cap ? first : cap) - (first + total));
+}
+
+// Block-aggregated reservation of `n` (0 or 1) slots per thread on `counter`: one atomicAdd per block.
+// Must be called by every thread of the block. Returns this thread's slot, or ULLONG_MAX past `cap` (the
+// pool error flag is set).
 __device__ __forceinline__ unsigned long long block_reserve_on(unsigned long long *counter, unsigned long long cap,
                                                               int *error, unsigned int n) {
     __shared__ unsigned int s_warp[32];
     __shared__ unsigned long long s_base;
-    __shared__ int s_ok;
     // the launch's own warp count (callers launch with different block sizes)
     const unsigned int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     unsigned int incl = n;
@@ -158,16 +168,14 @@ __device__ __forceinline__ unsigned long long block_reserve_on(unsigned long lon
         unsigned int total = __shfl_sync(0xffffffffu, inc2, n_warps - 1);
         if (lane == 0) {
             unsigned long long b = total ? atomicAdd(counter, (unsigned long long)total) : 0ull;
-            s_ok = (b + total <= cap);
-            if (!s_ok)
-                atomicOr(error, kErrListOverflow);
+            reserved_past(counter, cap, error, b, total);
             s_base = b;
         }
     }
     __syncthreads();
-    unsigned long long r = s_ok ? s_base + s_warp[warp] + (incl - n) : ULLONG_MAX;
+    const unsigned long long r = s_base + s_warp[warp] + (incl - n);
     __syncthreads(); // s_warp / s_base are reused by the next call
-    return r;
+    return r < cap ? r : ULLONG_MAX;
 }
 
 __device__ __forceinline__ unsigned long long block_reserve(PoolState *P, int slot, unsigned int n) {
@@ -181,15 +189,13 @@ __device__ __forceinline__ unsigned long long warp_reserve(unsigned long long *c
     int lane = threadIdx.x & 31;
     int leader = __ffs(act) - 1;
     unsigned long long base = 0;
-    if (lane == leader)
+    if (lane == leader) {
         base = atomicAdd(counter, (unsigned long long)__popc(act));
-    base = __shfl_sync(act, base, leader);
-    unsigned long long r = base + __popc(act & ((1u << lane) - 1));
-    if (r >= cap) {
-        atomicOr(error, kErrListOverflow);
-        return ULLONG_MAX;
+        reserved_past(counter, cap, error, base, (unsigned long long)__popc(act));
     }
-    return r;
+    base = __shfl_sync(act, base, leader);
+    const unsigned long long r = base + __popc(act & ((1u << lane) - 1));
+    return r < cap ? r : ULLONG_MAX;
 }
 
 // Block-level sum of per-thread statistics into one shard of the pool counters.
@@ -913,7 +919,8 @@ __device__ __noinline__ unsigned int drop_nucleated(const DomainDesc &D, unsigne
 // claim pass needs (list position, cell, domain, liquid-neighbour mask, grown DiagonalLength), so the
 // claim pass needs no dependent load before its own round of loads.
 // Warp-aggregated reservation of n slots per lane on a global counter (every lane of the warp
-// calls). Returns this lane's first slot, or ULLONG_MAX past `cap` (the pool error flag is set).
+// calls). Returns this lane's first slot; the caller writes those of its slots that lie below `cap`
+// (where one does not, the pool error flag is set).
 __device__ __forceinline__ unsigned long long warp_reserve_n(unsigned long long *counter, unsigned long long cap,
                                                              int *error, unsigned int n) {
     const unsigned int lane = threadIdx.x & 31;
@@ -926,14 +933,11 @@ __device__ __forceinline__ unsigned long long warp_reserve_n(unsigned long long 
     }
     const unsigned int total = __shfl_sync(0xffffffffu, incl, 31);
     unsigned long long base = 0;
-    if (lane == 31 && total)
+    if (lane == 31 && total) {
         base = atomicAdd(counter, (unsigned long long)total);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    if (base + total > cap) {
-        if (lane == 31 && total)
-            atomicOr(error, kErrListOverflow);
-        return ULLONG_MAX;
+        reserved_past(counter, cap, error, base, total);
     }
+    base = __shfl_sync(0xffffffffu, base, 31);
     return base + incl - n;
 }
 
@@ -1222,11 +1226,12 @@ template <int kBatch>
 __device__ __forceinline__ void queue_flagged(PoolState *P, unsigned int shard, unsigned int nf, unsigned int flagged,
                                               const unsigned int *idx, const ActiveRec *r, const unsigned int *dom) {
     unsigned long long k = warp_reserve_n(&P->qcnt_s[shard].v, P->shard_cap, &P->error, nf);
-    if (nf && k != ULLONG_MAX) {
+    if (nf) {
+        const unsigned long long end = (shard + 1ull) * P->shard_cap;
         k += (unsigned long long)shard * P->shard_cap;
 #pragma unroll
         for (int q = 0; q < kBatch; q++) {
-            if (flagged & (1u << q)) {
+            if ((flagged & (1u << q)) && k < end) {
                 P->qpos[k] = idx[q];
                 P->qdom[k] = word_dom(dom[q]);
                 P->qmask[k] = r[q].stat;
@@ -1618,7 +1623,7 @@ __device__ __noinline__ void compact_pass(PoolState *P, const PassCtx &X, int cu
             }
         }
         const unsigned long long pos = warp_reserve_n(&P->cnt[nxt], X.capacity, &P->error, keep ? 1u : 0u);
-        if (!(keep && pos != ULLONG_MAX))
+        if (!(keep && pos < X.capacity))
             flag = false;
         else {
             to.rec[pos] = r;
@@ -1945,7 +1950,7 @@ __device__ void claim_pass(PoolState *P, PassCtx &X, BlockShared *B, int app, Cy
                     const unsigned int t = (unsigned int)((long long)cl.cell + nb_offset(l, D.mx * D.my, D.my));
                     atomicMin(D.claim + t, key);
                     D.ctype[t] = kTemporaryUpdate;
-                    if (pos != ULLONG_MAX)
+                    if (pos < cap)
                         P->tgt[shard * cap + pos++] = claim_entry_of(cl.dom, l, t);
                 }
                 st.claims += __popc(cl.reach);
@@ -2779,10 +2784,8 @@ __device__ __noinline__ void start_next(PoolState *P, BlockShared &B, unsigned i
         if (lane == 0) {
             slot0 = base + atomicAdd(appended, (unsigned long long)n_fire);
             atomicAdd(&B.n_appended, n_fire);
-            if (slot0 + n_fire > B.X.capacity) {
+            if (slot0 + n_fire > B.X.capacity)
                 atomicOr(&P->error, kErrListOverflow);
-                slot0 = ULLONG_MAX;
-            }
         }
         slot0 = __shfl_sync(0xffffffffu, slot0, 0);
         for (unsigned int todo = firing; todo; todo &= todo - 1) {
@@ -2790,7 +2793,7 @@ __device__ __noinline__ void start_next(PoolState *P, BlockShared &B, unsigned i
             const unsigned int rank = __popc(firing & ((1u << src) - 1u));
             nucleate_site(V, s.ctype, L, d,
                           (unsigned int)__shfl_sync(0xffffffffu, l, src), __shfl_sync(0xffffffffu, h, src),
-                          __shfl_sync(0xffffffffu, cts, src), slot0 == ULLONG_MAX ? ULLONG_MAX : slot0 + rank,
+                          __shfl_sync(0xffffffffu, cts, src), slot0 + rank < B.X.capacity ? slot0 + rank : ULLONG_MAX,
                           [&](unsigned int nb_pos, int) {
                               if (nb_pos < base)
                                   atomicOr(&L.rec[nb_pos].stat, kMaskNuc);
