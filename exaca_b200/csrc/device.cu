@@ -3562,13 +3562,13 @@ Pool::Pool(int device, size_t budget_bytes, unsigned long long list_capacity)
     }
     CUDA_OK(cudaMalloc(&dstate_, sizeof(PoolState)));
     CUDA_OK(cudaMalloc(&ddesc_, sizeof(DomainDesc) * (max_domains_ + 1)));
-    CUDA_OK(cudaMemset(ddesc_, 0, sizeof(DomainDesc) * (max_domains_ + 1)));
+    CUDA_OK(cudaMemsetAsync(ddesc_, 0, sizeof(DomainDesc) * (max_domains_ + 1), s));
     {
         // descriptor max_domains_ is a placeholder that is always finished
         DomainDesc ph;
         std::memset(&ph, 0, sizeof(ph));
         ph.done = 1;
-        CUDA_OK(cudaMemcpy(ddesc_ + max_domains_, &ph, sizeof(ph), cudaMemcpyHostToDevice));
+        CUDA_OK(cudaMemcpyAsync(ddesc_ + max_domains_, &ph, sizeof(ph), cudaMemcpyHostToDevice, s));
     }
     PoolState ps;
     std::memset(&ps, 0, sizeof(ps));
@@ -3595,7 +3595,7 @@ Pool::Pool(int device, size_t budget_bytes, unsigned long long list_capacity)
     ps.pending = 0;
     ps.n_domains = 0;
     ps.desc = ddesc_;
-    CUDA_OK(cudaMemcpy(dstate_, &ps, sizeof(ps), cudaMemcpyHostToDevice));
+    CUDA_OK(cudaMemcpyAsync(dstate_, &ps, sizeof(ps), cudaMemcpyHostToDevice, s));
     CUDA_OK(cudaMalloc(&census_buf_, sizeof(Census)));
 }
 
@@ -3655,8 +3655,12 @@ const DeviceTables &Pool::tables_for(const Problem &p) {
     DeviceTables t;
     CUDA_OK(cudaMalloc(&t.guv, p.guv.size() * sizeof(float)));
     CUDA_OK(cudaMalloc(&t.cdl_table, p.cdl_table.size() * sizeof(float)));
-    CUDA_OK(cudaMemcpy(t.guv, p.guv.data(), p.guv.size() * sizeof(float), cudaMemcpyHostToDevice));
-    CUDA_OK(cudaMemcpy(t.cdl_table, p.cdl_table.data(), p.cdl_table.size() * sizeof(float), cudaMemcpyHostToDevice));
+    // on the pool's stream, as everything that its kernels read: it does not wait for the legacy stream, where
+    // a copy from pageable memory may still be under way when the call returns
+    cudaStream_t st = S(stream_);
+    CUDA_OK(cudaMemcpyAsync(t.guv, p.guv.data(), p.guv.size() * sizeof(float), cudaMemcpyHostToDevice, st));
+    CUDA_OK(cudaMemcpyAsync(t.cdl_table, p.cdl_table.data(), p.cdl_table.size() * sizeof(float), cudaMemcpyHostToDevice,
+                            st));
     h2d_bytes_ += (p.guv.size() + p.cdl_table.size()) * sizeof(float);
     return tables_[p.cfg.orientation_file] = t;
 }
@@ -4762,8 +4766,13 @@ GrainStats Pool::grain_stats(int slot, const int *region) {
         }
         float *d = nullptr;
         CUDA_OK(cudaMalloc(&d, mis.size() * sizeof(float)));
+        // on the stream of the kernels that read it (tables_for); kept only once it is filled
+        const cudaError_t filled =
+            cudaMemcpyAsync(d, mis.data(), mis.size() * sizeof(float), cudaMemcpyHostToDevice, S(stream_));
+        if (filled != cudaSuccess)
+            cudaFree(d);
+        CUDA_OK(filled);
         tb.mis = d;
-        CUDA_OK(cudaMemcpy(d, mis.data(), mis.size() * sizeof(float), cudaMemcpyHostToDevice));
     }
     cudaStream_t st = S(stream_);
     const size_t N = g.domain_size;
