@@ -311,6 +311,13 @@ __device__ __forceinline__ float4 &body_head(RecordBody &b) { return *reinterpre
 //      list positions (the list slots of all firing sites are reserved under the first such round).
 // Reads that may see data other blocks of the same kernel wrote go through L2 (__ldcg).
 
+// Entries of a queue's shard: none where its counter went past the shard's slots, since the warps that crossed
+// the limit wrote none of theirs (the pool's overflow flag is set; what the shard held is not acted on).
+__device__ __forceinline__ unsigned long long shard_count(const ShardCounter &c, unsigned long long cap) {
+    const unsigned long long n = __ldcg(&c.v);
+    return n <= cap ? n : 0ull;
+}
+
 // Pool part (warp 0): when `close`, the records the last capture pass appended join the list the
 // next cycle reads, which ends the previous cycle; then the list swap, the compaction decision and
 // the per-cycle counters. One round of loads. The list this cycle reads goes to *cur_out if given.
@@ -319,7 +326,7 @@ __device__ __forceinline__ void lists_start(PoolState *P, bool close, int *cur_o
         static_assert(kShards == 32, "one lane per shard");
         const int lane = threadIdx.x;
         unsigned long long added = __ldcg(&P->tomb_s[lane].v);
-        unsigned long long appended = close ? __ldcg(&P->tcnt_s[lane].v) : 0ull;
+        unsigned long long appended = close ? shard_count(P->tcnt_s[lane], P->shard_cap) : 0ull;
         int prev = 0, cur = 0;
         unsigned long long cnt0 = 0, cnt1 = 0, tombs = 0, cap = 0;
         if (lane == 0) {
@@ -919,8 +926,8 @@ __device__ __noinline__ unsigned int drop_nucleated(const DomainDesc &D, unsigne
 // claim pass needs (list position, cell, domain, liquid-neighbour mask, grown DiagonalLength), so the
 // claim pass needs no dependent load before its own round of loads.
 // Warp-aggregated reservation of n slots per lane on a global counter (every lane of the warp
-// calls). Returns this lane's first slot; the caller writes those of its slots that lie below `cap`
-// (where one does not, the pool error flag is set).
+// calls). Returns this lane's first slot, or ULLONG_MAX past `cap` (the pool error flag is set, and the
+// counter stays past cap: shard_count).
 __device__ __forceinline__ unsigned long long warp_reserve_n(unsigned long long *counter, unsigned long long cap,
                                                              int *error, unsigned int n) {
     const unsigned int lane = threadIdx.x & 31;
@@ -933,11 +940,14 @@ __device__ __forceinline__ unsigned long long warp_reserve_n(unsigned long long 
     }
     const unsigned int total = __shfl_sync(0xffffffffu, incl, 31);
     unsigned long long base = 0;
-    if (lane == 31 && total) {
+    if (lane == 31 && total)
         base = atomicAdd(counter, (unsigned long long)total);
-        reserved_past(counter, cap, error, base, total);
-    }
     base = __shfl_sync(0xffffffffu, base, 31);
+    if (base + total > cap) {
+        if (lane == 31 && total)
+            atomicOr(error, kErrListOverflow);
+        return ULLONG_MAX;
+    }
     return base + incl - n;
 }
 
@@ -1226,12 +1236,11 @@ template <int kBatch>
 __device__ __forceinline__ void queue_flagged(PoolState *P, unsigned int shard, unsigned int nf, unsigned int flagged,
                                               const unsigned int *idx, const ActiveRec *r, const unsigned int *dom) {
     unsigned long long k = warp_reserve_n(&P->qcnt_s[shard].v, P->shard_cap, &P->error, nf);
-    if (nf) {
-        const unsigned long long end = (shard + 1ull) * P->shard_cap;
+    if (nf && k != ULLONG_MAX) {
         k += (unsigned long long)shard * P->shard_cap;
 #pragma unroll
         for (int q = 0; q < kBatch; q++) {
-            if ((flagged & (1u << q)) && k < end) {
+            if (flagged & (1u << q)) {
                 P->qpos[k] = idx[q];
                 P->qdom[k] = word_dom(dom[q]);
                 P->qmask[k] = r[q].stat;
@@ -1623,7 +1632,7 @@ __device__ __noinline__ void compact_pass(PoolState *P, const PassCtx &X, int cu
             }
         }
         const unsigned long long pos = warp_reserve_n(&P->cnt[nxt], X.capacity, &P->error, keep ? 1u : 0u);
-        if (!(keep && pos < X.capacity))
+        if (!(keep && pos != ULLONG_MAX))
             flag = false;
         else {
             to.rec[pos] = r;
@@ -1886,10 +1895,10 @@ __device__ __forceinline__ void add_tombs(PoolState *P, unsigned int tombs) {
 }
 
 // Exclusive prefix of the shard counts in shared memory (all threads of the block call).
-__device__ __forceinline__ void shard_prefix(const ShardCounter *cnt, unsigned long long *pre) {
+__device__ __forceinline__ void shard_prefix(const ShardCounter *cnt, unsigned long long cap, unsigned long long *pre) {
     if (threadIdx.x < 32) {
         const unsigned int lane = threadIdx.x;
-        const unsigned long long c = __ldcg(&cnt[lane].v);
+        const unsigned long long c = shard_count(cnt[lane], cap);
         unsigned long long incl = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -1921,9 +1930,9 @@ __device__ __forceinline__ unsigned long long shard_entry(const unsigned long lo
 template <bool kOwnClaims>
 __device__ void claim_pass(PoolState *P, PassCtx &X, BlockShared *B, int app, CycleStats &st, unsigned int &tombs) {
     __shared__ unsigned long long s_pre[kShards + 1];
-    shard_prefix(P->qcnt_s, s_pre);
-    const unsigned long long nq = s_pre[kShards];
     const unsigned long long cap = X.shard_cap;
+    shard_prefix(P->qcnt_s, cap, s_pre);
+    const unsigned long long nq = s_pre[kShards];
     const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned long long nw = (unsigned long long)gridDim.x * (kBlock / 32);
     const unsigned long long gw = (unsigned long long)warp * gridDim.x + blockIdx.x;
@@ -1950,7 +1959,7 @@ __device__ void claim_pass(PoolState *P, PassCtx &X, BlockShared *B, int app, Cy
                     const unsigned int t = (unsigned int)((long long)cl.cell + nb_offset(l, D.mx * D.my, D.my));
                     atomicMin(D.claim + t, key);
                     D.ctype[t] = kTemporaryUpdate;
-                    if (pos < cap)
+                    if (pos != ULLONG_MAX)
                         P->tgt[shard * cap + pos++] = claim_entry_of(cl.dom, l, t);
                 }
                 st.claims += __popc(cl.reach);
@@ -2518,10 +2527,10 @@ struct CaptureShared {
 };
 __device__ void capture_pass(PoolState *P, const PassCtx &X, CaptureShared &C, CycleStats &st) {
     __shared__ unsigned long long s_pre[kShards + 1];
-    shard_prefix(P->tcnt_s, s_pre);
+    const unsigned long long cap = P->shard_cap;
+    shard_prefix(P->tcnt_s, cap, s_pre);
     const int app = P->pending; // list of the next cycle
     const unsigned long long T = s_pre[kShards];
-    const unsigned long long cap = P->shard_cap;
     const unsigned long long base = P->cnt[app];
     if (base + T > P->capacity) {
         if (threadIdx.x == 0 && blockIdx.x == 0)
@@ -2567,7 +2576,7 @@ __device__ void capture_pass(PoolState *P, const PassCtx &X, CaptureShared &C, C
 // End of a cycle: the record slots of this cycle's claims join the list.
 __device__ void finish_capture(PoolState *P) {
     if (threadIdx.x < 32) {
-        unsigned long long T = __ldcg(&P->tcnt_s[threadIdx.x].v);
+        unsigned long long T = shard_count(P->tcnt_s[threadIdx.x], P->shard_cap);
 #pragma unroll
         for (int o = 16; o; o >>= 1)
             T += __shfl_down_sync(0xffffffffu, T, o);
@@ -2784,8 +2793,12 @@ __device__ __noinline__ void start_next(PoolState *P, BlockShared &B, unsigned i
         if (lane == 0) {
             slot0 = base + atomicAdd(appended, (unsigned long long)n_fire);
             atomicAdd(&B.n_appended, n_fire);
-            if (slot0 + n_fire > B.X.capacity)
+            if (slot0 + n_fire > B.X.capacity) {
                 atomicOr(&P->error, kErrListOverflow);
+                for (; slot0 < B.X.capacity; slot0++) // what is left of the list holds no record
+                    L.rec[slot0].stat = kMaskTomb;
+                slot0 = ULLONG_MAX;
+            }
         }
         slot0 = __shfl_sync(0xffffffffu, slot0, 0);
         for (unsigned int todo = firing; todo; todo &= todo - 1) {
@@ -2793,7 +2806,7 @@ __device__ __noinline__ void start_next(PoolState *P, BlockShared &B, unsigned i
             const unsigned int rank = __popc(firing & ((1u << src) - 1u));
             nucleate_site(V, s.ctype, L, d,
                           (unsigned int)__shfl_sync(0xffffffffu, l, src), __shfl_sync(0xffffffffu, h, src),
-                          __shfl_sync(0xffffffffu, cts, src), slot0 + rank < B.X.capacity ? slot0 + rank : ULLONG_MAX,
+                          __shfl_sync(0xffffffffu, cts, src), slot0 == ULLONG_MAX ? ULLONG_MAX : slot0 + rank,
                           [&](unsigned int nb_pos, int) {
                               if (nb_pos < base)
                                   atomicOr(&L.rec[nb_pos].stat, kMaskNuc);
