@@ -360,7 +360,8 @@ __device__ __forceinline__ void lists_start(PoolState *P, bool close, int *cur_o
             // the list the previous cycle left becomes current; when it was a compacted copy, the old
             // one is emptied and carries no dropped records any more
             const unsigned long long cnt_cur = cur ? cnt1 : cnt0;
-            tombs += added;
+            // the sum of what blocks of the persistent kernel had not told may be negative
+            tombs = (unsigned long long)max((long long)(tombs + added), 0ll);
             if (cur != prev) {
                 P->cnt[prev] = 0;
                 tombs = 0;
@@ -1858,8 +1859,7 @@ __device__ void grow_pass(PoolState *P, PassCtx &X, BlockShared *B, const Domain
         compact_pass(P, X, cur, gw, nw, n, dyn, st, kOwnClaims ? B : nullptr);
         if (kOwnClaims) {
             B->busy = 1;
-            unsigned int claim_tombs = 0; // a compacted list starts without dropped records
-            block_claims<kFamily>(P, *B, cur ^ 1, st, claim_tombs);
+            block_claims<kFamily>(P, *B, cur ^ 1, st, tombs);
         }
         return;
     }
@@ -2842,6 +2842,8 @@ __device__ __noinline__ void start_next(PoolState *P, BlockShared &B, unsigned i
         atomicAdd(&P->stat[blockIdx.x & (kStatShards - 1)][kStatNucleated], (unsigned long long)fired_total);
 }
 
+constexpr int kTellLeast = 16; // dropped records for which a block asks for a meeting (k_cycles)
+
 // n_cycles complete CA cycles (start, grow/claim, capture) in one cooperative launch.
 //
 // With one running domain a cycle is cut short where nothing is left of it. A cycle without claims
@@ -2909,6 +2911,11 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
         // compact when dropped records exceed a quarter of the list, as lists_start
         const bool compact = tombs * 4 > n;
         const int app = compact ? cur ^ 1 : cur; // list of the next cycle
+        if (compact && threadIdx.x == 0) {
+            // positions in the old list; counted again, for the new one, after grow_pass's block barrier
+            B.n_free = 0;
+            B.tombs = 0;
+        }
         // growth with each block's claims right after its own growth; the global claim pass only
         // when some block's queue overflowed this cycle (the same answer for every block)
         unsigned int dropped = 0;
@@ -2921,8 +2928,14 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
         dropped = __reduce_add_sync(0xffffffffu, dropped);
         if ((threadIdx.x & 31) == 0 && dropped)
             atomicAdd(&B.tombs, (int)dropped);
-        // sums: first claims of the hot domain, blocks whose queue overflowed, blocks that are busy
-        constexpr int kOverflowShift = 40, kBusyShift = 48;
+        // sums: first claims of the hot domain (32 bits, as cell indices), blocks that would tell, blocks whose
+        // queue overflowed, blocks that are busy. A block tells its dropped records at the meeting after the
+        // captures, which a lone domain's cycle without claims leaves out; it asks for that meeting when the
+        // list would be due for compaction if every block had dropped as many as itself: were it due, a block
+        // with the mean or more would ask. Fewer than kTellLeast wait for the next meeting or the launch's end
+        // (all blocks' together are at most one more group of 32 for a few of the warps; three-layer spots
+        // lost 1 % to the meetings that they asked for).
+        constexpr int kTellShift = 32, kOverflowShift = 40, kBusyShift = 48;
         int *const grid_min = reinterpret_cast<int *>(&P->meet.min_cts[passes % 3].v);
         const auto claim_share = [&] {
             const unsigned long long v = B.n_first;
@@ -2932,23 +2945,22 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
         ok = grid_meet(
             P, meet, tl, 3 * c + 1,
             [&] {
-                const unsigned long long v = claim_share() + (B.n_items > (unsigned int)kBlockQueue ? 1ull << kOverflowShift : 0ull) +
+                // (the difference wraps to a large one in a cycle that compacts)
+                const bool tell = B.tombs >= kTellLeast && (unsigned int)B.tombs * gridDim.x > (unsigned int)(n >> 2) - (unsigned int)tombs;
+                const unsigned long long v = claim_share() + (tell ? 1ull << kTellShift : 0ull) +
+                                             (B.n_items > (unsigned int)kBlockQueue ? 1ull << kOverflowShift : 0ull) +
                                              ((unsigned long long)B.busy << kBusyShift);
                 if (!B.busy && B.min_cts != INT_MAX)
                     atomicMin(grid_min, B.min_cts);
                 B.n_items = B.busy = 0;
                 B.min_cts = INT_MAX;
-                if (compact) {
-                    // positions in the old list
-                    B.n_free = 0;
-                    B.tombs = 0;
-                }
                 return v;
             },
             total);
         if (!ok)
             break;
-        unsigned long long claimed = total & ((1ull << kOverflowShift) - 1);
+        unsigned long long claimed = total & 0xffffffffull;
+        const bool asked = (total & ((1ull << kBusyShift) - 1)) != 0; // claims, drops to tell, an overflow
         const bool overflow = ((total >> kOverflowShift) & 0xffu) != 0, busy = (total >> kBusyShift) != 0;
         if (blockIdx.x == 0 && threadIdx.x == 0) // read after the previous cycle's meeting, used two cycles on
             *reinterpret_cast<int *>(&P->meet.min_cts[(passes + 2) % 3].v) = INT_MAX;
@@ -2971,7 +2983,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
             if (overflow)
                 P->qcnt_s[threadIdx.x].v = 0;
         }
-        started = !solo || claimed || overflow || (!dyn.done && c + 1 < n_cycles && dyn.cycle + 1 >= dyn.next_start);
+        started = !solo || asked || (!dyn.done && c + 1 < n_cycles && dyn.cycle + 1 >= dyn.next_start);
         if (!started) {
             n = base;
             if (compact)
@@ -3027,6 +3039,9 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
         tombs = (unsigned long long)max((long long)(compact ? 0 : tombs) + change, 0ll);
         cur = app;
     }
+    // what the block has not told, for the next launch's start (lists_start)
+    if (ok && threadIdx.x == 0 && B.tombs)
+        atomicAdd(&P->tomb_s[blockIdx.x % kShards].v, (unsigned long long)(long long)B.tombs);
     if (ok && blockIdx.x == 0 && threadIdx.x == 0) {
         P->cur = P->pending = cur;
         P->cnt[cur] = n;

@@ -59,3 +59,23 @@ def test_at_the_capacity(lib):
     assert res[0][0] == res[1][0]
     for a, b in zip(res[0][1:], res[1][1:]):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("chunk", [1, 7, 1000])
+def test_dropped_records_leave_the_list(lib, chunk):
+    # solves one after the other in a list of 2.4 times their 1024 records, of which no cell ever claims another:
+    # the records dropped in cycles without claims, and in the last cycles of a launch, make room too
+    p = problem(nx=30, ny=30, nz=1, density=0.0)
+    pool = ex.Pool(0, list_capacity=2500)
+    try:
+        for solve in range(5):
+            slot = pool.admit(p, device_check=False)
+            for _ in range(max(1, 35 // chunk)):
+                pool.step(chunk)
+            st = pool.status(slot)
+            assert st.error == 0, f"solve {solve}"
+            _, ct = pool.copy_out(slot)
+            assert not np.any(ct == 2)
+            pool.retire(slot)
+    finally:
+        pool.close()
