@@ -142,6 +142,7 @@ SIGNATURES = {
     "exaca_pool_set_config": ([_P, _I], _I),
     "exaca_pool_set_grid": ([_P, _I], _I),
     "exaca_pool_autotune": ([_P, _I, ctypes.POINTER(_I), ctypes.POINTER(ctypes.c_double)], _I),
+    "exaca_pool_config_cycles": ([_P, ctypes.POINTER(ctypes.c_uint64)], _I),
     "exaca_problem_pin": ([_P], _I),
     "exaca_census_cells": ([_I, _P, ctypes.POINTER(CellFieldsT), _I, ctypes.POINTER(CensusT)], _I),
 }
@@ -404,6 +405,12 @@ class Pool:
         t = (ctypes.c_double * STEP_CONFIGS)()
         _check(load_library().exaca_pool_autotune(self._h, trial_cycles, ctypes.byref(c), t))
         return c.value, list(t)
+
+    def config_cycles(self) -> list:
+        """Cycles launched so far in each step configuration."""
+        c = (ctypes.c_uint64 * STEP_CONFIGS)()
+        _check(load_library().exaca_pool_config_cycles(self._h, c))
+        return list(c)
 
     def timed_step(self, n_cycles: int) -> float:
         """step(n_cycles) (one persistent launch) timed with CUDA events; waits; returns ms."""

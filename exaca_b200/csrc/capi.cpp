@@ -353,7 +353,7 @@ int exaca_pool_set_config(exaca_pool *pool, int config) {
 
 int exaca_pool_set_grid(exaca_pool *pool, int divisor) {
     if (!pool || divisor < 0 || divisor > 32)
-        return fail(EXACA_ERR_ARG, "grid divisor must be 0 (automatic) or 1-32");
+        return fail(EXACA_ERR_ARG, "grid divisor must be 0 (all co-resident blocks) or 1-32");
     return guarded([&] { pool->pool->set_grid(divisor); });
 }
 
@@ -365,6 +365,14 @@ int exaca_pool_autotune(exaca_pool *pool, int trial_cycles, int *config, double 
         if (config)
             *config = c;
     });
+}
+
+int exaca_pool_config_cycles(exaca_pool *pool, uint64_t *cycles) {
+    if (!pool || !cycles)
+        return fail(EXACA_ERR_ARG, "null argument");
+    for (int c = 0; c < exaca::Pool::kStepConfigs; c++)
+        cycles[c] = pool->pool->config_cycles(c);
+    return EXACA_OK;
 }
 
 int exaca_pool_timed_step(exaca_pool *pool, int n_cycles, double *ms) {

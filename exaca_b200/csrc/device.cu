@@ -4016,15 +4016,16 @@ void Pool::launch_persistent(int n) {
         if (host_desc_[alive.idx[i]].active_size > host_desc_[alive.idx[0]].active_size)
             std::swap(alive.idx[0], alive.idx[i]);
     void *args[] = {&ps, &n, &alive};
-    const int v = config_fixed_ && !(tuned_records_ && last_records_ && last_records_ * 4 < tuned_records_)
-                      ? variant_
-                      : shape_for(last_records_);
+    const bool fixed =
+        trial_ || (config_fixed_ && !(tuned_records_ && last_records_ && last_records_ * 4 < tuned_records_));
+    const int v = fixed ? variant_ : shape_for(last_records_);
     const int grid = std::max(1, std::min(kMeetMaxGrid, grid_cycles_[v]) / std::max(1, grid_fixed_));
     // many domains: a round of loads more per cycle for the views, which up to kSerialDomains do not repay
     // (a map of 96: 14.5 -> 15.5 us per cycle with seven running)
     const void *const kernel = alive.n < 0 ? kStepKernel[v].cycles_many : kStepKernel[v].cycles;
     CUDA_OK(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kBlock), args, 0, st));
     launches_ += 1;
+    config_cycles_[v] += (unsigned long long)n;
 }
 
 // n cycles as separate pass kernels: the start of cycles 2..n runs in the last block of the
@@ -4087,6 +4088,7 @@ void Pool::step(int n) {
             CUDA_OK(cudaGraphLaunch((cudaGraphExec_t)graph_exec_, st));
         launches_ += (unsigned long long)full * (1 + 3ull * graph_steps_);
         launch_passes(rest);
+        config_cycles_[config()] += (unsigned long long)n;
     }
     CUDA_OK(cudaGetLastError());
 }
@@ -4276,7 +4278,8 @@ void Pool::apply_config(int config) {
     if (config < 0 || config >= kStepConfigs)
         throw std::invalid_argument("step configuration out of range");
     const int mode = config / kStepVariants, variant = config % kStepVariants;
-    if (variant != variant_ && graph_exec_) {
+    // the graph holds the pass kernels, which two shapes share
+    if (kStepKernel[variant].grow != kStepKernel[variant_].grow && graph_exec_) {
         CUDA_OK(cudaStreamSynchronize(S(stream_)));
         CUDA_OK(cudaGraphExecDestroy((cudaGraphExec_t)graph_exec_));
         graph_exec_ = nullptr;
@@ -4286,19 +4289,35 @@ void Pool::apply_config(int config) {
 }
 
 int Pool::autotune(int trial_cycles, double *ms_per_cycle) {
-    int best = config();
-    double best_ms = 1e300;
-    for (int c = 0; c < kStepConfigs; c++) {
-        apply_config(c);
-        if (step_mode_ == 1)
-            build_graph(); // outside the timed trial
-        const double ms = timed_step(trial_cycles) / std::max(trial_cycles, 1);
-        if (ms_per_cycle)
-            ms_per_cycle[c] = ms;
-        if (ms < best_ms) {
-            best_ms = ms;
-            best = c;
+    // The active list grows from trial to trial. Half of each configuration's cycles are run in this order and
+    // half in the reverse, so that each has the same mean place in it (in one pass the first one won
+    // whatever it was). Graph shapes that share their kernels are neighbours: three graphs are built.
+    constexpr int kOrder[kStepConfigs] = {0, 1, 2, 3, 4, 6, 5, 7};
+    struct Trial {
+        bool &on;
+        explicit Trial(bool &f) : on(f) { on = true; }
+        ~Trial() { on = false; }
+    };
+    double ms[kStepConfigs] = {};
+    const int half[2] = {trial_cycles - trial_cycles / 2, trial_cycles / 2};
+    {
+        const Trial trial(trial_); // every launch takes the configuration that is timed
+        for (int k = 0; k < 2 * kStepConfigs; k++) {
+            const int c = kOrder[k < kStepConfigs ? k : 2 * kStepConfigs - 1 - k], n = half[k / kStepConfigs];
+            if (n == 0)
+                continue;
+            apply_config(c);
+            if (step_mode_ == 1)
+                build_graph(); // outside the timed trial
+            ms[c] += timed_step(n) / trial_cycles;
         }
+    }
+    int best = 0;
+    for (int c = 0; c < kStepConfigs; c++) {
+        if (ms_per_cycle)
+            ms_per_cycle[c] = ms[c];
+        if (ms[c] < ms[best])
+            best = c;
     }
     set_config(best);
     sync_state();

@@ -276,14 +276,16 @@ class Pool {
     // step(n) with CUDA events around the launches; returns their device time in ms
     double timed_step(int n);
     // Step configurations: config = mode * kStepVariants + variant. set_config switches; autotune
-    // runs trial_cycles real cycles with every configuration (the pool's domains advance), keeps
-    // the fastest and returns it; ms_per_cycle (kStepConfigs entries, may be null) gets the trials.
+    // runs trial_cycles (at least one) real cycles with every configuration (the pool's domains advance),
+    // keeps the fastest and returns it; ms_per_cycle (kStepConfigs entries, may be null) gets the trials.
     // Without either, every persistent launch takes the shape for the list's length (shape_for).
     static constexpr int kStepConfigs = 2 * kStepVariants;
     void set_config(int config);
     // Persistent grid: divisor d runs 1/d of the co-resident blocks; 0, all of them.
     void set_grid(int divisor);
     int config() const { return step_mode_ * kStepVariants + variant_; }
+    // cycles launched in configuration c (the shape that a launch took, whoever chose it)
+    unsigned long long config_cycles(int c) const { return config_cycles_[c]; }
     int autotune(int trial_cycles, double *ms_per_cycle);
     // Steps every admitted domain in chunks of `chunk` cycles until each one has ended on the device
     // (admitted with check_mode 1); returns the cycles stepped. Throws past max_cycles.
@@ -337,6 +339,8 @@ class Pool {
     int step_mode_ = 0;
     int variant_ = kStepVariants - 1;
     bool config_fixed_ = false; // set_config or autotune chose the configuration
+    bool trial_ = false;        // autotune times variant_
+    unsigned long long config_cycles_[kStepConfigs] = {};
     int grid_fixed_ = 0; // set_grid's divisor, 0 for every co-resident block
     unsigned long long last_records_ = 0;  // length of the active list at the last state read
     unsigned long long tuned_records_ = 0; // and at autotune's; its choice holds down to a quarter of it

@@ -145,9 +145,13 @@ int exaca_pool_set_config(exaca_pool *pool, int config);
 /* Grid of the persistent kernel (no counterpart in the reference): divisor d in 1-32 runs 1/d of
  * the co-resident blocks, 0 (the default) all of them. Results do not depend on it. */
 int exaca_pool_set_grid(exaca_pool *pool, int divisor);
-/* Autotuner: runs trial_cycles real cycles of the pool's domains in every configuration, keeps the
- * fastest; ms_per_cycle (EXACA_STEP_CONFIGS entries, may be NULL) receives the trial times. */
+/* Autotuner: runs trial_cycles real cycles of the pool's domains in every configuration (half of them in
+ * each of two passes over the configurations, the second in reverse order), keeps the fastest;
+ * ms_per_cycle (EXACA_STEP_CONFIGS entries, may be NULL) receives the trial times. */
 int exaca_pool_autotune(exaca_pool *pool, int trial_cycles, int *config, double *ms_per_cycle);
+/* Cycles launched so far in each configuration (EXACA_STEP_CONFIGS entries): those of exaca_pool_step and
+ * of what steps through it. */
+int exaca_pool_config_cycles(exaca_pool *pool, uint64_t *cycles);
 /* exaca_pool_step with CUDA events around the launch: waits and returns its device time in ms. */
 int exaca_pool_timed_step(exaca_pool *pool, int n_cycles, double *ms);
 /* exaca_pool_step with the persistent kernel's device timeline on (globaltimer at every grid-wide
