@@ -395,7 +395,8 @@ class Pool:
         _check(load_library().exaca_pool_set_config(self._h, config))
 
     def set_grid(self, divisor: int) -> None:
-        """Persistent kernel grid: divisor d in 1-32 runs 1/d of the co-resident blocks, 0 all of them."""
+        """Persistent kernel grid: divisor d in 1-32 runs 1/d of the co-resident blocks, 0 all of them, or fewer
+        in launches of up to 250 cycles on lists that need fewer."""
         _check(load_library().exaca_pool_set_grid(self._h, divisor))
 
     def autotune(self, trial_cycles: int = 100):

@@ -3950,6 +3950,7 @@ int Pool::admit(std::shared_ptr<const Problem> pp, int check_mode) {
     CUDA_OK(cudaGetLastError());
     bytes_in_use_ += s.bytes;
     // the list's length until the next state read: as then, with the new domain's first active cells
+    list_read_ = false;
     last_records_ += p.dir.used ? p.dir.active.size() : 0;
     return slot;
 }
@@ -3986,15 +3987,30 @@ void Pool::retire(int slot) {
 // list with two / four records per lane, middle, short: 2.9e4 records 14.9 / 15.8 / 11.9 / 11.7, 5.9e4 15.5
 // / 16.7 / 13.0 / 15.0, 1.7e5 19.7 / 19.9 / 17.5 / 18.8, 3.6e5 24.1 / 25.0 / 24.4 / 26.6, 5e5 27.7 / 28.2
 // / 29.2 / 31.2; whole solves: 64^3 (7e3) 9.9 / 10.2 / 7.9 / 7.6, 512^3 (1e6) 38.4 / 36.8 / 40.5 / 42.1.
-// All co-resident blocks are as fast as fewer, or faster, from 5e3 records on (half of them: 5.4 -> 6.3
-// on 3x3 spot melts), and within 2 % below.
 int Pool::shape_for(unsigned long long n) {
     if (n == 0)
         return 2;
     return n < (1ull << 15) ? 3 : (n < 350000 ? 2 : (n < 700000 ? 0 : 1));
 }
 
-// One cooperative launch of k_cycles over n cycles (the grid is exactly the co-resident blocks).
+// Blocks of a persistent launch of n cycles, of the `full` co-resident ones. A launch that holds every SM
+// keeps out those of other pools that a program steps beside it, and a short list gains nothing by more
+// than a block per 64 records: us per cycle of a lone 32^3 domain (1.6e3 records) 9.1 on all blocks and 8.9 on a
+// quarter, 48^3 (4.2e3) 9.3 and 9.2 on half, 64^3 (7.5e3) 9.5 and 9.6. Eight pools of 32^3 stepped from as many
+// threads: 7.1 -> 2.7 us per cycle and pool, of 48^3 8.3 -> 6.6. A list grows during a launch, so the rule
+// takes short launches only, and a quarter at least: from a few records to 1e5 within 1000 cycles, such
+// launches took 20-36 % longer on a quarter of the blocks than on all; of 250 cycles, as long.
+constexpr int kShortLaunch = 250;
+int Pool::grid_for(int n, int full, bool many) const {
+    if (grid_fixed_)
+        return std::max(1, full / grid_fixed_);
+    if (!list_read_ || n > kShortLaunch)
+        return full;
+    const unsigned long long least = std::max<unsigned long long>((full + 3) / 4, many ? n_domains_ : 0); // a warp starts a domain
+    return (int)std::min<unsigned long long>(full, std::max(last_records_ / 64 + 1, least));
+}
+
+// One cooperative launch of k_cycles over n cycles (at most the co-resident blocks).
 void Pool::launch_persistent(int n) {
     cudaStream_t st = S(stream_);
     // the meeting point starts at zero arrivals (a launch that gave up waiting may have left some)
@@ -4019,7 +4035,7 @@ void Pool::launch_persistent(int n) {
     const bool fixed =
         trial_ || (config_fixed_ && !(tuned_records_ && last_records_ && last_records_ * 4 < tuned_records_));
     const int v = fixed ? variant_ : shape_for(last_records_);
-    const int grid = std::max(1, std::min(kMeetMaxGrid, grid_cycles_[v]) / std::max(1, grid_fixed_));
+    const int grid = grid_for(n, std::min(kMeetMaxGrid, grid_cycles_[v]), alive.n < 0);
     // many domains: a round of loads more per cycle for the views, which up to kSerialDomains do not repay
     // (a map of 96: 14.5 -> 15.5 us per cycle with seven running)
     const void *const kernel = alive.n < 0 ? kStepKernel[v].cycles_many : kStepKernel[v].cycles;
@@ -4109,6 +4125,7 @@ void Pool::sync_state() {
     std::memcpy(cnt, lists, sizeof(cnt));
     std::memcpy(&cur, lists + (offsetof(PoolState, cur) - kCnt), sizeof(cur));
     last_records_ = cnt[cur & 1];
+    list_read_ = true;
 }
 
 int Pool::check_bounded_wait() {
@@ -4270,7 +4287,7 @@ void Pool::set_config(int config) {
 
 void Pool::set_grid(int divisor) {
     if (divisor < 0 || divisor > 32)
-        throw std::invalid_argument("grid divisor must be 0 (automatic) or 1-32");
+        throw std::invalid_argument("grid divisor must be 0 (the default rule) or 1-32");
     grid_fixed_ = divisor;
 }
 

@@ -281,7 +281,8 @@ class Pool {
     // Without either, every persistent launch takes the shape for the list's length (shape_for).
     static constexpr int kStepConfigs = 2 * kStepVariants;
     void set_config(int config);
-    // Persistent grid: divisor d runs 1/d of the co-resident blocks; 0, all of them.
+    // Persistent grid: divisor d runs 1/d of the co-resident blocks; 0, all of them, or in short launches
+    // on short lists as many as those need (grid_for).
     void set_grid(int divisor);
     int config() const { return step_mode_ * kStepVariants + variant_; }
     // cycles launched in configuration c (the shape that a launch took, whoever chose it)
@@ -341,10 +342,12 @@ class Pool {
     bool config_fixed_ = false; // set_config or autotune chose the configuration
     bool trial_ = false;        // autotune times variant_
     unsigned long long config_cycles_[kStepConfigs] = {};
-    int grid_fixed_ = 0; // set_grid's divisor, 0 for every co-resident block
+    int grid_fixed_ = 0; // set_grid's divisor, 0 for grid_for's rule
     unsigned long long last_records_ = 0;  // length of the active list at the last state read
+    bool list_read_ = false;               // no admission since
     unsigned long long tuned_records_ = 0; // and at autotune's; its choice holds down to a quarter of it
     static int shape_for(unsigned long long records);
+    int grid_for(int n, int full, bool many) const;
     void apply_config(int config);
     int grid_cycles_[kStepVariants] = {}; // co-resident blocks of each persistent kernel
     int grid_grow_[kStepVariants] = {};

@@ -143,7 +143,9 @@ int exaca_pool_run_all(exaca_pool *pool, int chunk_cycles, int64_t max_cycles, i
 #define EXACA_STEP_CONFIGS 8
 int exaca_pool_set_config(exaca_pool *pool, int config);
 /* Grid of the persistent kernel (no counterpart in the reference): divisor d in 1-32 runs 1/d of
- * the co-resident blocks, 0 (the default) all of them. Results do not depend on it. */
+ * the co-resident blocks, 0 (the default) all of them, or in launches of up to 250 cycles one per 64
+ * records of the list read since the last admission (a quarter at least), so that pools stepped from
+ * several threads run side by side. Results do not depend on it. */
 int exaca_pool_set_grid(exaca_pool *pool, int divisor);
 /* Autotuner: runs trial_cycles real cycles of the pool's domains in every configuration (half of them in
  * each of two passes over the configurations, the second in reverse order), keeps the fastest;
