@@ -53,21 +53,22 @@ WORKLOAD = dict(G=1e6, R=1e6, n_ratio=25, nucleation_density=100.0, dTN=3.0, dTs
 REF_BENCH = os.path.join(ROOT, "oracle", "_ref", "ref_bench")
 PORT_LIB = os.path.join(ROOT, "oracle", "_port", "liboracle.so")
 
-# Algorithmic bytes of each pass per unit of work (the bytes the pass must read or write, each
-# counted once per use, no cache reuse credited):
-#   grow/claim: record 16 + domain 4 + liquid mask 4 + growth-table entry 8 per listed record;
-#               diagonal/min-length write 8 per grown record; tombstone 16 + DiagonalLength 4 per
-#               dropped record; critical-length row 104 + min write 4 per flagged record; 26
-#               neighbour types + mask write 4 per fresh mask; 8 per claim + its TemporaryUpdate
-#               CellType byte 1; 8 per listed target
-#   capture:    per capture: claim 8, target 8, GrainID 4+4, centres 12+12, orientation 36,
-#               DiagonalLength 4, 26 critical lengths 104, mask 4, record 16+4, CellType 1,
-#               CritTimeStep 4, and per neighbour direction CellType 1 + two mask atomics 8; per
-#               solidifying re-check CellType 1 + mask 4 (the mask word says whether it was grown)
+# Algorithmic bytes of each pass of the persistent kernel per unit of work (the bytes of global memory the
+# pass must read or write, each counted once per use, no cache reuse credited; flagged records and listed
+# claims stay in shared memory, the growth tables and descriptors in L1 or shared memory):
+#   grow:    record 16 + domain word 4 + second bound 4 per listed record; DiagonalLength 4 per grown
+#            one; status 4 + DiagonalLength 4 + CellType 1 per dropped one
+#   claim:   body 128 + cell 4 read, the two bounds and the domain word 12 written per flagged record; 26
+#            neighbour types + mask 4 per fresh mask; claim word 8 + TemporaryUpdate byte 1 per claim
+#   capture: claim word 8 + CritTimeStep 4 + the claimant's GrainID and centre 16 per claim; per capture the
+#            orientation 36, the body 128, the cell's own critical lengths 104, GrainID 4, DiagonalLength
+#            4 and centre 12, the record 16 + cell 4 + domain word 4 + second bound 4, list position 4,
+#            CellType 1, and CellType 1 + list position 4 of 26 neighbours (the mask atomics of those that are
+#            active are not counted); per solidifying re-check CellType 1 + mask 4
 PASS_BYTES = {
-    "grow": dict(listed=24, grown=8, dropped=20, flagged=20),
-    "claim": dict(flagged=20 + 104 + 4, fresh=30, claims=8 + 1 + 8),
-    "capture": dict(claims=8 + 8, captured=221 + 26 * 9, rechecks=5),
+    "grow": dict(listed=24, grown=4, dropped=9),
+    "claim": dict(flagged=128 + 4 + 12, fresh=30, claims=8 + 1),
+    "capture": dict(claims=8 + 4 + 16, captured=321 + 26 * 5, rechecks=5),
 }
 
 
@@ -424,6 +425,7 @@ def b200_arm(args, rank, world, local):
     # the 1000-cycle census) on a bounded stretch of the solve: one launch, CUDA events around it
     slot = pool.admit(prob, device_check=False)
     pool.step(args.profile_at)
+    pool.status(slot)  # the launch shape follows the list's length at the last state read, as in the solve
     pa = pool.stats()
     launch_ms = pool.timed_step(args.profile_cycles)
     pb = pool.stats()
@@ -469,9 +471,8 @@ def b200_arm(args, rank, world, local):
                          "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                          "traffic_source": "not measured in this run: ncu DRAM bytes per cycle of a 1000-cycle "
                                            "k_cycles launch (profiles/traffic_per_launch.txt) x the cycles of "
-                                           "this launch; the 512^3 figure is from an earlier kernel version "
-                                           "(the current one moves 32 % fewer DRAM bytes per cycle at 288^3, "
-                                           "profiles/k_cycles_dirsolid288_dram.md)",
+                                           "this launch; less than the algorithmic bytes, since most of the list "
+                                           "and its bodies stay in L2 from cycle to cycle",
                          "algorithmic_bytes_per_launch": launch_bytes, "launch_ms": launch_ms,
                          "sample": f"one launch over cycles {args.profile_at + 1}-{args.profile_at + args.profile_cycles}",
                          "pass_bytes_per_launch": pass_bytes,

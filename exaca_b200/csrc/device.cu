@@ -981,8 +981,8 @@ struct ClaimLane {
 // The claim step of one flagged record by eight lanes (on: the group has one; every lane of the warp calls,
 // src/CAupdate.cpp:320-352): lanes 1-7 read four critical lengths each (lane 0 the rest
 // of the body), so a record is one 128-byte line in one load instruction of its group, and each lane compares four
-// lengths. (A record per lane, 26 lengths compared in turn from seven uncoalesced 16-byte loads, took
-// 3.7 us of a 256^3 cycle, its code 3000 instructions.)
+// lengths. A record per lane, 26 lengths compared in turn from seven uncoalesced 16-byte loads, is the longer
+// chain where a block has few of them (block_claims).
 __device__ __forceinline__ ClaimLane claim_group(const PassCtx &X, int app, const ClaimItem &it, bool on, CycleStats &st,
                                                  unsigned int &tombs) {
     const unsigned int lane = threadIdx.x & 31, sub = lane & 7u, group = 0xffu << (lane & 24u);
@@ -1523,9 +1523,9 @@ __device__ __forceinline__ void make_claims(PoolState *P, BlockShared &B, const 
 
 // The block's claim step over its queue (all threads of the block call, after the block's growth). In the
 // families for shorter lists a warp per record where there are no more of them than warps, else eight lanes per
-// record, consecutive records on different warps. Without it a record per lane: at 512^3 (270 flagged
-// records per block and cycle) 39.0 us per cycle against 45.2 with eight lanes, whose four rounds wait for
-// memory in turn; at 256^3 (67) eight lanes take 18.95 against 20.0.
+// record, consecutive records on different warps. In the one for long lists a record per lane: at 512^3 (270
+// flagged records per block and cycle) 36.3 us per cycle against 40.1 with eight lanes, whose four rounds wait
+// for memory in turn; at 256^3 (67) eight lanes take 16.9 against 17.9 with one.
 template <int kFamily>
 __device__ __forceinline__ void block_claims(PoolState *P, BlockShared &B, int app, CycleStats &st, unsigned int &tombs) {
     __syncthreads();
@@ -1651,10 +1651,6 @@ __device__ __noinline__ void compact_pass(PoolState *P, const PassCtx &X, int cu
     }
 }
 
-// Active records are handed out to warps in groups of 32 consecutive records (one coalesced load),
-// group g to warp g % (number of warps of the grid), consecutive warps on different blocks: the
-// records appended by the last capture pass, which all need a fresh mask and claims, spread over
-// every SM. No block-wide synchronisation.
 // The position of a dropped record, for one of the block's later captures.
 __device__ __forceinline__ void push_free(BlockShared &B, unsigned int pos) {
     const unsigned int e = atomicAdd(&B.n_free, 1u);
@@ -1704,7 +1700,9 @@ __device__ __noinline__ GrowResult grow_slow(const PassCtx &X, BlockShared *B, D
     return grow_any<kOwnClaims>(X, B, dyn, cur, idx, r, cell, word, min2, st);
 }
 
-// Growth of the list's groups of 32 records, kBatch groups per warp in flight (see grow_pass). A record
+// Growth of the list's groups of 32 consecutive records (one coalesced load), group g by warp g % (number of
+// warps of the grid), consecutive warps on different blocks, so that records appended together spread over
+// every SM; kBatch groups per warp in flight. No block-wide synchronisation. A record
 // costs 24 bytes read (its 16-byte vector with the status word, its domain word and the second bound)
 // and 4 written. Nearly every record of the hot domain takes the short path below (about 70 instead of
 // 250 instructions per group of 32): eligible or waiting, with liquid neighbours. The others go through
@@ -3983,10 +3981,11 @@ void Pool::retire(int slot) {
     s = SlotHost();
 }
 
-// The persistent shape for a list of n records (0: not known). us per cycle of directional solves, long
-// list with two / four records per lane, middle, short: 2.9e4 records 14.9 / 15.8 / 11.9 / 11.7, 5.9e4 15.5
-// / 16.7 / 13.0 / 15.0, 1.7e5 19.7 / 19.9 / 17.5 / 18.8, 3.6e5 24.1 / 25.0 / 24.4 / 26.6, 5e5 27.7 / 28.2
-// / 29.2 / 31.2; whole solves: 64^3 (7e3) 9.9 / 10.2 / 7.9 / 7.6, 512^3 (1e6) 38.4 / 36.8 / 40.5 / 42.1.
+// The persistent shape for a list of n records (0: not known). us per cycle of whole directional solves
+// (records in the mean; a front is longest in mid-solve), long list with two / four records per lane, middle,
+// short: 64^3 (7.0e3) 11.3 / 12.0 / 9.2 / 8.7, 128^3 (3.5e4) 12.6 / 13.3 / 10.3 / 10.4, 192^3 (8.7e4) 14.5 / 14.9
+// / 12.2 / 13.0, 320^3 (2.9e5) 21.5 / 21.9 / 20.8 / 21.8, 400^3 (4.7e5) 26.9 / 27.3 / 28.0 / 29.2, 512^3 (8.0e5)
+// 36.8 / 36.8 / 40.5 / 42.1; by this rule 8.7, 10.2, 12.3, 20.8, 26.5, 36.4.
 int Pool::shape_for(unsigned long long n) {
     if (n == 0)
         return 2;

@@ -6,7 +6,7 @@ had time to form:
 
     python -m exaca_b200.profile_passes 256 --warm 3000 --cycles 3
     python -m exaca_b200.profile_passes 288 --warm 4000 --launch 1000   # four k_cycles launches
-    python -m exaca_b200.profile_passes 288 --warm 4000 --launch 1000 --config 0   # 4 lanes, 2 records
+    python -m exaca_b200.profile_passes 288 --warm 4000 --launch 1000 --config 2   # the middle shape, as its list takes
     ncu --set full --clock-control none -k regex:k_grow -s 1 -c 1 -o prof_grow256 \\
         python -m exaca_b200.profile_passes 256 --warm 3000 --cycles 3
 """
