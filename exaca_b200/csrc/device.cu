@@ -1227,7 +1227,7 @@ struct BlockShared {
     unsigned int n_free, n_taken;
     int tombs; // change of the list's number of dropped records, not yet told to the grid
     unsigned int free_slots[kFreeSlots];
-    unsigned int busy;       // a record of the block was grown or dropped this cycle
+    unsigned int busy;       // 1: a record of the block was grown or dropped this cycle; kTellFlag beside it
     int min_cts;             // smallest CritTimeStep of the block's other records, while it is not busy
     PassCtx X;
 };
@@ -2840,7 +2840,8 @@ __device__ __noinline__ void start_next(PoolState *P, BlockShared &B, unsigned i
         atomicAdd(&P->stat[blockIdx.x & (kStatShards - 1)][kStatNucleated], (unsigned long long)fired_total);
 }
 
-constexpr int kTellLeast = 16; // dropped records for which a block asks for a meeting (k_cycles)
+constexpr int kTellLeast = 16;              // dropped records for which a block asks for a meeting (k_cycles)
+constexpr unsigned int kTellFlag = 1u << 8; // in BlockShared::busy: it does
 
 // n_cycles complete CA cycles (start, grow/claim, capture) in one cooperative launch.
 //
@@ -2924,16 +2925,22 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
         }
         grow_pass<kBatch, true, kFamily, kMany>(P, B.X, &B, dyn, cur, n, compact, passes == 0, st, dropped, views);
         dropped = __reduce_add_sync(0xffffffffu, dropped);
-        if ((threadIdx.x & 31) == 0 && dropped)
-            atomicAdd(&B.tombs, (int)dropped);
-        // sums: first claims of the hot domain (32 bits, as cell indices), blocks that would tell, blocks whose
-        // queue overflowed, blocks that are busy. A block tells its dropped records at the meeting after the
-        // captures, which a lone domain's cycle without claims leaves out; it asks for that meeting when the
-        // list would be due for compaction if every block had dropped as many as itself: were it due, a block
-        // with the mean or more would ask. Fewer than kTellLeast wait for the next meeting or the launch's end
-        // (all blocks' together are at most one more group of 32 for a few of the warps; three-layer spots
-        // lost 1 % to the meetings that they asked for).
-        constexpr int kTellShift = 32, kOverflowShift = 40, kBusyShift = 48;
+        // A block tells its dropped records at the meeting after the captures, which a lone domain's cycle without
+        // claims leaves out; it asks for that meeting when the list would be due for compaction if every block
+        // had dropped as many as itself: were it due, a block with the mean or more would ask. Fewer than
+        // kTellLeast wait for the next meeting or the launch's end (all blocks' together are at most one more
+        // group of 32 for a few of the warps). The warp that adds last sees the sum (asked by thread 0 on its way
+        // to the meeting instead: three-layer spots 0.2 % slower, melt tracks 0.3 %). (In a cycle that compacts the difference wraps
+        // to a large one.)
+        if ((threadIdx.x & 31) == 0 && dropped) {
+            const unsigned int untold = (unsigned int)(atomicAdd(&B.tombs, (int)dropped) + (int)dropped);
+            if ((int)untold >= kTellLeast && untold * gridDim.x > (unsigned int)(n >> 2) - (unsigned int)tombs)
+                atomicOr(&B.busy, kTellFlag); // every store of 1 lies before grow_pass's block barrier
+        }
+        // sums: first claims of the hot domain (32 bits, as cell indices), blocks whose queue overflowed, blocks that
+        // are busy, blocks that would tell
+        constexpr int kOverflowShift = 32, kBusyShift = 40;
+        static_assert(kTellFlag == 1u << 8, "the byte above the busy blocks");
         int *const grid_min = reinterpret_cast<int *>(&P->meet.min_cts[passes % 3].v);
         const auto claim_share = [&] {
             const unsigned long long v = B.n_first;
@@ -2943,10 +2950,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
         ok = grid_meet(
             P, meet, tl, 3 * c + 1,
             [&] {
-                // (the difference wraps to a large one in a cycle that compacts)
-                const bool tell = B.tombs >= kTellLeast && (unsigned int)B.tombs * gridDim.x > (unsigned int)(n >> 2) - (unsigned int)tombs;
-                const unsigned long long v = claim_share() + (tell ? 1ull << kTellShift : 0ull) +
-                                             (B.n_items > (unsigned int)kBlockQueue ? 1ull << kOverflowShift : 0ull) +
+                const unsigned long long v = claim_share() + (B.n_items > (unsigned int)kBlockQueue ? 1ull << kOverflowShift : 0ull) +
                                              ((unsigned long long)B.busy << kBusyShift);
                 if (!B.busy && B.min_cts != INT_MAX)
                     atomicMin(grid_min, B.min_cts);
@@ -2958,8 +2962,8 @@ __global__ void __launch_bounds__(kBlock, 1) k_cycles(PoolState *P, int n_cycles
         if (!ok)
             break;
         unsigned long long claimed = total & 0xffffffffull;
-        const bool asked = (total & ((1ull << kBusyShift) - 1)) != 0; // claims, drops to tell, an overflow
-        const bool overflow = ((total >> kOverflowShift) & 0xffu) != 0, busy = (total >> kBusyShift) != 0;
+        const bool asked = (total & ~(0xffull << kBusyShift)) != 0; // claims, an overflow, drops to tell
+        const bool overflow = ((total >> kOverflowShift) & 0xffu) != 0, busy = ((total >> kBusyShift) & 0xffu) != 0;
         if (blockIdx.x == 0 && threadIdx.x == 0) // read after the previous cycle's meeting, used two cycles on
             *reinterpret_cast<int *>(&P->meet.min_cts[(passes + 2) % 3].v) = INT_MAX;
         if (overflow) {
