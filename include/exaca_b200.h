@@ -209,7 +209,9 @@ int exaca_pool_copy_out(exaca_pool *pool, int slot, int32_t *grain_id, int32_t *
 int exaca_pool_copy_out_concurrent(exaca_pool *pool, int slot, int32_t *grain_id, int32_t *cell_type);
 /* Active-window octahedron state (DiagonalLength, DOCenter x3, CritDiagonalLength x26) of the
  * slot's current layer: window_nz * mx * my cells from plane window_z_lo (exaca_pool_status), the
- * reference's window arrays (src/runCA.cpp:147-151, resized per layer at :352-356). */
+ * reference's window arrays (src/runCA.cpp:147-151, resized per layer at :352-356). Centres and critical
+ * lengths of cells whose DiagonalLength is 0, which never had an octahedron, are unspecified in the first
+ * layer (as in the reference, which allocates those arrays uninitialised). */
 int exaca_pool_copy_octahedra(exaca_pool *pool, int slot, float *dl, float *doc, float *cdl);
 /* Frees a slot's device memory. */
 int exaca_pool_retire(exaca_pool *pool, int slot);
